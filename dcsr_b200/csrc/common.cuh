@@ -123,6 +123,14 @@ struct Mat {
 // marks the area's fault word with the kernel's epoch (the other waits of
 // that kernel then give up early instead of each spinning to the limit) and
 // sets the operation's status word (when it has one) to DCSR_TIMEOUT.
+struct LookbackGlobals {
+  unsigned long long faults;  // waits that ran out of iterations (dcsr_spin_faults)
+  int spin_limit;             // a wait's iteration limit
+  int stall;                  // test switch: the first tile of every single-pass kernel does not publish
+};
+// The current device's LookbackGlobals (prims.cu; looked up once per device).
+int lookback_globals(LookbackGlobals **out);
+
 struct Lookback {
   unsigned long long *epoch;
   unsigned *tiles, *done;
@@ -131,6 +139,7 @@ struct Lookback {
   unsigned long long *flag;   // look-back words
   unsigned long long slots;   // entries of flag
   long long *status;          // the operation's status word, or null
+  LookbackGlobals *g;         // the device's wait limit, test switch and fault count
 };
 constexpr size_t LB_HEADER = 64 + 8 * 256 * 4;
 
@@ -173,7 +182,7 @@ struct Arena {
     out->flag = (unsigned long long *)(lb + LB_HEADER);
     out->slots = lb_slots;
     out->status = status;
-    return DCSR_OK;
+    return lookback_globals(&out->g);
   }
   int reserve(size_t bytes, cudaStream_t s) {
     used = 0;

@@ -6,24 +6,50 @@
 
 namespace dcsr {
 
-// Lay out a matrix from a CSR whose row_ptr is int64 on the device (rows
-// already canonical for the handle's mode): policy capacities, fresh pool,
-// content copy.  Synchronises once (pool size).
-int load_from_csr64(dcsr_handle h, const long long *rp, const int32_t *cols, const void *vals, cudaStream_t s);
-size_t load_scratch_bytes(dcsr_handle h);
+// Entry-parallel copies between CSR order and a matrix's pool (flat.cu).
+// Offsets of the layout policy's capacities of rows given by a row pointer
+// (caps_scan) or by counts (counts_scan, which also makes the row pointer):
+// caps[n+1]; their sum, the pool top the rows need, goes to the handle's
+// ST_TOTAL word.
+int caps_scan(dcsr_handle h, const int32_t *rp, int32_t *caps, Arena &ar, cudaStream_t s);
+int counts_scan(dcsr_handle h, const int32_t *cnt, int32_t *rp, int32_t *caps, Arena &ar, cudaStream_t s);
+// The CSR's rows become the matrix's content: layout (layer 0 from caps) and
+// entries into the handle's pool; nnz bounds the entries, tile_row holds
+// flat_tiles(nnz) words of scratch.
+int place_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const int32_t *cols, const void *vals,
+              int64_t nnz, int32_t *tile_row, cudaStream_t s);
+// Staged rows (row r: lens[r] entries from src_off[r]) likewise: the layout
+// with its offsets, then the entries; bound bounds their number.
+int place_rows_scan(dcsr_handle h, const long long *lens, int32_t *off, int32_t *caps, int32_t *tile_row,
+                    int64_t bound, Arena &ar, cudaStream_t s);
+int place_rows_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, const int32_t *tile_row,
+                    const long long *src_off, const int32_t *scols, const void *svals, int64_t bound, cudaStream_t s);
+// Compaction: the offsets of the current content and of its policy
+// capacities (sum to ST_TOTAL), then the entries into the new pool (cap
+// entries) and the new layout.  tile_row: flat_tiles(pool_cap) words.
+int compact_scan(dcsr_handle h, int32_t *off, int32_t *caps, int32_t *tile_row, Arena &ar, cudaStream_t s);
+int compact_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, const int32_t *tile_row, int32_t *cols,
+                 void *vals, int64_t cap, cudaStream_t s);
+// Export: the row pointer (off, n+1 words) and every row's entries in CSR
+// order, optionally with their rows; entries at positions >= limit are not
+// written.  tile_row: flat_tiles(pool_cap) words.
+int export_rows(dcsr_handle h, int32_t *off, int32_t *tile_row, int32_t *cols, void *vals, int32_t *rows,
+                int64_t limit, Arena &ar, cudaStream_t s);
+
 // Rows staged elsewhere (row r: lens[r] entries at src_off[r]) become the
 // matrix's content with policy capacities, in a pool allocated at cap_bound
-// entries (an upper bound of the pool capacity the rows need); synchronises
-// once at the end (pool top).  Uses the handle's scratch arena.
+// entries (an upper bound of the pool capacity the rows need; bound: of their
+// entries); synchronises once at the end (pool top).  Uses the handle's
+// scratch arena.
 int load_from_rows(dcsr_handle h, const long long *src_off, const long long *lens, const int32_t *scols,
-                   const void *svals, int64_t cap_bound, cudaStream_t s);
+                   const void *svals, int64_t bound, int64_t cap_bound, cudaStream_t s);
 
 // Sort + group a COO batch (any order) into CSR form in the arena:
 // MERGE: sorted by (row, col), duplicates summed in input order;
-// APPEND: stably sorted by row.  *rp has n_rows+1 entries.  Sets BAD_INDEX in
-// *bad (device int) for out-of-range input.
-int coo_to_csr64(dcsr_handle h, const int32_t *rows, const int32_t *cols, const void *vals, int64_t nnz, bool merge,
-                 Arena &ar, long long **rp, int32_t **ocols, void **ovals, int *bad, cudaStream_t s);
+// APPEND: stably sorted by row.  *rp and *caps (counts_scan) have n_rows+1
+// entries.  Out-of-range input sets AUX_BAD_INDEX in the handle's ST_AUX word.
+int coo_to_csr(dcsr_handle h, const int32_t *rows, const int32_t *cols, const void *vals, int64_t nnz, bool merge,
+               Arena &ar, int32_t **rp, int32_t **caps, int32_t **ocols, void **ovals, cudaStream_t s);
 size_t coo_to_csr_scratch(dcsr_handle h, int64_t nnz);
 
 // Per-call operators that take a scratch arena (default: the handle's own);
@@ -99,12 +125,6 @@ template <typename V>
 RowItem<V> row_item(dcsr_handle h, const void *x, void *y, int64_t ldx, int64_t ldy, double alpha, double beta);
 // Size the handle's chunk table and chunk partials (K results per chunk).
 int ensure_part(dcsr_handle h, int K, cudaStream_t s);
-// Copy every row's logical entries to dst_off[r] (optionally COO row ids and
-// an int32 row pointer); entries at positions >= limit are not written.
-// Builds the schedule first if needed (so callers must not hold arena memory
-// across this call unless the schedule is valid).
-int copy_rows(dcsr_handle h, const long long *dst_off, int32_t *out_cols, void *out_vals, int32_t *out_rows,
-              int32_t *out_rowptr, cudaStream_t s, int64_t limit = INT64_MAX);
 // DCSR -> CSR writing at most `limit` entries (the row pointer is complete).
 int export_csr(dcsr_handle h, int32_t *row_ptr, int32_t *cols, void *vals, int64_t limit, cudaStream_t s,
                Arena *ar = nullptr);

@@ -1,0 +1,282 @@
+// lookback.cuh -- device side of the single-pass kernels (decoupled
+// look-back) and the scan over a row or entry function that the load, export,
+// schedule and update kernels are built from.
+#pragma once
+#include "common.cuh"
+
+namespace dcsr {
+
+// ------------------------------------------------- decoupled look-back
+//
+// Single-pass kernels: every block takes the next tile number from a device
+// counter (so all tiles before it are running or finished), publishes its
+// tile's aggregate, adds the aggregates of the tiles before it back to the
+// nearest published inclusive prefix, and publishes its own inclusive prefix.
+// A wait is only ever on an earlier tile, which therefore always finishes;
+// every wait still has an iteration limit, after which it counts a fault and
+// stops waiting.
+
+__device__ __forceinline__ unsigned long long ld_vol(const unsigned long long *p) {
+  return *(const volatile unsigned long long *)p;
+}
+
+// Look-back words are packed: a tag (the epoch's low 30 bits, a 2-bit kind)
+// above a 32-bit value, so a word is published with one store and read with
+// one load -- no fences, no second load.  A sort's word per (tile, digit)
+// holds a count (kind 1: the tile's aggregate, 2: its inclusive prefix); a
+// scan's words per tile hold the halves of its 64-bit aggregates and
+// inclusive prefixes (kind 1: written).  A word is current when its tag is the
+// kernel's; the tag repeats every 2^30 kernels on one area, so the kernel
+// whose last block advances the epoch to such a multiple clears the area
+// (lb_advance) and a stale word never matches.
+constexpr unsigned long long LB_EMASK = (1ull << 30) - 1;
+__device__ __forceinline__ unsigned long long lb_pack(unsigned long long e, int kind, unsigned v) {
+  return ((e & LB_EMASK) << 34) | ((unsigned long long)kind << 32) | v;
+}
+
+// A wait that gave up: count it, mark the area's fault word with this
+// kernel's epoch (its other waits then give up early) and report
+// DCSR_TIMEOUT in the operation's status word.
+__device__ __forceinline__ void lb_give_up(const Lookback &lb, unsigned long long e) {
+  atomicAdd(&lb.g->faults, 1ull);
+  *(volatile unsigned long long *)lb.fault = (e & LB_EMASK) + 1;
+  if (lb.status) atomicCAS(reinterpret_cast<unsigned long long *>(lb.status), 0ull, (unsigned long long)DCSR_TIMEOUT);
+}
+// True when another wait of this kernel (epoch e) gave up already.
+__device__ __forceinline__ bool lb_faulted(const Lookback &lb, unsigned long long e) {
+  return ld_vol(lb.fault) == (e & LB_EMASK) + 1;
+}
+
+// Thread 0 of every block: the block's tile and the kernel's epoch.
+__device__ __forceinline__ void lb_begin(const Lookback &lb, unsigned *tile, unsigned long long *ep) {
+  if (threadIdx.x == 0) {
+    *tile = atomicAdd(lb.tiles, 1u);
+    *ep = ld_vol(lb.epoch);
+  }
+}
+
+// End of every block (all threads): true in the last block to finish.
+__device__ __forceinline__ bool lb_end(const Lookback &lb) {
+  __shared__ int last;
+  __syncthreads();
+  // (no fence: this block's results reach later kernels at the launch boundary)
+  if (threadIdx.x == 0) last = atomicAdd(lb.done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  return last;
+}
+
+// The last block (all its threads): reset the counters and advance the
+// epoch; at a multiple of 2^30 clear the slots first (packed radix tags).
+__device__ __forceinline__ void lb_advance(const Lookback &lb) {
+  __shared__ unsigned long long next;
+  if (threadIdx.x == 0) next = ld_vol(lb.epoch) + 1;
+  __syncthreads();
+  if ((next & LB_EMASK) == 0)
+    for (unsigned long long i = threadIdx.x; i < lb.slots; i += blockDim.x) lb.flag[i] = 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *(volatile unsigned *)lb.tiles = 0;
+    *(volatile unsigned *)lb.done = 0;
+    __threadfence();
+    *(volatile unsigned long long *)lb.epoch = next;
+  }
+}
+
+// Warp 0 of tile t (the first tile of its sequence is t0): publish the NS
+// aggregates agg (in every lane), look back over 32 earlier tiles at a time,
+// publish the inclusive prefixes; excl receives the sums of the tiles before
+// t (in every lane).  Slot words of tile t: 4*NS of them -- per sum the
+// halves of its aggregate, then per sum the halves of its inclusive prefix,
+// each a packed word written once per epoch, so a reader that sees all halves
+// of one kind current has consistent values.
+template <int NS>
+__device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long long e, int64_t t, int64_t t0,
+                                            const long long (&agg)[NS], long long (&excl)[NS]) {
+  const int lane = lane_id();
+  const unsigned long long tag = e & LB_EMASK;
+  unsigned long long *w = lb.flag;
+  auto cur = [&](unsigned long long x) { return (x >> 34) == tag && ((x >> 32) & 3) == 1; };
+  auto put = [&](int64_t tile, int kind, const long long (&v)[NS]) {  // kind 0: aggregates, 1: inclusive prefixes
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 0; q < NS; q++) {
+        volatile unsigned long long *p = w + 4 * NS * tile + 2 * NS * kind + 2 * q;
+        p[0] = lb_pack(e, 1, (unsigned)(unsigned long long)v[q]);
+        p[1] = lb_pack(e, 1, (unsigned)((unsigned long long)v[q] >> 32));
+      }
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < NS; q++) excl[q] = 0;
+  if (t == t0) {
+    if (!(lb.g->stall && t == 0)) put(t, 1, agg);
+    return;
+  }
+  put(t, 0, agg);
+  int idle = 0;
+  const int limit = lb.g->spin_limit;
+  for (int64_t j = t - 1;;) {
+    const int64_t r = j - lane;  // lane 0: the nearest earlier tile
+    bool ready = true, inc = true;
+    long long v[NS];
+#pragma unroll
+    for (int q = 0; q < NS; q++) v[q] = 0;
+    if (r >= t0) {  // before the first tile: an inclusive prefix of 0
+      unsigned long long x[4 * NS];
+#pragma unroll
+      for (int q = 0; q < 4 * NS; q++) x[q] = ld_vol(w + 4 * NS * r + q);
+      bool a = true;
+#pragma unroll
+      for (int q = 0; q < 2 * NS; q++) {
+        a = a && cur(x[q]);
+        inc = inc && cur(x[2 * NS + q]);
+      }
+      ready = inc || a;
+#pragma unroll
+      for (int q = 0; q < NS; q++) {
+        const unsigned long long lo = inc ? x[2 * NS + 2 * q] : x[2 * q], hi = inc ? x[2 * NS + 2 * q + 1] : x[2 * q + 1];
+        v[q] = (long long)(((hi & 0xffffffffull) << 32) | (lo & 0xffffffffull));
+      }
+    }
+    const unsigned rm = __ballot_sync(FULL, ready), im = __ballot_sync(FULL, ready && inc);
+    const int first = im ? __ffs(im) - 1 : 32;  // nearest inclusive prefix in this window
+    const unsigned need = first >= 31 ? FULL : ((2u << first) - 1u);
+    if ((rm & need) == need) {  // everything up to it published
+#pragma unroll
+      for (int q = 0; q < NS; q++) excl[q] += warp_sum(lane <= first ? v[q] : 0ll);
+      if (first < 32) break;
+      j -= 32;
+      idle = 0;
+      continue;
+    }
+    if (++idle >= limit || ((idle & 1023) == 1023 && __any_sync(FULL, lb_faulted(lb, e)))) {
+      if (lane == 0) lb_give_up(lb, e);
+      break;
+    }
+    if (idle >= 32) __nanosleep(64);
+  }
+  long long inclv[NS];
+#pragma unroll
+  for (int q = 0; q < NS; q++) inclv[q] = excl[q] + agg[q];
+  put(t, 1, inclv);
+}
+
+// ------------------------------------------------------- scan over a function
+//
+// One kernel computes a value (NS of them) per item i in [0, n), scans it
+// exclusively and hands every item its prefix, so an operator needs no array
+// of flags, no scan of it and no pass over the result.  F supplies
+//   static constexpr int NS;
+//   struct State;                    what load leaves for emit (registers)
+//   load(i, ok, st, v[NS])           value of item i (ok false: past the end, v must be 0)
+//   emit(i, ok, st, excl[NS], v[NS]) item i's prefix; called by whole warps
+//   total(tot[NS])                   one thread, the totals
+// A warp takes 32*SM_ITEMS consecutive items, item j*32 + lane in lane's j-th
+// step (coalesced, and every step's prefix by a warp scan in registers -- no
+// staging through shared memory).  One block (no look-back) up to
+// SM_ONE items; else tiles of SM_THREADS*SM_ITEMS.
+constexpr int SM_ITEMS = 8;
+constexpr int SM_THREADS = 256;
+constexpr int SM_ONE_THREADS = 1024;
+constexpr int64_t SM_ONE = SM_ONE_THREADS * SM_ITEMS;
+
+template <int TH, class F>
+__global__ void __launch_bounds__(TH) k_scan_map(F f, int64_t n, Lookback lb) {
+  constexpr int NS = F::NS, NW = TH / 32;
+  __shared__ long long wsum[NS][NW];
+  __shared__ long long sh_prefix[NS];
+  __shared__ unsigned sh_tile;
+  __shared__ unsigned long long sh_ep;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool single = gridDim.x == 1;
+  int64_t t = 0;
+  unsigned long long e = 0;
+  if (!single) {
+    lb_begin(lb, &sh_tile, &sh_ep);
+    __syncthreads();
+    t = sh_tile;
+    e = sh_ep;
+    if (t >= gridDim.x) {  // a tile counter left non-zero (a bug): report it, touch nothing
+      if (threadIdx.x == 0) lb_give_up(lb, e);
+      if (lb_end(lb)) lb_advance(lb);
+      return;
+    }
+  }
+  const int64_t base = t * (TH * SM_ITEMS) + (int64_t)w * (32 * SM_ITEMS) + lane;
+  typename F::State st[SM_ITEMS];
+  typename F::T v[SM_ITEMS][NS], ex[SM_ITEMS][NS];
+  long long run[NS];
+#pragma unroll
+  for (int q = 0; q < NS; q++) run[q] = 0;
+#pragma unroll
+  for (int j = 0; j < SM_ITEMS; j++) {
+    const int64_t i = base + 32 * j;
+    f.load(i, i < n, st[j], v[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < SM_ITEMS; j++)
+#pragma unroll
+    for (int q = 0; q < NS; q++) {
+      const typename F::T inc = warp_incl_scan(v[j][q]);
+      ex[j][q] = (typename F::T)run[q] + inc - v[j][q];
+      run[q] += __shfl_sync(FULL, inc, 31);
+    }
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < NS; q++) wsum[q][w] = run[q];
+  __syncthreads();
+  long long before[NS], agg[NS];
+#pragma unroll
+  for (int q = 0; q < NS; q++) {
+    long long x = lane < NW ? wsum[q][lane] : 0;  // NW <= 32 warps
+    agg[q] = warp_sum(x);
+    before[q] = warp_sum(lane < w ? x : 0ll);
+  }
+  if (!single) {
+    if (w == 0) {
+      long long excl[NS];
+      lb_lookback<NS>(lb, e, t, 0, agg, excl);
+      if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NS; q++) sh_prefix[q] = excl[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NS; q++) before[q] += sh_prefix[q];
+  }
+#pragma unroll
+  for (int j = 0; j < SM_ITEMS; j++) {
+    const int64_t i = base + 32 * j;
+    long long p[NS];
+#pragma unroll
+    for (int q = 0; q < NS; q++) p[q] = before[q] + (long long)ex[j][q];
+    f.emit(i, i < n, st[j], p, v[j]);
+  }
+  if (threadIdx.x == 0 && t == (int64_t)gridDim.x - 1) {
+    long long tot[NS];
+#pragma unroll
+    for (int q = 0; q < NS; q++) tot[q] = (single ? 0 : sh_prefix[q]) + agg[q];
+    f.total(tot);
+  }
+  if (!single && lb_end(lb)) lb_advance(lb);
+}
+
+// n >= 1 items.  Needs 4*NS look-back slots per SM_THREADS*SM_ITEMS items
+// (lookback_slots covers NS <= 2).
+template <class F>
+static int scan_map(const F &f, int64_t n, Arena &ar, cudaStream_t s) {
+  Lookback lb;
+  std::memset(&lb, 0, sizeof(lb));
+  if (n <= SM_THREADS * SM_ITEMS) {
+    DCSR_LAUNCH((k_scan_map<SM_THREADS, F>), 1, SM_THREADS, 0, s, f, n, lb);
+  } else if (n <= SM_ONE) {
+    DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
+  } else {
+    const int64_t nt = div_up(n, SM_THREADS * SM_ITEMS);
+    DCSR_TRY(ar.lookback((size_t)(4 * F::NS * nt), s, &lb));
+    DCSR_LAUNCH((k_scan_map<SM_THREADS, F>), (unsigned)nt, SM_THREADS, 0, s, f, n, lb);
+  }
+  return DCSR_OK;
+}
+
+}  // namespace dcsr

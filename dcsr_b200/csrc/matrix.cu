@@ -1,176 +1,91 @@
 // matrix.cu -- DCSR handle lifecycle, CSR/COO/HYB -> DCSR loading, DCSR ->
 // CSR/COO export, compaction (defragmentation), pool growth, SpMV row bins,
 // the synchronous update repair policy and the status API.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
 #include <vector>
 
+#include "flat.cuh"
 #include "internal.cuh"
 
 namespace dcsr {
 
-enum { AUX_BAD_INDEX = 1, AUX_NONCANON = 4, AUX_BAD_ROWPTR = 8 };
+enum { AUX_BAD_INDEX = 1, AUX_BAD_ROWPTR = 8 };
 
 // ------------------------------------------------------------- kernels
 
-// caps[r] = policy_cap(len_r) with len_r from an int64 row pointer, caps[n] = 0.
-__global__ void k_caps_from_rp(const long long *rp, int32_t n, dcsr_opts o, long long *caps) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += stride)
-    caps[r] = r < n ? policy_cap(o, rp[r + 1] - rp[r]) : 0;
-}
-__global__ void k_caps_from_sizes(const int32_t *row_sizes, int32_t n, dcsr_opts o, long long *caps) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += stride)
-    caps[r] = r < n ? policy_cap(o, row_sizes[r]) : 0;
-}
-
-// Layer 0 = (off, off+cap), other layers cleared; row_sizes from lens (rp
-// diff) when rp != nullptr; pool top = offs[n].
-__global__ void k_layout(int32_t *seg, int32_t *row_sizes, int32_t n, int32_t pitch, int max_segs,
-                         const long long *offs, const long long *rp) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += stride) {
-    if (r == n) {
-      row_sizes[n] = (int32_t)offs[n];
-      continue;
-    }
-    *reinterpret_cast<int2 *>(seg + 2 * r) = make_int2((int32_t)offs[r], (int32_t)offs[r + 1]);
-    for (int l = 1; l < max_segs; l++) *reinterpret_cast<int2 *>(seg + (int64_t)l * pitch + 2 * r) = make_int2(-1, -1);
-    if (rp) row_sizes[r] = (int32_t)(rp[r + 1] - rp[r]);
-  }
-}
-
-// Copy CSR rows into their new layer-0 segments (warp per row, grid-stride).
-// CSR rows into their pool segments: a warp per row, four windows of 32
-// entries in flight.  A row longer than COPY_LONG entries is cut into pieces
-// of COPY_LONG entries, listed here as (row, piece) and copied a CTA per
-// piece by k_copy_csr_pieces: one warp would copy a power-law graph's
-// hottest rows alone, and the whole load would wait for it.
-constexpr int COPY_LONG = 4096;
-template <typename V>
-__global__ void k_copy_csr(int32_t n, const long long *__restrict__ offs, const long long *__restrict__ rp,
-                           const int32_t *__restrict__ cols, const V *__restrict__ vals, int32_t *__restrict__ pcols,
-                           V *__restrict__ pvals, unsigned long long *pieces, int32_t *piece_count) {
-  constexpr int U = 4;
+// CSR input check, by rows and by entries: the row pointer starts at 0, does
+// not decrease and ends at nnz; columns in range; rows strictly ascending.
+// The last by counting: *desc receives the number of entries whose column
+// does not exceed the one before, less those that start a row -- zero when
+// every row is strictly ascending (each term is counted where it is read,
+// coalesced, and no entry needs its row: 17M entries of a power-law graph
+// took 350 us with a warp per row, its hub rows alone).
+__global__ void k_csr_check(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ cols, int32_t n,
+                            int32_t n_cols, int64_t nnz, long long *stat) {
+  constexpr int U = 8;
   const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
-    const int64_t s = rp[r], L = rp[r + 1] - s, d = offs[r];
-    if (L > COPY_LONG) {
-      const int np = (int)((L + COPY_LONG - 1) / COPY_LONG);
-      int base = 0;
-      if (lane == 0) base = atomicAdd(piece_count, np);
-      base = __shfl_sync(FULL, base, 0);
-      for (int q = lane; q < np; q += 32) pieces[base + q] = ((unsigned long long)(uint32_t)r << 32) | (uint32_t)q;
-      continue;
-    }
-    for (int64_t j0 = 0; j0 < L; j0 += 32 * U) {
-      int32_t c[U];
-      V v[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t j = j0 + 32 * u + lane;
-        if (j < L) {
-          c[u] = __ldcs(cols + s + j);
-          v[u] = __ldcs(vals + s + j);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t j = j0 + 32 * u + lane;
-        if (j < L) {
-          pcols[d + j] = c[u];
-          pvals[d + j] = v[u];
-        }
-      }
-    }
-  }
-}
-
-// The listed pieces of long rows, a CTA per piece.
-template <typename V>
-__global__ void k_copy_csr_pieces(const unsigned long long *pieces, const int32_t *piece_count,
-                                  const long long *__restrict__ offs, const long long *__restrict__ rp,
-                                  const int32_t *__restrict__ cols, const V *__restrict__ vals,
-                                  int32_t *__restrict__ pcols, V *__restrict__ pvals) {
-  constexpr int U = 4;
-  const int32_t cnt = *piece_count;
-  const int nt = blockDim.x;
-  for (int64_t b = blockIdx.x; b < cnt; b += gridDim.x) {
-    const unsigned long long pc = pieces[b];
-    const int32_t r = (int32_t)(pc >> 32);
-    const int64_t q = (int64_t)(uint32_t)pc;
-    const int64_t s = rp[r], L = rp[r + 1] - s, d = offs[r];
-    const int64_t j1 = (q + 1) * COPY_LONG < L ? (q + 1) * COPY_LONG : L;
-    for (int64_t jb = q * COPY_LONG + threadIdx.x; jb < j1; jb += (int64_t)U * nt) {
-      int32_t c[U];
-      V v[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t j = jb + (int64_t)u * nt;
-        if (j < j1) {
-          c[u] = __ldcs(cols + s + j);
-          v[u] = __ldcs(vals + s + j);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t j = jb + (int64_t)u * nt;
-        if (j < j1) {
-          pcols[d + j] = c[u];
-          pvals[d + j] = v[u];
-        }
-      }
-    }
-  }
-}
-
-// CSR input check: row pointer monotone, columns in range, rows strictly
-// ascending (canonical); converts row_ptr to int64.
-__global__ void k_csr_check(const int32_t *row_ptr, const int32_t *cols, int32_t n, int32_t n_cols, long long *rp64,
-                            long long *stat) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned long long flags = 0;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  unsigned flags = 0;
+  int desc = 0;
+  for (int64_t r = tid; r < n; r += stride) {
     const int32_t s = row_ptr[r], e = row_ptr[r + 1];
-    if (lane == 0) {
-      rp64[r] = s;
-      if (r == n - 1) rp64[n] = e;
-      if (e < s || (r == 0 && s != 0)) flags |= AUX_BAD_ROWPTR;
+    if (e < s || s < 0 || (r == 0 && s != 0) || (r == n - 1 && e != nnz)) flags |= AUX_BAD_ROWPTR;
+    if (e > s && s > 0 && s < nnz && cols[s - 1] >= cols[s]) desc--;
+  }
+  const int64_t nw = stride >> 5;
+  for (int64_t b = (tid >> 5) * (32 * U); b < nnz; b += nw * (32 * U)) {
+    int32_t c[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t j = b + 32 * u + lane;
+      c[u] = j < nnz ? cols[j] : 0;
     }
-    if (e < s) continue;
-    for (int32_t j = s + lane; j < e; j += 32) {
-      const int32_t c = cols[j];
-      if (c < 0 || c >= n_cols) flags |= AUX_BAD_INDEX;
-      if (j > s && cols[j - 1] >= c) flags |= AUX_NONCANON;
+    int32_t last = lane == 31 && b > 0 ? cols[b - 1] : 0;  // the entry before the window, in lane 31
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t j = b + 32 * u + lane;
+      const int32_t up = __shfl_up_sync(FULL, c[u], 1), wrap = __shfl_sync(FULL, last, 31);
+      const int32_t prev = lane == 0 ? wrap : up;
+      if (j < nnz) {
+        if (c[u] < 0 || c[u] >= n_cols) flags |= AUX_BAD_INDEX;
+        if (j > 0 && prev >= c[u]) desc++;
+      }
+      last = c[u];
     }
   }
-  flags = __reduce_or_sync(FULL, (unsigned)flags);
-  if (lane == 0 && flags) atomicOr((unsigned long long *)&stat[ST_AUX], flags);
+  flags = __reduce_or_sync(FULL, flags);
+  desc = warp_sum(desc);
+  if (lane == 0) {
+    if (flags) atomicOr((unsigned long long *)&stat[ST_AUX], (unsigned long long)flags);
+    if (desc) atomicAdd((unsigned long long *)&stat[ST_SCRATCH], (unsigned long long)(long long)desc);
+  }
 }
 
-__global__ void k_expand_rows(const long long *rp, int32_t n, int32_t *rows) {
+__global__ void k_expand_rows(const int32_t *rp, int32_t n, int32_t *rows) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += nw)
     for (int64_t j = rp[r] + lane; j < rp[r + 1]; j += 32) rows[j] = (int32_t)r;
 }
 
-__global__ void k_lens(const int32_t *row_sizes, int32_t n, long long *out) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += stride)
-    out[r] = r < n ? row_sizes[r] : 0;
-}
-
-__global__ void k_sum_lens(const int32_t *row_sizes, int32_t n, long long *out) {
+// Sum of the row lengths: one atomic per block (with one per warp of a full
+// grid, 19k atomics on a single word took 12 of the 15 us at 2^20 rows).
+__global__ void __launch_bounds__(256) k_sum_lens(const int32_t *__restrict__ row_sizes, int32_t n, long long *out) {
+  __shared__ long long ws[8];
   long long s = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) s += row_sizes[r];
   s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0 && s) atomicAdd((unsigned long long *)out, (unsigned long long)s);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) s += ws[w];
+    if (s) atomicAdd((unsigned long long *)out, (unsigned long long)s);
+  }
 }
 
 // HYB -> COO: valid ELL slots (column-major, -1 padding) in (row, slot)
@@ -267,35 +182,23 @@ static void free_pool(dcsr_handle h, cudaStream_t s) {
 }
 
 static int clear_status(dcsr_handle h, cudaStream_t s);
+static int read_stat(dcsr_handle h, cudaStream_t s, long long *host);
 
-size_t load_scratch_bytes(dcsr_handle h) {
-  return arena_bytes(h->n_rows + 2, 8) + arena_bytes(1, 8) + scan_scratch_bytes(h->n_rows + 1);
+static size_t load_scratch_bytes(dcsr_handle h, int64_t nnz) {
+  return arena_bytes(h->n_rows + 2, 4) + arena_bytes(flat_tiles(nnz) + 1, 4) + scan_scratch_bytes(h->n_rows + 1);
 }
 
-int load_from_csr64(dcsr_handle h, const long long *rp, const int32_t *cols, const void *vals, cudaStream_t s) {
-  Arena &ar = h->scratch;  // caller reserved load_scratch_bytes() beyond its own use
-  const int32_t n = h->n_rows;
-  long long *caps = ar.take<long long>(n + 2);
-  int32_t *piece_count = ar.take<int32_t>(1);  // pieces of long rows listed by k_copy_csr
-  if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  DCSR_CUDA(cudaMemsetAsync(piece_count, 0, sizeof(int32_t), s));
-  DCSR_LAUNCH(k_caps_from_rp, grid_for(n + 1, 256), 256, 0, s, rp, n, h->o, caps);
-  DCSR_TRY(scan_i64(caps, caps, n + 1, h->stat + ST_TOTAL, ar, s));
-  long long host[ST_WORDS];
-  DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
-  DCSR_CUDA(cudaStreamSynchronize(s));
-  if (host[ST_STATUS] == DCSR_TIMEOUT) {  // a look-back wait of the sort or scan gave up
-    DCSR_TRY(clear_status(h, s));
-    return DCSR_TIMEOUT;
-  }
-  if (host[ST_AUX] & AUX_BAD_INDEX) {
-    DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
-    return DCSR_BAD_INDEX;
-  }
+// The end of a CSR or COO load, after the host has read the status words
+// (host): a fresh pool for the policy capacities (caps), the layout and the
+// entries.  nnz bounds the row pointer's entries.
+static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const int32_t *cols, const void *vals,
+                    int64_t nnz, const long long *host, cudaStream_t s) {
   const int64_t top = host[ST_TOTAL];
   if (top > 0x7fffffffLL) return DCSR_OOM;
   int64_t cap = pool_capacity(h->o, top);
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
+  int32_t *tile_row = h->scratch.take<int32_t>(flat_tiles(nnz) + 1);
+  if (h->scratch.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   int32_t *nc;
   void *nv;
   int64_t got;
@@ -305,23 +208,7 @@ int load_from_csr64(dcsr_handle h, const long long *rp, const int32_t *cols, con
   h->vals = nv;
   h->buf_cap = got;
   h->pool_cap = cap;
-  DCSR_LAUNCH(k_layout, grid_for(n + 1, 256), 256, 0, s, h->seg, h->row_sizes, n, h->pitch, h->o.max_segs, caps, rp);
-  // pieces of rows longer than COPY_LONG: at most 2 * top / COPY_LONG
-  unsigned long long *pieces = nullptr;
-  DCSR_CUDA(dcsr::dev_alloc(&pieces, sizeof(unsigned long long) * (size_t)(2 * top / COPY_LONG + 1), s));
-  const unsigned gp = (unsigned)(8 * sm_count());  // the pieces' grid
-  if (h->dtype == DCSR_F32) {
-    DCSR_LAUNCH(k_copy_csr<float>, grid_for((int64_t)n * 32, 256), 256, 0, s, n, caps, rp, cols, (const float *)vals,
-                h->cols, (float *)h->vals, pieces, piece_count);
-    DCSR_LAUNCH(k_copy_csr_pieces<float>, gp, 256, 0, s, pieces, piece_count, caps, rp, cols, (const float *)vals,
-                h->cols, (float *)h->vals);
-  } else {
-    DCSR_LAUNCH(k_copy_csr<double>, grid_for((int64_t)n * 32, 256), 256, 0, s, n, caps, rp, cols,
-                (const double *)vals, h->cols, (double *)h->vals, pieces, piece_count);
-    DCSR_LAUNCH(k_copy_csr_pieces<double>, gp, 256, 0, s, pieces, piece_count, caps, rp, cols, (const double *)vals,
-                h->cols, (double *)h->vals);
-  }
-  DCSR_CUDA(dcsr::dev_free(pieces, s));
+  DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, tile_row, s));
   h->bins_valid = false;
   // A load is a one-off: a resident matrix keeps no load-sized scratch (the
   // stream-ordered pool keeps the memory for the next allocation).
@@ -335,58 +222,16 @@ int load_from_csr64(dcsr_handle h, const long long *rp, const int32_t *cols, con
 // the pool is allocated at cap_bound entries (the caller's upper bound of
 // pool_capacity(top)), the rows are placed, and one synchronisation reads
 // the pool top to set the pool capacity.
-template <typename V>
-__global__ void k_place_rows(int32_t n, const long long *__restrict__ offs, const long long *__restrict__ src_off,
-                             const long long *__restrict__ lens, const int32_t *__restrict__ scols,
-                             const V *__restrict__ svals, int32_t *__restrict__ pcols, V *__restrict__ pvals) {
-  constexpr int U = 4;  // windows of 32 entries whose loads are in flight together
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
-    const int64_t s0 = src_off[r], L = lens[r], d = offs[r];
-    for (int64_t j0 = 0; j0 < L; j0 += 32 * U) {
-      int32_t c[U];
-      V v[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t j = j0 + 32 * u + lane;
-        if (j < L) {
-          c[u] = __ldcs(scols + s0 + j);
-          v[u] = __ldcs(svals + s0 + j);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t j = j0 + 32 * u + lane;
-        if (j < L) {
-          pcols[d + j] = c[u];
-          pvals[d + j] = v[u];
-        }
-      }
-    }
-  }
-}
-__global__ void k_caps_from_lens(const long long *lens, int32_t n, dcsr_opts o, long long *caps) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += stride)
-    caps[r] = r < n ? policy_cap(o, lens[r]) : 0;
-}
-__global__ void k_sizes_from_lens(const long long *lens, int32_t n, int32_t *row_sizes) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) row_sizes[r] = (int32_t)lens[r];
-}
-
 int load_from_rows(dcsr_handle h, const long long *src_off, const long long *lens, const int32_t *scols,
-                   const void *svals, int64_t cap_bound, cudaStream_t s) {
+                   const void *svals, int64_t bound, int64_t cap_bound, cudaStream_t s) {
   const int32_t n = h->n_rows;
   Arena &ar = h->scratch;
   ar.status = h->stat + ST_STATUS;
-  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) + scan_scratch_bytes(n + 1), s));
-  long long *caps = ar.take<long long>(n + 2);
+  DCSR_TRY(ar.reserve(2 * arena_bytes(n + 2, 4) + arena_bytes(flat_tiles(bound) + 1, 4) + scan_scratch_bytes(n + 1), s));
+  int32_t *off = ar.take<int32_t>(n + 2), *caps = ar.take<int32_t>(n + 2);
+  int32_t *tile_row = ar.take<int32_t>(flat_tiles(bound) + 1);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   if (cap_bound > 0x7fffffffLL) return DCSR_OOM;
-  DCSR_LAUNCH(k_caps_from_lens, grid_for(n + 1, 256), 256, 0, s, lens, n, h->o, caps);
-  DCSR_TRY(scan_i64(caps, caps, n + 1, h->stat + ST_TOTAL, ar, s));
   int32_t *nc;
   void *nv;
   int64_t got;
@@ -395,17 +240,8 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   h->cols = nc;
   h->vals = nv;
   h->buf_cap = got;
-  DCSR_LAUNCH(k_layout, grid_for(n + 1, 256), 256, 0, s, h->seg, h->row_sizes, n, h->pitch, h->o.max_segs, caps,
-              (const long long *)nullptr);
-  if (n > 0) DCSR_LAUNCH(k_sizes_from_lens, grid_for(n, 256), 256, 0, s, lens, n, h->row_sizes);
-  if (n > 0) {
-    if (h->dtype == DCSR_F32)
-      DCSR_LAUNCH(k_place_rows<float>, grid_for((int64_t)n * 32, 256), 256, 0, s, n, caps, src_off, lens, scols,
-                  (const float *)svals, h->cols, (float *)h->vals);
-    else
-      DCSR_LAUNCH(k_place_rows<double>, grid_for((int64_t)n * 32, 256), 256, 0, s, n, caps, src_off, lens, scols,
-                  (const double *)svals, h->cols, (double *)h->vals);
-  }
+  DCSR_TRY(place_rows_scan(h, lens, off, caps, tile_row, bound, ar, s));
+  DCSR_TRY(place_rows_copy(h, off, caps, tile_row, src_off, scols, svals, bound, s));
   long long host[ST_WORDS];
   DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
@@ -484,12 +320,11 @@ int compact(dcsr_handle h, cudaStream_t s) {
   const int32_t n = h->n_rows;
   Arena &ar = h->scratch;
   ar.status = h->stat + ST_STATUS;
-  if (!h->bins_valid) DCSR_TRY(build_schedule(h, s));  // before taking arena memory
-  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) + scan_scratch_bytes(n + 1), s));
-  long long *caps = ar.take<long long>(n + 2);
+  DCSR_TRY(ar.reserve(2 * arena_bytes(n + 2, 4) + arena_bytes(flat_tiles(h->pool_cap) + 1, 4) + scan_scratch_bytes(n + 1), s));
+  int32_t *off = ar.take<int32_t>(n + 2), *caps = ar.take<int32_t>(n + 2);
+  int32_t *tile_row = ar.take<int32_t>(flat_tiles(h->pool_cap) + 1);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  DCSR_LAUNCH(k_caps_from_sizes, grid_for(n + 1, 256), 256, 0, s, h->row_sizes, n, h->o, caps);
-  DCSR_TRY(scan_i64(caps, caps, n + 1, h->stat + ST_TOTAL, ar, s));
+  DCSR_TRY(compact_scan(h, off, caps, tile_row, ar, s));
   long long host[ST_WORDS];
   DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
@@ -503,9 +338,7 @@ int compact(dcsr_handle h, cudaStream_t s) {
   void *nv;
   int64_t got;
   DCSR_TRY(alloc_pool(h, cap, &nc, &nv, &got, s));
-  DCSR_TRY(copy_rows(h, caps, nc, nv, nullptr, nullptr, s));
-  DCSR_LAUNCH(k_layout, grid_for(n + 1, 256), 256, 0, s, h->seg, h->row_sizes, n, h->pitch, h->o.max_segs, caps,
-              (const long long *)nullptr);
+  DCSR_TRY(compact_copy(h, off, caps, tile_row, nc, nv, cap, s));
   free_pool(h, s);
   h->cols = nc;
   h->vals = nv;
@@ -655,41 +488,39 @@ int dcsr_from_csr(dcsr_handle h, const int32_t *row_ptr, const int32_t *cols, co
   if (!h || !row_ptr || (nnz > 0 && (!cols || !vals)) || nnz < 0 || nnz > 0x7fffffffLL) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const int32_t n = h->n_rows;
+  if (n == 0 && nnz != 0) return DCSR_BAD_ARG;
   Arena &ar = h->scratch;
-  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) + load_scratch_bytes(h), s));
-  long long *rp = ar.take<long long>(n + 2);
+  ar.status = h->stat + ST_STATUS;
+  DCSR_TRY(ar.reserve(load_scratch_bytes(h, nnz), s));
+  int32_t *caps = ar.take<int32_t>(n + 2);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
-  if (n > 0) DCSR_LAUNCH(k_csr_check, grid_for((int64_t)n * 32, 256), 256, 0, s, row_ptr, cols, n, h->n_cols, rp, h->stat);
-  else DCSR_CUDA(cudaMemsetAsync(rp, 0, sizeof(long long), s));
-  long long host[ST_WORDS], total = 0;
-  DCSR_CUDA(cudaMemcpyAsync(&total, rp + n, sizeof(total), cudaMemcpyDeviceToHost, s));
+  // the check and the capacities' scan together, then one read of both
+  static_assert(ST_SCRATCH == ST_AUX + 1, "the check's words are cleared together");
+  DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, 2 * sizeof(long long), s));
+  if (n > 0)
+    DCSR_LAUNCH(k_csr_check, grid_for(std::max<int64_t>(n, div_up(nnz, 8)), 256), 256, 0, s, row_ptr, cols, n,
+                h->n_cols, nnz, h->stat);
+  DCSR_TRY(caps_scan(h, row_ptr, caps, ar, s));
+  long long host[ST_WORDS];
   DCSR_TRY(read_stat(h, s, host));
   const long long aux = host[ST_AUX];
-  if (total != nnz) {
-    DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
-    return DCSR_BAD_ARG;
-  }
-  DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
+  if (aux || host[ST_SCRATCH]) DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, 2 * sizeof(long long), s));
   if (aux & AUX_BAD_ROWPTR) return DCSR_BAD_ARG;
   if (aux & AUX_BAD_INDEX) return DCSR_BAD_INDEX;
-  if ((aux & AUX_NONCANON) && h->o.mode == DCSR_MERGE) {
-    // canonicalise through the COO path (sort by (row,col), sum duplicates)
-    DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) + arena_bytes(nnz + 1, 4) + coo_to_csr_scratch(h, nnz) +
-                            load_scratch_bytes(h), s));
-    long long *rp2 = ar.take<long long>(n + 2);
-    int32_t *rows = ar.take<int32_t>(nnz + 1);
-    if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-    DCSR_LAUNCH(k_csr_check, grid_for((int64_t)n * 32, 256), 256, 0, s, row_ptr, cols, n, h->n_cols, rp2, h->stat);
-    DCSR_LAUNCH(k_expand_rows, grid_for((int64_t)n * 32, 256), 256, 0, s, rp2, n, rows);
-    DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
-    long long *crp;
-    int32_t *cc;
-    void *cv;
-    DCSR_TRY(coo_to_csr64(h, rows, cols, vals, nnz, true, ar, &crp, &cc, &cv, nullptr, s));
-    return load_from_csr64(h, crp, cc, cv, s);
+  if (host[ST_STATUS] == DCSR_TIMEOUT) {  // the scan's look-back gave up
+    DCSR_TRY(clear_status(h, s));
+    return DCSR_TIMEOUT;
   }
-  return load_from_csr64(h, rp, cols, vals, s);
+  if (host[ST_SCRATCH] != 0 && h->o.mode == DCSR_MERGE) {
+    // canonicalise through the COO path (sort by (row,col), sum duplicates)
+    int32_t *rows = nullptr;
+    DCSR_CUDA(dcsr::dev_alloc((void **)&rows, sizeof(int32_t) * (nnz + 1), s));
+    DCSR_LAUNCH(k_expand_rows, grid_for((int64_t)n * 32, 256), 256, 0, s, row_ptr, n, rows);
+    const int st = dcsr_from_coo(h, rows, cols, vals, nnz, stream);
+    DCSR_CUDA(dcsr::dev_free(rows, s));
+    return st;
+  }
+  return load_csr(h, row_ptr, caps, cols, vals, nnz, host, s);
 }
 
 int dcsr_from_coo(dcsr_handle h, const int32_t *rows, const int32_t *cols, const void *vals, int64_t nnz,
@@ -697,13 +528,23 @@ int dcsr_from_coo(dcsr_handle h, const int32_t *rows, const int32_t *cols, const
   if (!h || nnz < 0 || nnz > 0x7fffffffLL || (nnz > 0 && (!rows || !cols || !vals))) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   Arena &ar = h->scratch;
-  DCSR_TRY(ar.reserve(coo_to_csr_scratch(h, nnz) + load_scratch_bytes(h), s));
+  ar.status = h->stat + ST_STATUS;
+  DCSR_TRY(ar.reserve(coo_to_csr_scratch(h, nnz) + load_scratch_bytes(h, nnz), s));
   DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
-  long long *rp;
-  int32_t *cc;
+  int32_t *rp, *caps, *cc;
   void *cv;
-  DCSR_TRY(coo_to_csr64(h, rows, cols, vals, nnz, h->o.mode == DCSR_MERGE, ar, &rp, &cc, &cv, nullptr, s));
-  return load_from_csr64(h, rp, cc, cv, s);
+  DCSR_TRY(coo_to_csr(h, rows, cols, vals, nnz, h->o.mode == DCSR_MERGE, ar, &rp, &caps, &cc, &cv, s));
+  long long host[ST_WORDS];
+  DCSR_TRY(read_stat(h, s, host));
+  if (host[ST_STATUS] == DCSR_TIMEOUT) {  // a look-back wait of the sort or scan gave up
+    DCSR_TRY(clear_status(h, s));
+    return DCSR_TIMEOUT;
+  }
+  if (host[ST_AUX] & AUX_BAD_INDEX) {
+    DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
+    return DCSR_BAD_INDEX;
+  }
+  return load_csr(h, rp, caps, cc, cv, nnz, host, s);
 }
 
 int dcsr_from_hyb(dcsr_handle h, const int32_t *ell_cols, const void *ell_vals, int32_t ell_width, int64_t ell_pitch,
@@ -759,7 +600,7 @@ int dcsr_nnz(dcsr_handle h, int64_t *nnz, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX + 1, 0, sizeof(long long), s));
   if (h->n_rows > 0)
-    DCSR_LAUNCH(k_sum_lens, grid_for(h->n_rows, 256), 256, 0, s, h->row_sizes, h->n_rows, h->stat + ST_AUX + 1);
+    DCSR_LAUNCH(k_sum_lens, std::min(grid_for(h->n_rows, 1024), 2 * sm_count()), 256, 0, s, h->row_sizes, h->n_rows, h->stat + ST_AUX + 1);
   long long v = 0;
   DCSR_CUDA(cudaMemcpyAsync(&v, h->stat + ST_AUX + 1, sizeof(v), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
@@ -772,15 +613,12 @@ static int export_impl(dcsr_handle h, int32_t *row_ptr, int32_t *rows, int32_t *
   const int32_t n = h->n_rows;
   Arena &ar = arp ? *arp : h->scratch;
   ar.status = h->stat + ST_STATUS;
-  if (!h->bins_valid) DCSR_TRY(build_schedule(h, s, arp));  // before taking arena memory
-  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) + scan_scratch_bytes(n + 1), s));
-  long long *rp = ar.take<long long>(n + 2);
+  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 4) + arena_bytes(flat_tiles(h->pool_cap) + 1, 4) + scan_scratch_bytes(n + 1), s));
+  int32_t *off = row_ptr ? row_ptr : ar.take<int32_t>(n + 2);
+  int32_t *tile_row = ar.take<int32_t>(flat_tiles(h->pool_cap) + 1);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  DCSR_LAUNCH(k_lens, grid_for(n + 1, 256), 256, 0, s, h->row_sizes, n, rp);
-  DCSR_TRY(scan_i64(rp, rp, n + 1, nullptr, ar, s));
-  return copy_rows(h, rp, cols, vals, rows, row_ptr, s, limit);
+  return export_rows(h, off, tile_row, cols, vals, rows, limit, ar, s);
 }
-
 
 int dcsr_to_csr(dcsr_handle h, int32_t *row_ptr, int32_t *cols, void *vals, void *stream) {
   if (!h || !row_ptr) return DCSR_BAD_ARG;

@@ -2,9 +2,10 @@
 // (key, value) pairs, and the public segmented primitives
 // (count_sorted_indices, reduce_by_key).  All hand-written for sm_100a.
 #include <algorithm>
+#include <cstddef>
 #include <mutex>
 
-#include "common.cuh"
+#include "lookback.cuh"
 
 namespace dcsr {
 
@@ -71,101 +72,42 @@ __device__ __forceinline__ T block_excl_scan(T v, T *total) {
   return out;
 }
 
-// ------------------------------------------------- decoupled look-back
-//
-// Single-pass kernels: every block takes the next tile number from a device
-// counter (so all tiles before it are running or finished), publishes its
-// tile's aggregate, adds the aggregates of the tiles before it back to the
-// nearest published inclusive prefix, and publishes its own inclusive prefix.
-// A wait is only ever on an earlier tile, which therefore always finishes;
-// every wait still has an iteration limit, after which it counts a fault and
-// stops waiting.
-
-__device__ unsigned long long g_spin_faults = 0;
 constexpr int SPIN_LIMIT = 1 << 22;
-// Wait limit of the look-back kernels (SPIN_LIMIT unless a test lowered it)
-// and a test switch that keeps the first tile of every single-pass kernel
-// from publishing, so the waits on it run out (dcsr_debug_lookback).
-__device__ int g_spin_limit = SPIN_LIMIT;
-__device__ int g_lb_stall = 0;
+// Wait limit of the look-back kernels (SPIN_LIMIT unless a test lowered it),
+// the test switch that keeps the first tile of every single-pass kernel
+// from publishing so the waits on it run out (dcsr_debug_lookback), and the
+// count of waits that did.  Kernels of every file reach it through Lookback.
+__device__ LookbackGlobals g_lookback = {0ull, SPIN_LIMIT, 0};
 constexpr int LB_W = 8;  // earlier tiles whose flags one radix look-back step loads together
 
-__device__ __forceinline__ unsigned long long ld_vol(const unsigned long long *p) {
-  return *(const volatile unsigned long long *)p;
-}
-
-// Look-back words are packed: a tag (the epoch's low 30 bits, a 2-bit kind)
-// above a 32-bit value, so a word is published with one store and read with
-// one load -- no fences, no second load.  A sort's word per (tile, digit)
-// holds a count (kind 1: the tile's aggregate, 2: its inclusive prefix); a
-// scan's four words per tile hold the halves of its 64-bit aggregate and
-// inclusive prefix (kind 1: written).  A word is current when its tag is the
-// kernel's; the tag repeats every 2^30 kernels on one area, so the kernel
-// whose last block advances the epoch to such a multiple clears the area
-// (lb_advance) and a stale word never matches.
-constexpr unsigned long long LB_EMASK = (1ull << 30) - 1;
-__device__ __forceinline__ unsigned long long lb_pack(unsigned long long e, int kind, unsigned v) {
-  return ((e & LB_EMASK) << 34) | ((unsigned long long)kind << 32) | v;
-}
-
-// A wait that gave up: count it, mark the area's fault word with this
-// kernel's epoch (its other waits then give up early) and report
-// DCSR_TIMEOUT in the operation's status word.
-__device__ __forceinline__ void lb_give_up(const Lookback &lb, unsigned long long e) {
-  atomicAdd(&g_spin_faults, 1ull);
-  *(volatile unsigned long long *)lb.fault = (e & LB_EMASK) + 1;
-  if (lb.status) atomicCAS(reinterpret_cast<unsigned long long *>(lb.status), 0ull, (unsigned long long)DCSR_TIMEOUT);
-}
-// True when another wait of this kernel (epoch e) gave up already.
-__device__ __forceinline__ bool lb_faulted(const Lookback &lb, unsigned long long e) {
-  return ld_vol(lb.fault) == (e & LB_EMASK) + 1;
-}
-
-// Thread 0 of every block: the block's tile and the kernel's epoch.
-__device__ __forceinline__ void lb_begin(const Lookback &lb, unsigned *tile, unsigned long long *ep) {
-  if (threadIdx.x == 0) {
-    *tile = atomicAdd(lb.tiles, 1u);
-    *ep = ld_vol(lb.epoch);
+int lookback_globals(LookbackGlobals **out) {
+  static std::mutex mu;
+  static std::atomic<LookbackGlobals *> ptr[128] = {};
+  int dev = 0;
+  DCSR_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 128) return DCSR_NOT_SUPPORTED;
+  LookbackGlobals *g = ptr[dev].load();
+  if (!g) {
+    std::lock_guard<std::mutex> lock(mu);
+    void *p = nullptr;
+    DCSR_CUDA(cudaGetSymbolAddress(&p, g_lookback));
+    g = (LookbackGlobals *)p;
+    ptr[dev].store(g);
   }
-}
-
-// End of every block (all threads): true in the last block to finish.
-__device__ __forceinline__ bool lb_end(const Lookback &lb) {
-  __shared__ int last;
-  __syncthreads();
-  // (no fence: this block's results reach later kernels at the launch boundary)
-  if (threadIdx.x == 0) last = atomicAdd(lb.done, 1u) == gridDim.x - 1;
-  __syncthreads();
-  return last;
-}
-
-// The last block (all its threads): reset the counters and advance the
-// epoch; at a multiple of 2^30 clear the slots first (packed radix tags).
-__device__ __forceinline__ void lb_advance(const Lookback &lb) {
-  __shared__ unsigned long long next;
-  if (threadIdx.x == 0) next = ld_vol(lb.epoch) + 1;
-  __syncthreads();
-  if ((next & LB_EMASK) == 0)
-    for (unsigned long long i = threadIdx.x; i < lb.slots; i += blockDim.x) lb.flag[i] = 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *(volatile unsigned *)lb.tiles = 0;
-    *(volatile unsigned *)lb.done = 0;
-    __threadfence();
-    *(volatile unsigned long long *)lb.epoch = next;
-  }
+  *out = g;
+  return DCSR_OK;
 }
 
 long long spin_faults() {
-  unsigned long long v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_spin_faults, sizeof(v)) != cudaSuccess) return -1;
-  return (long long)v;
+  LookbackGlobals v;
+  if (cudaMemcpyFromSymbol(&v, g_lookback, sizeof(v)) != cudaSuccess) return -1;
+  return (long long)v.faults;
 }
 
 int debug_lookback(int spin_limit, int stall) {
   const int lim = spin_limit > 0 ? spin_limit : SPIN_LIMIT;
-  DCSR_CUDA(cudaMemcpyToSymbol(g_spin_limit, &lim, sizeof(int)));
-  DCSR_CUDA(cudaMemcpyToSymbol(g_lb_stall, &stall, sizeof(int)));
+  DCSR_CUDA(cudaMemcpyToSymbol(g_lookback, &lim, sizeof(int), offsetof(LookbackGlobals, spin_limit)));
+  DCSR_CUDA(cudaMemcpyToSymbol(g_lookback, &stall, sizeof(int), offsetof(LookbackGlobals, stall)));
   DCSR_CUDA(cudaDeviceSynchronize());
   return DCSR_OK;
 }
@@ -217,60 +159,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_1p(ScanArgs a, Lookback l
   long long bt;
   long long ex = block_excl_scan(sum, &bt);
   if (threadIdx.x < 32) {
-    // look-back: slot words 4t..4t+3 hold the tile's aggregate (low, high
-    // half) and inclusive prefix (low, high half), each a packed word written
-    // once per epoch, so a reader that sees both halves of one pair current
-    // has a consistent value -- no fences
     const int lane = threadIdx.x;
-    const unsigned long long tag = e & LB_EMASK;
-    unsigned long long *w = lb.flag;
-    auto cur = [&](unsigned long long x) { return (x >> 34) == tag && ((x >> 32) & 3) == 1; };
-    long long excl = 0;
-    if (t == t0) {
-      if (lane == 0 && !(g_lb_stall && t == 0)) {
-        *(volatile unsigned long long *)(w + 4 * t + 2) = lb_pack(e, 1, (unsigned)bt);
-        *(volatile unsigned long long *)(w + 4 * t + 3) = lb_pack(e, 1, (unsigned)((unsigned long long)bt >> 32));
-      }
-    } else {
-      if (lane == 0) {
-        *(volatile unsigned long long *)(w + 4 * t + 0) = lb_pack(e, 1, (unsigned)bt);
-        *(volatile unsigned long long *)(w + 4 * t + 1) = lb_pack(e, 1, (unsigned)((unsigned long long)bt >> 32));
-      }
-      int idle = 0;
-      for (int64_t j = t - 1;;) {
-        const int64_t q = j - lane;  // lane 0: the nearest earlier tile
-        bool ready = true, inc = true;
-        long long v = 0;
-        if (q >= t0) {  // before the array's first tile: an inclusive prefix of 0
-          const unsigned long long a0 = ld_vol(w + 4 * q), a1 = ld_vol(w + 4 * q + 1);
-          const unsigned long long i0 = ld_vol(w + 4 * q + 2), i1 = ld_vol(w + 4 * q + 3);
-          inc = cur(i0) && cur(i1);
-          ready = inc || (cur(a0) && cur(a1));
-          const unsigned long long lo = inc ? i0 : a0, hi = inc ? i1 : a1;
-          v = (long long)(((hi & 0xffffffffull) << 32) | (lo & 0xffffffffull));
-        }
-        const unsigned rm = __ballot_sync(FULL, ready), im = __ballot_sync(FULL, ready && inc);
-        const int first = im ? __ffs(im) - 1 : 32;  // nearest inclusive prefix in this window
-        const unsigned need = first >= 31 ? FULL : ((2u << first) - 1u);
-        if ((rm & need) == need) {  // everything up to it published
-          excl += warp_sum(lane <= first ? v : 0ll);
-          if (first < 32) break;
-          j -= 32;
-          idle = 0;
-          continue;
-        }
-        if (++idle >= g_spin_limit || ((idle & 1023) == 1023 && __any_sync(FULL, lb_faulted(lb, e)))) {
-          if (lane == 0) lb_give_up(lb, e);
-          break;
-        }
-        if (idle >= 32) __nanosleep(64);
-      }
-      if (lane == 0) {
-        const unsigned long long p = (unsigned long long)(excl + bt);
-        *(volatile unsigned long long *)(w + 4 * t + 2) = lb_pack(e, 1, (unsigned)p);
-        *(volatile unsigned long long *)(w + 4 * t + 3) = lb_pack(e, 1, (unsigned)(p >> 32));
-      }
-    }
+    const long long agg[1] = {bt};
+    long long before[1];
+    lb_lookback<1>(lb, e, t, t0, agg, before);
+    const long long excl = before[0];
     if (lane == 0) sh_prefix = excl;
   }
   __syncthreads();
@@ -544,7 +437,7 @@ __global__ void __launch_bounds__(OS_THREADS, MIN_BLOCKS) k_radix_onesweep(const
   if (d >= RS_BINS) {
     // no digit: nothing to look back for
   } else if (t == 0) {
-    if (!g_lb_stall) *(volatile unsigned long long *)(lb.flag + slot) = lb_pack(e, 2, run);
+    if (!lb.g->stall) *(volatile unsigned long long *)(lb.flag + slot) = lb_pack(e, 2, run);
   } else {
     *(volatile unsigned long long *)(lb.flag + slot) = lb_pack(e, 1, run);
     const unsigned long long tag = e & LB_EMASK;
@@ -567,7 +460,7 @@ __global__ void __launch_bounds__(OS_THREADS, MIN_BLOCKS) k_radix_onesweep(const
       }
       q -= used;
       if (used == 0) {  // the nearest tile has not published yet
-        if (++idle >= g_spin_limit || ((idle & 1023) == 1023 && lb_faulted(lb, e))) {
+        if (++idle >= lb.g->spin_limit || ((idle & 1023) == 1023 && lb_faulted(lb, e))) {
           lb_give_up(lb, e);
           break;
         }

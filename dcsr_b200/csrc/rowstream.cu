@@ -72,14 +72,6 @@ constexpr int CHUNK = DCSR_CHUNK;
 #ifndef DCSR_K1B_U
 #define DCSR_K1B_U 4
 #endif
-// Blocks per SM the copy pass (export, compaction) is compiled for.
-#ifndef DCSR_COPY_MINB
-#define DCSR_COPY_MINB 3
-#endif
-// Entries a thread copies per unit and pass (FP64: half).
-#ifndef DCSR_COPY_EPT
-#define DCSR_COPY_EPT 8
-#endif
 constexpr int STEP = 4096;    // entries a CTA has in flight per step
 enum { P_BLOCKS = 0, P_CHUNKS = 1, P_MED = 2 };
 
@@ -1288,156 +1280,6 @@ __global__ void __launch_bounds__(RS_THREADS_, DCSR_K1B_MINB) k_rows1_blocks(Src
   }
 }
 
-// -------------------------------------------------------------- copy pass
-// Copies each row's logical entries to dst_off[r] in (out_cols, out_vals),
-// optionally writing COO row ids and an int32 row pointer (one matrix).
-
-template <typename V, int PART>
-__global__ void __launch_bounds__(RS_THREADS_, DCSR_COPY_MINB) k_rows_copy(RowItem<V> it, const long long *__restrict__ dst_off,
-                                                           int32_t *__restrict__ out_cols, V *__restrict__ out_vals,
-                                                           int32_t *__restrict__ out_rows,
-                                                           int32_t *__restrict__ out_rowptr, int64_t limit) {
-  constexpr int U = 4;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const Mat<V> &m = it.m;
-  RowOne<V> src{it};
-  const int64_t units = src.units(PART);
-  if (PART == P_BLOCKS && out_rowptr && blockIdx.x == 0 && threadIdx.x == 0)
-    out_rowptr[m.n_rows] = (int32_t)dst_off[m.n_rows];
-  if constexpr (PART == P_CHUNKS || PART == P_MED) {
-    // Long-row chunks (a CTA each) or medium rows (a warp each), two per
-    // step (unit u and the one a grid stride later): both units' descriptor
-    // chains (unit -> row -> length, segments, destination) and then all
-    // their entries are in flight together -- one unit alone left the warps
-    // waiting on its chain for a fraction of the data.
-    static_assert(CHUNK % RS_THREADS_ == 0, "whole chunks per thread");
-    constexpr bool CH = PART == P_CHUNKS;
-    constexpr int NTHR = CH ? RS_THREADS_ : 32;
-    // a thread's entries per unit and pass: chunks DCSR_COPY_EPT, medium rows
-    // (shorter, a warp each) half that, FP64 half again (8 / 4 measured
-    // 217 us for the R-MAT 2^20 stream matrix's export, 8 / 8 with spills
-    // 267 us, 4 / 4 219 us; one unit per step 244 us)
-    constexpr int EMAX = (CH ? DCSR_COPY_EPT : DCSR_COPY_EPT / 2) / (sizeof(V) == 8 ? 2 : 1);
-    constexpr int EPT = CH && CHUNK / RS_THREADS_ < EMAX ? CHUNK / RS_THREADS_ : EMAX;
-    const int tid = CH ? threadIdx.x : lane;
-    // unit numbers: chunks per CTA, medium rows per warp
-    const int64_t n_units = CH ? units : it.info[2];
-    const int64_t first = CH ? blockIdx.x : (int64_t)blockIdx.x * RS_WARPS + w;
-    const int64_t stride = CH ? gridDim.x : (int64_t)gridDim.x * RS_WARPS;
-    for (int64_t u = first; u < n_units; u += 2 * stride) {
-      int32_t row[2];
-      int64_t c0[2], c1[2], d[2];
-      Chain ch[2];
-      bool fast[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int64_t uu = u + h * stride;
-        row[h] = -1;
-        c0[h] = c1[h] = d[h] = 0;
-        fast[h] = true;
-        ch[h].ns = 0;
-        if (uu < n_units) {
-          int64_t L;
-          if (CH) {
-            const int2 rl = it.chunk_rl[uu];
-            row[h] = rl.x;
-            L = m.row_sizes[rl.x];
-            const int64_t chunk = L <= CHUNK ? 0 : uu - it.long_off[rl.y];
-            c0[h] = chunk * CHUNK;
-            c1[h] = c0[h] + CHUNK < L ? c0[h] + CHUNK : L;
-          } else {
-            row[h] = it.med_desc[uu].x;
-            L = m.row_sizes[row[h]];
-            c1[h] = L;
-          }
-          ch[h] = load_chain(m, row[h]);
-          d[h] = dst_off[row[h]];
-          fast[h] = ch[h].cp[0] >= c1[h];
-          if (out_rowptr && c0[h] == 0 && tid == 0) out_rowptr[row[h]] = (int32_t)d[h];
-        }
-      }
-      const int64_t span = CH ? CHUNK : (c1[0] > c1[1] ? c1[0] : c1[1]);  // medium rows start at 0
-      for (int64_t s0 = 0; s0 < span; s0 += (int64_t)EPT * NTHR) {
-        int32_t cv[2 * EPT];
-        V vv[2 * EPT];
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-          for (int g = 0; g < EPT; g++) {
-            const int64_t p = c0[h] + s0 + tid + (int64_t)g * NTHR;
-            if (p < c1[h]) {
-              const int64_t q = fast[h] ? (int64_t)ch[h].st[0] + p : ch[h].phys(p);
-              cv[h * EPT + g] = __ldcs(m.cols + q);
-              vv[h * EPT + g] = __ldcs(m.vals + q);
-            }
-          }
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-          for (int g = 0; g < EPT; g++) {
-            const int64_t p = c0[h] + s0 + tid + (int64_t)g * NTHR;
-            if (p < c1[h] && d[h] + p < limit) {
-              out_cols[d[h] + p] = cv[h * EPT + g];
-              out_vals[d[h] + p] = vv[h * EPT + g];
-              if (out_rows) out_rows[d[h] + p] = row[h];
-            }
-          }
-      }
-    }
-  } else {
-    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {  // a block of 32 short rows per warp
-      const int64_t blk = u * RS_WARPS + w;
-      if (blk * 32 >= m.n_rows) continue;
-      const int64_t r0 = blk * 32;
-      const RowBlock rb = load_block(m, r0, lane, it.short_max);
-      const int64_t dme = rb.row >= 0 ? dst_off[rb.row] : 0;
-      if (out_rowptr && rb.row >= 0 && rb.len <= it.short_max) out_rowptr[rb.row] = (int32_t)dme;
-      int64_t cum = 0;
-      for (int l = 0; l < m.max_segs; l++) {
-        const int64_t dl = dme + cum;  // destination of this layer's part
-        int32_t len_l, st_l;
-        next_layer(m, rb, l, cum, len_l, st_l);
-        if (!__any_sync(FULL, len_l > 0)) break;
-        const int32_t incl = warp_incl_scan(len_l);
-        const int32_t excl = incl - len_l;
-        const int32_t E = __shfl_sync(FULL, incl, 31);
-        for (int32_t base = 0; base < E; base += 32 * U) {
-          int64_t q[U], dst[U];
-          int jw[U];
-#pragma unroll
-          for (int i = 0; i < U; i++) {
-            const int32_t w0 = base + 32 * i;
-            const int j = owner_lane(excl, w0 + lane);
-            const int32_t ej = __shfl_sync(FULL, excl, j);
-            const int32_t sj = __shfl_sync(FULL, st_l, j);
-            const int64_t dj = __shfl_sync(FULL, dl, j);
-            const bool ok = w0 + lane < E;
-            const int32_t off = ok ? w0 + lane - ej : 0;
-            jw[i] = ok ? j : -1;
-            q[i] = (int64_t)sj + off;
-            dst[i] = dj + off;
-          }
-          int32_t cv[U];
-          V vv[U];
-#pragma unroll
-          for (int i = 0; i < U; i++) {
-            cv[i] = __ldcs(m.cols + q[i]);
-            vv[i] = __ldcs(m.vals + q[i]);
-          }
-#pragma unroll
-          for (int i = 0; i < U; i++) {
-            if (jw[i] >= 0 && dst[i] < limit) {
-              out_cols[dst[i]] = cv[i];
-              out_vals[dst[i]] = vv[i];
-              if (out_rows) out_rows[dst[i]] = (int32_t)(r0 + jw[i]);
-            }
-          }
-        }
-      }
-    }
-  }
-}
-
 static int grid_of(const void *k) { return persistent_grid(k, RS_THREADS_, 0); }
 
 template <typename V, int K, int OP, bool VEC, typename Src>
@@ -1568,30 +1410,6 @@ int unit_prefix_many(const void *const *items, const int *counts, long long *con
   if (n > MAX_PREFIX_JOBS) return DCSR_BAD_ARG;
   if (dtype == DCSR_F32) return unit_prefix_many_t<float>(items, counts, prefs, splits, n, s);
   return unit_prefix_many_t<double>(items, counts, prefs, splits, n, s);
-}
-
-template <typename V>
-static int launch_copy(dcsr_handle h, const long long *dst_off, int32_t *out_cols, V *out_vals, int32_t *out_rows,
-                       int32_t *out_rowptr, int64_t limit, cudaStream_t s) {
-  static const int g0 = grid_of((const void *)k_rows_copy<V, P_BLOCKS>);
-  static const int g1 = grid_of((const void *)k_rows_copy<V, P_CHUNKS>);
-  static const int g2 = grid_of((const void *)k_rows_copy<V, P_MED>);
-  const RowItem<V> it = row_item<V>(h, nullptr, nullptr, 0, 0, 0.0, 0.0);
-  DCSR_LAUNCH((k_rows_copy<V, P_CHUNKS>), g1, RS_THREADS_, 0, s, it, dst_off, out_cols, out_vals, out_rows, out_rowptr,
-              limit);
-  DCSR_LAUNCH((k_rows_copy<V, P_MED>), g2, RS_THREADS_, 0, s, it, dst_off, out_cols, out_vals, out_rows, out_rowptr,
-              limit);
-  DCSR_LAUNCH((k_rows_copy<V, P_BLOCKS>), g0, RS_THREADS_, 0, s, it, dst_off, out_cols, out_vals, out_rows,
-              out_rowptr, limit);
-  return DCSR_OK;
-}
-
-int copy_rows(dcsr_handle h, const long long *dst_off, int32_t *out_cols, void *out_vals, int32_t *out_rows,
-              int32_t *out_rowptr, cudaStream_t s, int64_t limit) {
-  if (!h->bins_valid) DCSR_TRY(build_schedule(h, s));
-  if (h->dtype == DCSR_F32)
-    return launch_copy<float>(h, dst_off, out_cols, (float *)out_vals, out_rows, out_rowptr, limit, s);
-  return launch_copy<double>(h, dst_off, out_cols, (double *)out_vals, out_rows, out_rowptr, limit, s);
 }
 
 }  // namespace dcsr

@@ -631,7 +631,7 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
   }
   // C's rows go straight from the staging area into C's pool (policy
   // capacities); the second and last synchronisation reads C's pool top
-  const int st = load_from_rows(hC, ub, ucnt, tcol, tval, cap_bound, s);
+  const int st = load_from_rows(hC, ub, ucnt, tcol, tval, P, cap_bound, s);
   gg.release(s);
   ar.release(s);
   dcsr::dev_free(tcol, s);

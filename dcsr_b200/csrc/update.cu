@@ -767,7 +767,7 @@ __global__ void k_group(const unsigned long long *keys, int64_t n, int merge, lo
 template <typename V>
 __global__ void k_group_emit(const unsigned long long *keys, const unsigned *perm, const int32_t *cols,
                              const V *vals, int64_t n, int cb, int merge, int32_t n_cols, const long long *pos,
-                             int32_t *ocols, V *ovals, long long *rowcnt) {
+                             int32_t *ocols, V *ovals, int32_t *rowcnt) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const unsigned long long cmask = (1ull << cb) - 1;
   const int lane = threadIdx.x & 31;
@@ -792,28 +792,30 @@ __global__ void k_group_emit(const unsigned long long *keys, const unsigned *per
     // warp's entries are a few runs of one row each (a power-law graph's
     // hottest rows otherwise took one atomic per entry on a single word)
     const unsigned peers = __match_any_sync(FULL, r);
-    if (r >= 0 && __ffs(peers) - 1 == lane) atomicAdd((unsigned long long *)&rowcnt[r], (unsigned long long)__popc(peers));
+    if (r >= 0 && __ffs(peers) - 1 == lane) atomicAdd(&rowcnt[r], __popc(peers));
   }
 }
 
 size_t coo_to_csr_scratch(dcsr_handle h, int64_t T) {
   return 2 * arena_bytes(T, 8) + 2 * arena_bytes(T, 4) + arena_bytes(T + 1, 8) + arena_bytes(T, 4) +
-         arena_bytes(T, 8) + arena_bytes(h->n_rows + 2, 8) + radix_scratch_bytes(T) +
+         arena_bytes(T, 8) + 3 * arena_bytes(h->n_rows + 2, 4) + radix_scratch_bytes(T) +
          scan_scratch_bytes(std::max<int64_t>(T, h->n_rows + 1));
 }
 
 template <typename V>
 static int coo_impl(dcsr_handle h, const int32_t *rows, const int32_t *cols, const V *vals, int64_t T, bool merge,
-                    Arena &ar, long long **rp, int32_t **ocols, void **ovals, cudaStream_t s) {
+                    Arena &ar, int32_t **rp, int32_t **caps, int32_t **ocols, void **ovals, cudaStream_t s) {
   const int cb = bits_for(h->n_cols), rb = bits_for(h->n_rows);
   unsigned long long *k0 = ar.take<unsigned long long>(T), *k1 = ar.take<unsigned long long>(T);
   unsigned *p0 = ar.take<unsigned>(T), *p1 = ar.take<unsigned>(T);
   long long *flag = ar.take<long long>(T + 1);
   int32_t *oc = ar.take<int32_t>(T);
   V *ov = (V *)ar.take<double>(T);
-  long long *cnt = ar.take<long long>(h->n_rows + 2);
+  int32_t *cnt = ar.take<int32_t>(h->n_rows + 2);
+  *rp = ar.take<int32_t>(h->n_rows + 2);
+  *caps = ar.take<int32_t>(h->n_rows + 2);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  DCSR_CUDA(cudaMemsetAsync(cnt, 0, sizeof(long long) * (h->n_rows + 2), s));
+  DCSR_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (h->n_rows + 2), s));
   if (T > 0) {
     DCSR_LAUNCH(k_coo_keys, grid_for(T, 256), 256, 0, s, rows, cols, T, h->n_rows, h->n_cols, cb, merge ? 1 : 0, k0,
                 p0, h->stat);
@@ -823,19 +825,17 @@ static int coo_impl(dcsr_handle h, const int32_t *rows, const int32_t *cols, con
     DCSR_LAUNCH(k_group_emit<V>, grid_for(T, 256), 256, 0, s, k0, p0, cols, vals, T, cb, merge ? 1 : 0, h->n_cols,
                 flag, oc, ov, cnt);
   }
-  DCSR_TRY(scan_i64(cnt, cnt, h->n_rows + 1, nullptr, ar, s));
-  *rp = cnt;
+  DCSR_TRY(counts_scan(h, cnt, *rp, *caps, ar, s));
   *ocols = oc;
   *ovals = ov;
   return DCSR_OK;
 }
 
-int coo_to_csr64(dcsr_handle h, const int32_t *rows, const int32_t *cols, const void *vals, int64_t nnz, bool merge,
-                 Arena &ar, long long **rp, int32_t **ocols, void **ovals, int *bad, cudaStream_t s) {
-  (void)bad;
+int coo_to_csr(dcsr_handle h, const int32_t *rows, const int32_t *cols, const void *vals, int64_t nnz, bool merge,
+               Arena &ar, int32_t **rp, int32_t **caps, int32_t **ocols, void **ovals, cudaStream_t s) {
   if (h->dtype == DCSR_F32)
-    return coo_impl<float>(h, rows, cols, (const float *)vals, nnz, merge, ar, rp, ocols, ovals, s);
-  return coo_impl<double>(h, rows, cols, (const double *)vals, nnz, merge, ar, rp, ocols, ovals, s);
+    return coo_impl<float>(h, rows, cols, (const float *)vals, nnz, merge, ar, rp, caps, ocols, ovals, s);
+  return coo_impl<double>(h, rows, cols, (const double *)vals, nnz, merge, ar, rp, caps, ocols, ovals, s);
 }
 
 }  // namespace dcsr
