@@ -443,9 +443,10 @@ int scan2_i64(const long long *in0, long long *out0, long long *total0, const lo
               long long *total1, int64_t n, Arena &ar, cudaStream_t s);
 size_t scan_scratch_bytes(int64_t n);
 
-// Stable LSD radix sort of (uint64 key, uint32 value) pairs on bits [0, bits).
-// Sorted output lands in (*keys, *vals) -- the pointers are swapped with the
-// tmp buffers as passes ping-pong.
+// Stable LSD radix sort on bits [0, bits) of uint64 keys (no higher bit set),
+// each with its input position: *vals holds 0, 1, .., n-1 on entry.  Sorted
+// keys and positions land in (*keys, *vals) -- the pointers are swapped with
+// the tmp buffers as passes ping-pong.
 int radix_sort_pairs(unsigned long long **keys, unsigned **vals, unsigned long long **keys_tmp,
                      unsigned **vals_tmp, int64_t n, int bits, Arena &ar, cudaStream_t s);
 size_t radix_scratch_bytes(int64_t n);

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <mutex>
+#include <utility>
 
 #include "lookback.cuh"
 
@@ -78,7 +79,10 @@ constexpr int SPIN_LIMIT = 1 << 22;
 // from publishing so the waits on it run out (dcsr_debug_lookback), and the
 // count of waits that did.  Kernels of every file reach it through Lookback.
 __device__ LookbackGlobals g_lookback = {0ull, SPIN_LIMIT, 0};
-constexpr int LB_W = 8;  // earlier tiles whose flags one radix look-back step loads together
+#ifndef DCSR_LB_W
+#define DCSR_LB_W 8
+#endif
+constexpr int LB_W = DCSR_LB_W;  // earlier tiles whose flags one radix look-back step loads together
 
 int lookback_globals(LookbackGlobals **out) {
   static std::mutex mu;
@@ -250,35 +254,43 @@ int scan2_i64(const long long *in0, long long *out0, long long *total0, const lo
 
 // ------------------------------------------------------------ radix sort
 //
-// Stable LSD radix sort, 8-bit digits.  Up to RS_MID = 2^22 keys, one pass
-// over the keys per digit plus one histogram pass (a 1M-triple update's sort
-// ran 12 % faster this way than with the three-kernel passes below): (1) one kernel counts the digits of every
-// pass at once into per-pass histograms; (2) per pass, one scatter kernel:
-// each block takes the next tile, ranks its items per warp with match_any
-// (ties keep input order), orders its warps by a per-digit prefix, and finds
-// the items of each digit in the tiles before it by decoupled look-back (one
-// thread per digit, LB_W earlier tiles per step); the digit's global start is
-// the exclusive scan of the pass's histogram.  Larger inputs use three
-// kernels per pass (tile histograms, the exclusive scan of the digit-major
-// histogram table, a scatter with the same ranking and the scanned offsets),
-// which bounds the look-back area (one slot per tile and digit) for the
-// largest sorts and for sorts above RS_MID inside a stream capture.
+// Stable LSD radix sort of (key, input index) by 8-bit digits.  Where key and
+// index fit in 64 bits together (every update and load whose
+// row, column and triple count do: 40-bit keys of a 2^20 x 2^20 matrix with up
+// to 2^24 triples) the sort moves one packed word per item -- the first pass
+// packs, the last one unpacks -- else a key and an index.
+//   up to RS_SMALL items  one CTA, the words in registers, every pass a rank
+//                         and a scatter through shared memory;
+//   up to RS_BIG          one histogram kernel for all digits (its last block
+//                         scans them), then per pass one scatter kernel: a
+//                         block takes the next tile, ranks its items per warp
+//                         with match_any (ties keep input order), publishes
+//                         its digit counts, orders the tile in shared memory,
+//                         finds the items of each digit in the tiles before
+//                         it by decoupled look-back (one thread per digit,
+//                         LB_W earlier tiles per step) and writes whole digit
+//                         runs;
+//   larger                three kernels per pass (tile histograms, the scan of
+//                         the digit-major table, a scatter), which bounds the
+//                         look-back area.
+// Measured, 40-bit keys (five passes): 1.05M items 15.5 us a pass and 14 us
+// the histograms (35 and 11 us with key-index pairs, match_any and a scatter
+// straight from registers in tiles of 2048), 16.8M items 142-156 us a pass and
+// 57 us (350 and 67 us).  A pass moves 16 bytes an item (a floor of 40 us at
+// 16.8M); it is bound by the rank chains through shared memory at 24 warps
+// per SM.  Tiles of 2048, 3072 and 8192 items, 8 or 16 look-back words a step
+// and four blocks per SM (spills) were within 3% or slower.
 
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_BINS = 256;
-// items per lane: 16 for large inputs (three kernels per pass), 8 up to RS_MID
-// items (single-pass scatter)
 #ifndef DCSR_RS_MID_LOG2
 #define DCSR_RS_MID_LOG2 22
 #endif
+// Sorts above RS_MID may take the three-kernel passes inside a stream capture
+// (when the look-back area, one word per tile and digit, was not sized before
+// it), sorts above RS_BIG always do.  Either tier gives the same order.
 constexpr int64_t RS_MID = int64_t(1) << DCSR_RS_MID_LOG2;
-// Outside a stream capture the single-pass tier also takes sorts of up to
-// RS_BIG keys: its look-back area (one slot per tile and digit, 16 MB at
-// 2^24 keys) is grown on demand there, and the 16.1M-key sort of an R-MAT
-// 2^20 COO load ran 0.8 ms faster than with three kernels per pass.  Inside
-// a capture the tier stops at RS_MID, whose area a batch reserves before
-// capturing.  Either tier gives the same (stable) order.
 constexpr int64_t RS_BIG = int64_t(1) << 25;
 
 __device__ __forceinline__ unsigned lanemask_lt() {
@@ -359,40 +371,104 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const unsigned lon
 
 // Digit histograms of every pass (keys read once), into the look-back
 // area's histogram table (zero on entry: the previous sort's last pass left
-// it cleared).
+// it cleared); the last block turns each pass's counts into the digits' first
+// positions.
 __global__ void __launch_bounds__(RS_THREADS) k_radix_hist_all(const unsigned long long *keys, int64_t n,
                                                                 int passes, Lookback lb) {
   __shared__ unsigned h[8 * RS_BINS];
   for (int i = threadIdx.x; i < 8 * RS_BINS; i += RS_THREADS) h[i] = 0;
   __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RS_THREADS) {
-    const unsigned long long k = keys[i];
-    for (int p = 0; p < passes; p++) atomicAdd(&h[p * RS_BINS + (unsigned)((k >> (8 * p)) & 0xff)], 1u);
+  constexpr int U = 4;  // keys in flight per thread
+  const int64_t stride = (int64_t)gridDim.x * RS_THREADS;
+  for (int64_t i = (int64_t)blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += U * stride) {
+    unsigned long long k[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) k[u] = i + u * stride < n ? __ldg(keys + i + u * stride) : 0ull;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i + u * stride < n) {
+#pragma unroll
+        for (int p = 0; p < 8; p++)
+          if (p < passes) atomicAdd(&h[p * RS_BINS + (unsigned)((k[u] >> (8 * p)) & 0xff)], 1u);
+      }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < passes * RS_BINS; i += RS_THREADS)
     if (h[i]) atomicAdd(lb.hist + i, h[i]);
+  __threadfence();
+  if (lb_end(lb)) {
+    static_assert(RS_THREADS == RS_BINS, "a thread per digit");
+    __threadfence();
+    for (int p = 0; p < passes; p++) {
+      int all;
+      const int c = (int)__ldcg(lb.hist + p * RS_BINS + threadIdx.x);
+      lb.hist[p * RS_BINS + threadIdx.x] = (unsigned)block_excl_scan(c, &all);
+    }
+    if (threadIdx.x == 0) *(volatile unsigned *)lb.done = 0;
+  }
 }
 
-template <int OS_THREADS, int RS_ITEMS, int MIN_BLOCKS>
-__global__ void __launch_bounds__(OS_THREADS, MIN_BLOCKS) k_radix_onesweep(const unsigned long long *keys,
-                                                                   const unsigned *vals, unsigned long long *keys_out,
-                                                                   unsigned *vals_out, int64_t n, int pass,
-                                                                   int last_pass, Lookback lb) {
-  constexpr int RS_TILE = OS_THREADS * RS_ITEMS, OS_WARPS = OS_THREADS / 32;
-  __shared__ unsigned wcnt[OS_WARPS][RS_BINS];
-  __shared__ long long boff[RS_BINS];
+// Ranks of a warp's IT items (digit dg(j) of item j*32 + lane, for ok(j))
+// among the warp's items of the same digit, in input order; cnt (RS_BINS
+// counters, zero on entry) receives the warp's digit counts.  The lanes with
+// the same digit are found through a table of lane masks in shared memory
+// (RS_BINS words of the warp's own, zero on entry and on return): about ten
+// instructions, against forty for a ballot per bit; match_any ran at half the
+// ballots' speed.
+template <int IT, typename C, typename D, typename O>
+__device__ __forceinline__ void warp_digit_ranks(D &&dg, O &&ok, unsigned (&rank)[IT], C *cnt, unsigned *mask) {
+  const unsigned lt = lanemask_lt(), me = 1u << lane_id();
+#pragma unroll
+  for (int j = 0; j < IT; j++) {
+    const bool v = ok(j);
+    const unsigned d = dg(j);
+    if (v) atomicOr(&mask[d], me);
+    __syncwarp();
+    const unsigned peers = v ? mask[d] : 0u, pre = v ? cnt[d] : 0u;
+    const unsigned below = peers & lt;
+    rank[j] = pre + __popc(below);
+    __syncwarp();
+    if (v && below == 0) {
+      cnt[d] = (C)(pre + __popc(peers));
+      mask[d] = 0;
+    }
+    __syncwarp();
+  }
+}
+
+#ifndef DCSR_OS_MINB
+#define DCSR_OS_MINB 3
+#endif
+// One pass of the mid tier (the first RS_BINS threads own a digit each in the
+// middle).  PACK: keys_in holds key << ib | index words, or (FIRST) the bare
+// keys, packed here with their input positions; LAST unpacks to keys_out and
+// vals_out.  Not PACK: keys and indices side by side.
+template <int TH, int IT, bool PACK, bool FIRST, bool LAST>
+__global__ void __launch_bounds__(TH, DCSR_OS_MINB) k_radix_onesweep(const unsigned long long *__restrict__ keys,
+                                                           const unsigned *__restrict__ vals,
+                                                           unsigned long long *__restrict__ keys_out,
+                                                           unsigned *__restrict__ vals_out, int64_t n, int pass,
+                                                           int ib, int last_pass, Lookback lb) {
+  constexpr int TILE = TH * IT, WARPS = TH / 32;
+  static_assert(TH >= RS_BINS && TILE >= 2 * WARPS * RS_BINS * 4 / 8, "rank tables fit the tile's room");
+  extern __shared__ __align__(16) unsigned char os_sm[];
+  unsigned long long *sw = reinterpret_cast<unsigned long long *>(os_sm);  // the tile in digit order
+  unsigned *sv = reinterpret_cast<unsigned *>(sw + TILE);                   // (not PACK) its indices
+  unsigned(*mask)[RS_BINS] = reinterpret_cast<unsigned(*)[RS_BINS]>(os_sm);  // lane masks, before the tile is there
+  __shared__ unsigned wcnt[WARPS][RS_BINS];
+  __shared__ unsigned dstart[RS_BINS];  // a digit's first position in the ordered tile
+  __shared__ int goff[RS_BINS];         // its output position less that
   __shared__ unsigned sh_tile;
   __shared__ unsigned long long sh_ep;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
-  const int shift = 8 * pass;
+  const bool owner = TH == RS_BINS || d < RS_BINS;
   lb_begin(lb, &sh_tile, &sh_ep);
-  for (int i = threadIdx.x; i < OS_WARPS * RS_BINS; i += OS_THREADS) (&wcnt[0][0])[i] = 0;
-  // the digit's first position in the output: exclusive scan of the
-  // histogram (thread d < RS_BINS owns digit d from here on)
-  long long all;
-  const long long gbase =
-      block_excl_scan((long long)(d < RS_BINS ? __ldcg(lb.hist + pass * RS_BINS + d) : 0u), &all);
+  for (int i = lane; i < RS_BINS; i += 32) {
+    wcnt[warp][i] = 0;
+    mask[warp][i] = 0;
+  }
+  const unsigned gbase = owner ? __ldcg(lb.hist + pass * RS_BINS + d) : 0u;
+  __syncthreads();
   const int64_t t = sh_tile;
   const unsigned long long e = sh_ep;
   if (t >= gridDim.x) {  // a tile counter left non-zero (a bug): report it, touch nothing
@@ -400,179 +476,215 @@ __global__ void __launch_bounds__(OS_THREADS, MIN_BLOCKS) k_radix_onesweep(const
     if (lb_end(lb)) lb_advance(lb);
     return;
   }
-  const int64_t base = t * RS_TILE + (int64_t)warp * (32 * RS_ITEMS);
-  unsigned long long k[RS_ITEMS];
-  unsigned rank[RS_ITEMS], val[RS_ITEMS];
-  const unsigned lt = lanemask_lt();
+  const int64_t t0 = t * TILE;
+  const int cnt = n - t0 < TILE ? (int)(n - t0) : TILE;
+  const int wbase = warp * (32 * IT) + lane;
+  const int shift = 8 * pass + (PACK ? ib : 0);
+  unsigned long long k[IT];
+  unsigned val[PACK ? 1 : IT];
 #pragma unroll
-  for (int j = 0; j < RS_ITEMS; j++) {  // keys and values in one round of loads
-    const int64_t i = base + j * 32 + lane;
-    k[j] = i < n ? keys[i] : ~0ull;
-    val[j] = i < n ? vals[i] : 0u;
+  for (int j = 0; j < IT; j++) {
+    const int p = wbase + 32 * j;
+    k[j] = 0;
+    if constexpr (!PACK) val[j] = 0;
+    if (p < cnt) {
+      k[j] = __ldcs(keys + t0 + p);
+      if constexpr (!PACK) val[j] = __ldcs(vals + t0 + p);
+      if constexpr (PACK && FIRST) k[j] = (k[j] << ib) | (unsigned long long)(t0 + p);
+    }
   }
-#pragma unroll
-  for (int j = 0; j < RS_ITEMS; j++) {
-    const int64_t i = base + j * 32 + lane;
-    const unsigned dg = i < n ? (unsigned)((k[j] >> shift) & 0xff) : 0x100u;
-    const unsigned peers = __match_any_sync(FULL, dg);
-    const unsigned pre = dg < 0x100u ? wcnt[warp][dg] : 0u;
-    rank[j] = pre + __popc(peers & lt);
-    __syncwarp();
-    if (dg < 0x100u && (__ffs(peers) - 1) == lane) wcnt[warp][dg] = pre + __popc(peers);
-    __syncwarp();
-  }
+  auto digit = [&](int j) { return (unsigned)(k[j] >> shift) & 0xffu; };
+  auto valid = [&](int j) { return wbase + 32 * j < cnt; };
+  unsigned rank[IT];
+  warp_digit_ranks<IT>(digit, valid, rank, wcnt[warp], mask[warp]);
   __syncthreads();
   unsigned run = 0;  // exclusive prefix across warps per digit; run = the tile's count of digit d
-  if (d < RS_BINS)
-    for (int w = 0; w < OS_WARPS; w++) {
+  const int64_t slot = t * RS_BINS + d;
+  const unsigned tag2 = (unsigned)(e & LB_EMASK) << 2;  // a current look-back word's upper half, less its kind
+  auto publish = [&](unsigned kind, unsigned v) {
+    *(volatile unsigned long long *)(lb.flag + slot) = ((unsigned long long)(tag2 | kind) << 32) | v;
+  };
+  if (owner) {
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) {
       const unsigned c = wcnt[w][d];
       wcnt[w][d] = run;
       run += c;
     }
+    // published before the tile is put in order: later tiles can look back
+    if (t > 0) publish(1, run);
+    else if (!lb.g->stall) publish(2, run);
+  }
+  unsigned all;
+  const unsigned ds = block_excl_scan(run, &all);
+  if (owner) dstart[d] = ds;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < IT; j++) {
+    if (valid(j)) {
+      const unsigned dg = digit(j);
+      const unsigned lp = dstart[dg] + wcnt[warp][dg] + rank[j];
+      sw[lp] = k[j];
+      if constexpr (!PACK) sv[lp] = val[j];
+    }
+  }
   // items of digit d in the tiles before this one: look back over windows of
   // LB_W earlier tiles (their flags loaded together), consuming published
   // aggregates up to the nearest published inclusive prefix
-  long long excl = 0;
-  const int64_t slot = t * RS_BINS + d;
-  if (d >= RS_BINS) {
-    // no digit: nothing to look back for
-  } else if (t == 0) {
-    if (!lb.g->stall) *(volatile unsigned long long *)(lb.flag + slot) = lb_pack(e, 2, run);
-  } else {
-    *(volatile unsigned long long *)(lb.flag + slot) = lb_pack(e, 1, run);
-    const unsigned long long tag = e & LB_EMASK;
-    int64_t q = t - 1;
-    int idle = 0;
-    bool done = false;
-    while (!done) {
-      unsigned long long f[LB_W];
+  if (owner) {
+    unsigned excl = 0;
+    if (t > 0) {
+      const int limit = lb.g->spin_limit;
+      int q = (int)t - 1, idle = 0;
+      bool done = false;
+      while (!done) {
+        const unsigned long long *f0 = lb.flag + (int64_t)q * RS_BINS + d;
+        unsigned long long f[LB_W];
 #pragma unroll
-      for (int j = 0; j < LB_W; j++)
-        f[j] = q - j >= 0 ? ld_vol(lb.flag + (q - j) * RS_BINS + d) : lb_pack(e, 2, 0);  // before tile 0: 0
-      int used = 0;
+        for (int j = 0; j < LB_W; j++)  // before tile 0: an inclusive prefix of 0
+          f[j] = q >= j ? ld_vol(f0 - j * RS_BINS) : (unsigned long long)(tag2 | 2u) << 32;
+        int used = 0;
+        bool live = true;
 #pragma unroll
-      for (int j = 0; j < LB_W; j++) {
-        // stop at the first tile that has not published in this epoch
-        if (done || used < j || (f[j] >> 34) != tag || ((f[j] >> 32) & 3) == 0) continue;
-        excl += (long long)(f[j] & 0xffffffffull);
-        used = j + 1;
-        done = ((f[j] >> 32) & 3) == 2;
-      }
-      q -= used;
-      if (used == 0) {  // the nearest tile has not published yet
-        if (++idle >= lb.g->spin_limit || ((idle & 1023) == 1023 && lb_faulted(lb, e))) {
-          lb_give_up(lb, e);
-          break;
+        for (int j = 0; j < LB_W; j++) {
+          const unsigned kind = (unsigned)(f[j] >> 32) - tag2;  // 1, 2, or not published in this epoch
+          live = live && kind - 1u < 2u;
+          if (live) {
+            excl += (unsigned)f[j];
+            used = j + 1;
+            done = kind == 2u;
+            live = !done;
+          }
         }
-        if (idle >= 32) __nanosleep(64);
+        q -= used;
+        if (used == 0) {  // the nearest tile has not published yet
+          if (++idle >= limit || ((idle & 1023) == 1023 && lb_faulted(lb, e))) {
+            lb_give_up(lb, e);
+            break;
+          }
+          if (idle >= 32) __nanosleep(64);
+        }
       }
+      publish(2, excl + run);
     }
-    *(volatile unsigned long long *)(lb.flag + slot) = lb_pack(e, 2, (unsigned)(excl + run));
+    goff[d] = (int)(gbase + excl - ds);
   }
-  if (d < RS_BINS) boff[d] = gbase + excl;
   __syncthreads();
+  const unsigned long long imask = (1ull << ib) - 1;
 #pragma unroll
-  for (int j = 0; j < RS_ITEMS; j++) {
-    const int64_t i = base + j * 32 + lane;
-    if (i < n) {
-      const unsigned dg = (unsigned)((k[j] >> shift) & 0xff);
-      const int64_t pos = boff[dg] + wcnt[warp][dg] + rank[j];
-      keys_out[pos] = k[j];
-      vals_out[pos] = val[j];
+  for (int j = 0; j < IT; j++) {
+    const int lp = j * TH + threadIdx.x;
+    if (lp < cnt) {
+      const unsigned long long w = sw[lp];
+      const unsigned pos = (unsigned)(goff[(unsigned)(w >> shift) & 0xffu] + lp);
+      if constexpr (PACK && LAST) {
+        keys_out[pos] = w >> ib;
+        vals_out[pos] = (unsigned)(w & imask);
+      } else {
+        keys_out[pos] = w;
+        if constexpr (!PACK) vals_out[pos] = sv[lp];
+      }
     }
   }
   if (lb_end(lb)) {
     if (last_pass)  // leave the histogram table cleared for the next sort
-      for (int i = threadIdx.x; i < 8 * RS_BINS; i += OS_THREADS) lb.hist[i] = 0;
+      for (int i = threadIdx.x; i < 8 * RS_BINS; i += TH) lb.hist[i] = 0;
     __syncthreads();
     lb_advance(lb);
   }
 }
 
-// Small inputs (n <= RS_SMALL): one 1024-thread block runs every pass in
-// shared memory on (key, 16-bit input index) pairs -- per pass a digit
-// histogram, its scan, and a stable scatter in rounds of 1024 consecutive
-// items (warp ranks from match_any, warps ordered by a per-digit prefix) --
-// then gathers the values by index.  Same order as the multi-block sort.
+// Small inputs (n <= RS_SMALL, key and a 13-bit index within 64 bits): one
+// 1024-thread block keeps IT packed words per thread in registers and runs
+// every pass as rank (per-warp digit counters), prefix over warps and digits,
+// scatter to and reload from shared memory.  8192 keys of 24 bits: 56 us with
+// eight rounds of 1024 items per pass before.
 constexpr int RS_SMALL = 8192;
-constexpr size_t RS_SMALL_SMEM = (size_t)RS_SMALL * (2 * 8 + 2 * 2) + 32 * RS_BINS * 4 + 2 * RS_BINS * 4;
+constexpr int RS_SMALL_BITS = 13;
+constexpr int RS_SMALL_T = 1024;
 
-__global__ void __launch_bounds__(1024) k_radix_small(const unsigned long long *keys, const unsigned *vals,
-                                                       unsigned long long *keys_out, unsigned *vals_out, int n,
-                                                       int bits) {
-  extern __shared__ __align__(16) unsigned char sm[];
-  unsigned long long *ka = (unsigned long long *)sm;
-  unsigned long long *kb = ka + RS_SMALL;
-  unsigned short *ia = (unsigned short *)(kb + RS_SMALL);
-  unsigned short *ib = ia + RS_SMALL;
-  unsigned *wc = (unsigned *)(ib + RS_SMALL);  // [32][256]
-  unsigned *base = wc + 32 * RS_BINS;          // running digit offsets
-  unsigned *rtot = base + RS_BINS;             // this round's digit totals
+template <int IT>
+__global__ void __launch_bounds__(RS_SMALL_T) k_radix_small(const unsigned long long *__restrict__ keys,
+                                                            unsigned long long *__restrict__ keys_out,
+                                                            unsigned *__restrict__ vals_out, int n, int bits) {
+  constexpr int WARPS = RS_SMALL_T / 32, TILE = RS_SMALL_T * IT;
+  extern __shared__ __align__(16) unsigned char rs_sm[];
+  unsigned long long *sw = reinterpret_cast<unsigned long long *>(rs_sm);
+  unsigned *mask = reinterpret_cast<unsigned *>(sw + TILE);                      // [WARPS][RS_BINS] lane masks
+  unsigned short *wc = reinterpret_cast<unsigned short *>(mask + WARPS * RS_BINS);  // [WARPS][RS_BINS] counts
+  __shared__ unsigned quad[4][RS_BINS];  // digit counts of each quarter of the warps
+  __shared__ unsigned dstart[RS_BINS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned lt = lanemask_lt();
-  for (int i = tid; i < n; i += 1024) {
-    ka[i] = keys[i];
-    ia[i] = (unsigned short)i;
+  const int wbase = warp * (32 * IT) + lane;
+  const unsigned long long imask = (1ull << RS_SMALL_BITS) - 1;
+  unsigned long long k[IT];
+#pragma unroll
+  for (int j = 0; j < IT; j++) {
+    const int p = wbase + 32 * j;
+    k[j] = p < n ? (keys[p] << RS_SMALL_BITS) | (unsigned long long)p : ~0ull;
   }
-  for (int shift = 0; shift < bits; shift += 8) {
-    if (tid < RS_BINS) base[tid] = 0;
+  for (int i = tid; i < WARPS * RS_BINS; i += RS_SMALL_T) mask[i] = 0;
+  for (int shift = RS_SMALL_BITS; shift < bits + RS_SMALL_BITS; shift += 8) {
+    unsigned *wz = reinterpret_cast<unsigned *>(wc);
+    for (int i = tid; i < WARPS * RS_BINS / 2; i += RS_SMALL_T) wz[i] = 0;
     __syncthreads();
-    for (int i = tid; i < n; i += 1024) atomicAdd(&base[(unsigned)(ka[i] >> shift) & 0xff], 1u);
+    auto digit = [&](int j) { return (unsigned)(k[j] >> shift) & 0xffu; };
+    auto valid = [&](int j) { return wbase + 32 * j < n; };
+    unsigned rank[IT];
+    warp_digit_ranks<IT>(digit, valid, rank, wc + warp * RS_BINS, mask + warp * RS_BINS);
     __syncthreads();
-    if (warp == 0) {  // exclusive scan of the 256 digit counts (8 per lane)
-      unsigned v[8], t = 0;
+    // prefix over the warps: a thread per digit and quarter of the warps
+    const int dd = tid & (RS_BINS - 1), q = tid >> 8;
+    unsigned run = 0;
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        v[j] = base[lane * 8 + j];
-        t += v[j];
-      }
-      unsigned ex = warp_incl_scan(t) - t;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        base[lane * 8 + j] = ex;
-        ex += v[j];
-      }
+    for (int w = 0; w < WARPS / 4; w++) {
+      unsigned short *c = wc + (q * (WARPS / 4) + w) * RS_BINS + dd;
+      const unsigned x = *c;
+      *c = (unsigned short)run;
+      run += x;
     }
+    quad[q][dd] = run;
     __syncthreads();
-    for (int r0 = 0; r0 < n; r0 += 1024) {
-      const int i = r0 + tid;
-      for (int q = tid; q < 32 * RS_BINS; q += 1024) wc[q] = 0;
-      __syncthreads();
-      const unsigned long long k = i < n ? ka[i] : 0ull;
-      const unsigned d = i < n ? (unsigned)(k >> shift) & 0xff : 0x100u;
-      const unsigned peers = __match_any_sync(FULL, d);
-      const unsigned rank = __popc(peers & lt);
-      if (d < 0x100u && (__ffs(peers) - 1) == lane) wc[warp * RS_BINS + d] = __popc(peers);
-      __syncthreads();
-      if (tid < RS_BINS) {  // prefix across warps for digit tid
-        unsigned run = 0;
-        for (int w = 0; w < 32; w++) {
-          const unsigned c = wc[w * RS_BINS + tid];
-          wc[w * RS_BINS + tid] = run;
-          run += c;
+    if (warp == 0) {  // digit totals (8 per lane) -> first positions; quarters -> their offsets
+      unsigned tot[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        unsigned c[4], o = 0;
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          c[x] = quad[x][lane * 8 + j];
+          quad[x][lane * 8 + j] = o;
+          o += c[x];
         }
-        rtot[tid] = run;
+        tot[j] = o;
+        sum += o;
       }
-      __syncthreads();
-      if (d < 0x100u) {
-        const unsigned pos = base[d] + wc[warp * RS_BINS + d] + rank;
-        kb[pos] = k;
-        ib[pos] = ia[i];
+      unsigned ex = warp_incl_scan(sum) - sum;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        dstart[lane * 8 + j] = ex;
+        ex += tot[j];
       }
-      __syncthreads();
-      if (tid < RS_BINS) base[tid] += rtot[tid];
-      __syncthreads();
     }
-    unsigned long long *tk = ka;
-    ka = kb;
-    kb = tk;
-    unsigned short *ti = ia;
-    ia = ib;
-    ib = ti;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < IT; j++)
+      if (valid(j)) {
+        const unsigned dg = digit(j);
+        sw[dstart[dg] + quad[warp / (WARPS / 4)][dg] + wc[warp * RS_BINS + dg] + rank[j]] = k[j];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < IT; j++) k[j] = wbase + 32 * j < n ? sw[wbase + 32 * j] : ~0ull;
+    // (the next pass syncs before it writes the shared words)
   }
-  for (int i = tid; i < n; i += 1024) {
-    keys_out[i] = ka[i];
-    vals_out[i] = vals[ia[i]];
+#pragma unroll
+  for (int j = 0; j < IT; j++) {
+    const int p = wbase + 32 * j;
+    if (p < n) {
+      keys_out[p] = k[j] >> RS_SMALL_BITS;
+      vals_out[p] = (unsigned)(k[j] & imask);
+    }
   }
 }
 
@@ -581,12 +693,22 @@ size_t radix_scratch_bytes(int64_t n) {
   return arena_bytes(div_up(n, RS_THREADS * 16) * RS_BINS, 8);
 }
 
+// Items per thread of the single-pass scatter's tiles.
+#ifndef DCSR_OS_I
+#define DCSR_OS_I 16
+#endif
+#ifndef DCSR_OS_T
+#define DCSR_OS_T 256
+#endif
+constexpr int OS_I = DCSR_OS_I, OS_T = DCSR_OS_T;
+constexpr int OS_TILE = OS_T * OS_I;
+
 size_t lookback_slots(int64_t n) {
-  // mid-size sorts: one slot per (tile, digit); large sorts: the scan of their
-  // histogram table; scans: one slot per tile
-  const int64_t sort = n <= RS_MID ? div_up(n, RS_THREADS * 8) * RS_BINS
-                                   : div_up(div_up(n, RS_THREADS * 16) * RS_BINS, SCAN_TILE);
-  return (size_t)(std::max<int64_t>(sort, 8 * div_up(n, SCAN_TILE)) + 1);  // two-array scans: 4 words x 2 tiles
+  // single-pass sorts: one slot per (tile, digit); larger ones: the scan of
+  // their histogram table; scans: eight words per tile (two sums)
+  const int64_t sort = n <= RS_BIG ? div_up(n, OS_TILE) * RS_BINS
+                                   : 4 * div_up(div_up(n, RS_THREADS * 16) * RS_BINS, SCAN_TILE);
+  return (size_t)(std::max<int64_t>(sort, 8 * div_up(n, SCAN_TILE)) + 1);
 }
 
 // Large inputs: three kernels per pass (tile histograms, table scan, scatter).
@@ -613,56 +735,78 @@ static int radix_passes_table(unsigned long long **keys, unsigned **vals, unsign
   return DCSR_OK;
 }
 
+template <bool PACK, bool FIRST, bool LAST>
+static int launch_onesweep(const unsigned long long *ki, const unsigned *vi, unsigned long long *ko, unsigned *vo,
+                           int64_t n, int pass, int ib, bool last, const Lookback &lb, cudaStream_t s) {
+  constexpr size_t smem = (size_t)OS_TILE * (PACK ? 8 : 12);
+  static const cudaError_t attr = cudaFuncSetAttribute(k_radix_onesweep<OS_T, OS_I, PACK, FIRST, LAST>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  DCSR_CUDA(attr);
+  DCSR_LAUNCH((k_radix_onesweep<OS_T, OS_I, PACK, FIRST, LAST>), (unsigned)div_up(n, OS_TILE), OS_T, smem, s, ki, vi, ko,
+              vo, n, pass, ib, last ? 1 : 0, lb);
+  return DCSR_OK;
+}
+
 // Mid-size inputs: one histogram kernel, then one single-pass scatter per pass.
-// Tile shape of the single-pass scatter: OS_T threads x OS_I keys per thread
-// (tiles of 4096 and 8192 keys, with 256-1024 threads, ran no faster: the
-// pass time is the chain of memory round trips of one tile, not its size).
-constexpr int OS_T = 256, OS_I = 8, OS_MB = 2;
 static int radix_passes_onesweep(unsigned long long **keys, unsigned **vals, unsigned long long **keys_tmp,
                                  unsigned **vals_tmp, int64_t n, int bits, Arena &ar, cudaStream_t s) {
-  constexpr int ITEMS = OS_T * OS_I / RS_THREADS;  // keys per tile / RS_THREADS
-  const int passes = (int)div_up(bits, 8);
+  const int passes = (int)div_up(bits, 8), ib = bits_for(n);
   if (passes <= 0) return DCSR_OK;
-  const int64_t nt = div_up(n, RS_THREADS * ITEMS);
+  const bool pack = bits + ib <= 64;
   Lookback lb;
-  DCSR_TRY(ar.lookback((size_t)(nt * RS_BINS), s, &lb));
-  const int gh = (int)std::min<int64_t>(div_up(n, RS_THREADS * 8), 4 * sm_count());
+  DCSR_TRY(ar.lookback((size_t)(div_up(n, OS_TILE) * RS_BINS), s, &lb));
+  const int gh = (int)std::min<int64_t>(div_up(n, RS_THREADS * 8), 6 * sm_count());
   DCSR_LAUNCH(k_radix_hist_all, gh, RS_THREADS, 0, s, *keys, n, passes, lb);
   for (int p = 0; p < passes; p++) {
-    DCSR_LAUNCH((k_radix_onesweep<OS_T, OS_I, OS_MB>), (unsigned)nt, OS_T, 0, s, *keys, *vals, *keys_tmp, *vals_tmp,
-                n, p,
-                p == passes - 1 ? 1 : 0, lb);
-    unsigned long long *tk = *keys;
-    *keys = *keys_tmp;
-    *keys_tmp = tk;
-    unsigned *tv = *vals;
-    *vals = *vals_tmp;
-    *vals_tmp = tv;
+    const bool first = p == 0, last = p == passes - 1;
+    if (!pack)
+      DCSR_TRY((launch_onesweep<false, false, false>(*keys, *vals, *keys_tmp, *vals_tmp, n, p, 0, last, lb, s)));
+    else if (first && last)
+      DCSR_TRY((launch_onesweep<true, true, true>(*keys, *vals, *keys_tmp, *vals_tmp, n, p, ib, last, lb, s)));
+    else if (first)
+      DCSR_TRY((launch_onesweep<true, true, false>(*keys, *vals, *keys_tmp, *vals_tmp, n, p, ib, last, lb, s)));
+    else if (last)
+      DCSR_TRY((launch_onesweep<true, false, true>(*keys, *vals, *keys_tmp, *vals_tmp, n, p, ib, last, lb, s)));
+    else
+      DCSR_TRY((launch_onesweep<true, false, false>(*keys, *vals, *keys_tmp, *vals_tmp, n, p, ib, last, lb, s)));
+    std::swap(*keys, *keys_tmp);
+    if (!pack || last) std::swap(*vals, *vals_tmp);
   }
+  return DCSR_OK;
+}
+
+template <int IT>
+static int launch_small(const unsigned long long *ki, unsigned long long *ko, unsigned *vo, int64_t n, int bits,
+                        cudaStream_t s) {
+  constexpr size_t smem = (size_t)RS_SMALL_T * IT * 8 + RS_SMALL_T / 32 * RS_BINS * 6;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_radix_small<IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  DCSR_CUDA(attr);
+  DCSR_LAUNCH(k_radix_small<IT>, 1, RS_SMALL_T, smem, s, ki, ko, vo, (int)n, bits);
   return DCSR_OK;
 }
 
 int radix_sort_pairs(unsigned long long **keys, unsigned **vals, unsigned long long **keys_tmp,
                      unsigned **vals_tmp, int64_t n, int bits, Arena &ar, cudaStream_t s) {
   if (n <= 1) return DCSR_OK;
-  if (n <= RS_SMALL) {
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_radix_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMALL_SMEM);
-    DCSR_CUDA(attr);
-    DCSR_LAUNCH(k_radix_small, 1, 1024, RS_SMALL_SMEM, s, *keys, *vals, *keys_tmp, *vals_tmp, (int)n, bits);
-    unsigned long long *tk = *keys;
-    *keys = *keys_tmp;
-    *keys_tmp = tk;
-    unsigned *tv = *vals;
-    *vals = *vals_tmp;
-    *vals_tmp = tv;
+  if (n <= RS_SMALL && bits + RS_SMALL_BITS <= 64) {
+    if (n <= RS_SMALL_T) DCSR_TRY(launch_small<1>(*keys, *keys_tmp, *vals_tmp, n, bits, s));
+    else if (n <= 2 * RS_SMALL_T) DCSR_TRY(launch_small<2>(*keys, *keys_tmp, *vals_tmp, n, bits, s));
+    else if (n <= 4 * RS_SMALL_T) DCSR_TRY(launch_small<4>(*keys, *keys_tmp, *vals_tmp, n, bits, s));
+    else DCSR_TRY(launch_small<8>(*keys, *keys_tmp, *vals_tmp, n, bits, s));
+    std::swap(*keys, *keys_tmp);
+    std::swap(*vals, *vals_tmp);
     return DCSR_OK;
   }
   if (n <= RS_MID) return radix_passes_onesweep(keys, vals, keys_tmp, vals_tmp, n, bits, ar, s);
   if (n <= RS_BIG) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    DCSR_CUDA(cudaStreamIsCapturing(s, &cs));
-    if (cs == cudaStreamCaptureStatusNone) return radix_passes_onesweep(keys, vals, keys_tmp, vals_tmp, n, bits, ar, s);
+    bool fits = ar.lb && ar.lb_slots >= (size_t)(div_up(n, OS_TILE) * RS_BINS);
+    if (!fits) {  // the area is grown on demand, but not inside a capture
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      DCSR_CUDA(cudaStreamIsCapturing(s, &cs));
+      fits = cs == cudaStreamCaptureStatusNone;
+    }
+    if (fits) return radix_passes_onesweep(keys, vals, keys_tmp, vals_tmp, n, bits, ar, s);
   }
   return radix_passes_table(keys, vals, keys_tmp, vals_tmp, n, bits, ar, s);
 }
