@@ -75,7 +75,7 @@ __host__ __device__ inline int64_t policy_cap(const dcsr_opts &o, int64_t len) {
   int64_t c = (len * o.factor_x16 + 15) / 16;
   if (c < o.min_cap) c = o.min_cap;
   if (c < len) c = len;
-  return align_up(c, o.align);
+  return (c + o.align - 1) & ~(int64_t)(o.align - 1);  // align is a power of two (checked at creation)
 }
 __host__ __device__ inline int64_t pool_capacity(const dcsr_opts &o, int64_t top) {
   int64_t spare = top * o.spare_x16 / 16;
@@ -94,8 +94,10 @@ enum StatWord {
   ST_AUX = 6,      // per-update flags (bad index, layer overflow)
   ST_SCRATCH = 7,  // one-off device-side result words
   ST_TOP = 8,      // pool top before the current update
-  ST_T0 = 9,       // this matrix's touched-row range [T0, T1) in the batch
-  ST_T1 = 10,
+  ST_A0 = 9,       // this matrix's new segments take [A0, A1) of the batch's allocation order
+  ST_A1 = 10,
+  ST_LISTS = 11,   // rows of the batch's apply lists, small | big << 32 (batch-global word)
+  ST_RELOC = 12,   // relocated rows of the current batch (batch-global word)
   ST_WORDS = 16
 };
 
@@ -142,6 +144,7 @@ struct Lookback {
   LookbackGlobals *g;         // the device's wait limit, test switch and fault count
 };
 constexpr size_t LB_HEADER = 64 + 8 * 256 * 4;
+static_assert(LB_HEADER % 16 == 0, "look-back words of 16 bytes follow the header");
 
 // Stream-ordered scratch arena: one device buffer, bump-allocated per
 // operation, grown (stream-ordered free + malloc) when an operation needs more;

@@ -20,7 +20,7 @@ namespace {
 
 // Row lengths -> CSR row pointer and tile rows.
 struct OffsetsScan {
-  static constexpr int NS = 1;
+  static constexpr int NS = 1, IT = SM_LIGHT;
   using T = int32_t;
   struct State {};
   const int32_t *sizes;
@@ -39,7 +39,7 @@ struct OffsetsScan {
 // Row lengths -> CSR row pointer, tile rows and the offsets of the policy's
 // capacities (compaction); the capacities' sum goes to *top.
 struct CompactScan {
-  static constexpr int NS = 2;
+  static constexpr int NS = 2, IT = SM_LIGHT;
   using T = long long;
   struct State {};
   const int32_t *sizes;
@@ -69,7 +69,7 @@ struct CompactScan {
 
 // CSR row pointer -> offsets of the policy's capacities; their sum to *top.
 struct CapsScan {
-  static constexpr int NS = 1;
+  static constexpr int NS = 1, IT = SM_LIGHT;
   using T = long long;
   struct State {};
   const int32_t *rp;
@@ -93,7 +93,7 @@ struct CapsScan {
 // Row counts of a grouped COO batch -> CSR row pointer and the offsets of the
 // policy's capacities; the capacities' sum to *top.
 struct CountScan {
-  static constexpr int NS = 2;
+  static constexpr int NS = 2, IT = SM_LIGHT;
   using T = long long;
   struct State {};
   const int32_t *cnt;
@@ -122,7 +122,7 @@ struct CountScan {
 // Staged rows of given lengths -> CSR offsets, tile rows, capacity offsets and
 // the new layout itself (row lengths, layer 0, other layers cleared).
 struct PlaceScan {
-  static constexpr int NS = 2;
+  static constexpr int NS = 2, IT = SM_LIGHT;
   using T = long long;
   struct State {};
   const long long *lens;

@@ -2,6 +2,8 @@
 // look-back) and the scan over a row or entry function that the load, export,
 // schedule and update kernels are built from.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace dcsr {
@@ -24,8 +26,8 @@ __device__ __forceinline__ unsigned long long ld_vol(const unsigned long long *p
 // above a 32-bit value, so a word is published with one store and read with
 // one load -- no fences, no second load.  A sort's word per (tile, digit)
 // holds a count (kind 1: the tile's aggregate, 2: its inclusive prefix); a
-// scan's words per tile hold the halves of its 64-bit aggregates and
-// inclusive prefixes (kind 1: written).  A word is current when its tag is the
+// scan has one 128-bit word per tile, tag and kind above up to two 48-bit
+// sums, stored and loaded whole.  A word is current when its tag is the
 // kernel's; the tag repeats every 2^30 kernels on one area, so the kernel
 // whose last block advances the epoch to such a multiple clears the area
 // (lb_advance) and a stale word never matches.
@@ -82,70 +84,98 @@ __device__ __forceinline__ void lb_advance(const Lookback &lb) {
   }
 }
 
+// A scan's 128-bit look-back word (16-byte aligned), written and read as one
+// relaxed access: hi = tag | kind | 32 bits, lo = 64 bits; the 96 bits hold
+// one 64-bit sum or two of 48 bits.
+struct LbWord {
+  unsigned long long lo, hi;
+};
+__device__ __forceinline__ LbWord lb_load(const unsigned long long *p) {
+  LbWord w;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(w.lo), "=l"(w.hi)
+               : "l"(p)
+               : "memory");
+  return w;
+}
+__device__ __forceinline__ void lb_store(unsigned long long *p, const LbWord &w) {
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%0, %1};\n\tst.relaxed.gpu.global.b128 [%2], q;\n\t}" ::"l"(w.lo),
+               "l"(w.hi), "l"(p)
+               : "memory");
+}
+template <int NS>
+__device__ __forceinline__ LbWord lb_word(unsigned long long e, int kind, const long long (&v)[NS]) {
+  static_assert(NS == 1 || NS == 2, "one or two sums");
+  LbWord w;
+  w.lo = (unsigned long long)v[0];
+  w.hi = lb_pack(e, kind, 0);
+  if constexpr (NS == 2) {
+    const unsigned long long b = (unsigned long long)v[1];
+    w.lo = (w.lo & 0xffffffffffffull) | (b << 48);
+    w.hi |= (b >> 16) & 0xffffffffull;
+  }
+  return w;
+}
+template <int NS>
+__device__ __forceinline__ long long lb_sum(const LbWord &w, int q) {
+  if constexpr (NS == 1) return (long long)w.lo;
+  return q == 0 ? (long long)(w.lo & 0xffffffffffffull) : (long long)((w.lo >> 48) | ((w.hi & 0xffffffffull) << 16));
+}
+// Look-back words (8 bytes) that a scan of `tiles` tiles needs.
+constexpr int LB_SCAN_WORDS = 2;
+
 // Warp 0 of tile t (the first tile of its sequence is t0): publish the NS
-// aggregates agg (in every lane), look back over 32 earlier tiles at a time,
-// publish the inclusive prefixes; excl receives the sums of the tiles before
-// t (in every lane).  Slot words of tile t: 4*NS of them -- per sum the
-// halves of its aggregate, then per sum the halves of its inclusive prefix,
-// each a packed word written once per epoch, so a reader that sees all halves
-// of one kind current has consistent values.
+// aggregates agg (in every lane), look back over the earlier tiles, publish
+// the inclusive prefixes; excl receives the sums of the tiles before t (in
+// every lane).  A step loads 32 * LB_U tiles' words together: when all tiles
+// of a scan run at once (up to about 2^20 items) the look-back is a chain of
+// such round trips, and the 512 tiles of a 2^20-row scan took 10 of its 16 us
+// with 32 tiles and four 64-bit words each a step.
+constexpr int LB_U = 4;
 template <int NS>
 __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long long e, int64_t t, int64_t t0,
                                             const long long (&agg)[NS], long long (&excl)[NS]) {
   const int lane = lane_id();
-  const unsigned long long tag = e & LB_EMASK;
+  const unsigned tag2 = (unsigned)(e & LB_EMASK) << 2;  // a current word's upper 32 bits, less its kind
   unsigned long long *w = lb.flag;
-  auto cur = [&](unsigned long long x) { return (x >> 34) == tag && ((x >> 32) & 3) == 1; };
-  auto put = [&](int64_t tile, int kind, const long long (&v)[NS]) {  // kind 0: aggregates, 1: inclusive prefixes
-    if (lane == 0) {
-#pragma unroll
-      for (int q = 0; q < NS; q++) {
-        volatile unsigned long long *p = w + 4 * NS * tile + 2 * NS * kind + 2 * q;
-        p[0] = lb_pack(e, 1, (unsigned)(unsigned long long)v[q]);
-        p[1] = lb_pack(e, 1, (unsigned)((unsigned long long)v[q] >> 32));
-      }
-    }
-  };
 #pragma unroll
   for (int q = 0; q < NS; q++) excl[q] = 0;
   if (t == t0) {
-    if (!(lb.g->stall && t == 0)) put(t, 1, agg);
+    if (lane == 0 && !(lb.g->stall && t == 0)) lb_store(w + 2 * t, lb_word<NS>(e, 2, agg));
     return;
   }
-  put(t, 0, agg);
+  if (lane == 0) lb_store(w + 2 * t, lb_word<NS>(e, 1, agg));
   int idle = 0;
   const int limit = lb.g->spin_limit;
-  for (int64_t j = t - 1;;) {
-    const int64_t r = j - lane;  // lane 0: the nearest earlier tile
-    bool ready = true, inc = true;
-    long long v[NS];
+  bool done = false;
+  for (int64_t j = t - 1; !done;) {
+    LbWord x[LB_U];
 #pragma unroll
-    for (int q = 0; q < NS; q++) v[q] = 0;
-    if (r >= t0) {  // before the first tile: an inclusive prefix of 0
-      unsigned long long x[4 * NS];
+    for (int u = 0; u < LB_U; u++) {
+      const int64_t r = j - 32 * u - lane;  // u = 0, lane 0: the nearest earlier tile
+      if (r >= t0) x[u] = lb_load(w + 2 * r);
+      else x[u] = LbWord{0, lb_pack(e, 2, 0)};  // before the first tile: an inclusive prefix of 0
+    }
+    int used = 0;
+    bool live = true;
 #pragma unroll
-      for (int q = 0; q < 4 * NS; q++) x[q] = ld_vol(w + 4 * NS * r + q);
-      bool a = true;
+    for (int u = 0; u < LB_U; u++) {
+      if (!live) continue;
+      const unsigned kind = (unsigned)(x[u].hi >> 32) - tag2;  // 1, 2, or not published in this epoch
+      const unsigned rm = __ballot_sync(FULL, kind - 1u < 2u), im = __ballot_sync(FULL, kind == 2u);
+      const int first = im ? __ffs(im) - 1 : 32;  // nearest inclusive prefix among these 32
+      const unsigned need = first >= 31 ? FULL : ((2u << first) - 1u);
+      live = (rm & need) == need;  // everything up to it published
+      if (live) {
 #pragma unroll
-      for (int q = 0; q < 2 * NS; q++) {
-        a = a && cur(x[q]);
-        inc = inc && cur(x[2 * NS + q]);
-      }
-      ready = inc || a;
-#pragma unroll
-      for (int q = 0; q < NS; q++) {
-        const unsigned long long lo = inc ? x[2 * NS + 2 * q] : x[2 * q], hi = inc ? x[2 * NS + 2 * q + 1] : x[2 * q + 1];
-        v[q] = (long long)(((hi & 0xffffffffull) << 32) | (lo & 0xffffffffull));
+        for (int q = 0; q < NS; q++) excl[q] += warp_sum(lane <= first ? lb_sum<NS>(x[u], q) : 0ll);
+        used = u + 1;
+        done = first < 32;
+        live = !done;
       }
     }
-    const unsigned rm = __ballot_sync(FULL, ready), im = __ballot_sync(FULL, ready && inc);
-    const int first = im ? __ffs(im) - 1 : 32;  // nearest inclusive prefix in this window
-    const unsigned need = first >= 31 ? FULL : ((2u << first) - 1u);
-    if ((rm & need) == need) {  // everything up to it published
-#pragma unroll
-      for (int q = 0; q < NS; q++) excl[q] += warp_sum(lane <= first ? v[q] : 0ll);
-      if (first < 32) break;
-      j -= 32;
+    j -= 32 * used;
+    if (used) {
       idle = 0;
       continue;
     }
@@ -158,7 +188,7 @@ __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long lo
   long long inclv[NS];
 #pragma unroll
   for (int q = 0; q < NS; q++) inclv[q] = excl[q] + agg[q];
-  put(t, 1, inclv);
+  if (lane == 0) lb_store(w + 2 * t, lb_word<NS>(e, 2, inclv));
 }
 
 // ------------------------------------------------------- scan over a function
@@ -166,23 +196,36 @@ __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long lo
 // One kernel computes a value (NS of them) per item i in [0, n), scans it
 // exclusively and hands every item its prefix, so an operator needs no array
 // of flags, no scan of it and no pass over the result.  F supplies
-//   static constexpr int NS;
+//   static constexpr int NS, IT;     sums; items per thread
 //   struct State;                    what load leaves for emit (registers)
-//   load(i, ok, st, v[NS])           value of item i (ok false: past the end, v must be 0)
-//   emit(i, ok, st, excl[NS], v[NS]) item i's prefix; called by whole warps
+//   load(i, ok, st, v[NS])           value of item i (ok false: past the end, v must be 0),
+//                                    or, with a member LOAD_ALL, load_all(base, n, st[], v[][NS])
+//                                    for the thread's items base + 32*j at once
+//   emit(i, ok, st, excl[NS], v[NS]) item i's prefix; called by whole warps (with a member
+//                                    EMIT_ALL after emit_all(base, n, st[], v[][NS]))
 //   total(tot[NS])                   one thread, the totals
-// A warp takes 32*SM_ITEMS consecutive items, item j*32 + lane in lane's j-th
-// step (coalesced, and every step's prefix by a warp scan in registers -- no
-// staging through shared memory).  One block (no look-back) up to
-// SM_ONE items; else tiles of SM_THREADS*SM_ITEMS.
-constexpr int SM_ITEMS = 8;
+// A warp takes 32*IT consecutive items, item j*32 + lane in lane's j-th step
+// (coalesced, and every step's prefix by a warp scan in registers -- no
+// staging through shared memory), a block SM_THREADS*IT.  Light functions
+// (IT = 8) of up to SM_ONE items run in one block without look-back; heavy
+// ones (IT = 4: searches, plans) spread over blocks from 1024 items on.
+constexpr int SM_LIGHT = 8, SM_HEAVY = 4;
 constexpr int SM_THREADS = 256;
 constexpr int SM_ONE_THREADS = 1024;
-constexpr int64_t SM_ONE = SM_ONE_THREADS * SM_ITEMS;
+constexpr int64_t SM_ONE = SM_ONE_THREADS * SM_LIGHT;
+
+template <class F, class = void>
+struct ScanHasEmitAll : std::false_type {};
+template <class F>
+struct ScanHasEmitAll<F, std::void_t<decltype(F::EMIT_ALL)>> : std::true_type {};
+template <class F, class = void>
+struct ScanHasLoadAll : std::false_type {};
+template <class F>
+struct ScanHasLoadAll<F, std::void_t<decltype(F::LOAD_ALL)>> : std::true_type {};
 
 template <int TH, class F>
-__global__ void __launch_bounds__(TH) k_scan_map(F f, int64_t n, Lookback lb) {
-  constexpr int NS = F::NS, NW = TH / 32;
+__global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY ? 3 : 4) k_scan_map(F f, int64_t n, Lookback lb) {
+  constexpr int NS = F::NS, NW = TH / 32, SM_ITEMS = F::IT;
   __shared__ long long wsum[NS][NW];
   __shared__ long long sh_prefix[NS];
   __shared__ unsigned sh_tile;
@@ -208,10 +251,14 @@ __global__ void __launch_bounds__(TH) k_scan_map(F f, int64_t n, Lookback lb) {
   long long run[NS];
 #pragma unroll
   for (int q = 0; q < NS; q++) run[q] = 0;
+  if constexpr (ScanHasLoadAll<F>::value) {
+    f.load_all(base, n, st, v);
+  } else {
 #pragma unroll
-  for (int j = 0; j < SM_ITEMS; j++) {
-    const int64_t i = base + 32 * j;
-    f.load(i, i < n, st[j], v[j]);
+    for (int j = 0; j < SM_ITEMS; j++) {
+      const int64_t i = base + 32 * j;
+      f.load(i, i < n, st[j], v[j]);
+    }
   }
 #pragma unroll
   for (int j = 0; j < SM_ITEMS; j++)
@@ -244,6 +291,7 @@ __global__ void __launch_bounds__(TH) k_scan_map(F f, int64_t n, Lookback lb) {
 #pragma unroll
     for (int q = 0; q < NS; q++) before[q] += sh_prefix[q];
   }
+  if constexpr (ScanHasEmitAll<F>::value) f.emit_all(base, n, st, v);
 #pragma unroll
   for (int j = 0; j < SM_ITEMS; j++) {
     const int64_t i = base + 32 * j;
@@ -261,21 +309,24 @@ __global__ void __launch_bounds__(TH) k_scan_map(F f, int64_t n, Lookback lb) {
   if (!single && lb_end(lb)) lb_advance(lb);
 }
 
-// n >= 1 items.  Needs 4*NS look-back slots per SM_THREADS*SM_ITEMS items
-// (lookback_slots covers NS <= 2).
+// n >= 1 items.  Needs LB_SCAN_WORDS look-back slots per SM_THREADS*IT items.
 template <class F>
 static int scan_map(const F &f, int64_t n, Arena &ar, cudaStream_t s) {
   Lookback lb;
   std::memset(&lb, 0, sizeof(lb));
-  if (n <= SM_THREADS * SM_ITEMS) {
+  const int64_t nt = div_up(n, SM_THREADS * F::IT);
+  if (nt == 1) {
     DCSR_LAUNCH((k_scan_map<SM_THREADS, F>), 1, SM_THREADS, 0, s, f, n, lb);
-  } else if (n <= SM_ONE) {
-    DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
-  } else {
-    const int64_t nt = div_up(n, SM_THREADS * SM_ITEMS);
-    DCSR_TRY(ar.lookback((size_t)(4 * F::NS * nt), s, &lb));
-    DCSR_LAUNCH((k_scan_map<SM_THREADS, F>), (unsigned)nt, SM_THREADS, 0, s, f, n, lb);
+    return DCSR_OK;
   }
+  if constexpr (F::IT == SM_LIGHT) {
+    if (n <= SM_ONE) {
+      DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
+      return DCSR_OK;
+    }
+  }
+  DCSR_TRY(ar.lookback((size_t)(LB_SCAN_WORDS * nt), s, &lb));
+  DCSR_LAUNCH((k_scan_map<SM_THREADS, F>), (unsigned)nt, SM_THREADS, 0, s, f, n, lb);
   return DCSR_OK;
 }
 

@@ -229,7 +229,7 @@ int scan_i64(const long long *in, long long *out, int64_t n, long long *total, A
     return DCSR_OK;
   }
   Lookback lb;
-  DCSR_TRY(ar.lookback((size_t)(4 * a.nt), s, &lb));  // four look-back words per tile
+  DCSR_TRY(ar.lookback((size_t)(LB_SCAN_WORDS * a.nt), s, &lb));
   DCSR_LAUNCH(k_scan_1p, (unsigned)a.nt, SCAN_THREADS, 0, s, a, lb);
   return DCSR_OK;
 }
@@ -247,7 +247,7 @@ int scan2_i64(const long long *in0, long long *out0, long long *total0, const lo
     return DCSR_OK;
   }
   Lookback lb;
-  DCSR_TRY(ar.lookback((size_t)(8 * a.nt), s, &lb));
+  DCSR_TRY(ar.lookback((size_t)(2 * LB_SCAN_WORDS * a.nt), s, &lb));
   DCSR_LAUNCH(k_scan_1p, (unsigned)(2 * a.nt), SCAN_THREADS, 0, s, a, lb);
   return DCSR_OK;
 }
@@ -705,10 +705,10 @@ constexpr int OS_TILE = OS_T * OS_I;
 
 size_t lookback_slots(int64_t n) {
   // single-pass sorts: one slot per (tile, digit); larger ones: the scan of
-  // their histogram table; scans: eight words per tile (two sums)
+  // their histogram table; scans: a two-slot word per (smallest) tile, of two arrays
   const int64_t sort = n <= RS_BIG ? div_up(n, OS_TILE) * RS_BINS
-                                   : 4 * div_up(div_up(n, RS_THREADS * 16) * RS_BINS, SCAN_TILE);
-  return (size_t)(std::max<int64_t>(sort, 8 * div_up(n, SCAN_TILE)) + 1);
+                                   : LB_SCAN_WORDS * div_up(div_up(n, RS_THREADS * 16) * RS_BINS, SCAN_TILE);
+  return (size_t)(std::max<int64_t>(sort, 2 * LB_SCAN_WORDS * div_up(n, SM_THREADS * SM_HEAVY)) + 1);
 }
 
 // Large inputs: three kernels per pass (tile histograms, table scan, scatter).
@@ -906,8 +906,9 @@ static int rbk_launch(const int32_t *keys, const V *vals, int64_t n, long long *
 // looked up once per device.
 constexpr size_t NOALLOC_POS_BYTES = (size_t)DCSR_NOALLOC_MAX_KEYS * sizeof(long long);
 constexpr size_t NOALLOC_PART_BYTES = (size_t)(DCSR_NOALLOC_MAX_KEYS / RBK_PIECE + 1) * sizeof(double);
-constexpr size_t NOALLOC_LB_SLOTS = 4 * ((DCSR_NOALLOC_MAX_KEYS + SCAN_TILE - 1) / SCAN_TILE) + 4;
-constexpr size_t NOALLOC_ARENA_BYTES = NOALLOC_POS_BYTES + 256 + NOALLOC_PART_BYTES + 256;
+constexpr size_t NOALLOC_LB_SLOTS = LB_SCAN_WORDS * ((DCSR_NOALLOC_MAX_KEYS + SCAN_TILE - 1) / SCAN_TILE) + 4;
+// (a multiple of 256: the look-back area behind it holds 16-byte words)
+constexpr size_t NOALLOC_ARENA_BYTES = (NOALLOC_POS_BYTES + 256 + NOALLOC_PART_BYTES + 256 + 255) / 256 * 256;
 constexpr size_t NOALLOC_BYTES = NOALLOC_ARENA_BYTES + LB_HEADER + 8 * NOALLOC_LB_SLOTS;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 

@@ -1,0 +1,83 @@
+"""In-place insertion, relocation and list edges of the update's apply step:
+rows whose changed stretch is 1, 31..33, 255..257 and several times 256
+positions, insertions before the first, between two and after the last entry
+(many at one place), more new columns than lanes, rows in several segments,
+and relocations of short, long and empty rows; bit-exact against the oracle."""
+import numpy as np
+import pytest
+
+from helpers import assert_content_equal, assert_layout_equal, make_pair
+
+pytestmark = pytest.mark.gpu
+
+M = 100_000
+
+
+def build(rng, lens):
+    """Rows with the columns 10, 20, 30, ... so that insertions can be aimed."""
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = np.concatenate([10 * np.arange(1, L + 1) for L in lens if L]).astype(np.int32)
+    return rp, cols, rng.uniform(-1, 1, cols.size)
+
+
+def aimed(rng, lens, kind):
+    r, c = [], []
+    for i, L in enumerate(lens):
+        if kind == "front":
+            k = [1 + j for j in range(1 + i % 9)]
+        elif kind == "back":
+            k = [10 * L + 11 + j for j in range(1 + i % 9)]
+        elif kind == "one_place":
+            k = [10 * (L // 2) + 1 + j for j in range(9)]
+        elif kind == "spread":
+            k = [10 * q + 5 for q in range(0, L + 1, max(1, L // 7))]
+        elif kind == "many":
+            k = [10 * q + 1 + j for q in range(0, L + 1, max(1, L // 20)) for j in range(5)]
+        else:  # existing and new mixed, duplicates
+            k = list(rng.integers(1, 10 * L + 30, 12)) + [10 * (1 + q % max(L, 1)) for q in range(5)] * 2
+        r += [i] * len(k)
+        c += k
+    order = rng.permutation(len(r))
+    return np.asarray(r, np.int32)[order], np.asarray(c, np.int32)[order], rng.uniform(-1, 1, len(r))
+
+
+LENS = [0, 1, 2, 7, 8, 22, 23, 24, 30, 31, 32, 33, 63, 64, 95, 96, 97, 246, 247, 248, 255, 256, 257, 300, 503, 511, 512,
+        513, 1000, 2047, 2048, 2049, 2600, 5000]
+
+
+@pytest.mark.parametrize("kind", ["front", "back", "one_place", "spread", "many", "mixed"])
+@pytest.mark.parametrize("dtype,reloc_min", [(0, 2048), (1, 2048), (0, 0), (1, 20), (1, 1 << 20)])
+def test_aimed_insertions(dcsr, kind, dtype, reloc_min):
+    rng = np.random.default_rng(len(kind) + reloc_min)
+    lens = LENS
+    rp, cols, vals = build(rng, lens)
+    vals = vals.astype(np.float32) if dtype == 0 else vals
+    dev, orc = make_pair(dcsr, len(lens), M, dtype, 0, reloc_min=reloc_min, min_cap=2)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals.astype(np.float64)) == 0
+    for it in range(4):  # later rounds meet rows in several segments
+        r, c, v = aimed(rng, lens, kind if it % 2 == 0 else "mixed")
+        c = np.minimum(c + it, M - 1).astype(np.int32)
+        v = v.astype(np.float32) if dtype == 0 else v
+        assert dev.update(r, c, v) == orc.update_auto(r, c, v.astype(np.float64)) == 0
+        assert_layout_equal(dev, orc, f"round {it}")
+        assert_content_equal(dev, orc, f"round {it}")
+
+
+@pytest.mark.parametrize("T", [1, 1023, 1024, 1025, 2048, 5000])
+def test_batch_sizes_around_the_scan_tiles(dcsr, T):
+    rng = np.random.default_rng(T)
+    n = 300
+    lens = rng.integers(0, 60, n)
+    rp, cols, vals = build(rng, lens)
+    for mode in (0, 1):
+        dev, orc = make_pair(dcsr, n, M, 1, mode)
+        dev.from_csr(rp, cols, vals)
+        assert orc.load_csr(rp, cols, vals) == 0
+        for _ in range(2):
+            r = rng.integers(0, n, T).astype(np.int32)
+            c = rng.integers(0, 700, T).astype(np.int32)
+            v = rng.uniform(-1, 1, T)
+            assert dev.update(r, c, v) == orc.update_auto(r, c, v) == 0
+            assert_layout_equal(dev, orc, f"T={T}")
+            assert_content_equal(dev, orc, f"T={T}")
