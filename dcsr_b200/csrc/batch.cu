@@ -74,6 +74,7 @@ void fill_image(const BatchCore &b, unsigned char *img) {
   }
   for (auto &g : b.groups) {
     RowItem<V> *gi = (RowItem<V> *)(img + g.off);
+    row0 = 0;  // a flat group's own row space (flat_many)
     for (size_t j = 0; j < g.idx.size(); j++) {
       const int i = g.idx[j];
       const dcsr_batch_item &it = b.items[i];
@@ -84,6 +85,8 @@ void fill_image(const BatchCore &b, unsigned char *img) {
       // the largest power of two (<= 32) dividing the row size
       const size_t rb = it.k * sizeof(V), al = (rb & (0 - rb)) >= 32 ? 32 : (rb & (0 - rb));
       r.vec = it.k > 1 && it.k % 2 == 0 && it.ldx == it.k && ((uintptr_t)it.x % al) == 0;
+      r.row0 = row0;
+      row0 += it.matrix->n_rows;
       gi[j] = r;
     }
   }
@@ -148,8 +151,7 @@ int BatchCore::plan(const dcsr_batch_item *its, int n, cudaStream_t s, bool all_
   for (int i = 0; i < n; i++) {
     const dcsr_batch_item &it = its[i];
     if (!it.x || it.matrix->n_rows == 0) continue;
-    // k families 1 (large matrices), 2 (k <= 2; k = 1 of small matrices), 4, 8
-    const int gk = it.k == 1 ? (it.matrix->n_rows <= K1_GROUP_ROWS ? 2 : 1) : it.k <= 2 ? 2 : it.k <= 4 ? 4 : 8;
+    const int gk = it.k == 1 ? 1 : it.k <= 2 ? 2 : it.k <= 4 ? 4 : 8;
     int gi = -1;
     for (size_t q = 0; q < groups.size(); q++)
       if (groups[q].k == gk) gi = (int)q;
@@ -160,19 +162,27 @@ int BatchCore::plan(const dcsr_batch_item *its, int n, cudaStream_t s, bool all_
     }
     groups[gi].idx.push_back(i);
   }
-  // schedules to rebuild: every matrix, or the updated ones and those whose
-  // schedule is stale (after sizing their schedule buffers, which can
-  // invalidate a schedule); the SpMVs of the others may run beside the update
+  // row classes (k >= 2) and flat tables (k = 1) to rebuild for this run's
+  // SpMVs: every matrix's, or the updated ones' and the stale ones (after
+  // sizing their buffers, which can invalidate them); the SpMVs of the others
+  // may run beside the update
   DCSR_TRY(ensure_buffers(s));
   sched.clear();
   R = 0;
   std::vector<char> in_sched(n, 0);
-  for (int i = 0; i < n; i++)
-    if (all_schedules || its[i].nnz > 0 || !its[i].matrix->bins_valid) {
+  R1 = 0;
+  for (int i = 0; i < n; i++) {
+    if (!its[i].x || its[i].matrix->n_rows == 0) continue;
+    const bool flat = its[i].k == 1;
+    if (!all_schedules && its[i].nnz == 0 && (flat ? its[i].matrix->flat_valid : its[i].matrix->bins_valid)) continue;
+    in_sched[i] = 1;
+    if (flat) {
+      R1 += its[i].matrix->n_rows;
+    } else {
       sched.push_back(i);
-      in_sched[i] = 1;
       R += its[i].matrix->n_rows;
     }
+  }
   {
     std::vector<Group> split;
     for (auto &g : groups) {
@@ -193,10 +203,10 @@ int BatchCore::plan(const dcsr_batch_item *its, int n, cudaStream_t s, bool all_
     g.off = off;
     off = align_up((int64_t)(off + g.idx.size() * desc_size(dtype, true)), 256);
     g.pref_off = poff;
-    poff += 3 * (g.idx.size() + 1) + 2;  // unit prefixes + the k = 1 passes' counter words
+    poff += 3 * (g.idx.size() + 1);  // unit prefixes
     int64_t blocks = 0;
     for (int i : g.idx) blocks += div_up(its[i].matrix->n_rows, 32);
-    g.split = split_force > 0 && g.k >= 2 ? split_force : short_split(blocks, g.k);
+    g.split = g.k == 1 ? 0 : split_force > 0 ? split_force : short_split(blocks, g.k);  // 0: flat units
   }
   img_bytes = off;
   if (img_bytes > img_cap) {
@@ -244,8 +254,7 @@ int BatchCore::reserve_items(int n, int dt, cudaStream_t s) {
 
 int BatchCore::ensure_buffers(cudaStream_t s) {
   for (auto &g : groups)
-    for (int i : g.idx) DCSR_TRY(ensure_part(items[i].matrix, g.k, s));
-  for (int i = 0; i < count; i++) DCSR_TRY(ensure_part(items[i].matrix, 1, s));
+    for (int i : g.idx) DCSR_TRY(g.k == 1 ? ensure_flat(items[i].matrix, s) : ensure_part(items[i].matrix, g.k, s));
   return DCSR_OK;
 }
 
@@ -265,12 +274,12 @@ int BatchCore::upload(cudaStream_t s, bool sync, bool force) {
 
 int BatchCore::reserve_scratch(cudaStream_t s) {
   const size_t upd = T > 0 ? update_scratch_bytes(T, dtype == DCSR_F64 ? 8 : 4) : 0;
-  const size_t sch = schedule_scratch_bytes(R);
+  const size_t sch = std::max(schedule_scratch_bytes(R), flat_scratch_bytes(R1));
   DCSR_TRY(ar.reserve(upd > sch ? upd : sch, s));
   // look-back area for the update's sort and scans and the schedule's scans
   // (sized here, outside any stream capture)
   Lookback lb;
-  return ar.lookback(lookback_slots((T > R ? T : R) + 2), s, &lb);
+  return ar.lookback(lookback_slots(std::max(T, std::max(R, R1)) + 2), s, &lb);
 }
 
 int BatchCore::enqueue(cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEvent_t join) {
@@ -319,6 +328,11 @@ int BatchCore::enqueue(cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEv
     DCSR_TRY(ar.reserve(schedule_scratch_bytes(R), s));
     DCSR_TRY(schedule_many(img_dev + off_row, dtype, (int)sched.size(), R, ar, s));
   }
+  for (auto &g : groups)
+    if (g.k == 1 && !g.side) {
+      DCSR_TRY(ar.reserve(flat_scratch_bytes(R1), s));
+      DCSR_TRY(flat_many(img_dev + g.off, dtype, (int)g.idx.size(), R1, ar, s));
+    }
   DCSR_TRY(prefixes(false));
   for (auto &g : groups)
     if (!g.side || !beside)
@@ -341,7 +355,10 @@ int BatchCore::status_async(long long *host, cudaStream_t s) {
 }
 
 void BatchCore::mark_scheduled() {
-  for (auto &it : items) it.matrix->bins_valid = true;
+  for (auto &it : items)
+    if (it.nnz > 0) it.matrix->bins_valid = it.matrix->flat_valid = false;
+  for (auto &g : groups)
+    for (int i : g.idx) (g.k == 1 ? items[i].matrix->flat_valid : items[i].matrix->bins_valid) = true;
 }
 
 void BatchCore::release() {

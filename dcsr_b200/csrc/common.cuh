@@ -236,8 +236,8 @@ struct dcsr_matrix_s {
   int32_t *cols = nullptr;
   void *vals = nullptr;
   long long *stat = nullptr;
-  // Row-pass schedule (handle-local; the reference used a global __constant__
-  // bin table): long rows with their chunk offsets, medium rows.
+  // Row-pass schedule of the k >= 2 SpMV (handle-local; the reference used a
+  // global __constant__ bin table): long rows with their chunk offsets, medium rows.
   int32_t *long_rows = nullptr;  // [n_rows + 1]
   long long *long_off = nullptr; // [n_rows + 2] chunk offsets of long rows
   int32_t *long_cnt = nullptr;   // [n_rows + 1] chunk-finisher counters
@@ -246,14 +246,19 @@ struct dcsr_matrix_s {
   int64_t part_cap = 0;
   int2 *chunk_rl = nullptr;      // (row, long-row index) of every chunk
   int64_t chunk_cap = 0;
-  // medium-length rows, one descriptor each: (row, length, layer-0 start,
-  // layer-0 capacity)
-  int4 *med_desc = nullptr;      // [n_rows + 1]
-  int4 *chunk_desc = nullptr;    // [chunk_cap] per chunk: its row's (row, length, layer-0 start, capacity)
+  int32_t *med_rows = nullptr;   // [n_rows + 1] medium-length rows
   // Row-class thresholds of the row passes (rows of at most short_max
   // entries are streamed by row blocks, rows above long_min are chunked).
   int32_t short_max = 64, long_min = 512;
   bool bins_valid = false;
+  // Flat tables (one value per entry: k = 1 SpMV, row reductions; export):
+  // the rows' CSR offsets, the row of every tile of 256 entries, two partial
+  // sums per tile.  They depend on the row lengths alone.
+  int32_t *flat_off = nullptr;   // [n_rows + 2]
+  int32_t *flat_tile = nullptr;  // [flat_tiles]
+  double *flat_part = nullptr;   // [2 * flat_tiles]
+  int64_t flat_tiles = 0;
+  bool flat_valid = false;
   dcsr::Arena scratch;
   // Pool buffers: buf_cap >= pool_cap entries are allocated.  The buffers a
   // compaction or growth replaced stay as this matrix's spare (within a

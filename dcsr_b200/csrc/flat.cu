@@ -253,7 +253,31 @@ __global__ void __launch_bounds__(FT_THREADS) k_flat_copy(FlatCopy<V> a) {
       }
     }
     const bool marked = r1 - r0 <= FT_ROWS;
-    if (marked) {
+    // a tile inside one row (and its first segment): one distance, no marks
+    // (copies into the pool know their sources at once and gain nothing)
+    bool inner = false;
+    if constexpr (SRC == AT_POOL)
+      inner = r0 == r1 && e0 + cnt - __shfl_sync(FULL, cur.o, 0) <=
+                           __shfl_sync(FULL, cur.sg.y, 0) - __shfl_sync(FULL, cur.sg.x, 0) &&
+              __shfl_sync(FULL, cur.sg.x, 0) >= 0;
+    if (inner) {
+      const int32_t o = __shfl_sync(FULL, cur.o, 0), dd = __shfl_sync(FULL, cur.dd, 0) - o;
+      const SD sd = SRC == AT_POOL ? (SD)(__shfl_sync(FULL, cur.sg.x, 0) - o) : (SD)(__shfl_sync(FULL, cur.so, 0) - o);
+#pragma unroll
+      for (int i = 0; i < FT_WIN; i++) {
+        const int p = 32 * i + lane;
+        dst[i] = 0xffffffffu;
+        if (p < cnt) {
+          if constexpr (SRC != AT_FLAT) {
+            const SD src = (SD)(e0 + p) + sd;
+            c[i] = __ldcs(a.scols + src);
+            v[i] = __ldcs(a.svals + src);
+          }
+          dst[i] = (unsigned)(DST == AT_FLAT ? e0 + p : e0 + p + dd);
+          if constexpr (ROWS) row[i] = r0;
+        }
+      }
+    } else if (marked) {
       if (lane < FT_WIN) mask[lane] = 0;
       __syncwarp();
       auto mark_row = [&](int32_t r, const FlatRows &d) {
@@ -523,10 +547,13 @@ int compact_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, const i
   return DCSR_OK;
 }
 
-int export_rows(dcsr_handle h, int32_t *off, int32_t *tile_row, int32_t *cols, void *vals, int32_t *rows,
-                int64_t limit, Arena &ar, cudaStream_t s) {
-  const OffsetsScan f{h->row_sizes, h->n_rows, off, tile_row, flat_tiles(h->pool_cap)};
-  DCSR_TRY(scan_map(f, h->n_rows > 0 ? h->n_rows : 1, ar, s));
+int flat_offsets(dcsr_handle h, int32_t *off, int32_t *tile_row, int64_t tiles, Arena &ar, cudaStream_t s) {
+  const OffsetsScan f{h->row_sizes, h->n_rows, off, tile_row, tiles};
+  return scan_map(f, h->n_rows > 0 ? h->n_rows : 1, ar, s);
+}
+
+int export_rows(dcsr_handle h, const int32_t *off, const int32_t *tile_row, int32_t *cols, void *vals, int32_t *rows,
+                int64_t limit, cudaStream_t s) {
   if (h->dtype == DCSR_F32) return export_t<float>(h, off, tile_row, cols, (float *)vals, rows, limit, s);
   return export_t<double>(h, off, tile_row, cols, (double *)vals, rows, limit, s);
 }

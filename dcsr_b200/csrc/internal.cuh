@@ -30,11 +30,10 @@ int place_rows_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, cons
 int compact_scan(dcsr_handle h, int32_t *off, int32_t *caps, int32_t *tile_row, Arena &ar, cudaStream_t s);
 int compact_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, const int32_t *tile_row, int32_t *cols,
                  void *vals, int64_t cap, cudaStream_t s);
-// Export: the row pointer (off, n+1 words) and every row's entries in CSR
-// order, optionally with their rows; entries at positions >= limit are not
-// written.  tile_row: flat_tiles(pool_cap) words.
-int export_rows(dcsr_handle h, int32_t *off, int32_t *tile_row, int32_t *cols, void *vals, int32_t *rows,
-                int64_t limit, Arena &ar, cudaStream_t s);
+// Export: every row's entries in CSR order (off, tile_row: flat_offsets),
+// optionally with their rows; entries at positions >= limit are not written.
+int export_rows(dcsr_handle h, const int32_t *off, const int32_t *tile_row, int32_t *cols, void *vals, int32_t *rows,
+                int64_t limit, cudaStream_t s);
 
 // Rows staged elsewhere (row r: lens[r] entries at src_off[r]) become the
 // matrix's content with policy capacities, in a pool allocated at cap_bound
@@ -83,8 +82,7 @@ struct RowItem {
   const int32_t *long_rows;
   const long long *long_off;
   const int2 *chunk_rl;   // per chunk: (row, long-row index)
-  const int4 *chunk_desc; // per chunk: (row, length, layer-0 start, layer-0 capacity)
-  const int4 *med_desc;   // per medium row: the same descriptor
+  const int32_t *med_rows; // medium rows
   int32_t *info;  // [0] long rows, [1] chunks, [2] medium rows
   int32_t *long_cnt;
   double *part;
@@ -93,6 +91,10 @@ struct RowItem {
   int64_t ldx, ldy;
   double alpha, beta;
   long long row0;             // first row of this matrix in the batch's row space
+  // flat pass (k = 1, row reductions): CSR offsets, tile rows, tile partials, tiles the tables hold
+  const int32_t *off, *tile_row;
+  double *fpart;
+  long long tiles;
   int32_t short_max, long_min; // row classes: short <= short_max < medium <= long_min < long
   const int32_t *skip;        // batch: nonzero -> this matrix's pass is skipped (may be null)
   int32_t k, vec;             // runtime-k passes: right-hand sides, x rows loadable as vectors
@@ -103,20 +105,26 @@ struct RowItem {
 int schedule_many(const void *items_dev, int dtype, int count, int64_t R, Arena &ar, cudaStream_t s);
 size_t schedule_scratch_bytes(int64_t R);
 // y = A x for `count` matrices (items: device RowItem<V>[count]) of one k
-// family: kf = 1, 2, 4 or 8, every item's k <= kf (each item's own k / vec
-// are read by the kernel); pref: device scratch of 3*(count+1)+2 long longs
-// (the unit prefixes, then the k = 1 passes' counter words).
+// family: kf = 1 (flat pass), 2, 4 or 8, every item's k <= kf (each item's own
+// k / vec are read by the kernel); pref: device scratch of 3*(count+1) long
+// longs (the unit prefixes).
 // prefixed: the group's unit prefixes were computed already (unit_prefix_many,
 // with the same split); split: warps per 32-row block of short rows (short_split)
 int spmv_many(const void *items_dev, int dtype, int count, int k, long long *pref, cudaStream_t s,
               bool prefixed = false, int split = 1);
 // Warps per 32-row short-row block for an SpMV pass over `blocks` blocks with k RHS.
 int short_split(int64_t blocks, int k);
-// A k = 1 SpMV of a matrix of at most this many rows runs in the runtime-k
-// (k <= 2) pass -- row groups of G lanes, blocks split across warps -- instead
-// of the one-value stream, whose 32-row blocks leave a small matrix to a few
-// dozen warps.  A per-matrix rule, so the per-call and batched paths agree.
-constexpr int32_t K1_GROUP_ROWS = 32768;
+// Flat tables of a handle (row offsets, tile rows, tile partials): sized for
+// its pool; built from its row lengths when they are not valid.
+int ensure_flat(dcsr_handle h, cudaStream_t s);
+int build_flat(dcsr_handle h, cudaStream_t s, Arena *ar = nullptr);
+// Of `count` matrices at once (items: device RowItem<V>[count], row0 = their
+// first rows in a common row space of R rows).  Needs flat_scratch_bytes(R)
+// free in the arena.
+int flat_many(const void *items_dev, int dtype, int count, int64_t R, Arena &ar, cudaStream_t s);
+size_t flat_scratch_bytes(int64_t R);
+// The offsets and tile rows of a matrix (flat.cu): off n_rows+1 words.
+int flat_offsets(dcsr_handle h, int32_t *off, int32_t *tile_row, int64_t tiles, Arena &ar, cudaStream_t s);
 // The unit prefixes of up to MAX_PREFIX_JOBS SpMV groups in one launch.
 constexpr int MAX_PREFIX_JOBS = 8;
 int unit_prefix_many(const void *const *items, const int *counts, long long *const *prefs, const int *splits, int n,
@@ -152,12 +160,13 @@ struct BatchCore {
     size_t pref_off = 0;   // unit-prefix offset in pref
   };
   int count = 0, dtype = 0, mode = 0;
+  int64_t R1 = 0;       // rows of the flat (k = 1) items whose tables the run rebuilds
   int split_force = 0;  // > 0: warps per short-row block of every k >= 2 group (else short_split)
   std::vector<dcsr_batch_item> items;
   int64_t T = 0, R = 0;
   int rb = 1, cb = 1;
   std::vector<Group> groups;
-  std::vector<int> sched;   // items whose schedules the run rebuilds
+  std::vector<int> sched;   // items whose row classes the run rebuilds (k >= 2)
   std::vector<int> upd;     // items with update triples (the update pipeline's items)
   std::vector<int> upd_of;  // per item: its index in upd, or -1
   // image: BatchItem[upd] | RowItem[sched] (row space) | group RowItems

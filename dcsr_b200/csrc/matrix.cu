@@ -209,7 +209,7 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   h->buf_cap = got;
   h->pool_cap = cap;
   DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, tile_row, s));
-  h->bins_valid = false;
+  h->bins_valid = h->flat_valid = false;
   // A load is a one-off: a resident matrix keeps no load-sized scratch (the
   // stream-ordered pool keeps the memory for the next allocation).
   h->scratch.release(s);
@@ -245,7 +245,7 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   long long host[ST_WORDS];
   DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
-  h->bins_valid = false;
+  h->bins_valid = h->flat_valid = false;
   h->scratch.release(s);
   if (host[ST_STATUS] == DCSR_TIMEOUT) {
     DCSR_TRY(clear_status(h, s));
@@ -344,7 +344,8 @@ int compact(dcsr_handle h, cudaStream_t s) {
   h->vals = nv;
   h->buf_cap = got;
   h->pool_cap = cap;
-  // the schedule's row descriptors hold segment starts, which moved
+  // the schedule's row descriptors hold segment starts, which moved (the
+  // flat tables follow the row lengths, which did not change)
   h->bins_valid = false;
   // the scratch (sized by this matrix's earlier updates) stays for the
   // update a repair runs next: re-allocating it there stalled repairs
@@ -417,7 +418,7 @@ int dcsr_create(dcsr_handle *out, int32_t n_rows, int32_t n_cols, int32_t dtype,
       dcsr::dev_alloc((void **)&h->long_rows, sizeof(int32_t) * (n_rows + 1), ls) != cudaSuccess ||
       dcsr::dev_alloc((void **)&h->long_off, sizeof(long long) * (n_rows + 2), ls) != cudaSuccess ||
       dcsr::dev_alloc((void **)&h->long_cnt, sizeof(int32_t) * (n_rows + 1), ls) != cudaSuccess ||
-      dcsr::dev_alloc((void **)&h->med_desc, sizeof(int4) * (n_rows + 1), ls) != cudaSuccess ||
+      dcsr::dev_alloc((void **)&h->med_rows, sizeof(int32_t) * (n_rows + 1), ls) != cudaSuccess ||
       dcsr::dev_alloc((void **)&h->sched_info, sizeof(int32_t) * 32, ls) != cudaSuccess)
     st = DCSR_OOM;
   if (st == DCSR_OK) {
@@ -449,7 +450,7 @@ int dcsr_destroy(dcsr_handle h) {
   h->scratch.release(s0);
   drop_spare(h, s0);
   void *bufs[] = {h->cols, h->vals, h->row_sizes, h->seg, h->stat, h->long_rows, h->long_off,
-                  h->long_cnt, h->med_desc, h->sched_info, h->part, h->chunk_rl, h->chunk_desc};
+                  h->long_cnt, h->med_rows, h->sched_info, h->part, h->chunk_rl, h->flat_off, h->flat_tile, h->flat_part};
   for (void *p : bufs)
     if (p) dcsr::dev_free(p, s0);
   if (h->spare_ev) cudaEventDestroy(h->spare_ev);
@@ -598,6 +599,13 @@ int dcsr_from_hyb(dcsr_handle h, const int32_t *ell_cols, const void *ell_vals, 
 int dcsr_nnz(dcsr_handle h, int64_t *nnz, void *stream) {
   if (!h || !nnz) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
+  if (h->flat_valid) {  // the offsets' last word
+    int32_t t = 0;
+    DCSR_CUDA(cudaMemcpyAsync(&t, h->flat_off + h->n_rows, sizeof(t), cudaMemcpyDeviceToHost, s));
+    DCSR_CUDA(cudaStreamSynchronize(s));
+    *nnz = t;
+    return DCSR_OK;
+  }
   DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX + 1, 0, sizeof(long long), s));
   if (h->n_rows > 0)
     DCSR_LAUNCH(k_sum_lens, std::min(grid_for(h->n_rows, 1024), 2 * sm_count()), 256, 0, s, h->row_sizes, h->n_rows, h->stat + ST_AUX + 1);
@@ -611,13 +619,12 @@ int dcsr_nnz(dcsr_handle h, int64_t *nnz, void *stream) {
 static int export_impl(dcsr_handle h, int32_t *row_ptr, int32_t *rows, int32_t *cols, void *vals, cudaStream_t s,
                        int64_t limit = INT64_MAX, Arena *arp = nullptr) {
   const int32_t n = h->n_rows;
-  Arena &ar = arp ? *arp : h->scratch;
-  ar.status = h->stat + ST_STATUS;
-  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 4) + arena_bytes(flat_tiles(h->pool_cap) + 1, 4) + scan_scratch_bytes(n + 1), s));
-  int32_t *off = row_ptr ? row_ptr : ar.take<int32_t>(n + 2);
-  int32_t *tile_row = ar.take<int32_t>(flat_tiles(h->pool_cap) + 1);
-  if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  return export_rows(h, off, tile_row, cols, vals, rows, limit, ar, s);
+  // the flat tables are the export's offsets too; built here when stale (a
+  // later SpMV or reduction finds them)
+  if (!h->flat_valid) DCSR_TRY(build_flat(h, s, arp));
+  if (row_ptr)
+    DCSR_CUDA(cudaMemcpyAsync(row_ptr, h->flat_off, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, s));
+  return export_rows(h, h->flat_off, h->flat_tile, cols, vals, rows, limit, s);
 }
 
 int dcsr_to_csr(dcsr_handle h, int32_t *row_ptr, int32_t *cols, void *vals, void *stream) {
@@ -796,14 +803,15 @@ int dcsr_restore(dcsr_handle h, const void *host_buf, int64_t buf_bytes, void *s
     p += 4 * (size_t)hd.top;
     DCSR_CUDA(cudaMemcpyAsync(h->vals, p, h->vsize() * (size_t)hd.top, cudaMemcpyHostToDevice, s));
   }
-  h->bins_valid = false;
+  h->bins_valid = h->flat_valid = false;
   DCSR_CUDA(cudaStreamSynchronize(s));  // the host buffer may be released on return
   return DCSR_OK;
 }
 
 int dcsr_bin_rows(dcsr_handle h, void *stream) {
   if (!h) return DCSR_BAD_ARG;
-  return build_schedule(h, (cudaStream_t)stream);
+  DCSR_TRY(build_schedule(h, (cudaStream_t)stream));
+  return build_flat(h, (cudaStream_t)stream);
 }
 
 int dcsr_set_row_classes(dcsr_handle h, int32_t short_max, int32_t long_min) {

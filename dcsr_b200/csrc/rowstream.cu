@@ -1,34 +1,27 @@
-// rowstream.cu -- row-parallel passes over one DCSR matrix or a set of them:
-// SpMV (1..8 RHS), row reductions, DCSR -> CSR/COO export, compaction copy.
+// rowstream.cu -- passes over the rows of one DCSR matrix or a set of them:
+// SpMV (1..8 RHS) and row reductions.
 //
-// Rows are split into three classes by the schedule (rebuilt lazily after
-// any change of row lengths), each with its own launch so each has its own
-// register budget and its units carry bounded work:
-//   short  (<= short_max entries)  a warp takes 32 consecutive rows.  With
-//          one value per entry (SpMV k=1, row reductions, the copy pass) it
-//          streams each segment layer's entries across its lanes, U windows
-//          of 32 entries at a time with every window's loads issued first; a
-//          lane's row is found by a binary search over the lanes' row
-//          offsets and sums use a segmented scan whose segment test is one
-//          compare with the start of the lane's row in the window -- uneven
-//          rows cost nothing extra.
-//          With k >= 2 values per entry (where the scan's k shuffles per
-//          step would dominate) the warp splits into groups of G lanes, G in
-//          {1..16} from the block's mean row length; a group walks one row
-//          with four loads in flight per lane and reduces over its lanes with
-//          log2(G) shuffles.
+// One value per entry (SpMV with one right-hand side, row reductions): the
+// flat pass, a warp per tile of 256 consecutive entries (k_flat_rows).
+//
+// SpMV with k >= 2: rows are split into three classes by the schedule (rebuilt
+// lazily after any change of row lengths), each with its own launch so each
+// has its own register budget and its units carry bounded work:
+//   short  (<= short_max entries)  a warp takes 32 consecutive rows and splits
+//          into groups of G lanes, G in {1..16} from the block's mean row
+//          length; a group walks one row with several loads in flight per
+//          lane and reduces over its lanes with log2(G) shuffles.
 //   medium (<= long_min)          one warp per row, lanes strided, U loads in
 //          flight per lane, one warp reduction per row.
 //   long                          CHUNK-entry chunks, one CTA per chunk,
 //          STEP entries in flight per CTA step (128-bit loads when aligned);
 //          multi-chunk rows combine their partials in chunk order (the CTA
 //          that finishes the last chunk sums them).
-// A row's result depends only on the row (its length picks its class, the
-// block's lengths pick G), never on which launch or batch it runs in.
-// Products accumulate in FP64 per lane (fused multiply-add); the k=1
-// stream's per-window partials use the matrix type (FP32 partials of at
-// most 32 products, then FP64); every rounding step is an explicit
-// round-to-nearest intrinsic.
+// A row's result depends only on the row and its matrix (its length picks its
+// class, the block's lengths pick G, its position its tiles), never on which
+// launch or batch it runs in.  Sums are FP64, products too (k = 1: FP32 products
+// exact for matrices of up to FLAT_EXACT_ROWS rows, rounded to FP32 above);
+// every rounding step is an explicit round-to-nearest intrinsic.
 //
 // Reference: spmv_dcsr_bin* include/spmv.inl:364-622 (seven bin kernels on
 // seven streams, rows read with stale Prow_sizes), CompactIndices
@@ -37,43 +30,26 @@
 #include <cstring>
 #include <type_traits>
 
+#include "flat.cuh"
 #include "internal.cuh"
+#include "lookback.cuh"
 
 namespace dcsr {
 
 constexpr int RS_THREADS_ = 256;
 constexpr int RS_WARPS = RS_THREADS_ / 32;
-// Long-row entries per chunk unit: one warp's unit in the k = 1 pass
-// (k_rows1), one CTA's in the k >= 2 and copy passes.  Small enough that a
-// power-law matrix's hottest rows spread over many warps; multi-chunk rows
-// combine their partials in chunk order.
+// Long-row entries per chunk unit (a CTA's).  Small enough that a power-law
+// matrix's hottest rows spread over many CTAs; multi-chunk rows combine their
+// partials in chunk order.
 #ifndef DCSR_CHUNK
 #define DCSR_CHUNK 2048
 #endif
 constexpr int CHUNK = DCSR_CHUNK;
-// Windows of 32 entries a warp has in flight per step, and blocks per SM the
-// k = 1 pass is compiled for.
-#ifndef DCSR_K1_UN
-#define DCSR_K1_UN 4
-#endif
-// The same for the k = 1 row reductions (sum, max, min, count), which hold
-// no columns: twice the SpMV's (149 against 156 us for the row sums of the
-// R-MAT 2^20 stream matrix; 16 spills).
-#ifndef DCSR_K1_UN_RED
-#define DCSR_K1_UN_RED 8
-#endif
-#ifndef DCSR_K1_MINB
-#define DCSR_K1_MINB 3
-#endif
-#ifndef DCSR_K1B_MINB
-#define DCSR_K1B_MINB 4
-#endif
-// Windows of 32 entries whose loads a short-row block has in flight.
-#ifndef DCSR_K1B_U
-#define DCSR_K1B_U 4
-#endif
 constexpr int STEP = 4096;    // entries a CTA has in flight per step
 enum { P_BLOCKS = 0, P_CHUNKS = 1, P_MED = 2 };
+// The flat pass's units (one value per entry): tiles; blocks of FT_THREADS
+// tiles and rows for k_flat_fix.
+enum { P_TILES = 0, P_TBLOCKS = 1, P_RBLOCKS = 2 };
 
 // ------------------------------------------------------------- sources
 // A row pass runs over one matrix (RowOne, descriptor passed by value) or a
@@ -87,13 +63,6 @@ template <typename V>
 struct RowOne {
   RowItem<V> it;
   int split = 1;
-  // unit counter and finished-warp counter of the k = 1 passes (the handle's
-  // schedule words 8, 9 for the streamed units, 10, 11 for the short-row
-  // blocks: zeroed by the schedule rebuild, reset by the last warp of every
-  // pass)
-  __device__ __forceinline__ unsigned *ctr(int which) const {
-    return reinterpret_cast<unsigned *>(it.info + 8 + 2 * which);
-  }
   __device__ __forceinline__ int n_items() const { return 1; }
   __device__ __forceinline__ const RowItem<V> &item(int) const { return it; }
   __device__ __forceinline__ int find_row(int64_t) const { return 0; }
@@ -108,17 +77,29 @@ struct RowOne {
   }
 };
 
+// One matrix of a flat pass.
+template <typename V>
+struct FlatOne {
+  RowItem<V> it;
+  __device__ __forceinline__ const RowItem<V> &item(int) const { return it; }
+  __device__ __forceinline__ int find_row(int64_t) const { return 0; }
+  __device__ __forceinline__ int64_t units(int part) const {
+    if (part == P_RBLOCKS) return div_up(it.m.n_rows, FT_THREADS);
+    const int64_t tiles = div_up(it.off[it.m.n_rows], FT_TILE);
+    return part == P_TILES ? tiles : div_up(tiles, FT_THREADS);
+  }
+  __device__ __forceinline__ int locate(int, int64_t u, int64_t &lu) const {
+    lu = u;
+    return 0;
+  }
+};
+
 template <typename V>
 struct RowMany {
   const RowItem<V> *its;
   int count;
-  const long long *pref;  // [3][count+1] unit prefixes per class (short blocks counted split times),
-                          // then two words: the unit and finished-warp counters of the
-                          // k = 1 passes (streamed units, short-row blocks)
+  const long long *pref;  // [3][count+1] unit prefixes per class (short blocks counted split times)
   int split = 1;
-  __device__ __forceinline__ unsigned *ctr(int which) const {
-    return reinterpret_cast<unsigned *>(const_cast<long long *>(pref + 3 * (count + 1) + which));
-  }
   __device__ __forceinline__ int n_items() const { return count; }
   __device__ __forceinline__ const RowItem<V> &item(int i) const { return its[i]; }
   __device__ __forceinline__ int find_row(int64_t g) const {  // matrix holding global row g
@@ -177,10 +158,6 @@ __global__ void k_sched_emit(Src src, int64_t R, const long long *lscan, const l
     const int64_t r = g - it.row0;
     const int32_t L = it.m.row_sizes[r];
     if (L > it.short_max) {
-      // unit descriptors of the k = 1 pass: (row, length, pool slot of the
-      // unit's first entry when the unit lies in layer 0 else -1, chunk number)
-      const int2 s0 = *reinterpret_cast<const int2 *>(it.m.seg + 2 * r);  // layer 0
-      const int32_t cap0 = s0.y - s0.x;
       if (L > it.long_min) {
         const long long s = lscan[g] - lscan[it.row0];
         const int32_t li = (int32_t)(s >> 32);
@@ -188,15 +165,9 @@ __global__ void k_sched_emit(Src src, int64_t R, const long long *lscan, const l
         const_cast<int32_t *>(it.long_rows)[li] = (int32_t)r;
         const_cast<long long *>(it.long_off)[li] = c0;
         it.long_cnt[li] = 0;
-        for (long long c = c0; c < c0 + nc; c++) {
-          const int32_t k = (int32_t)(c - c0);
-          const int32_t e = (k + 1) * CHUNK < L ? (k + 1) * CHUNK : L;
-          const_cast<int2 *>(it.chunk_rl)[c] = make_int2((int32_t)r, li);
-          const_cast<int4 *>(it.chunk_desc)[c] = make_int4((int32_t)r, L, e <= cap0 ? s0.x + k * CHUNK : -1, k);
-        }
+        for (long long c = c0; c < c0 + nc; c++) const_cast<int2 *>(it.chunk_rl)[c] = make_int2((int32_t)r, li);
       } else {
-        const_cast<int4 *>(it.med_desc)[mscan[g] - mscan[it.row0]] =
-            make_int4((int32_t)r, L, L <= cap0 ? s0.x : -1, 0);
+        const_cast<int32_t *>(it.med_rows)[mscan[g] - mscan[it.row0]] = (int32_t)r;
       }
     }
   }
@@ -216,7 +187,6 @@ __global__ void k_sched_info(Src src, const long long *lscan, const long long *m
       it.info[0] = n_long;
       it.info[1] = n_chunks;
       it.info[2] = (int32_t)(mscan[b] - mscan[a]);
-      for (int q = 8; q < 12; q++) it.info[q] = 0;  // k = 1 pass counters
       const_cast<long long *>(it.long_off)[n_long] = n_chunks;
     }
   }
@@ -227,11 +197,8 @@ static int64_t max_chunks(dcsr_handle h) { return h->pool_cap / CHUNK + h->pool_
 int ensure_part(dcsr_handle h, int K, cudaStream_t s) {
   if (max_chunks(h) > h->chunk_cap) {
     if (h->chunk_rl) DCSR_CUDA(dcsr::dev_free(h->chunk_rl, s));
-    if (h->chunk_desc) DCSR_CUDA(dcsr::dev_free(h->chunk_desc, s));
     h->chunk_rl = nullptr;
-    h->chunk_desc = nullptr;
     DCSR_CUDA(dcsr::dev_alloc((void **)&h->chunk_rl, sizeof(int2) * max_chunks(h), s));
-    DCSR_CUDA(dcsr::dev_alloc((void **)&h->chunk_desc, sizeof(int4) * max_chunks(h), s));
     h->chunk_cap = max_chunks(h);
     h->bins_valid = false;  // the chunk table is gone
   }
@@ -252,8 +219,7 @@ RowItem<V> row_item(dcsr_handle h, const void *x, void *y, int64_t ldx, int64_t 
   it.long_rows = h->long_rows;
   it.long_off = h->long_off;
   it.chunk_rl = h->chunk_rl;
-  it.med_desc = h->med_desc;
-  it.chunk_desc = h->chunk_desc;
+  it.med_rows = h->med_rows;
   it.info = h->sched_info;
   it.long_cnt = h->long_cnt;
   it.part = h->part;
@@ -264,6 +230,10 @@ RowItem<V> row_item(dcsr_handle h, const void *x, void *y, int64_t ldx, int64_t 
   it.alpha = alpha;
   it.beta = beta;
   it.row0 = 0;
+  it.off = h->flat_off;
+  it.tile_row = h->flat_tile;
+  it.fpart = h->flat_part;
+  it.tiles = h->flat_tiles;
   it.short_max = h->short_max;
   it.long_min = h->long_min;
   it.skip = nullptr;
@@ -319,6 +289,45 @@ int build_schedule(dcsr_handle h, cudaStream_t s, Arena *ar) {
   return build_schedule_t<double>(h, s, a);
 }
 
+// Flat tables: offsets, tile rows and tile partials of a matrix (one scan of
+// its row lengths), sized for its pool.
+int ensure_flat(dcsr_handle h, cudaStream_t s) {
+  const int64_t need = flat_tiles(h->pool_cap) + 1;
+  if (h->flat_off && need <= h->flat_tiles) return DCSR_OK;
+  if (!h->flat_off) DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_off, sizeof(int32_t) * ((size_t)h->n_rows + 2), s));
+  if (h->flat_tile) DCSR_CUDA(dcsr::dev_free(h->flat_tile, s));
+  if (h->flat_part) DCSR_CUDA(dcsr::dev_free(h->flat_part, s));
+  h->flat_tile = nullptr;
+  h->flat_part = nullptr;
+  h->flat_tiles = 0;
+  h->flat_valid = false;
+  const int64_t want = need + need / 4;
+  DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_tile, sizeof(int32_t) * want, s));
+  DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_part, sizeof(double) * 2 * want, s));
+  h->flat_tiles = want;
+  return DCSR_OK;
+}
+
+int build_flat(dcsr_handle h, cudaStream_t s, Arena *ar) {
+  Arena &a = ar ? *ar : h->scratch;
+  a.status = h->stat + ST_STATUS;
+  DCSR_TRY(ensure_flat(h, s));
+  DCSR_TRY(flat_offsets(h, h->flat_off, h->flat_tile, h->flat_tiles, a, s));
+  h->flat_valid = true;
+  return DCSR_OK;
+}
+
+size_t flat_scratch_bytes(int64_t R) { return arena_bytes(R + 2, 4); }
+
+template <typename V>
+static int flat_many_t(const RowItem<V> *its, int count, int64_t R, Arena &ar, cudaStream_t s);
+
+int flat_many(const void *items_dev, int dtype, int count, int64_t R, Arena &ar, cudaStream_t s) {
+  if (count == 0 || R == 0) return DCSR_OK;
+  if (dtype == DCSR_F32) return flat_many_t<float>((const RowItem<float> *)items_dev, count, R, ar, s);
+  return flat_many_t<double>((const RowItem<double> *)items_dev, count, R, ar, s);
+}
+
 // Exclusive prefix over the matrices of each class's unit count (one block
 // of 1024 threads, 1024 matrices per round).
 template <typename V>
@@ -331,7 +340,12 @@ __device__ __forceinline__ void unit_prefix_block(const RowItem<V> *its, int cou
   for (int b = 0; b < count; b += 1024) {
     const int i = b + threadIdx.x;
     long long u[3] = {0, 0, 0}, inc[3];
-    if (i < count) {
+    if (i < count && split == 0) {  // a flat group
+      const int64_t tiles = div_up(its[i].off[its[i].m.n_rows], FT_TILE);
+      u[P_TILES] = tiles;
+      u[P_TBLOCKS] = div_up(tiles, FT_THREADS);
+      u[P_RBLOCKS] = div_up(its[i].m.n_rows, FT_THREADS);
+    } else if (i < count) {
       u[P_BLOCKS] = div_up(div_up(its[i].m.n_rows, 32) * split, RS_WARPS);
       u[P_CHUNKS] = its[i].info[1];
       u[P_MED] = div_up(its[i].info[2], RS_WARPS);
@@ -355,7 +369,6 @@ __device__ __forceinline__ void unit_prefix_block(const RowItem<V> *its, int cou
     __syncthreads();
   }
   if (threadIdx.x < 3) pref[threadIdx.x * (count + 1) + count] = carry[threadIdx.x];
-  if (threadIdx.x < 2) pref[3 * (count + 1) + threadIdx.x] = 0;  // the k = 1 passes' counters
 }
 
 template <typename V>
@@ -393,40 +406,6 @@ __device__ __forceinline__ RowBlock load_block(const Mat<V> &m, int64_t r0, int 
   b.len = b.row >= 0 ? __ldg(m.row_sizes + r) : 0;
   b.stream = b.len > 0 && b.len <= smax;
   return b;
-}
-
-// Entries of the lane's row in segment layer l (coalesced pair loads across
-// the block); cum accumulates the capacity of layers < l.
-template <typename V>
-__device__ __forceinline__ void next_layer(const Mat<V> &m, const RowBlock &b, int l, int64_t &cum, int32_t &len_l,
-                                           int32_t &st_l) {
-  len_l = 0;
-  st_l = 0;
-  if (b.stream && cum < b.len) {
-    const int2 sg = __ldg(reinterpret_cast<const int2 *>(m.seg + (int64_t)l * m.pitch + 2 * (int64_t)b.row));
-    if (sg.x >= 0) {
-      const int64_t cap = sg.y - sg.x;
-      len_l = (int32_t)(b.len - cum < cap ? b.len - cum : cap);
-      st_l = sg.x;
-      cum += cap;
-    } else {
-      cum = b.len;
-    }
-  }
-}
-
-// The lane whose row holds block position p: the last lane whose row starts
-// at or before p (excl, the rows' exclusive offsets, never decreases across
-// the lanes; an empty row shares its offset with the next row, so the last
-// lane found is the non-empty one), by a binary search over the lanes.
-__device__ __forceinline__ int owner_lane(int32_t excl, int32_t p) {
-  int lo = 0;
-#pragma unroll
-  for (int st = 16; st > 0; st >>= 1) {
-    const int c = lo + st;  // <= 31
-    if (__shfl_sync(FULL, excl, c) <= p) lo = c;
-  }
-  return lo;
 }
 
 // Lanes per row for a block of 32 short rows: the largest power of two
@@ -586,107 +565,6 @@ __device__ __forceinline__ void write_y(V *y, int64_t ldy, int32_t row, const do
   }
 }
 
-// ------------------------------------------------- k = 1 short-row block
-// One warp, one block of 32 consecutive rows: one value per entry (SpMV
-// k = 1, row reductions), the block's entries streamed across the lanes in
-// windows of 32, U windows' loads in flight (windows past the block's end
-// skipped); a lane's row comes from a binary search over the lanes' row
-// offsets, sums use a segmented warp scan.
-// d0: the lane's row, its length and its layer-0 segment (start, capacity),
-// loaded ahead by the caller (row -1 past the matrix's end).
-template <typename V, int OP, bool XU>
-__device__ __forceinline__ void short_block_k1(const RowItem<V> &it, int4 d0, int lane) {
-  using P = typename std::conditional<sizeof(V) == 4, float, double>::type;  // window partials
-  constexpr int U = DCSR_K1B_U;
-  const Mat<V> &m = it.m;
-  const V *__restrict__ x = it.x;
-  RowBlock rb;
-  rb.row = d0.x;
-  rb.len = d0.y;
-  rb.stream = rb.len > 0 && rb.len <= it.short_max;
-  double acc = op_init<double, OP>();
-  int64_t cum = 0;  // capacity of this lane's row in the layers before l
-  for (int l = 0; l < m.max_segs; l++) {
-    int32_t len_l = 0, st_l = 0;
-    if (l == 0) {
-      if (rb.stream) {  // the layer-0 segment came with the descriptor
-        len_l = rb.len < d0.w ? rb.len : d0.w;
-        st_l = d0.z;
-        cum = d0.w;
-      }
-    } else {
-      next_layer(m, rb, l, cum, len_l, st_l);
-    }
-    if (!__any_sync(FULL, len_l > 0)) break;
-    const int32_t incl = warp_incl_scan(len_l);  // block-local (<= 32 * short_max)
-    const int32_t excl = incl - len_l;
-    const int32_t E = __shfl_sync(FULL, incl, 31);
-    for (int32_t base = 0; base < E; base += 32 * U) {
-      int32_t q[U];
-      int32_t rs[U];  // the window lane where the lane's row starts (0: it runs in from before)
-      bool ok[U];
-      // windows past the block's end (warp-uniform) are skipped whole
-#pragma unroll
-      for (int i = 0; i < U; i++) {
-        const int32_t w0 = base + 32 * i, p = w0 + lane;
-        q[i] = rs[i] = 0;
-        ok[i] = false;
-        if (w0 >= E) continue;
-        const int j = owner_lane(excl, p);
-        const int32_t ej = __shfl_sync(FULL, excl, j);
-        const int32_t sj = __shfl_sync(FULL, st_l, j);
-        ok[i] = p < E;
-        rs[i] = ej > w0 ? ej - w0 : 0;
-        q[i] = sj + (ok[i] ? p - ej : 0);
-      }
-      V a[U];
-      int32_t col[U];
-#pragma unroll
-      for (int i = 0; i < U; i++) {
-        a[i] = V(0);
-        col[i] = 0;
-        if (base + 32 * i >= E) continue;
-        a[i] = __ldcs(m.vals + q[i]);
-        col[i] = OP == OP_SPMV ? __ldcs(m.cols + q[i]) : 0;
-      }
-      // every window's x gathers issued before the first scan (lanes past
-      // the block's end loaded a valid entry: their columns are valid)
-      V xv[U];
-#pragma unroll
-      for (int i = 0; i < U; i++)
-        xv[i] = OP != OP_SPMV || base + 32 * i >= E ? V(0)
-                : XU                                ? __ldg(x + col[i])
-                                                    : __ldg(x + (int64_t)col[i] * it.ldx);
-#pragma unroll
-      for (int i = 0; i < U; i++) {
-        if (base + 32 * i >= E) continue;
-        P c = op_init<P, OP>();
-        if (ok[i]) {
-          if constexpr (OP == OP_SPMV) c = mul_rn((P)a[i], (P)xv[i]);
-          else c = OP == OP_COUNT ? (P)1 : (P)a[i];
-        }
-        // segmented inclusive scan: lanes p-d and p share a row when p-d is
-        // at or past the start of p's row in this window
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const P co = __shfl_up_sync(FULL, c, d);
-          if (lane - d >= rs[i]) c = op_comb<P, OP>(c, co);
-        }
-        // lane j collects the tail of its row's run in this window
-        const int32_t w0 = base + 32 * i;
-        const bool hit = len_l > 0 && excl < w0 + 32 && incl > w0;
-        const int tail = (incl < w0 + 32 ? incl : w0 + 32) - 1 - w0;
-        const P got = __shfl_sync(FULL, c, hit ? tail : 0);
-        if (hit) acc = op_comb<double, OP>(acc, (double)got);
-      }
-    }
-  }
-  if (rb.row >= 0 && rb.len <= it.short_max) {
-    const double accs[1] = {acc};
-    write_y<V, 1, OP>(it.y, it.ldy, rb.row, accs, it.alpha, it.beta, rb.len, 1);
-  }
-}
-
 // --------------------------------------------------------- reduction pass
 
 // Blocks per SM the row pass is compiled for: the runtime-k families hold up
@@ -812,7 +690,7 @@ __global__ void __launch_bounds__(RS_THREADS_, RowsMinBlocks<K>::N) k_rows_reduc
       // ---- one medium row per warp, UN loads in flight per lane
       const int64_t mi = lu * RS_WARPS + w;
       if (mi >= it.info[2]) continue;
-      const int32_t row = it.med_desc[mi].x;
+      const int32_t row = it.med_rows[mi];
       const int64_t L = m.row_sizes[row];
       const Chain ch = load_chain(m, row);
       double acc[KA];
@@ -851,20 +729,12 @@ __global__ void __launch_bounds__(RS_THREADS_, RowsMinBlocks<K>::N) k_rows_reduc
       if (lane == 0) write_y<V, K, OP>(it.y, it.ldy, row, acc, it.alpha, it.beta, (int32_t)L, kr);
     } else {
       // ---- short rows: a warp takes 32 consecutive rows
-      const int S = K == 1 ? 1 : src.split;  // warps per 32-row block (k >= 2 pass only)
+      const int S = src.split;  // warps per 32-row block
       const int64_t wu = lu * RS_WARPS + w;
       const int64_t blk = wu / S;
       const int sub = (int)(wu - blk * S);
       if (blk * 32 >= m.n_rows) continue;
-      if constexpr (K == 1) {
-        const int64_t r = blk * 32 + lane;
-        int4 d0 = make_int4(-1, 0, 0, 0);
-        if (r < m.n_rows) {
-          const int2 s0 = __ldg(reinterpret_cast<const int2 *>(m.seg + 2 * r));
-          d0 = make_int4((int32_t)r, __ldg(m.row_sizes + r), s0.x, s0.y - s0.x);
-        }
-        short_block_k1<V, OP, false>(it, d0, lane);
-      } else {
+      {
         // K values per entry: G lanes per row
         const RowBlock rb = load_block(m, blk * 32, lane, it.short_max);
         const Chain own = load_chain_used(m, rb.row >= 0 ? rb.row : 0, rb.stream ? rb.len : 0);
@@ -907,400 +777,498 @@ __global__ void __launch_bounds__(RS_THREADS_, RowsMinBlocks<K>::N) k_rows_reduc
   }
 }
 
-// ---------------------------------------------------- k = 1 single pass
-// SpMV with one right-hand side and the row reductions: every class in one
-// launch of warp units, taken from a device counter (longest first: long-row
-// chunks, then medium rows, then 32-row short blocks), so no class waits for
-// another's tail and a warp's next unit number is fetched while it works on
-// the current one.  A chunk or medium row is streamed lane-consecutively
-// (UN windows of 32 entries in flight per warp), the products of one window
-// step summed in the matrix type in a fixed order and the step sums
-// accumulated in FP64; a row of several chunks combines their partials in
-// chunk order (the warp that finishes its last chunk does it).  The pass is
-// bound by the x gathers (random 4-byte reads of x, one L1 line each).
+// --------------------------------------------- one value per entry: flat pass
+// SpMV with one right-hand side and the row reductions: a warp per tile of 256
+// consecutive entries (flat.cuh), whatever the rows' lengths.  The entries are
+// loaded striped (coalesced along each row), x gathered, the products put in
+// tile order through shared memory so that each lane holds eight consecutive
+// entries; a lane sums its pieces of rows left to right in FP64, a segmented
+// scan over the lanes carries the open piece on, and every row that lies in
+// the tile is written.  A row over several tiles leaves its sums in part[2t]
+// (the part of a row that began in an earlier tile) and part[2t+1] (the part
+// of one that goes on in the next); k_flat_fix adds them in tile order and
+// writes the empty rows.  A row's result depends on the row and on its
+// position among the matrix's entries, never on the launch or batch it runs in.
+//
+// Bound by the x gathers (random reads of x, a sector each) and the per-entry
+// instructions; the row classes it replaces (32-row blocks with a segmented
+// scan per window of 32 entries, streamed long and medium rows taken from a
+// counter) left it to latency: the R-MAT 2^20 stream matrix (17.8M entries,
+// FP32) took 118 + 63 us.
 
-// Entries [c0, c1) of a row (chain ch) streamed across the warp; returns the
-// lane's partial.
-
-
-// Entries [c0, c1) of a row whose range lies in one segment starting at pool
-// slot st: two sets of UN windows, the loads of the next set in flight while
-// the current set's x values are gathered and summed.  Returns the lane's
-// partial.
-template <typename V, int OP>
-__device__ __forceinline__ double stream_seg(const RowItem<V> &it, int64_t st, int64_t c0, int64_t c1, int lane) {
-  using P = typename std::conditional<sizeof(V) == 4, float, double>::type;
-  constexpr int UN = sizeof(V) == 8 && DCSR_K1_UN > 1 ? DCSR_K1_UN / 2 : DCSR_K1_UN;  // FP64: half the windows
-  const V *__restrict__ vals = it.m.vals + st;
-  const int32_t *__restrict__ cols = it.m.cols + st;
-  const V *__restrict__ x = it.x;
-  V a[UN], an[UN];
-  int32_t col[UN], coln[UN];
-#pragma unroll
-  for (int i = 0; i < UN; i++) {
-    const int64_t p = c0 + 32 * i + lane, q = p < c1 ? p : c0;
-    a[i] = __ldcs(vals + q);
-    col[i] = OP == OP_SPMV ? __ldcs(cols + q) : 0;
-  }
-  double acc = op_init<double, OP>();
-  for (int64_t b0 = c0; b0 < c1; b0 += 32 * UN) {
-    const int64_t nb = b0 + 32 * UN;
-    if (nb < c1) {
-#pragma unroll
-      for (int i = 0; i < UN; i++) {
-        const int64_t p = nb + 32 * i + lane, q = p < c1 ? p : c0;
-        an[i] = __ldcs(vals + q);
-        coln[i] = OP == OP_SPMV ? __ldcs(cols + q) : 0;
-      }
-    }
-    P w = op_init<P, OP>();
-#pragma unroll
-    for (int i = 0; i < UN; i++) {
-      if (b0 + 32 * i + lane < c1) {
-        P t;
-        if constexpr (OP == OP_SPMV) t = mul_rn((P)a[i], (P)__ldg(x + (int64_t)col[i] * it.ldx));
-        else t = OP == OP_COUNT ? (P)1 : (P)a[i];
-        w = op_comb<P, OP>(w, t);
-      }
-    }
-    acc = op_comb<double, OP>(acc, (double)w);
-#pragma unroll
-    for (int i = 0; i < UN; i++) {
-      a[i] = an[i];
-      col[i] = coln[i];
-    }
-  }
-  return acc;
-}
-
-// The same over a range that crosses segments (a chained row): UN windows
-// per step, each entry's slot found through the chain.  Same summation
-// order as the single-segment stream.  Not inlined (chained units are rare;
-// their registers stay out of the streaming loop); takes plain pointers.
-template <typename V, int OP>
-__device__ __forceinline__ double stream_chain(const V *vals, const int32_t *cols, const V *x, int64_t ldx, Chain ch,
-                                            int64_t c0, int64_t c1, int lane) {
-  using P = typename std::conditional<sizeof(V) == 4, float, double>::type;
-  constexpr int UN = sizeof(V) == 8 && DCSR_K1_UN > 1 ? DCSR_K1_UN / 2 : DCSR_K1_UN;
-  const int64_t first = ch.phys(c0);
-  double acc = op_init<double, OP>();
-  for (int64_t b0 = c0; b0 < c1; b0 += 32 * UN) {
-    V a[UN];
-    int32_t col[UN];
-#pragma unroll
-    for (int i = 0; i < UN; i++) {
-      const int64_t p = b0 + 32 * i + lane;
-      const int64_t q = p < c1 ? ch.phys(p) : first;
-      a[i] = __ldcs(vals + q);
-      col[i] = OP == OP_SPMV ? __ldcs(cols + q) : 0;
-    }
-    P w = op_init<P, OP>();
-#pragma unroll
-    for (int i = 0; i < UN; i++) {
-      if (b0 + 32 * i + lane < c1) {
-        P t;
-        if constexpr (OP == OP_SPMV) t = mul_rn((P)a[i], (P)__ldg(x + (int64_t)col[i] * ldx));
-        else t = OP == OP_COUNT ? (P)1 : (P)a[i];
-        w = op_comb<P, OP>(w, t);
-      }
-    }
-    acc = op_comb<double, OP>(acc, (double)w);
-  }
-  return acc;
-}
-
-template <int OP>
-__device__ __forceinline__ double warp_comb(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = op_comb<double, OP>(v, __shfl_xor_sync(FULL, v, o));
-  return v;
-}
-
-// A unit of the k = 1 pass, decoded, with its descriptor loaded.  A long-row
-// chunk or a medium row is a "streamed" unit: every lane holds (row, row
-// length, pool slot of the unit's first entry or -1 when the unit crosses a
-// segment boundary, chunk number within the row).  A block of short rows
-// holds, in each lane, that lane's row: (row or -1, length, layer-0 start,
-// layer-0 capacity).
-enum { U1_CHUNK = 0, U1_MED = 1, U1_BLOCK = 2, U1_NONE = 3 };
-struct Unit1 {
-  int32_t u;   // unit number (>= total: past the end)
-  int32_t lu;  // chunk index within the matrix's chunk table (chunks)
-  int kind;
-  int item;    // matrix of the unit
-  int4 d;
+// A tile of a flat pass: its matrix, its entries, and the row data of its
+// first 32 rows, one per lane (loaded ahead).
+struct FlatTile {
+  int32_t item, lt;  // matrix; tile within it
+  int32_t r0, r1;    // rows that hold its first entry and the next tile's
+  int32_t cnt;       // entries (0: past the end, or a skipped matrix)
+  int32_t nnz;       // of the matrix
+  int32_t o, o1;     // the lane's row: offsets
+  int2 sg;           // and first segment
 };
 
 template <typename V, typename Src>
-__device__ __forceinline__ Unit1 unit1_load(const Src &src, int64_t u, int64_t NC, int64_t NM, int64_t total,
-                                            int lane) {
-  Unit1 x;
-  x.u = (int32_t)(u < total ? u : total);
-  x.kind = U1_NONE;
+__device__ __forceinline__ void flat_tile_head(const Src &src, int64_t t, int64_t total, FlatTile &x) {
   x.item = 0;
-  x.lu = 0;
-  x.d = make_int4(-1, 0, -1, 0);
-  if (u >= total) return x;
-  int64_t lu;
-  if (u < NC) {
-    x.item = src.locate(P_CHUNKS, u, lu);
-    const RowItem<V> &it = src.item(x.item);
-    if (it.skip && *it.skip) return x;
-    x.kind = U1_CHUNK;
-    x.lu = (int32_t)lu;
-    x.d = it.chunk_desc[lu];
-  } else if (u < NC + NM) {
-    x.item = src.locate(P_MED, (u - NC) / RS_WARPS, lu);
-    const RowItem<V> &it = src.item(x.item);
-    const int64_t mi = lu * RS_WARPS + (u - NC) % RS_WARPS;
-    if ((it.skip && *it.skip) || mi >= it.info[2]) return x;
-    x.kind = U1_MED;
-    x.d = it.med_desc[mi];
-  } else {
-    const int64_t bu = u - NC - NM;
-    x.item = src.locate(P_BLOCKS, bu / RS_WARPS, lu);
-    const RowItem<V> &it = src.item(x.item);
-    const int64_t blk = lu * RS_WARPS + bu % RS_WARPS;
-    if ((it.skip && *it.skip) || blk * 32 >= it.m.n_rows) return x;
-    x.kind = U1_BLOCK;
-    const int64_t r = blk * 32 + lane;
-    if (r < it.m.n_rows) {
-      const int2 s0 = __ldg(reinterpret_cast<const int2 *>(it.m.seg + 2 * r));
-      x.d = make_int4((int32_t)r, __ldg(it.m.row_sizes + r), s0.x, s0.y - s0.x);
-    }
-  }
-  return x;
+  x.lt = 0;
+  x.cnt = 0;
+  x.r0 = 0;
+  x.r1 = -1;
+  x.nnz = 0;
+  if (t >= total) return;
+  int64_t lt;
+  x.item = src.locate(P_TILES, t, lt);
+  const RowItem<V> &it = src.item(x.item);
+  if (it.skip && *it.skip) return;
+  x.lt = (int32_t)lt;
+  x.nnz = __ldg(it.off + it.m.n_rows);
+  const int64_t e0 = lt * FT_TILE, left = x.nnz - e0;
+  if (left <= 0) return;
+  x.cnt = left < FT_TILE ? (int32_t)left : FT_TILE;
+  x.r0 = max(__ldg(it.tile_row + lt), 0);
+  x.r1 = left > FT_TILE ? min(__ldg(it.tile_row + lt + 1), it.m.n_rows - 1) : it.m.n_rows - 1;
 }
 
-__device__ __forceinline__ bool streamed(const Unit1 &x) { return x.kind == U1_CHUNK || x.kind == U1_MED; }
-// The entry range [c0, c1) of a streamed unit within its row.
-__device__ __forceinline__ void unit_range(const Unit1 &x, int64_t &c0, int64_t &c1) {
-  if (x.kind == U1_CHUNK) {
-    c0 = (int64_t)x.d.w * CHUNK;
-    c1 = c0 + CHUNK < x.d.y ? c0 + CHUNK : x.d.y;
-  } else {
-    c0 = 0;
-    c1 = x.d.y;
+template <typename V, typename Src>
+__device__ __forceinline__ void flat_tile_rows(const Src &src, FlatTile &x) {
+  const int32_t r = x.r0 + lane_id();
+  x.o = x.o1 = 0;
+  x.sg = make_int2(-1, -1);
+  if (r <= x.r1) {
+    const RowItem<V> &it = src.item(x.item);
+    x.o = __ldg(it.off + r);
+    x.o1 = __ldg(it.off + r + 1);
+    x.sg = __ldg(reinterpret_cast<const int2 *>(it.m.seg + 2 * (int64_t)r));
   }
 }
 
-// Loads of one step (UN windows of 32 entries) of a streamed unit lying in
-// one segment (first pool slot d.z), entries [o, o + 32*UN) of the unit.
-template <typename V, int UN, int OP>
-__device__ __forceinline__ void load_step(const Mat<V> &m, int32_t base, int32_t n, int32_t o, int lane, V (&a)[UN],
-                                          int32_t (&col)[UN]) {
-#pragma unroll
-  for (int i = 0; i < UN; i++) {
-    const int32_t p = o + 32 * i + lane, q = base + (p < n ? p : 0);  // pool slots are below 2^31
-    a[i] = __ldcs(m.vals + q);
-    col[i] = OP == OP_SPMV ? __ldcs(m.cols + q) : 0;
-  }
-}
-
-// The end of a streamed unit: its total (t, in every lane) is the row's
-// result, or one chunk's partial; the warp that adds the row's last chunk
-// combines the partials in chunk order.
 template <typename V, int OP>
-__device__ __forceinline__ void finish_unit(const RowItem<V> &it, const Unit1 &x, double t, int lane) {
-  const int32_t row = x.d.x, L = x.d.y;
-  const int64_t nch = x.kind == U1_CHUNK ? (L + CHUNK - 1) / CHUNK : 1;
-  if (nch == 1) {
-    if (lane == 0) {
-      const double o[1] = {t};
-      write_y<V, 1, OP>(it.y, it.ldy, row, o, it.alpha, it.beta, L, 1);
-    }
-    return;
-  }
-  const int64_t p0 = x.lu - x.d.w;  // the row's first chunk (chunks of a row are consecutive)
-  int last = 0;
-  if (lane == 0) {
-    const int32_t li = it.chunk_rl[x.lu].y;
-    it.part[x.lu] = t;
-    __threadfence();
-    last = atomicAdd(&it.long_cnt[li], 1) == nch - 1;
-    if (last) it.long_cnt[li] = 0;
-  }
-  if (__shfl_sync(FULL, last, 0)) {
-    // every chunk's partial is published: lanes take partials lane,
-    // lane+32, ... in order, then a fixed xor tree
-    __threadfence();
-    double v = op_init<double, OP>();
-    for (int64_t q = lane; q < nch; q += 32) v = op_comb<double, OP>(v, __ldcg(it.part + p0 + q));
-    v = warp_comb<OP>(v);
-    if (lane == 0) {
-      const double o[1] = {v};
-      write_y<V, 1, OP>(it.y, it.ldy, row, o, it.alpha, it.beta, L, 1);
-    }
-  }
+__device__ __forceinline__ void write_row(const RowItem<V> &it, int32_t row, double v) {
+  const double o[1] = {v};
+  write_y<V, 1, OP>(it.y, it.ldy, row, o, it.alpha, it.beta, 1, 1);  // (length 1: not empty)
 }
 
-// The streamed units (long-row chunks, then medium rows) of a k = 1 pass.
-template <typename V, int OP, typename Src, bool XU>
-__global__ void __launch_bounds__(RS_THREADS_, DCSR_K1_MINB) k_rows1(Src src) {
-  using P = typename std::conditional<sizeof(V) == 4, float, double>::type;
-  constexpr int UNO = OP == OP_SPMV ? DCSR_K1_UN : DCSR_K1_UN_RED;
-  constexpr int UN = sizeof(V) == 8 && UNO > 1 ? UNO / 2 : UNO;
-  constexpr int W = 32 * UN;  // entries of one step
-  const int lane = threadIdx.x & 31;
-  const int64_t NC = src.units(P_CHUNKS), NM = src.units(P_MED) * RS_WARPS;
-  const int64_t total = NC + NM;
-  unsigned *ctr = src.ctr(0);
-  // A unit number is taken by lane 0 with an atomic and broadcast only when
-  // it is needed, one unit later: the atomic's round trip overlaps a unit.
-  unsigned pend = 0;
-  auto fetch_issue = [&]() {
-    if (lane == 0) pend = atomicAdd(ctr, 1u);
-  };
-  auto fetch_take = [&]() -> int64_t { return (int64_t)__shfl_sync(FULL, pend, 0); };
-  // Units in flight per warp: cur (streamed step by step), nx (its
-  // descriptor loaded or in flight) and the number of the one after.  Two
-  // register buffers take turns: the loads of the next step go into one
-  // while the current step's x values are gathered from the other (no copy
-  // between them, so nothing waits for a load before its data is used), and
-  // the next step may be the next unit's first -- the stream does not stop at
-  // unit ends.
-  fetch_issue();
-  Unit1 cur = unit1_load<V>(src, fetch_take(), NC, NM, total, lane);
-  fetch_issue();
-  Unit1 nx = unit1_load<V>(src, fetch_take(), NC, NM, total, lane);
-  fetch_issue();
-  V a0[UN], a1[UN];
-  int32_t k0[UN], k1[UN];
-  int64_t c0 = 0, c1 = 0;  // cur's range
-  int32_t o = 0;           // the current step's offset in it
-  if (streamed(cur)) {
-    unit_range(cur, c0, c1);
-    if (cur.d.z >= 0) load_step<V, UN, OP>(src.item(cur.item).m, cur.d.z, (int32_t)(c1 - c0), 0, lane, a0, k0);
-  }
-  double acc = op_init<double, OP>();
-  // One step: consume (ca, cc), loading the following step into (na, nc).
-  auto step = [&](V(&ca)[UN], int32_t(&cc)[UN], V(&na)[UN], int32_t(&nc)[UN]) {
-    bool advance = true;
-    if (streamed(cur)) {
-      const RowItem<V> &it = src.item(cur.item);
-      if (cur.d.z < 0) {
-        // a unit across segment boundaries (a chained row): streamed on its own
-        const double t = warp_comb<OP>(
-            stream_chain<V, OP>(it.m.vals, it.m.cols, it.x, it.ldx, load_chain(it.m, cur.d.x), c0, c1, lane));
-        finish_unit<V, OP>(it, cur, t, lane);
-        if (streamed(nx) && nx.d.z >= 0) {  // the next unit's first step, into the buffer consumed next
-          int64_t d0, d1;
-          unit_range(nx, d0, d1);
-          load_step<V, UN, OP>(src.item(nx.item).m, nx.d.z, (int32_t)(d1 - d0), 0, lane, na, nc);
-        }
-      } else {
-        const int32_t n = (int32_t)(c1 - c0);
-        const bool last = o + W >= n;
-        if (!last) {
-          load_step<V, UN, OP>(it.m, cur.d.z, n, o + W, lane, na, nc);
-        } else if (streamed(nx) && nx.d.z >= 0) {
-          int64_t d0, d1;
-          unit_range(nx, d0, d1);
-          load_step<V, UN, OP>(src.item(nx.item).m, nx.d.z, (int32_t)(d1 - d0), 0, lane, na, nc);
-        }
-        // every x gather of the step issued before the first is used (lanes
-        // past the unit's end loaded its first entry: their columns are valid)
-        V xv[UN];
+// FP32 matrices of at most this many rows sum exact products; larger ones
+// products rounded to FP32 (summed in FP64 either way), where the gathers and
+// instructions of many tiles count: 99 against 112 us on the R-MAT matrix, its
+// error against 64 bits 3.7e-8 (2.6e-8 with exact products, most of it the
+// result's own rounding).
+constexpr int32_t FLAT_EXACT_ROWS = 32768;
+
+#ifndef DCSR_FLAT_MINB
+#define DCSR_FLAT_MINB 4
+#endif
+// EXACT (FP32 SpMV): products are kept with their rounding errors.
+template <typename V, int OP, typename Src, bool XU, bool EXACT>
+__global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src src) {
+  __shared__ __align__(16) unsigned s_run[FT_WARPS][FT_WIN], s_row[FT_WARPS][FT_WIN];
+  // Products in tile order; before them, in an SpMV, the distances from an
+  // entry's number to its slot, by run; and the rows by their first entries.
+  // Shared memory is kept small: what it takes, the x gathers' L1 loses (33 KB
+  // a block ran 118 us on the R-MAT matrix where 25 KB ran 102, 17 KB 99).  EXACT
+  // adds each product's rounding error (one fused multiply-add), 112 us;
+  // FP64 products (two more conversions per entry) took 132 us.
+  constexpr bool OWN = OP != OP_SPMV, ERR = EXACT && OP == OP_SPMV && sizeof(V) == 4;
+  __shared__ __align__(16) V s_prod[FT_WARPS][FT_TILE];
+  __shared__ __align__(16) float s_err[ERR ? FT_WARPS : 1][ERR ? FT_TILE : 4];
+  __shared__ int32_t s_sdel[OWN ? FT_WARPS : 1][OWN ? FT_TILE : 1];  // (the reductions': room of their own)
+  __shared__ int32_t s_hrow[FT_WARPS][FT_TILE];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned *runs = s_run[w], *starts = s_row[w];
+  int32_t *hrow = s_hrow[w], *sdel = OWN ? s_sdel[OWN ? w : 0] : reinterpret_cast<int32_t *>(s_prod[w]);
+  V *prod = s_prod[w];
+  float *err = s_err[ERR ? w : 0];
+  const int64_t total = src.units(P_TILES), nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
+  FlatTile cur, nx;
+  flat_tile_head<V>(src, t, total, cur);
+  flat_tile_rows<V>(src, cur);
+  flat_tile_head<V>(src, t + nw, total, nx);
+  for (; t < total; t += nw) {
+    const RowItem<V> &it = src.item(cur.item);
+    const int32_t e0 = cur.lt * FT_TILE, cnt = cur.cnt, r0 = cur.r0, r1 = cur.r1;
+    // a tile inside one row's first segment: no marks, one sum (half of the
+    // tiles of a power-law matrix)
+    const int32_t o0 = __shfl_sync(FULL, cur.o, 0), o01 = __shfl_sync(FULL, cur.o1, 0);
+    const int32_t sx = __shfl_sync(FULL, cur.sg.x, 0), sy = __shfl_sync(FULL, cur.sg.y, 0);
+    const bool inner = cnt > 0 && r0 == r1 && sx >= 0 && e0 + cnt - o0 <= sy - sx;
+    const bool cont = o0 < e0;  // its first row began in an earlier tile
+    const bool exact = ERR && it.m.n_rows <= FLAT_EXACT_ROWS;  // (a set's larger matrices: as on their own)
+    double isum = op_init<double, OP>();
+    float ierr = 0.0f;
+    if (inner) {
+      const int32_t base = sx + (e0 - o0) + lane;
+      V a[FT_WIN];
+      int32_t col[FT_WIN];
 #pragma unroll
-        for (int i = 0; i < UN; i++)
-          xv[i] = OP != OP_SPMV ? V(0) : XU ? __ldg(it.x + cc[i]) : __ldg(it.x + (int64_t)cc[i] * it.ldx);
-        P w = op_init<P, OP>();
-#pragma unroll
-        for (int i = 0; i < UN; i++) {
-          if (o + 32 * i + lane < n) {
-            P t;
-            if constexpr (OP == OP_SPMV) t = mul_rn((P)ca[i], (P)xv[i]);
-            else t = OP == OP_COUNT ? (P)1 : (P)ca[i];
-            w = op_comb<P, OP>(w, t);
-          }
-        }
-        acc = op_comb<double, OP>(acc, (double)w);
-        if (last) {
-          finish_unit<V, OP>(it, cur, warp_comb<OP>(acc), lane);
-          acc = op_init<double, OP>();
-        } else {
-          o += W;
-          advance = false;
+      for (int i = 0; i < FT_WIN; i++) {
+        a[i] = V(0);
+        col[i] = 0;
+        if (32 * i + lane < cnt) {
+          a[i] = __ldcs(it.m.vals + base + 32 * i);
+          col[i] = OP == OP_SPMV ? __ldcs(it.m.cols + base + 32 * i) : 0;
         }
       }
-    } else if (streamed(nx) && nx.d.z >= 0) {  // a skipped unit: the next one's first step
-      int64_t d0, d1;
-      unit_range(nx, d0, d1);
-      load_step<V, UN, OP>(src.item(nx.item).m, nx.d.z, (int32_t)(d1 - d0), 0, lane, na, nc);
+      if constexpr (OP == OP_SPMV) {
+        const V *__restrict__ x = it.x;
+        V xv[FT_WIN];
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++)
+          xv[i] = 32 * i + lane < cnt ? (XU ? __ldg(x + col[i]) : __ldg(x + (int64_t)col[i] * it.ldx)) : V(0);
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++)
+          if (32 * i + lane < cnt) {
+            const V p = mul_rn(a[i], xv[i]);
+            isum = __dadd_rn((double)p, isum);
+            if constexpr (ERR) ierr = __fadd_rn(ierr, exact ? __fmaf_rn(a[i], xv[i], -p) : 0.0f);
+          }
+        if constexpr (ERR) isum = __dadd_rn(isum, (double)ierr);
+      } else {
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++)
+          if (32 * i + lane < cnt) isum = op_comb<double, OP>(OP == OP_COUNT ? 1.0 : (double)a[i], isum);
+      }
+    } else if (cnt > 0) {
+      // ---- runs and row starts
+      if (lane < FT_WIN) runs[lane] = starts[lane] = 0;
+      __syncwarp();
+      auto mark_row = [&](int32_t r, int32_t o, int32_t o1, int2 sg) {
+        if (o1 <= o || o - e0 >= cnt) return;
+        hrow[o > e0 ? o - e0 : 0] = r;
+        if (o > e0) atomicOr(&starts[(o - e0) >> 5], 1u << ((o - e0) & 31));  // (position 0 needs no bit)
+        int32_t pos = o;
+        for (int l = 1; sg.x >= 0; l++) {
+          const int32_t len = min(sg.y - sg.x, o1 - pos);
+          const int a = pos - e0, b = a + len;
+          if (b > 0 && a < cnt && len > 0) {
+            const int p = a > 0 ? a : 0;
+            atomicOr(&runs[p >> 5], 1u << (p & 31));
+            sdel[p] = sg.x - pos;
+          }
+          pos += len;
+          if (pos >= o1 || l >= it.m.max_segs) break;
+          sg = __ldg(reinterpret_cast<const int2 *>(it.m.seg + (int64_t)l * it.m.pitch + 2 * (int64_t)r));
+        }
+      };
+      if (r1 - r0 <= FT_ROWS) {
+        mark_row(r0 + lane, cur.o, cur.o1, cur.sg);
+        for (int32_t rb = r0 + 32; rb <= r1; rb += 128) {  // past the first 32 rows: 128 at a time
+          int32_t o[4], o1[4];
+          int2 sg[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const int32_t r = rb + 32 * q + lane;
+            o[q] = o1[q] = 0;
+            sg[q] = make_int2(-1, -1);
+            if (r <= r1) {
+              o[q] = __ldg(it.off + r);
+              o1[q] = __ldg(it.off + r + 1);
+              sg[q] = __ldg(reinterpret_cast<const int2 *>(it.m.seg + 2 * (int64_t)r));
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 4; q++) mark_row(rb + 32 * q + lane, o[q], o1[q], sg[q]);
+        }
+      } else {  // a long stretch of empty rows: each entry's row by a search, marked by its first entry here
+        int32_t rows[FT_WIN];
+        flat_find_rows(it.off, e0, cnt, r0, r1, rows);
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++) {
+          const int p = 32 * i + lane;
+          if (p >= cnt) continue;
+          const int32_t r = rows[i], o = it.off[r];
+          if (p == 0 || e0 + p == o)
+            mark_row(r, o, it.off[r + 1], *reinterpret_cast<const int2 *>(it.m.seg + 2 * (int64_t)r));
+        }
+      }
+      __syncwarp();
+      // ---- entries
+      int h[FT_WIN];
+      flat_heads(runs, h);
+      V a[FT_WIN];
+      int32_t col[FT_WIN];
+#pragma unroll
+      for (int i = 0; i < FT_WIN; i++) {
+        const int p = 32 * i + lane;
+        a[i] = V(0);
+        col[i] = 0;
+        if (p < cnt) {
+          const int32_t q = e0 + p + sdel[h[i]];
+          a[i] = __ldcs(it.m.vals + q);
+          col[i] = OP == OP_SPMV ? __ldcs(it.m.cols + q) : 0;
+        }
+      }
+      if constexpr (!OWN) __syncwarp();  // the distances are read: the products take their place
+      if constexpr (OP == OP_SPMV) {
+        const V *__restrict__ x = it.x;
+        V xv[FT_WIN];
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++)
+          xv[i] = 32 * i + lane < cnt ? (XU ? __ldg(x + col[i]) : __ldg(x + (int64_t)col[i] * it.ldx)) : V(0);
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++) {
+          const bool in = 32 * i + lane < cnt;
+          const V p = mul_rn(a[i], xv[i]);
+          prod[32 * i + lane] = in ? p : V(0);
+          if constexpr (ERR) err[32 * i + lane] = in && exact ? __fmaf_rn(a[i], xv[i], -p) : 0.0f;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < FT_WIN; i++)
+          prod[32 * i + lane] = 32 * i + lane >= cnt ? op_init<V, OP>() : OP == OP_COUNT ? V(1) : a[i];
+      }
     }
-    if (advance) {
-      cur = nx;
-      nx = unit1_load<V>(src, fetch_take(), NC, NM, total, lane);
-      fetch_issue();
-      o = 0;
-      if (streamed(cur)) unit_range(cur, c0, c1);
+    // the next tile's rows and the tile after it, on their way meanwhile
+    FlatTile next = nx;
+    flat_tile_rows<V>(src, next);
+    flat_tile_head<V>(src, t + 2 * nw, total, nx);
+    if (inner) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) isum = op_comb<double, OP>(isum, __shfl_xor_sync(FULL, isum, o));
+      if (lane == 0) {
+        double *part = it.fpart + 2 * (int64_t)cur.lt;
+        if (cont) part[0] = isum;
+        else if (o01 > e0 + cnt) part[1] = isum;
+        else write_row<V, OP>(it, r0, isum);
+      }
+    } else if (cnt > 0) {
+      __syncwarp();
+      // ---- sums: lane l holds entries 8l .. 8l+7
+      V pv[FT_WIN];
+      float ev[ERR ? FT_WIN : 1];
+      auto eight = [&](const auto *b, auto &v) {
+        using U = typename std::remove_cv<typename std::remove_reference<decltype(*b)>::type>::type;
+#pragma unroll
+        for (int q = 0; q < FT_WIN; q += 16 / (int)sizeof(U)) {
+          if constexpr (sizeof(U) == 4) {
+            const float4 f = *reinterpret_cast<const float4 *>(b + q);
+            v[q] = f.x; v[q + 1] = f.y; v[q + 2] = f.z; v[q + 3] = f.w;
+          } else {
+            const double2 f = *reinterpret_cast<const double2 *>(b + q);
+            v[q] = f.x; v[q + 1] = f.y;
+          }
+        }
+      };
+      eight(prod + 8 * lane, pv);
+      if constexpr (ERR) eight(err + 8 * lane, ev);
+      const unsigned bits = (starts[lane >> 2] >> (8 * (lane & 3))) & 0xffu;
+      double acc = op_init<double, OP>(), first = acc;
+      float ea = 0.0f;  // the errors of acc's products
+      auto piece = [&]() -> double {
+        if constexpr (ERR) return __dadd_rn(acc, (double)ea);
+        return acc;
+      };
+      int at = -1;  // last row start in this lane
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if ((bits >> q) & 1) {
+          if (at < 0) first = piece();  // closes a row that began in an earlier lane (or the tile's first)
+          else write_row<V, OP>(it, hrow[at], piece());
+          at = 8 * lane + q;
+          acc = op_init<double, OP>();
+          ea = 0.0f;
+        }
+        acc = op_comb<double, OP>((double)pv[q], acc);
+        if constexpr (ERR) ea = __fadd_rn(ea, ev[q]);
+      }
+      // open pieces carried over the lanes; the last start before each lane
+      double open = piece();
+      bool seen = at >= 0;
+      int last = at < 0 ? 0 : at;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const double ov = __shfl_up_sync(FULL, open, d);
+        const int os = __shfl_up_sync(FULL, (int)seen, d), ol = __shfl_up_sync(FULL, last, d);
+        if (lane >= d) {
+          if (!seen) open = op_comb<double, OP>(open, ov);
+          seen = seen || os;
+          last = max(last, ol);
+        }
+      }
+      double carry = __shfl_up_sync(FULL, open, 1);
+      int before = __shfl_up_sync(FULL, last, 1);
+      if (lane == 0) {
+        carry = op_init<double, OP>();
+        before = 0;
+      }
+      double *part = it.fpart + 2 * (int64_t)cur.lt;
+      if (at >= 0) {  // the row open before this lane ends here
+        const double v = op_comb<double, OP>(first, carry);
+        if (before == 0 && cont) part[0] = v;
+        else write_row<V, OP>(it, hrow[before], v);
+      }
+      if (lane == 31) {  // the row open at the tile's end
+        const int32_t r = hrow[last];
+        if (last == 0 && cont) part[0] = open;
+        else if (it.off[r + 1] > e0 + cnt) part[1] = open;
+        else write_row<V, OP>(it, r, open);
+      }
+      __syncwarp();  // the tile's marks and products are free
     }
-  };
-  while (cur.u < total) {
-    step(a0, k0, a1, k1);
-    if (cur.u >= total) break;
-    step(a1, k1, a0, k0);
-  }
-  // the last warp to finish resets the counters for the next pass (the
-  // atomic still pending in lane 0 belongs to nobody: every number past
-  // the end is discarded)
-  if (lane == 0 && atomicAdd(ctr + 1, 1u) == gridDim.x * RS_WARPS - 1) {
-    ctr[0] = 0;
-    ctr[1] = 0;
+    cur = next;
   }
 }
 
-// The short-row blocks of a k = 1 pass: a warp per block of 32 rows, the
-// next block's descriptors (each lane's row length and layer-0 segment)
-// loaded while the current block runs.
-template <typename V, int OP, typename Src, bool XU>
-__global__ void __launch_bounds__(RS_THREADS_, DCSR_K1B_MINB) k_rows1_blocks(Src src) {
-  const int lane = threadIdx.x & 31;
-  const int64_t NB = src.units(P_BLOCKS) * RS_WARPS;
-  unsigned *ctr = src.ctr(1);
-  unsigned pend = 0;  // lane 0's atomic, broadcast one block later
-  auto fetch_issue = [&]() {
-    if (lane == 0) pend = atomicAdd(ctr, 1u);
-  };
-  auto fetch_take = [&]() -> int64_t { return (int64_t)__shfl_sync(FULL, pend, 0); };
-  // units numbered after the streamed ones (NC + NM): unit1_load decodes them as blocks
-  const int64_t base = src.units(P_CHUNKS) + src.units(P_MED) * RS_WARPS, total = base + NB;
-  fetch_issue();
-  Unit1 cur = unit1_load<V>(src, base + fetch_take(), base, 0, total, lane);
-  fetch_issue();
-  while (cur.u < total) {
-    const Unit1 nx = unit1_load<V>(src, base + fetch_take(), base, 0, total, lane);
-    fetch_issue();
-    if (cur.kind == U1_BLOCK) short_block_k1<V, OP, XU>(src.item(cur.item), cur.d, lane);
-    cur = nx;
+// Rows over several tiles (a thread per tile in which one begins, a warp for
+// more than 16 tiles) and empty rows (a thread per row).
+template <typename V, int OP, typename Src>
+__global__ void __launch_bounds__(FT_THREADS) k_flat_fix(Src src) {
+  const int64_t nt = src.units(P_TBLOCKS), total = nt + src.units(P_RBLOCKS);
+  for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
+    int64_t lu;
+    const bool tiles = u < nt;
+    const RowItem<V> &it = src.item(tiles ? src.locate(P_TBLOCKS, u, lu) : src.locate(P_RBLOCKS, u - nt, lu));
+    if (it.skip && *it.skip) continue;
+    const int64_t i = lu * FT_THREADS + threadIdx.x;
+    if (!tiles) {
+      if (i < it.m.n_rows && it.off[i] == it.off[i + 1]) {
+        const double z[1] = {op_init<double, OP>()};
+        write_y<V, 1, OP>(it.y, it.ldy, (int32_t)i, z, it.alpha, it.beta, 0, 1);
+      }
+      continue;
+    }
+    const int64_t nnz = it.off[it.m.n_rows], e1 = (i + 1) * FT_TILE;
+    int32_t r = -1, nh = 0;  // the row that begins in tile i and goes on, and in how many more tiles
+    if (e1 < nnz) {
+      r = it.tile_row[i + 1];
+      const int32_t o = it.off[r];
+      if (o >= e1 - FT_TILE && o < e1) nh = (int32_t)((it.off[r + 1] - 1) / FT_TILE - i);
+      else r = -1;
+    }
+    double v = 0.0;
+    if (r >= 0) {
+      v = it.fpart[2 * i + 1];
+      if (nh <= 16)
+        for (int32_t q = 1; q <= nh; q++) v = op_comb<double, OP>(it.fpart[2 * (i + q)], v);
+    }
+    unsigned big = __ballot_sync(FULL, nh > 16);
+    while (big) {  // lanes take heads lane, lane+32, ... in order, then a fixed tree
+      const int s = __ffs(big) - 1;
+      big &= big - 1;
+      const int64_t ti = __shfl_sync(FULL, i, s);
+      const int32_t n = __shfl_sync(FULL, nh, s);
+      double p = op_init<double, OP>();
+      for (int32_t q = 1 + lane_id(); q <= n; q += 32) p = op_comb<double, OP>(it.fpart[2 * (ti + q)], p);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) p = op_comb<double, OP>(p, __shfl_xor_sync(FULL, p, o));
+      if (lane_id() == s) v = op_comb<double, OP>(p, v);
+    }
+    if (r >= 0) write_row<V, OP>(it, r, v);
   }
-  if (lane == 0 && atomicAdd(ctr + 1, 1u) == gridDim.x * RS_WARPS - 1) {
-    ctr[0] = 0;
-    ctr[1] = 0;
+}
+
+// Row lengths -> offsets within a set of matrices' concatenated rows (mod
+// 2^32: only differences within one matrix are used).
+template <typename V, typename Src>
+struct FlatManyScan {
+  static constexpr int NS = 1, IT = SM_LIGHT;
+  using T = int32_t;
+  struct State {};
+  Src src;
+  int64_t R;
+  unsigned *tmp;
+  __device__ __forceinline__ void load(int64_t g, bool ok, State &, T (&v)[1]) const {
+    v[0] = 0;
+    if (ok) {
+      const RowItem<V> &it = src.item(src.find_row(g));
+      v[0] = it.m.row_sizes[g - it.row0];
+    }
   }
+  __device__ __forceinline__ void emit(int64_t g, bool ok, const State &, const long long (&p)[1], const T (&)[1]) const {
+    if (ok) tmp[g] = (unsigned)p[0];
+  }
+  __device__ __forceinline__ void total(const long long (&t)[1]) const { tmp[R] = (unsigned)t[0]; }
+};
+
+template <typename V, typename Src>
+__global__ void __launch_bounds__(256) k_flat_tables(Src src, int64_t R, const unsigned *tmp) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x; b < R; b += stride) {
+    const int64_t g = b + threadIdx.x;
+    int32_t r = 0, o = 0, len = 0;
+    int i = 0;
+    if (g < R) {
+      i = src.find_row(g);
+      const RowItem<V> &it = src.item(i);
+      r = (int32_t)(g - it.row0);
+      o = (int32_t)(tmp[g] - tmp[it.row0]);
+      len = (int32_t)(tmp[g + 1] - tmp[g]);
+      const_cast<int32_t *>(it.off)[r] = o;
+      if (r == it.m.n_rows - 1) const_cast<int32_t *>(it.off)[r + 1] = o + len;
+    }
+    // (a warp may hold rows of several matrices: tiles are marked per row)
+    const RowItem<V> &it = src.item(i);
+    const unsigned t0 = ((unsigned)o + (FT_TILE - 1)) / FT_TILE;
+    const unsigned t1 = len > 0 ? min(((unsigned)o + (unsigned)len - 1) / FT_TILE + 1, (unsigned)it.tiles) : 0;
+    const bool many = t1 > t0 && t1 - t0 > 16;
+    if (!many)
+      for (unsigned t = t0; t < t1; t++) const_cast<int32_t *>(it.tile_row)[t] = r;
+    unsigned big = __ballot_sync(FULL, many);
+    while (big) {
+      const int s = __ffs(big) - 1;
+      big &= big - 1;
+      const unsigned a = __shfl_sync(FULL, t0, s), z = __shfl_sync(FULL, t1, s);
+      const int32_t rr = __shfl_sync(FULL, r, s);
+      int32_t *tr = const_cast<int32_t *>(src.item(__shfl_sync(FULL, i, s)).tile_row);
+      for (unsigned t = a + lane_id(); t < z; t += 32) tr[t] = rr;
+    }
+  }
+}
+
+template <typename V>
+static int flat_many_t(const RowItem<V> *its, int count, int64_t R, Arena &ar, cudaStream_t s) {
+  const RowMany<V> src{its, count, nullptr};
+  unsigned *tmp = ar.take<unsigned>(R + 2);
+  if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
+  DCSR_TRY((scan_map(FlatManyScan<V, RowMany<V>>{src, R, tmp}, R, ar, s)));
+  DCSR_LAUNCH((k_flat_tables<V, RowMany<V>>), grid_for(R, 256), 256, 0, s, src, R, tmp);
+  return DCSR_OK;
 }
 
 static int grid_of(const void *k) { return persistent_grid(k, RS_THREADS_, 0); }
 
 template <typename V, int K, int OP, bool VEC, typename Src>
 static int launch_reduce_src(const Src &src, cudaStream_t s) {
-  if constexpr (K == 1) {  // one value per entry: streamed units, then short-row blocks
-    // VEC (k = 1): x has unit stride, gathered without the stride multiply
-    constexpr bool XU = VEC && OP == OP_SPMV;
-    static const int g = grid_of((const void *)k_rows1<V, OP, Src, XU>);
-    static const int gb = grid_of((const void *)k_rows1_blocks<V, OP, Src, XU>);
-    DCSR_LAUNCH((k_rows1<V, OP, Src, XU>), g, RS_THREADS_, 0, s, src);
-    DCSR_LAUNCH((k_rows1_blocks<V, OP, Src, XU>), gb, RS_THREADS_, 0, s, src);
-    return DCSR_OK;
-  } else {
-    static const int g0 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_BLOCKS, Src>);
-    static const int g1 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_CHUNKS, Src>);
-    static const int g2 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_MED, Src>);
-    DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_CHUNKS, Src>), g1, RS_THREADS_, 0, s, src);
-    DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_MED, Src>), g2, RS_THREADS_, 0, s, src);
-    DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_BLOCKS, Src>), g0, RS_THREADS_, 0, s, src);
-    return DCSR_OK;
+  static const int g0 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_BLOCKS, Src>);
+  static const int g1 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_CHUNKS, Src>);
+  static const int g2 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_MED, Src>);
+  DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_CHUNKS, Src>), g1, RS_THREADS_, 0, s, src);
+  DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_MED, Src>), g2, RS_THREADS_, 0, s, src);
+  DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_BLOCKS, Src>), g0, RS_THREADS_, 0, s, src);
+  return DCSR_OK;
+}
+
+// The flat pass over `tiles` tiles and `rows` rows at most (-1: not known on
+// the host).  Few tiles: two warps per block, so that they spread over the SMs.
+template <typename V, int OP, bool XU, bool EXACT, typename Src>
+static int launch_flat_src(const Src &src, int64_t tiles, int64_t rows, cudaStream_t s) {
+  static const int g = grid_of((const void *)k_flat_rows<V, OP, Src, XU, EXACT>);
+  static const int gf = grid_of((const void *)k_flat_fix<V, OP, Src>);
+  const int64_t cap = (int64_t)g * FT_WARPS;  // resident warps
+  int threads = FT_THREADS;
+  int64_t blocks = g, fix = gf;
+  if (tiles >= 0) {
+    if (tiles < cap / 4) threads = 64;
+    blocks = std::max<int64_t>(1, std::min<int64_t>(div_up(tiles, threads / 32), threads == 64 ? cap / 2 : g));
+    fix = std::max<int64_t>(1, std::min<int64_t>(div_up(tiles, FT_THREADS) + div_up(rows, FT_THREADS), gf));
   }
+  DCSR_LAUNCH((k_flat_rows<V, OP, Src, XU, EXACT>), (unsigned)blocks, threads, 0, s, src);
+  DCSR_LAUNCH((k_flat_fix<V, OP, Src>), (unsigned)fix, FT_THREADS, 0, s, src);
+  return DCSR_OK;
+}
+
+template <typename V, int OP>
+static int launch_flat(dcsr_handle h, const V *x, int64_t ldx, V *y, int64_t ldy, double alpha, double beta,
+                       cudaStream_t s) {
+  const FlatOne<V> src{row_item<V>(h, x, y, ldx, ldy, alpha, beta)};
+  const int64_t tiles = flat_tiles(h->pool_cap);
+  constexpr bool F32 = OP == OP_SPMV && sizeof(V) == 4;
+  if (OP == OP_SPMV && ldx == 1) {
+    if (F32 && h->n_rows <= FLAT_EXACT_ROWS) return launch_flat_src<V, OP, OP == OP_SPMV, F32>(src, tiles, h->n_rows, s);
+    return launch_flat_src<V, OP, OP == OP_SPMV, false>(src, tiles, h->n_rows, s);
+  }
+  if (F32 && h->n_rows <= FLAT_EXACT_ROWS) return launch_flat_src<V, OP, false, F32>(src, tiles, h->n_rows, s);
+  return launch_flat_src<V, OP, false, false>(src, tiles, h->n_rows, s);
 }
 
 // Warps per 32-row block of short rows for the k >= 2 pass: doubled (up to
@@ -1326,8 +1294,8 @@ template <typename V, int K>
 static int spmv_k(dcsr_handle h, const V *x, int64_t ldx, V *y, int64_t ldy, double alpha, double beta,
                   cudaStream_t s) {
   const size_t rb = K * sizeof(V), al = (rb & (0 - rb)) >= 32 ? 32 : (rb & (0 - rb));  // row alignment
-  // k >= 2: packed, aligned rows of x (vector loads); k = 1: x of unit stride
-  const bool vec = K == 1 ? ldx == 1 : (K % 2 == 0) && ldx == K && ((uintptr_t)x % al) == 0;
+  // packed, aligned rows of x: vector loads
+  const bool vec = (K % 2 == 0) && ldx == K && ((uintptr_t)x % al) == 0;
   if (vec) return launch_reduce<V, K, OP_SPMV, true>(h, x, ldx, y, ldy, alpha, beta, s);
   return launch_reduce<V, K, OP_SPMV, false>(h, x, ldx, y, ldy, alpha, beta, s);
 }
@@ -1335,13 +1303,8 @@ static int spmv_k(dcsr_handle h, const V *x, int64_t ldx, V *y, int64_t ldy, dou
 template <typename V>
 static int spmv_dispatch(dcsr_handle h, const V *x, int32_t k, int64_t ldx, V *y, int64_t ldy, double alpha,
                          double beta, cudaStream_t s) {
-  if (k == 1 && h->n_rows <= K1_GROUP_ROWS) {  // the runtime-k pass with the item's k = 1
-    RowOne<V> src{row_item<V>(h, x, y, ldx, ldy, alpha, beta)};
-    src.split = short_split(div_up(h->n_rows, 32), 2);
-    return launch_reduce_src<V, -2, OP_SPMV, false>(src, s);
-  }
   switch (k) {
-    case 1: return spmv_k<V, 1>(h, x, ldx, y, ldy, alpha, beta, s);
+    case 1: return launch_flat<V, OP_SPMV>(h, x, ldx, y, ldy, alpha, beta, s);
     case 2: return spmv_k<V, 2>(h, x, ldx, y, ldy, alpha, beta, s);
     case 3: return spmv_k<V, 3>(h, x, ldx, y, ldy, alpha, beta, s);
     case 4: return spmv_k<V, 4>(h, x, ldx, y, ldy, alpha, beta, s);
@@ -1356,10 +1319,10 @@ static int spmv_dispatch(dcsr_handle h, const V *x, int32_t k, int64_t ldx, V *y
 template <typename V>
 static int reduce_dispatch(dcsr_handle h, int32_t op, V *y, cudaStream_t s) {
   switch (op) {
-    case DCSR_REDUCE_SUM: return launch_reduce<V, 1, OP_SUM, false>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
-    case DCSR_REDUCE_MAX: return launch_reduce<V, 1, OP_MAX, false>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
-    case DCSR_REDUCE_MIN: return launch_reduce<V, 1, OP_MIN, false>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
-    case DCSR_REDUCE_COUNT: return launch_reduce<V, 1, OP_COUNT, false>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
+    case DCSR_REDUCE_SUM: return launch_flat<V, OP_SUM>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
+    case DCSR_REDUCE_MAX: return launch_flat<V, OP_MAX>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
+    case DCSR_REDUCE_MIN: return launch_flat<V, OP_MIN>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
+    case DCSR_REDUCE_COUNT: return launch_flat<V, OP_COUNT>(h, nullptr, 0, y, 1, 1.0, 0.0, s);
   }
   return DCSR_BAD_ARG;
 }
@@ -1369,11 +1332,11 @@ static int reduce_dispatch(dcsr_handle h, int32_t op, V *y, cudaStream_t s) {
 template <typename V>
 static int spmv_many_t(const RowItem<V> *its, int count, int kf, long long *pref, bool prefixed, int split,
                        cudaStream_t s) {
-  if (kf == 1) split = 1;
+  if (kf == 1) split = 0;  // flat units
   if (!prefixed) DCSR_LAUNCH(k_unit_prefix<V>, 1, 1024, 0, s, its, count, pref, split);
   RowMany<V> src{its, count, pref, split};
   switch (kf) {
-    case 1: return launch_reduce_src<V, 1, OP_SPMV, false>(src, s);
+    case 1: return launch_flat_src<V, OP_SPMV, false, sizeof(V) == 4>(src, -1, -1, s);
     case 2: return launch_reduce_src<V, -2, OP_SPMV, false>(src, s);
     case 4: return launch_reduce_src<V, -4, OP_SPMV, false>(src, s);
     case 8: return launch_reduce_src<V, -8, OP_SPMV, false>(src, s);
@@ -1420,8 +1383,12 @@ namespace dcsr {
 int spmv_call(dcsr_handle h, const void *x, int32_t k, int64_t ldx, void *y, int64_t ldy, double alpha, double beta,
               cudaStream_t s, Arena *ar) {
   if (h->n_rows == 0) return DCSR_OK;
-  DCSR_TRY(ensure_part(h, k == 1 && h->n_rows <= K1_GROUP_ROWS ? 2 : k, s));  // partials of the k <= 2 pass
-  if (!h->bins_valid) DCSR_TRY(build_schedule(h, s, ar));
+  if (k == 1) {
+    if (!h->flat_valid) DCSR_TRY(build_flat(h, s, ar));
+  } else {
+    DCSR_TRY(ensure_part(h, k, s));
+    if (!h->bins_valid) DCSR_TRY(build_schedule(h, s, ar));
+  }
   if (h->dtype == DCSR_F32)
     return spmv_dispatch<float>(h, (const float *)x, k, ldx, (float *)y, ldy, alpha, beta, s);
   return spmv_dispatch<double>(h, (const double *)x, k, ldx, (double *)y, ldy, alpha, beta, s);
@@ -1439,8 +1406,7 @@ extern "C" int dcsr_row_reduce(dcsr_handle h, int32_t op, void *y, void *stream)
   if (!h || (h->n_rows > 0 && !y) || op < 0 || op > 3) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   if (h->n_rows == 0) return DCSR_OK;
-  DCSR_TRY(ensure_part(h, 1, s));
-  if (!h->bins_valid) DCSR_TRY(build_schedule(h, s));
+  if (!h->flat_valid) DCSR_TRY(build_flat(h, s));
   if (h->dtype == DCSR_F32) return reduce_dispatch<float>(h, op, (float *)y, s);
   return reduce_dispatch<double>(h, op, (double *)y, s);
 }

@@ -6,7 +6,9 @@ several segments; layout, structure and values bit-exact against the oracle."""
 import numpy as np
 import pytest
 
-from helpers import assert_content_equal, assert_layout_equal, make_pair
+import torch
+
+from helpers import assert_content_equal, assert_layout_equal, make_pair, spmv_bound
 
 pytestmark = pytest.mark.gpu
 
@@ -59,6 +61,75 @@ def test_load_export_compact(dcsr, name, dtype, mode):
     orc.compact()
     assert_layout_equal(dev, orc, "compaction")
     assert_content_equal(dev, orc, "compaction")
+
+
+def check_rows(dcsr, dev, orc, rng, what):
+    """SpMV with one right-hand side (unit stride, strided, alpha and beta) and
+    the row reductions against the FP64 oracle: |error| within 1e-6 (FP32) or
+    1e-13 (FP64) of the sum of magnitudes."""
+    tol = {0: 1e-6, 1: 1e-13}[dev.dtype_code]
+    n, m = dev.n_rows, dev.n_cols
+    x = torch.tensor(rng.uniform(-1, 1, (m, 3)), dtype=dev.dtype).cuda()
+    y0 = torch.tensor(rng.uniform(-1, 1, (n, 2)), dtype=dev.dtype).cuda()
+    x64, y64 = x.cpu().double().numpy(), y0.cpu().double().numpy()
+    bound = spmv_bound(orc, x64[:, 0])
+    y = dev.spmv(x[:, 0].contiguous()).cpu().double().numpy()
+    assert np.all(np.abs(y - orc.spmv(x64[:, 0].copy())) <= tol * bound + 1e-300), what
+    # strided x and y, accumulating (the C ABI's ldx / ldy)
+    y = y0.clone()
+    assert dcsr.lib().dcsr_spmv(dev.h, x.data_ptr(), 1, 3, y.data_ptr(), 2, -1.5, 0.25,
+                                torch.cuda.current_stream().cuda_stream) == 0
+    y = y.cpu().double().numpy()
+    ref = orc.spmv(x64[:, 0].copy(), alpha=-1.5, beta=0.25, y=y64[:, 0].copy())
+    assert np.all(np.abs(y[:, 0] - ref) <= tol * (1.5 * bound + 0.25 * np.abs(y64[:, 0])) + 1e-300), what
+    np.testing.assert_array_equal(y[:, 1], y64[:, 1])
+    rp, _, v = orc.export_csr()
+    for op in (dcsr.REDUCE_SUM, dcsr.REDUCE_MAX, dcsr.REDUCE_MIN, dcsr.REDUCE_COUNT):
+        got = dev.row_reduce(op).cpu().double().numpy()
+        want = orc.row_reduce(op)
+        if op == dcsr.REDUCE_SUM:
+            mag = np.zeros(n)
+            np.add.at(mag, np.repeat(np.arange(n), np.diff(rp)), np.abs(v))
+            assert np.all(np.abs(got - want) <= tol * mag + 1e-300), what
+        else:
+            np.testing.assert_array_equal(got, want, err_msg=what)
+
+
+@pytest.mark.parametrize("name", list(LENS))
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_rows_over_tiles(dcsr, name, dtype):
+    lens = np.asarray(LENS[name], np.int64)
+    rng = np.random.default_rng(len(lens) + 1)
+    n, m = len(lens), 100_003
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(m, L, replace=False)) for L in lens if L]).astype(np.int32)
+    vals = rng.uniform(-1, 1, cols.size)
+    vals = vals.astype(np.float32) if dtype == 0 else vals
+    dev, orc = make_pair(dcsr, n, m, dtype, 0)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals.astype(np.float64)) == 0
+    check_rows(dcsr, dev, orc, rng, "loaded")
+    for it in range(2):
+        T = 700
+        r = np.where(rng.random(T) < 0.5, rng.choice(np.repeat(np.arange(n), lens), T),
+                     rng.integers(0, n, T)).astype(np.int32)
+        c = rng.integers(0, m, T).astype(np.int32)
+        v = rng.uniform(-1, 1, T)
+        v = v.astype(np.float32) if dtype == 0 else v
+        assert dev.update(r, c, v) == orc.update_auto(r, c, v.astype(np.float64)) == 0
+        check_rows(dcsr, dev, orc, rng, f"update {it}")
+    dev.compact()
+    orc.compact()
+    check_rows(dcsr, dev, orc, rng, "compacted")
+
+
+def test_empty_matrix_rows(dcsr):
+    """No entries: every row is written (0, or beta * y), the next state likewise."""
+    rng = np.random.default_rng(3)
+    dev, orc = make_pair(dcsr, 1000, 50, 1, 0)
+    check_rows(dcsr, dev, orc, rng, "empty")
+    dev.from_csr(np.zeros(1001, np.int32), np.zeros(0, np.int32), np.zeros(0))
+    check_rows(dcsr, dev, orc, rng, "loaded empty")
 
 
 @pytest.mark.parametrize("nnz", [1, 255, 256, 257, 4096, 70_001])
