@@ -81,10 +81,7 @@ void fill_image(const BatchCore &b, unsigned char *img) {
       RowItem<V> r = row_item<V>(it.matrix, it.x, it.y, it.ldx, it.ldy, it.alpha, it.beta);
       r.skip = b.upd_of[i] >= 0 ? b.skip + b.upd_of[i] : nullptr;  // only an update can be rejected
       r.k = it.k;
-      // x rows as 8/16/32-byte vectors: even k, packed rows, base aligned to
-      // the largest power of two (<= 32) dividing the row size
-      const size_t rb = it.k * sizeof(V), al = (rb & (0 - rb)) >= 32 ? 32 : (rb & (0 - rb));
-      r.vec = it.k > 1 && it.k % 2 == 0 && it.ldx == it.k && ((uintptr_t)it.x % al) == 0;
+      r.vec = rhs_vec(it.x, it.k, it.ldx, sizeof(V)) ? 1 : 0;
       r.row0 = row0;
       row0 += it.matrix->n_rows;
       gi[j] = r;
@@ -151,7 +148,7 @@ int BatchCore::plan(const dcsr_batch_item *its, int n, cudaStream_t s, bool all_
   for (int i = 0; i < n; i++) {
     const dcsr_batch_item &it = its[i];
     if (!it.x || it.matrix->n_rows == 0) continue;
-    const int gk = it.k == 1 ? 1 : it.k <= 2 ? 2 : it.k <= 4 ? 4 : 8;
+    const int gk = rhs_family(it.k);
     int gi = -1;
     for (size_t q = 0; q < groups.size(); q++)
       if (groups[q].k == gk) gi = (int)q;

@@ -5,16 +5,14 @@
 // flat pass, a warp per tile of 256 consecutive entries (k_flat_rows).
 //
 // SpMV with k >= 2: rows are split into three classes by the schedule (rebuilt
-// lazily after any change of row lengths), each with its own launch so each
-// has its own register budget and its units carry bounded work:
+// lazily after any change of row lengths), whose units carry bounded work:
 //   short  (<= short_max entries)  a warp takes 32 consecutive rows and splits
 //          into groups of G lanes, G in {1..16} from the block's mean row
 //          length; a group walks one row with several loads in flight per
 //          lane and reduces over its lanes with log2(G) shuffles.
 //   medium (<= long_min)          one warp per row, lanes strided, U loads in
 //          flight per lane, one warp reduction per row.
-//   long                          CHUNK-entry chunks, one CTA per chunk,
-//          STEP entries in flight per CTA step (128-bit loads when aligned);
+//   long                          CHUNK-entry chunks, one CTA per chunk;
 //          multi-chunk rows combine their partials in chunk order (the CTA
 //          that finishes the last chunk sums them).
 // A row's result depends only on the row and its matrix (its length picks its
@@ -45,7 +43,6 @@ constexpr int RS_WARPS = RS_THREADS_ / 32;
 #define DCSR_CHUNK 2048
 #endif
 constexpr int CHUNK = DCSR_CHUNK;
-constexpr int STEP = 4096;    // entries a CTA has in flight per step
 enum { P_BLOCKS = 0, P_CHUNKS = 1, P_MED = 2 };
 // The flat pass's units (one value per entry): tiles; blocks of FT_THREADS
 // tiles and rows for k_flat_fix.
@@ -416,51 +413,6 @@ __device__ __forceinline__ int group_width(int32_t total) {
   return mean < 8 ? 1 : mean < 16 ? 2 : mean < 32 ? 4 : mean < 64 ? 8 : 16;
 }
 
-// Visit the logical entries [0, len) of a row: lane j of a G-lane group takes
-// entries j, j+G, ...; f(st, p0, take, before) handles the UN entries
-// p0 + i*G (< take) of the layer starting at pool slot st, whose first entry
-// is logical position `before`.
-template <int UN, typename F>
-__device__ __forceinline__ void for_row_entries(const Chain &ch, int32_t len, int j, int G, F &&f) {
-  int32_t before = 0;
-#pragma unroll
-  for (int l = 0; l < MAX_SEGS; l++) {
-    if (l < ch.ns && before < len) {
-      const int32_t take = ch.cp[l] < len - before ? ch.cp[l] : len - before;
-      const int64_t st = ch.st[l];
-      for (int32_t p0 = j; p0 < take; p0 += UN * G) f(st, p0, take, before);
-      before += ch.cp[l];
-    }
-  }
-}
-
-// VEC: the rows of x are packed (ldx == K) and aligned to the largest power
-// of two (<= 32) dividing the row size, so a row is read with vector loads.
-template <typename T, typename V, int K, bool VEC>
-__device__ __forceinline__ void load_xk(const V *__restrict__ x, int64_t c, int64_t ldx, T (&xv)[K]) {
-  if constexpr (VEC && sizeof(V) == 4 && K == 8) {  // two 128-bit loads (measured faster than one 256-bit load)
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(x + c * 8));
-    const float4 u = __ldg(reinterpret_cast<const float4 *>(x + c * 8) + 1);
-    xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
-    xv[4] = u.x; xv[5] = u.y; xv[6] = u.z; xv[7] = u.w;
-  } else if constexpr (VEC && sizeof(V) == 4 && K == 4) {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(x + c * 4));
-    xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
-  } else if constexpr (VEC && sizeof(V) == 4 && K == 2) {
-    const float2 t = __ldg(reinterpret_cast<const float2 *>(x + c * 2));
-    xv[0] = t.x; xv[1] = t.y;
-  } else if constexpr (VEC && sizeof(V) == 8 && K % 2 == 0) {
-#pragma unroll
-    for (int k = 0; k < K; k += 2) {
-      const double2 t = __ldg(reinterpret_cast<const double2 *>(x + c * K + k));
-      xv[k] = (T)t.x; xv[k + 1] = (T)t.y;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < K; k++) xv[k] = (T)__ldg(x + c * ldx + k);
-  }
-}
-
 enum { OP_SPMV = 0, OP_SUM = 1, OP_MAX = 2, OP_MIN = 3, OP_COUNT = 4 };
 
 template <typename T, int OP>
@@ -483,296 +435,221 @@ __device__ __forceinline__ T op_comb(T a, T b) {
   return add_rn(a, b);
 }
 
-// acc (op) a*x for one entry with value a and column c (FP64 accumulators)
-template <typename V, int K, int OP, bool VEC>
-__device__ __forceinline__ void accum_entry(double a, int32_t c, const V *x, int64_t ldx, double (&acc)[K]) {
-  if constexpr (OP == OP_SPMV) {
-    double xv[K];
-    load_xk<double, V, K, VEC>(x, c, ldx, xv);
-#pragma unroll
-    for (int k = 0; k < K; k++) acc[k] = __fma_rn(a, xv[k], acc[k]);
-  } else {
-    acc[0] = op_comb<double, OP>(acc[0], OP == OP_COUNT ? 1.0 : a);
+// y[row*ldy + k] = alpha*v + beta*y (SpMV), or v.
+template <typename V, int OP>
+__device__ __forceinline__ void write_y(V *y, double v, double alpha, double beta) {
+  if (OP == OP_SPMV) {
+    v = mul_rn(v, alpha);
+    if (beta != 0.0) v = __fma_rn(beta, (double)*y, v);
   }
+  *y = (V)v;
 }
 
-// K < 0: the number of right-hand sides is a runtime value kr <= -K (one
-// launch serves matrices with different k); accumulators are sized for -K.
-template <int K>
-struct KArr {
-  static constexpr int N = K < 0 ? -K : K;
-};
-
-// acc (op) a*x for one entry, k from the template (K > 0) or the item (K < 0).
-template <typename V, int K, int OP, bool VEC>
-__device__ __forceinline__ void accum_k(double a, int32_t c, const V *x, int64_t ldx, int kr, bool vec,
-                                        double (&acc)[KArr<K>::N]) {
-  constexpr int N = KArr<K>::N;
-  if constexpr (K > 0) {
-    accum_entry<V, K, OP, VEC>(a, c, x, ldx, acc);
-  } else if constexpr (OP == OP_SPMV) {
-    const V *xr = x + (int64_t)c * ldx;
-    double xv[N];
-    if (vec && kr == N && N % (16 / (int)sizeof(V)) == 0) {  // whole 16-byte vectors
+// ------------------------------------------------------- k >= 2 right-hand sides
+// A lane takes an entry with all of its K right-hand sides (K accumulators; a
+// packed, aligned row of x in 16-byte loads): what counts is how many rows of
+// x a warp has in flight.  Sharing an entry among lanes (2 of 4 values each
+// for k = 8) touched half the cache lines per gather but left fewer rows in
+// flight: 131 against 101 us for 8M entries with k = 8 (FP32), 59 against 36 us
+// for 2M with k = 3 (FP64).  Kernels are compiled per family (k = 2, 3..4,
+// 5..8; one launch serves matrices of different k) and branch to the code of a
+// matrix's own K -- a runtime k in the inner loop ran the batched passes at
+// half the speed.
+template <typename V, int K, bool VEC>
+__device__ __forceinline__ void load_x(const V *__restrict__ p, V (&v)[K]) {
+  if constexpr (VEC && K * sizeof(V) >= 16) {
 #pragma unroll
-      for (int q = 0; q < N; q += 16 / (int)sizeof(V)) {
-        if constexpr (sizeof(V) == 4) {
-          const float4 t = __ldg(reinterpret_cast<const float4 *>(xr) + q / 4);
-          xv[q] = t.x; xv[q + 1] = t.y; xv[q + 2] = t.z; xv[q + 3] = t.w;
-        } else {
-          const double2 t = __ldg(reinterpret_cast<const double2 *>(xr) + q / 2);
-          xv[q] = t.x; xv[q + 1] = t.y;
-        }
-      }
-    } else if (vec) {  // even kr: pairs
-#pragma unroll
-      for (int q = 0; q < N; q += 2)
-        if (q < kr) {
-          if constexpr (sizeof(V) == 4) {
-            const float2 t = __ldg(reinterpret_cast<const float2 *>(xr) + q / 2);
-            xv[q] = t.x; xv[q + 1] = t.y;
-          } else {
-            const double2 t = __ldg(reinterpret_cast<const double2 *>(xr) + q / 2);
-            xv[q] = t.x; xv[q + 1] = t.y;
-          }
-        }
-    } else {
-#pragma unroll
-      for (int q = 0; q < N; q++)
-        if (q < kr) xv[q] = __ldg(xr + q);
-    }
-#pragma unroll
-    for (int q = 0; q < N; q++)
-      if (q < kr) acc[q] = __fma_rn(a, xv[q], acc[q]);
-  } else {
-    acc[0] = op_comb<double, OP>(acc[0], OP == OP_COUNT ? 1.0 : a);
-  }
-}
-
-template <typename V, int K, int OP>
-__device__ __forceinline__ void write_y(V *y, int64_t ldy, int32_t row, const double (&acc)[KArr<K>::N],
-                                        double alpha, double beta, int32_t len, int kr) {
-#pragma unroll
-  for (int k = 0; k < KArr<K>::N; k++) {
-    if (K < 0 && k >= kr) break;
-    double v = acc[k];
-    if ((OP == OP_MAX || OP == OP_MIN) && len == 0) v = 0.0;
-    if (OP == OP_SPMV) {
-      v = mul_rn(v, alpha);
-      if (beta != 0.0) v = __fma_rn(beta, (double)y[(int64_t)row * ldy + k], v);
-    }
-    y[(int64_t)row * ldy + k] = (V)v;
-  }
-}
-
-// --------------------------------------------------------- reduction pass
-
-// Blocks per SM the row pass is compiled for: the runtime-k families hold up
-// to 8 FP64 accumulators and 8 x values per entry in flight, which left them
-// at 2-3 blocks (16-24 warps) per SM, too few to hide the gather latency.
-// Three blocks for k families 8 and 4 and four for family 2 (a few spilled
-// registers) ran the batched SpMV pass of 512 matrices 9% faster than the
-// unconstrained build (7.6 vs 8.4 ms).
-template <int K>
-struct RowsMinBlocks {
-  static constexpr int N = K == -8 ? 3 : K == -4 ? 3 : K == -2 ? 4 : 1;
-};
-
-template <typename V, int K, int OP, bool VEC, int PART, typename Src>
-__global__ void __launch_bounds__(RS_THREADS_, RowsMinBlocks<K>::N) k_rows_reduce(Src src) {
-  constexpr int KA = KArr<K>::N;
-  __shared__ double red[RS_WARPS][KA];
-  __shared__ int last_flag;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t units = src.units(PART);
-  for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-    int64_t lu;
-    const RowItem<V> &it = src.item(src.locate(PART, u, lu));
-    if (it.skip && *it.skip) continue;  // a batch matrix whose update was rejected: y untouched
-    const Mat<V> &m = it.m;
-    const V *__restrict__ x = it.x;
-    const int64_t ldx = it.ldx;
-    const int kr = K < 0 ? it.k : K;
-    const bool vec = K < 0 ? it.vec != 0 : VEC;
-    if constexpr (PART == P_CHUNKS) {
-      // ---- one chunk of a long row, whole CTA (the chunk's row comes with
-      // it; its chunk number and the long-row tables only for multi-chunk rows)
-      const int2 rl = it.chunk_rl[lu];
-      const int32_t row = rl.x;
-      const int64_t li = rl.y;
-      const int64_t L = m.row_sizes[row];
-      const int64_t nch = (L + CHUNK - 1) / CHUNK;
-      const int64_t chunk = nch == 1 ? 0 : lu - it.long_off[li];
-      const Chain ch = load_chain(m, row);
-      const int64_t c0 = chunk * CHUNK, c1 = c0 + CHUNK < L ? c0 + CHUNK : L;
-      double acc[KA];
-#pragma unroll
-      for (int k = 0; k < KA; k++) acc[k] = op_init<double, OP>();
-      const bool fast = ch.cp[0] >= c1;  // chunk inside layer 0
-      if (K > 0 && fast && sizeof(V) == 4 && ((ch.st[0] + c0) & 3) == 0) {
-        constexpr int G = STEP / 4 / RS_THREADS_;
-        for (int64_t s0 = c0; s0 < c1; s0 += STEP) {
-          const int64_t s1 = s0 + STEP < c1 ? s0 + STEP : c1;
-          const int64_t base = ch.st[0] + s0;
-          const int nv = (int)((s1 - s0) >> 2);
-          float4 a4[G];
-          int4 c4[G] = {};
-#pragma unroll
-          for (int g = 0; g < G; g++) {
-            const int v = threadIdx.x + g * RS_THREADS_;
-            if (v < nv) {
-              a4[g] = __ldcs(reinterpret_cast<const float4 *>(m.vals + base) + v);
-              if (OP == OP_SPMV) c4[g] = __ldcs(reinterpret_cast<const int4 *>(m.cols + base) + v);
-            }
-          }
-#pragma unroll
-          for (int g = 0; g < G; g++) {
-            if (threadIdx.x + g * RS_THREADS_ < nv) {
-              accum_k<V, K, OP, VEC>(a4[g].x, c4[g].x, x, ldx, kr, vec, acc);
-              accum_k<V, K, OP, VEC>(a4[g].y, c4[g].y, x, ldx, kr, vec, acc);
-              accum_k<V, K, OP, VEC>(a4[g].z, c4[g].z, x, ldx, kr, vec, acc);
-              accum_k<V, K, OP, VEC>(a4[g].w, c4[g].w, x, ldx, kr, vec, acc);
-            }
-          }
-          for (int64_t p = s0 + ((int64_t)nv << 2) + threadIdx.x; p < s1; p += RS_THREADS_)
-            accum_k<V, K, OP, VEC>((double)__ldcs(m.vals + ch.st[0] + p),
-                                       OP == OP_SPMV ? __ldcs(m.cols + ch.st[0] + p) : 0, x, ldx, kr, vec, acc);
-        }
+    for (int q = 0; q < K; q += 16 / (int)sizeof(V)) {
+      if constexpr (sizeof(V) == 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(p + q));
+        v[q] = t.x; v[q + 1] = t.y; v[q + 2] = t.z; v[q + 3] = t.w;
       } else {
-        for (int64_t p = c0 + threadIdx.x; p < c1; p += RS_THREADS_) {
-          const int64_t q = fast ? (int64_t)ch.st[0] + p : ch.phys(p);
-          accum_k<V, K, OP, VEC>((double)__ldcs(m.vals + q), OP == OP_SPMV ? __ldcs(m.cols + q) : 0, x, ldx, kr, vec,
-                                     acc);
-        }
+        const double2 t = __ldg(reinterpret_cast<const double2 *>(p + q));
+        v[q] = t.x; v[q + 1] = t.y;
       }
+    }
+  } else if constexpr (VEC) {  // FP32, K = 2
+    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
+    v[0] = t.x; v[1] = t.y;
+  } else {
 #pragma unroll
-      for (int k = 0; k < KA; k++) {
-        if (K < 0 && k >= kr) break;
-        double v = acc[k];
+    for (int q = 0; q < K; q++) v[q] = __ldg(p + q);
+  }
+}
+
+// acc += a*x over logical entries [c0, c1) of a row, lane j of G: entries j,
+// j+G, ... of each segment, UN of them in flight.
+template <typename V, int K, bool VEC>
+__device__ __forceinline__ void accum_row(const Mat<V> &m, const V *__restrict__ x, int64_t ldx, const Chain &ch,
+                                          int32_t c0, int32_t c1, int j, int G, double (&acc)[K]) {
+  constexpr int UN = K <= 2 ? 8 : 4;
+  int32_t before = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = op_comb<double, OP>(v, __shfl_xor_sync(FULL, v, o));
-        if (lane == 0) red[w][k] = v;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double t[KA];
+  for (int l = 0; l < MAX_SEGS; l++) {
+    if (l < ch.ns && before < c1) {
+      const int32_t from = c0 > before ? c0 - before : 0, take = ch.cp[l] < c1 - before ? ch.cp[l] : c1 - before;
+      const int64_t st = ch.st[l];
+      for (int32_t p = from + j; p < take; p += UN * G) {
+        V a[UN];
+        int32_t col[UN];
 #pragma unroll
-        for (int k = 0; k < KA; k++) {
-        if (K < 0 && k >= kr) break;
-          t[k] = red[0][k];
-          for (int q = 1; q < RS_WARPS; q++) t[k] = op_comb<double, OP>(t[k], red[q][k]);
+        for (int i = 0; i < UN; i++) {
+          const int32_t pp = p + i * G;
+          const int64_t q = st + (pp < take ? pp : p);
+          a[i] = __ldcs(m.vals + q);
+          col[i] = __ldcs(m.cols + q);
         }
-        if (nch == 1) {  // the whole row in one unit: no partials
-          write_y<V, K, OP>(it.y, it.ldy, row, t, it.alpha, it.beta, (int32_t)L, kr);
-          last_flag = 0;
-        } else {
 #pragma unroll
-          for (int k = 0; k < KA; k++) it.part[(it.long_off[li] + chunk) * KA + k] = t[k];
-          __threadfence();
-          last_flag = atomicAdd(&it.long_cnt[li], 1) == nch - 1;
-        }
+        for (int i = 0; i < UN; i++)
+          if (p + i * G < take) {
+            V xv[K];
+            load_x<V, K, VEC>(x + (int64_t)col[i] * ldx, xv);
+#pragma unroll
+            for (int q = 0; q < K; q++) acc[q] = __fma_rn((double)a[i], (double)xv[q], acc[q]);
+          }
       }
-      __syncthreads();
-      if (last_flag && threadIdx.x == 0) {
+      before += ch.cp[l];
+    }
+  }
+}
+
+template <typename V, int K>
+__device__ __forceinline__ void write_rhs(const RowItem<V> &it, int32_t row, const double (&acc)[K]) {
+#pragma unroll
+  for (int q = 0; q < K; q++)
+    write_y<V, OP_SPMV>(it.y + (int64_t)row * it.ldy + q, acc[q], it.alpha, it.beta);
+}
+
+// One unit of a class (lu within matrix it).
+template <typename V, int K, bool VEC, int PART>
+__device__ __forceinline__ void rows_unit(const RowItem<V> &it, int64_t lu, int split, double (*red)[8],
+                                          int *last_flag) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const Mat<V> &m = it.m;
+  const V *__restrict__ x = it.x;
+  double acc[K];
+#pragma unroll
+  for (int q = 0; q < K; q++) acc[q] = 0.0;
+  auto reduce = [&](int G) {  // over the lanes of a group
+    for (int o = G >> 1; o > 0; o >>= 1) {
+#pragma unroll
+      for (int q = 0; q < K; q++) acc[q] = add_rn(acc[q], __shfl_xor_sync(FULL, acc[q], o));
+    }
+  };
+  if constexpr (PART == P_CHUNKS) {
+    // ---- one chunk of a long row, whole CTA
+    const int2 rl = it.chunk_rl[lu];
+    const int32_t row = rl.x, len = m.row_sizes[row];
+    const int64_t li = rl.y;
+    const int32_t nch = (len + CHUNK - 1) / CHUNK, chunk = nch == 1 ? 0 : (int32_t)(lu - it.long_off[li]);
+    const Chain ch = load_chain(m, row);
+    const int32_t c0 = chunk * CHUNK, c1 = len - c0 > CHUNK ? c0 + CHUNK : len;
+    accum_row<V, K, VEC>(m, x, it.ldx, ch, c0, c1, threadIdx.x, RS_THREADS_, acc);
+    reduce(32);
+    if (lane == 0)
+#pragma unroll
+      for (int q = 0; q < K; q++) red[w][q] = acc[q];
+    __syncthreads();
+    if (threadIdx.x < K) {  // a thread per right-hand side: warps in order
+      double t = red[0][threadIdx.x];
+      for (int q = 1; q < RS_WARPS; q++) t = add_rn(t, red[q][threadIdx.x]);
+      if (nch == 1) {
+        write_y<V, OP_SPMV>(it.y + (int64_t)row * it.ldy + threadIdx.x, t, it.alpha, it.beta);
+      } else {
+        it.part[(it.long_off[li] + chunk) * K + threadIdx.x] = t;
         __threadfence();
-        double out[KA];
-#pragma unroll
-        for (int k = 0; k < KA; k++) out[k] = op_init<double, OP>();
-        for (int64_t q = 0; q < nch; q++)
-#pragma unroll
-          for (int k = 0; k < KA; k++)
-            out[k] = op_comb<double, OP>(out[k], __ldcg(it.part + (it.long_off[li] + q) * KA + k));
-        write_y<V, K, OP>(it.y, it.ldy, row, out, it.alpha, it.beta, (int32_t)L, kr);
-        it.long_cnt[li] = 0;
       }
+    }
+    if (nch > 1) {
       __syncthreads();
-    } else if constexpr (PART == P_MED) {
-      // ---- one medium row per warp, UN loads in flight per lane
-      const int64_t mi = lu * RS_WARPS + w;
-      if (mi >= it.info[2]) continue;
-      const int32_t row = it.med_rows[mi];
-      const int64_t L = m.row_sizes[row];
-      const Chain ch = load_chain(m, row);
-      double acc[KA];
-#pragma unroll
-      for (int k = 0; k < KA; k++) acc[k] = op_init<double, OP>();
-      constexpr int UN = KArr<K>::N <= 2 ? 8 : 4;
-      int64_t before = 0;
-#pragma unroll
-      for (int l = 0; l < MAX_SEGS; l++) {
-        if (l < ch.ns && before < L) {
-          const int64_t take = (int64_t)ch.cp[l] < L - before ? (int64_t)ch.cp[l] : L - before;
-          const int64_t st = ch.st[l];
-          for (int64_t b0 = 0; b0 < take; b0 += 32 * UN) {
-            V a[UN];
-            int32_t col[UN];
-#pragma unroll
-            for (int i = 0; i < UN; i++) {
-              const int64_t p = b0 + 32 * i + lane;
-              const int64_t q = st + (p < take ? p : 0);
-              a[i] = __ldcs(m.vals + q);
-              col[i] = OP == OP_SPMV ? __ldcs(m.cols + q) : 0;
-            }
-#pragma unroll
-            for (int i = 0; i < UN; i++)
-              if (b0 + 32 * i + lane < take) accum_k<V, K, OP, VEC>((double)a[i], col[i], x, ldx, kr, vec, acc);
-          }
-          before += ch.cp[l];
-        }
+      if (threadIdx.x == 0) *last_flag = atomicAdd(&it.long_cnt[li], 1) == nch - 1;
+      __syncthreads();
+      if (*last_flag && threadIdx.x < K) {  // every chunk's sums are there: in chunk order
+        __threadfence();
+        double t = 0.0;
+        for (int32_t q = 0; q < nch; q++) t = add_rn(t, __ldcg(it.part + (it.long_off[li] + q) * K + threadIdx.x));
+        write_y<V, OP_SPMV>(it.y + (int64_t)row * it.ldy + threadIdx.x, t, it.alpha, it.beta);
+        if (threadIdx.x == 0) it.long_cnt[li] = 0;
       }
+    }
+    __syncthreads();
+  } else if constexpr (PART == P_MED) {
+    // ---- one medium row per warp
+    const int64_t mi = lu * RS_WARPS + w;
+    if (mi >= it.info[2]) return;
+    const int32_t row = it.med_rows[mi], len = m.row_sizes[row];
+    const Chain ch = load_chain_used(m, row, len);
+    accum_row<V, K, VEC>(m, x, it.ldx, ch, 0, len, lane, 32, acc);
+    reduce(32);
+    if (lane == 0) write_rhs<V, K>(it, row, acc);
+  } else {
+    // ---- short rows: a warp takes 32 consecutive rows, G lanes per row
+    const int64_t wu = lu * RS_WARPS + w;
+    const int64_t blk = wu / split;
+    const int sub = (int)(wu - blk * split);
+    if (blk * 32 >= m.n_rows) return;
+    const RowBlock rb = load_block(m, blk * 32, lane, it.short_max);
+    const Chain own = load_chain_used(m, rb.row >= 0 ? rb.row : 0, rb.stream ? rb.len : 0);
+    const int G = group_width(warp_sum(rb.stream ? rb.len : 0));
+    const int per = 32 / G, j = lane & (G - 1), g = lane / G;
+    for (int pass = sub; pass < G; pass += split) {
+      const int owner = pass * per + g;
+      const int32_t row = __shfl_sync(FULL, rb.row, owner);
+      const int32_t len = __shfl_sync(FULL, rb.len, owner);
+      const Chain ch = shfl_chain(own, owner);
 #pragma unroll
-      for (int k = 0; k < KA; k++) {
-        if (K < 0 && k >= kr) break;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[k] = op_comb<double, OP>(acc[k], __shfl_xor_sync(FULL, acc[k], o));
-      }
-      if (lane == 0) write_y<V, K, OP>(it.y, it.ldy, row, acc, it.alpha, it.beta, (int32_t)L, kr);
+      for (int q = 0; q < K; q++) acc[q] = 0.0;
+      if (row >= 0 && len > 0 && len <= it.short_max) accum_row<V, K, VEC>(m, x, it.ldx, ch, 0, len, j, G, acc);
+      reduce(G);
+      if (j == 0 && row >= 0 && len <= it.short_max) write_rhs<V, K>(it, row, acc);
+    }
+  }
+}
+
+// Blocks per SM: three (80 registers) measured fastest for every family; the
+// compiler's own choice (94-158 registers) left two or one: 121 us for 8M
+// entries with k = 8 against 101, four blocks 106.
+#ifndef DCSR_RHS_MINB
+#define DCSR_RHS_MINB 3
+#endif
+template <typename V, int FAM, int PART>
+__device__ __forceinline__ void rows_unit_k(const RowItem<V> &it, int64_t lu, int split, double (*red)[8],
+                                            int *last_flag) {
+  if (it.skip && *it.skip) return;  // a batch matrix whose update was rejected: y untouched
+  if (it.vec) {  // k = 2, 4 or 8
+    rows_unit<V, FAM, true, PART>(it, lu, split, red, last_flag);
+  } else if constexpr (FAM == 2) {
+    rows_unit<V, 2, false, PART>(it, lu, split, red, last_flag);
+  } else if constexpr (FAM == 4) {
+    if (it.k == 3) rows_unit<V, 3, false, PART>(it, lu, split, red, last_flag);
+    else rows_unit<V, 4, false, PART>(it, lu, split, red, last_flag);
+  } else {
+    if (it.k == 5) rows_unit<V, 5, false, PART>(it, lu, split, red, last_flag);
+    else if (it.k == 6) rows_unit<V, 6, false, PART>(it, lu, split, red, last_flag);
+    else if (it.k == 7) rows_unit<V, 7, false, PART>(it, lu, split, red, last_flag);
+    else rows_unit<V, 8, false, PART>(it, lu, split, red, last_flag);
+  }
+}
+
+// All classes in one launch, the long rows' chunks first: a class of few units
+// (the batched matrices have hundreds of medium rows) no longer has the GPU
+// to itself for its tail.
+template <typename V, int FAM, typename Src>
+__global__ void __launch_bounds__(RS_THREADS_, DCSR_RHS_MINB) k_rows_rhs(Src src) {
+  __shared__ double red[RS_WARPS][8];
+  __shared__ int last_flag;
+  const int64_t nc = src.units(P_CHUNKS), nm = src.units(P_MED), total = nc + nm + src.units(P_BLOCKS);
+  for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
+    int64_t lu;
+    if (u < nc) {
+      const RowItem<V> &it = src.item(src.locate(P_CHUNKS, u, lu));
+      rows_unit_k<V, FAM, P_CHUNKS>(it, lu, src.split, red, &last_flag);
+    } else if (u < nc + nm) {
+      const RowItem<V> &it = src.item(src.locate(P_MED, u - nc, lu));
+      rows_unit_k<V, FAM, P_MED>(it, lu, src.split, red, &last_flag);
     } else {
-      // ---- short rows: a warp takes 32 consecutive rows
-      const int S = src.split;  // warps per 32-row block
-      const int64_t wu = lu * RS_WARPS + w;
-      const int64_t blk = wu / S;
-      const int sub = (int)(wu - blk * S);
-      if (blk * 32 >= m.n_rows) continue;
-      {
-        // K values per entry: G lanes per row
-        const RowBlock rb = load_block(m, blk * 32, lane, it.short_max);
-        const Chain own = load_chain_used(m, rb.row >= 0 ? rb.row : 0, rb.stream ? rb.len : 0);
-        const int G = group_width(warp_sum(rb.stream ? rb.len : 0));
-        const int per = 32 / G, j = lane & (G - 1), g = lane / G;
-        for (int pass = sub; pass < G; pass += S) {
-          const int owner = pass * per + g;
-          const int32_t row = __shfl_sync(FULL, rb.row, owner);
-          const int32_t len = __shfl_sync(FULL, rb.len, owner);
-          const Chain ch = shfl_chain(own, owner);
-          double acc[KA];
-#pragma unroll
-          for (int k = 0; k < KA; k++) acc[k] = op_init<double, OP>();
-          if (row >= 0 && len > 0 && len <= it.short_max) {
-            constexpr int UN = KArr<K>::N <= 2 ? 8 : 4;  // entries in flight per lane
-            for_row_entries<UN>(ch, len, j, G, [&](int64_t st, int32_t p0, int32_t take, int32_t) {
-              V a[UN];
-              int32_t col[UN];
-#pragma unroll
-              for (int i = 0; i < UN; i++) {
-                const int32_t p = p0 + i * G;
-                const int64_t q = st + (p < take ? p : 0);
-                a[i] = __ldcs(m.vals + q);
-                col[i] = OP == OP_SPMV ? __ldcs(m.cols + q) : 0;
-              }
-#pragma unroll
-              for (int i = 0; i < UN; i++)
-                if (p0 + i * G < take) accum_k<V, K, OP, VEC>((double)a[i], col[i], x, ldx, kr, vec, acc);
-            });
-          }
-#pragma unroll
-          for (int k = 0; k < KA; k++) {
-            if (K < 0 && k >= kr) break;
-            for (int o = G >> 1; o > 0; o >>= 1) acc[k] = op_comb<double, OP>(acc[k], __shfl_xor_sync(FULL, acc[k], o));
-          }
-          if (j == 0 && row >= 0 && len <= it.short_max) write_y<V, K, OP>(it.y, it.ldy, row, acc, it.alpha, it.beta, len, kr);
-        }
-      }
+      const RowItem<V> &it = src.item(src.locate(P_BLOCKS, u - nc - nm, lu));
+      rows_unit_k<V, FAM, P_BLOCKS>(it, lu, src.split, red, &last_flag);
     }
   }
 }
@@ -844,8 +721,7 @@ __device__ __forceinline__ void flat_tile_rows(const Src &src, FlatTile &x) {
 
 template <typename V, int OP>
 __device__ __forceinline__ void write_row(const RowItem<V> &it, int32_t row, double v) {
-  const double o[1] = {v};
-  write_y<V, 1, OP>(it.y, it.ldy, row, o, it.alpha, it.beta, 1, 1);  // (length 1: not empty)
+  write_y<V, OP>(it.y + (int64_t)row * it.ldy, v, it.alpha, it.beta);
 }
 
 // FP32 matrices of at most this many rows sum exact products; larger ones
@@ -1121,10 +997,7 @@ __global__ void __launch_bounds__(FT_THREADS) k_flat_fix(Src src) {
     if (it.skip && *it.skip) continue;
     const int64_t i = lu * FT_THREADS + threadIdx.x;
     if (!tiles) {
-      if (i < it.m.n_rows && it.off[i] == it.off[i + 1]) {
-        const double z[1] = {op_init<double, OP>()};
-        write_y<V, 1, OP>(it.y, it.ldy, (int32_t)i, z, it.alpha, it.beta, 0, 1);
-      }
+      if (i < it.m.n_rows && it.off[i] == it.off[i + 1]) write_row<V, OP>(it, (int32_t)i, 0.0);  // (max, min: 0 too)
       continue;
     }
     const int64_t nnz = it.off[it.m.n_rows], e1 = (i + 1) * FT_TILE;
@@ -1227,14 +1100,10 @@ static int flat_many_t(const RowItem<V> *its, int count, int64_t R, Arena &ar, c
 
 static int grid_of(const void *k) { return persistent_grid(k, RS_THREADS_, 0); }
 
-template <typename V, int K, int OP, bool VEC, typename Src>
-static int launch_reduce_src(const Src &src, cudaStream_t s) {
-  static const int g0 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_BLOCKS, Src>);
-  static const int g1 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_CHUNKS, Src>);
-  static const int g2 = grid_of((const void *)k_rows_reduce<V, K, OP, VEC, P_MED, Src>);
-  DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_CHUNKS, Src>), g1, RS_THREADS_, 0, s, src);
-  DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_MED, Src>), g2, RS_THREADS_, 0, s, src);
-  DCSR_LAUNCH((k_rows_reduce<V, K, OP, VEC, P_BLOCKS, Src>), g0, RS_THREADS_, 0, s, src);
+template <typename V, int FAM, typename Src>
+static int launch_rhs(const Src &src, cudaStream_t s) {
+  static const int g = grid_of((const void *)k_rows_rhs<V, FAM, Src>);
+  DCSR_LAUNCH((k_rows_rhs<V, FAM, Src>), g, RS_THREADS_, 0, s, src);
   return DCSR_OK;
 }
 
@@ -1282,36 +1151,23 @@ int short_split(int64_t blocks, int k) {
   return S;
 }
 
-template <typename V, int K, int OP, bool VEC>
-static int launch_reduce(dcsr_handle h, const V *x, int64_t ldx, V *y, int64_t ldy, double alpha, double beta,
-                         cudaStream_t s) {
-  RowOne<V> src{row_item<V>(h, x, y, ldx, ldy, alpha, beta)};
-  src.split = OP == OP_SPMV ? short_split(div_up(h->n_rows, 32), K) : 1;
-  return launch_reduce_src<V, K, OP, VEC>(src, s);
-}
-
-template <typename V, int K>
-static int spmv_k(dcsr_handle h, const V *x, int64_t ldx, V *y, int64_t ldy, double alpha, double beta,
-                  cudaStream_t s) {
-  const size_t rb = K * sizeof(V), al = (rb & (0 - rb)) >= 32 ? 32 : (rb & (0 - rb));  // row alignment
-  // packed, aligned rows of x: vector loads
-  const bool vec = (K % 2 == 0) && ldx == K && ((uintptr_t)x % al) == 0;
-  if (vec) return launch_reduce<V, K, OP_SPMV, true>(h, x, ldx, y, ldy, alpha, beta, s);
-  return launch_reduce<V, K, OP_SPMV, false>(h, x, ldx, y, ldy, alpha, beta, s);
+bool rhs_vec(const void *x, int32_t k, int64_t ldx, size_t vsize) {
+  const size_t rb = (size_t)k * vsize, al = rb >= 16 ? 16 : rb;  // a lane's load
+  return (k == 2 || k == 4 || k == 8) && ldx == k && (uintptr_t)x % al == 0;
 }
 
 template <typename V>
 static int spmv_dispatch(dcsr_handle h, const V *x, int32_t k, int64_t ldx, V *y, int64_t ldy, double alpha,
                          double beta, cudaStream_t s) {
-  switch (k) {
-    case 1: return launch_flat<V, OP_SPMV>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 2: return spmv_k<V, 2>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 3: return spmv_k<V, 3>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 4: return spmv_k<V, 4>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 5: return spmv_k<V, 5>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 6: return spmv_k<V, 6>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 7: return spmv_k<V, 7>(h, x, ldx, y, ldy, alpha, beta, s);
-    case 8: return spmv_k<V, 8>(h, x, ldx, y, ldy, alpha, beta, s);
+  if (k == 1) return launch_flat<V, OP_SPMV>(h, x, ldx, y, ldy, alpha, beta, s);
+  RowOne<V> src{row_item<V>(h, x, y, ldx, ldy, alpha, beta)};
+  src.it.k = k;
+  src.it.vec = rhs_vec(x, k, ldx, sizeof(V)) ? 1 : 0;
+  src.split = short_split(div_up(h->n_rows, 32), k);
+  switch (rhs_family(k)) {
+    case 2: return launch_rhs<V, 2>(src, s);
+    case 4: return launch_rhs<V, 4>(src, s);
+    case 8: return launch_rhs<V, 8>(src, s);
   }
   return DCSR_BAD_ARG;
 }
@@ -1337,9 +1193,9 @@ static int spmv_many_t(const RowItem<V> *its, int count, int kf, long long *pref
   RowMany<V> src{its, count, pref, split};
   switch (kf) {
     case 1: return launch_flat_src<V, OP_SPMV, false, sizeof(V) == 4>(src, -1, -1, s);
-    case 2: return launch_reduce_src<V, -2, OP_SPMV, false>(src, s);
-    case 4: return launch_reduce_src<V, -4, OP_SPMV, false>(src, s);
-    case 8: return launch_reduce_src<V, -8, OP_SPMV, false>(src, s);
+    case 2: return launch_rhs<V, 2>(src, s);
+    case 4: return launch_rhs<V, 4>(src, s);
+    case 8: return launch_rhs<V, 8>(src, s);
   }
   return DCSR_BAD_ARG;
 }
@@ -1386,7 +1242,7 @@ int spmv_call(dcsr_handle h, const void *x, int32_t k, int64_t ldx, void *y, int
   if (k == 1) {
     if (!h->flat_valid) DCSR_TRY(build_flat(h, s, ar));
   } else {
-    DCSR_TRY(ensure_part(h, k, s));
+    DCSR_TRY(ensure_part(h, rhs_family(k), s));
     if (!h->bins_valid) DCSR_TRY(build_schedule(h, s, ar));
   }
   if (h->dtype == DCSR_F32)

@@ -1,0 +1,52 @@
+"""SpMV with 2 to 8 right-hand sides over every row class and its edges, with
+packed, strided and misaligned x (the 16-byte loads and the value-by-value
+path), alpha and beta, rows in one and several segments: within 1e-6 (FP32) or
+1e-13 (FP64) of the sum of magnitudes of the FP64 oracle."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import make_pair, spmv_bound
+
+pytestmark = pytest.mark.gpu
+
+LENS = [0, 1, 5, 31, 32, 33, 63, 64, 65, 100, 255, 300, 511, 512, 513, 2047, 2048, 2049, 9000] + [3] * 50 + [40] * 70
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("layout", ["packed", "strided", "misaligned"])
+def test_right_hand_sides(dcsr, k, dtype, layout):
+    rng = np.random.default_rng(k)
+    n, m = len(LENS), 20_000
+    rp = np.concatenate([[0], np.cumsum(LENS)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(m, L, replace=False)) for L in LENS if L]).astype(np.int32)
+    vals = rng.uniform(-1, 1, cols.size)
+    vals = vals.astype(np.float32) if dtype == 0 else vals
+    dev, orc = make_pair(dcsr, n, m, dtype, 0, reloc_min=1 << 20)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals.astype(np.float64)) == 0
+    tol = {0: 1e-6, 1: 1e-13}[dtype]
+    ldx, ldy, off = {"packed": (k, k, 0), "strided": (k + 1, k + 2, 0), "misaligned": (k, k, 1)}[layout]
+    for it in range(2):
+        if it:  # rows in several segments
+            r = np.repeat(np.arange(n), 60).astype(np.int32)
+            c = rng.integers(0, m, r.size).astype(np.int32)
+            v = rng.uniform(-1, 1, r.size)
+            v = v.astype(np.float32) if dtype == 0 else v
+            assert dev.update(r, c, v) == orc.update_auto(r, c, v.astype(np.float64)) == 0
+        xb = torch.tensor(rng.uniform(-1, 1, m * ldx + off), dtype=dev.dtype).cuda()
+        yb = torch.tensor(rng.uniform(-1, 1, n * ldy), dtype=dev.dtype).cuda()
+        x = xb[off:].view(m, ldx)[:, :k].cpu().double().numpy()
+        y0 = yb.view(n, ldy).cpu().double().numpy()
+        bound = spmv_bound(orc, x, k)
+        for alpha, beta in ((1.0, 0.0), (-0.5, 0.25)):
+            y = yb.clone()
+            assert dcsr.lib().dcsr_spmv(dev.h, xb[off:].data_ptr(), k, ldx, y.data_ptr(), ldy, alpha, beta,
+                                        torch.cuda.current_stream().cuda_stream) == 0
+            got = y.view(n, ldy).cpu().double().numpy()
+            ref = orc.spmv(x.reshape(-1).copy(), k=k, alpha=alpha, beta=beta, y=y0[:, :k].reshape(-1).copy())
+            err = np.abs(got[:, :k] - ref.reshape(n, k))
+            lim = tol * (abs(alpha) * bound.reshape(n, k) + abs(beta) * np.abs(y0[:, :k])) + 1e-300
+            assert np.all(err <= lim), f"it {it} alpha {alpha}: {np.max(err / lim):.3g}"
+            np.testing.assert_array_equal(got[:, k:], y0[:, k:])
