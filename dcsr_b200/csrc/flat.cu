@@ -387,10 +387,10 @@ int launch_flat(const FlatCopy<V> &a, int64_t entries, cudaStream_t s) {
   return DCSR_OK;
 }
 
-// Layer 0 = [caps[r], caps[r+1]), other layers cleared, row lengths and tile
-// rows from the row pointer; pool top = caps[n].
+// Layer 0 = [caps[r], caps[r+1]), other layers cleared, row lengths and the
+// flat tables (offsets, tile rows) from the row pointer; pool top = caps[n].
 __global__ void k_layout_rp(int32_t *seg, int32_t *row_sizes, int32_t n, int32_t pitch, int max_segs,
-                            const int32_t *caps, const int32_t *rp, int32_t *tile_row, int64_t tiles) {
+                            const int32_t *caps, const int32_t *rp, int32_t *off, int32_t *tile_row, int64_t tiles) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x; r0 <= n; r0 += stride) {
     const int64_t r = r0 + threadIdx.x;
@@ -402,8 +402,11 @@ __global__ void k_layout_rp(int32_t *seg, int32_t *row_sizes, int32_t n, int32_t
       o = rp[r];
       len = rp[r + 1] - o;
       row_sizes[r] = len;
+      off[r] = o;
+      if (r == n - 1) off[n] = o + len;
     } else if (r == n) {
       row_sizes[n] = caps[n];
+      if (n == 0) off[0] = 0;
     }
     flat_mark_tiles((int32_t)r, o, len, tile_row, tiles);
   }
@@ -511,25 +514,24 @@ int counts_scan(dcsr_handle h, const int32_t *cnt, int32_t *rp, int32_t *caps, A
 }
 
 int place_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const int32_t *cols, const void *vals,
-              int64_t nnz, int32_t *tile_row, cudaStream_t s) {
+              int64_t nnz, cudaStream_t s) {
   DCSR_LAUNCH(k_layout_rp, grid_for((int64_t)h->n_rows + 1, 256), 256, 0, s, h->seg, h->row_sizes, h->n_rows, h->pitch,
-              h->o.max_segs, caps, rp, tile_row, flat_tiles(nnz));
-  if (h->dtype == DCSR_F32) return load_t<float>(h, rp, tile_row, caps, cols, (const float *)vals, nnz, s);
-  return load_t<double>(h, rp, tile_row, caps, cols, (const double *)vals, nnz, s);
+              h->o.max_segs, caps, rp, h->flat_off, h->flat_tile, h->flat_tiles);
+  if (h->dtype == DCSR_F32) return load_t<float>(h, h->flat_off, h->flat_tile, caps, cols, (const float *)vals, nnz, s);
+  return load_t<double>(h, h->flat_off, h->flat_tile, caps, cols, (const double *)vals, nnz, s);
 }
 
-int place_rows_scan(dcsr_handle h, const long long *lens, int32_t *off, int32_t *caps, int32_t *tile_row,
-                    int64_t bound, Arena &ar, cudaStream_t s) {
-  const PlaceScan f{lens, h->n_rows, h->o,     off,         tile_row,          caps, h->row_sizes,
-                    h->seg, h->pitch, h->o.max_segs, flat_tiles(bound), h->stat + ST_TOTAL};
+int place_rows_scan(dcsr_handle h, const long long *lens, int32_t *caps, Arena &ar, cudaStream_t s) {
+  const PlaceScan f{lens,   h->n_rows, h->o,          h->flat_off,   h->flat_tile,      caps, h->row_sizes,
+                    h->seg, h->pitch,  h->o.max_segs, h->flat_tiles, h->stat + ST_TOTAL};
   return scan_map(f, h->n_rows > 0 ? h->n_rows : 1, ar, s);
 }
 
-int place_rows_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, const int32_t *tile_row,
-                    const long long *src_off, const int32_t *scols, const void *svals, int64_t bound, cudaStream_t s) {
+int place_rows_copy(dcsr_handle h, const int32_t *caps, const long long *src_off, const int32_t *scols,
+                    const void *svals, int64_t bound, cudaStream_t s) {
   if (h->dtype == DCSR_F32)
-    return place_t<float>(h, off, tile_row, caps, src_off, scols, (const float *)svals, bound, s);
-  return place_t<double>(h, off, tile_row, caps, src_off, scols, (const double *)svals, bound, s);
+    return place_t<float>(h, h->flat_off, h->flat_tile, caps, src_off, scols, (const float *)svals, bound, s);
+  return place_t<double>(h, h->flat_off, h->flat_tile, caps, src_off, scols, (const double *)svals, bound, s);
 }
 
 int compact_scan(dcsr_handle h, int32_t *off, int32_t *caps, int32_t *tile_row, Arena &ar, cudaStream_t s) {

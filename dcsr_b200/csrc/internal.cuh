@@ -13,17 +13,17 @@ namespace dcsr {
 // ST_TOTAL word.
 int caps_scan(dcsr_handle h, const int32_t *rp, int32_t *caps, Arena &ar, cudaStream_t s);
 int counts_scan(dcsr_handle h, const int32_t *cnt, int32_t *rp, int32_t *caps, Arena &ar, cudaStream_t s);
-// The CSR's rows become the matrix's content: layout (layer 0 from caps) and
-// entries into the handle's pool; nnz bounds the entries, tile_row holds
-// flat_tiles(nnz) words of scratch.
+// The CSR's rows become the matrix's content: layout (layer 0 from caps), flat
+// tables (ensure_flat first) and entries into the handle's pool; nnz bounds
+// the entries.
 int place_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const int32_t *cols, const void *vals,
-              int64_t nnz, int32_t *tile_row, cudaStream_t s);
+              int64_t nnz, cudaStream_t s);
 // Staged rows (row r: lens[r] entries from src_off[r]) likewise: the layout
-// with its offsets, then the entries; bound bounds their number.
-int place_rows_scan(dcsr_handle h, const long long *lens, int32_t *off, int32_t *caps, int32_t *tile_row,
-                    int64_t bound, Arena &ar, cudaStream_t s);
-int place_rows_copy(dcsr_handle h, const int32_t *off, const int32_t *caps, const int32_t *tile_row,
-                    const long long *src_off, const int32_t *scols, const void *svals, int64_t bound, cudaStream_t s);
+// and tables with the capacities' offsets, then the entries; bound bounds
+// their number.
+int place_rows_scan(dcsr_handle h, const long long *lens, int32_t *caps, Arena &ar, cudaStream_t s);
+int place_rows_copy(dcsr_handle h, const int32_t *caps, const long long *src_off, const int32_t *scols,
+                    const void *svals, int64_t bound, cudaStream_t s);
 // Compaction: the offsets of the current content and of its policy
 // capacities (sum to ST_TOTAL), then the entries into the new pool (cap
 // entries) and the new layout.  tile_row: flat_tiles(pool_cap) words.
@@ -119,8 +119,9 @@ bool rhs_vec(const void *x, int32_t k, int64_t ldx, size_t vsize);
 // Warps per 32-row short-row block for an SpMV pass over `blocks` blocks with k RHS.
 int short_split(int64_t blocks, int k);
 // Flat tables of a handle (row offsets, tile rows, tile partials): sized for
-// its pool; built from its row lengths when they are not valid.
-int ensure_flat(dcsr_handle h, cudaStream_t s);
+// its pool (or for `entries`); built from its row lengths when they are not
+// valid.
+int ensure_flat(dcsr_handle h, cudaStream_t s, int64_t entries = 0);
 int build_flat(dcsr_handle h, cudaStream_t s, Arena *ar = nullptr);
 // Of `count` matrices at once (items: device RowItem<V>[count], row0 = their
 // first rows in a common row space of R rows).  Needs flat_scratch_bytes(R)

@@ -184,8 +184,8 @@ static void free_pool(dcsr_handle h, cudaStream_t s) {
 static int clear_status(dcsr_handle h, cudaStream_t s);
 static int read_stat(dcsr_handle h, cudaStream_t s, long long *host);
 
-static size_t load_scratch_bytes(dcsr_handle h, int64_t nnz) {
-  return arena_bytes(h->n_rows + 2, 4) + arena_bytes(flat_tiles(nnz) + 1, 4) + scan_scratch_bytes(h->n_rows + 1);
+static size_t load_scratch_bytes(dcsr_handle h) {
+  return arena_bytes(h->n_rows + 2, 4) + scan_scratch_bytes(h->n_rows + 1);
 }
 
 // The end of a CSR or COO load, after the host has read the status words
@@ -197,8 +197,6 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   if (top > 0x7fffffffLL) return DCSR_OOM;
   int64_t cap = pool_capacity(h->o, top);
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
-  int32_t *tile_row = h->scratch.take<int32_t>(flat_tiles(nnz) + 1);
-  if (h->scratch.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   int32_t *nc;
   void *nv;
   int64_t got;
@@ -208,8 +206,10 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   h->vals = nv;
   h->buf_cap = got;
   h->pool_cap = cap;
-  DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, tile_row, s));
   h->bins_valid = h->flat_valid = false;
+  DCSR_TRY(ensure_flat(h, s));
+  DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, s));
+  h->flat_valid = true;  // the load knows the offsets: the export and the row passes find them
   // A load is a one-off: a resident matrix keeps no load-sized scratch (the
   // stream-ordered pool keeps the memory for the next allocation).
   h->scratch.release(s);
@@ -227,9 +227,8 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   const int32_t n = h->n_rows;
   Arena &ar = h->scratch;
   ar.status = h->stat + ST_STATUS;
-  DCSR_TRY(ar.reserve(2 * arena_bytes(n + 2, 4) + arena_bytes(flat_tiles(bound) + 1, 4) + scan_scratch_bytes(n + 1), s));
-  int32_t *off = ar.take<int32_t>(n + 2), *caps = ar.take<int32_t>(n + 2);
-  int32_t *tile_row = ar.take<int32_t>(flat_tiles(bound) + 1);
+  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 4) + scan_scratch_bytes(n + 1), s));
+  int32_t *caps = ar.take<int32_t>(n + 2);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   if (cap_bound > 0x7fffffffLL) return DCSR_OOM;
   int32_t *nc;
@@ -240,12 +239,13 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   h->cols = nc;
   h->vals = nv;
   h->buf_cap = got;
-  DCSR_TRY(place_rows_scan(h, lens, off, caps, tile_row, bound, ar, s));
-  DCSR_TRY(place_rows_copy(h, off, caps, tile_row, src_off, scols, svals, bound, s));
+  h->bins_valid = h->flat_valid = false;
+  DCSR_TRY(ensure_flat(h, s, bound));
+  DCSR_TRY(place_rows_scan(h, lens, caps, ar, s));
+  DCSR_TRY(place_rows_copy(h, caps, src_off, scols, svals, bound, s));
   long long host[ST_WORDS];
   DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
-  h->bins_valid = h->flat_valid = false;
   h->scratch.release(s);
   if (host[ST_STATUS] == DCSR_TIMEOUT) {
     DCSR_TRY(clear_status(h, s));
@@ -255,6 +255,7 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
   if (cap > got) return DCSR_OOM;  // the caller's bound was not one (a bug)
   h->pool_cap = cap;
+  h->flat_valid = true;
   return DCSR_OK;
 }
 
@@ -492,7 +493,7 @@ int dcsr_from_csr(dcsr_handle h, const int32_t *row_ptr, const int32_t *cols, co
   if (n == 0 && nnz != 0) return DCSR_BAD_ARG;
   Arena &ar = h->scratch;
   ar.status = h->stat + ST_STATUS;
-  DCSR_TRY(ar.reserve(load_scratch_bytes(h, nnz), s));
+  DCSR_TRY(ar.reserve(load_scratch_bytes(h), s));
   int32_t *caps = ar.take<int32_t>(n + 2);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   // the check and the capacities' scan together, then one read of both
@@ -530,7 +531,7 @@ int dcsr_from_coo(dcsr_handle h, const int32_t *rows, const int32_t *cols, const
   cudaStream_t s = (cudaStream_t)stream;
   Arena &ar = h->scratch;
   ar.status = h->stat + ST_STATUS;
-  DCSR_TRY(ar.reserve(coo_to_csr_scratch(h, nnz) + load_scratch_bytes(h, nnz), s));
+  DCSR_TRY(ar.reserve(coo_to_csr_scratch(h, nnz) + load_scratch_bytes(h), s));
   DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX, 0, sizeof(long long), s));
   int32_t *rp, *caps, *cc;
   void *cv;

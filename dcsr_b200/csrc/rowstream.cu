@@ -288,8 +288,8 @@ int build_schedule(dcsr_handle h, cudaStream_t s, Arena *ar) {
 
 // Flat tables: offsets, tile rows and tile partials of a matrix (one scan of
 // its row lengths), sized for its pool.
-int ensure_flat(dcsr_handle h, cudaStream_t s) {
-  const int64_t need = flat_tiles(h->pool_cap) + 1;
+int ensure_flat(dcsr_handle h, cudaStream_t s, int64_t entries) {
+  const int64_t need = flat_tiles(std::max(h->pool_cap, entries)) + 1;
   if (h->flat_off && need <= h->flat_tiles) return DCSR_OK;
   if (!h->flat_off) DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_off, sizeof(int32_t) * ((size_t)h->n_rows + 2), s));
   if (h->flat_tile) DCSR_CUDA(dcsr::dev_free(h->flat_tile, s));
