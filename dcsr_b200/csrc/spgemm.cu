@@ -1,17 +1,23 @@
 // spgemm.cu -- C = A*B for DCSR matrices (expand - sort - reduce).
 //
-// 1. count   products per row P_i = sum_{k in A_i} |B_k| and a size class
+// 1. count   products per row P_i = sum_{k in A_i} |B_k|, rows per size class
 //            (reference CalcSortSizes_SPMM / SetBins_SPMM include/spmm.inl:951-1061)
-// 2. bucket  rows by class (one radix pass), scan P_i -> per-row staging offsets
+// 2. stage   one scan: per-row staging offsets, C's pool bound
 // 3. numeric per row: expand products a_ik*b_kj tagged with their product
 //            index p, sort by (column, p), sum equal columns left to right,
 //            write unique columns to the staging area:
-//              P_i <= 256   warp per row, bitonic sort in shared memory
+//              P_i <= 256   warp per row, bitonic sort in registers
+//              P_i <= 1024  the same, 16 or 32 keys a lane, where column and p
+//                           fit 32 bits (columns of up to 22 bits)
 //              P_i <= 4096  CTA per row, bitonic sort in shared memory
 //              P_i >  4096  all such rows together: global stable radix sort
 //                           of (row, column) keys (no row is skipped; the
 //                           reference left rows > 2048 products uncomputed,
 //                           include/spmm.h:368-389)
+//            The warp classes take the rows in row order and pass over those
+//            of other classes; the upper two have lists, built only where
+//            there are such rows (a sort of all rows by class and its
+//            searches cost 42 us of a product of 131072 rows).
 // 4. layout  C's rows placed straight from the staging area into C's pool
 //            with C's slack policy; the pool is allocated at an upper bound
 //            (the policy capacity of P_i per row) so nothing waits for the
@@ -23,22 +29,33 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "lookback.cuh"
 
 namespace dcsr {
 
 constexpr int SG_THREADS = 256;
 constexpr int SG_WARP_MAX = 256;   // products per warp-row
+constexpr int SG_WARP4_MAX = 1024; // products per warp-row of the class above (columns of up to 22 bits)
 constexpr int SG_CTA_MAX = 4096;   // products per CTA-row
-enum { SG_EMPTY = 0, SG_WARP = 1, SG_CTA = 2, SG_GLOBAL = 3 };
+enum { SG_EMPTY = 0, SG_WARP = 1, SG_WARP4 = 2, SG_CTA = 3, SG_GLOBAL = 4, SG_CLASSES = 5 };
+// Result words: the rows of each class, then
+enum { SG_R_GPROD = SG_CLASSES, SG_R_PROD, SG_R_CAPS, SG_R_STATUS, SG_R_NEXT, SG_R_NEXT4, SG_R_WORDS = 16 };
 
-// Per row: its product count P_i, its size class, and the capacity C's
-// layout policy gives a row of P_i entries (an upper bound of the row's
-// capacity, whatever its unique columns); the products of the rows of the
-// global class are added up in *gtotal.
+__host__ __device__ __forceinline__ int sg_class(int64_t p, int warp_max) {
+  return p == 0 ? SG_EMPTY : p <= SG_WARP_MAX ? SG_WARP : p <= warp_max ? SG_WARP4 : p <= SG_CTA_MAX ? SG_CTA : SG_GLOBAL;
+}
+
+// Per row its product count P_i; per class the number of rows, and the
+// products of the global class's.
 template <typename V>
-__global__ void k_sg_count(Mat<V> A, Mat<V> B, dcsr_opts co, long long *cnt, long long *capub,
-                           unsigned long long *cls, unsigned *rows, unsigned long long *gtotal) {
+__global__ void __launch_bounds__(SG_THREADS) k_sg_count(Mat<V> A, Mat<V> B, int warp_max, long long *cnt,
+                                                         long long *res) {
   constexpr int G = 8;  // lanes per row: a warp has four rows' loads in flight
+  __shared__ unsigned rows[SG_CLASSES];
+  __shared__ unsigned long long gprod;
+  if (threadIdx.x < SG_CLASSES) rows[threadIdx.x] = 0;
+  if (threadIdx.x == 0) gprod = 0;
+  __syncthreads();
   const int lane = threadIdx.x & 31, j = lane & (G - 1);
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t i0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 / G); i0 < A.n_rows;
@@ -54,82 +71,92 @@ __global__ void k_sg_count(Mat<V> A, Mat<V> B, dcsr_opts co, long long *cnt, lon
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
     if (j == 0 && i < A.n_rows) {
       cnt[i] = s;
-      capub[i] = policy_cap(co, s);
-      const int c = s == 0 ? SG_EMPTY : s <= SG_WARP_MAX ? SG_WARP : s <= SG_CTA_MAX ? SG_CTA : SG_GLOBAL;
-      cls[i] = c;
-      rows[i] = (unsigned)i;
-      if (c == SG_GLOBAL) atomicAdd(gtotal, (unsigned long long)s);
+      const int c = sg_class(s, warp_max);
+      atomicAdd(&rows[c], 1u);
+      if (c == SG_GLOBAL) atomicAdd(&gprod, (unsigned long long)s);
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    cnt[A.n_rows] = 0;
-    capub[A.n_rows] = 0;
-  }
+  __syncthreads();
+  if (threadIdx.x < SG_CLASSES && rows[threadIdx.x])
+    atomicAdd((unsigned long long *)&res[threadIdx.x], (unsigned long long)rows[threadIdx.x]);
+  if (threadIdx.x == 0 && gprod) atomicAdd((unsigned long long *)&res[SG_R_GPROD], gprod);
 }
 
-// class starts [0..4] from the sorted class keys
-__global__ void k_sg_classes(const unsigned long long *keys, int32_t n, long long *starts) {
-  const int c = threadIdx.x;
-  if (c <= 4) {
-    int64_t lo = 0, hi = n;
-    while (lo < hi) {
-      int64_t mid = (lo + hi) >> 1;
-      if (keys[mid] < (unsigned long long)c) lo = mid + 1;
-      else hi = mid;
+// Staging offsets ub (n + 1) from the product counts, and the capacities that
+// C's layout policy gives rows of P_i entries added up (an upper bound of the
+// pool, whatever the rows' unique columns); no unique columns yet.
+struct StageScan {
+  static constexpr int NS = 2, IT = SM_LIGHT;
+  using T = long long;
+  struct State {};
+  const long long *cnt;
+  dcsr_opts o;
+  long long *ub, *ucnt, *res;
+  int32_t n;
+  __device__ __forceinline__ void load(int64_t i, bool ok, State &, T (&v)[2]) const {
+    v[0] = ok ? cnt[i] : 0;
+    v[1] = ok ? policy_cap(o, v[0]) : 0;
+  }
+  __device__ __forceinline__ void emit(int64_t i, bool ok, const State &, const long long (&p)[2],
+                                       const T (&)[2]) const {
+    if (ok) {
+      ub[i] = p[0];
+      ucnt[i] = 0;
     }
-    starts[c] = c == 4 ? n : lo;
   }
-}
-
-// Expand row i's products into (key = col<<32 | p, prod[p]) over `nthr`
-// cooperating threads (tid in [0, nthr)); returns the product count.
-template <typename V>
-__device__ __forceinline__ int64_t sg_expand(const Mat<V> &A, const Mat<V> &B, int64_t i, int tid, int nthr,
-                                             unsigned long long *key, V *prod) {
-  const Chain ca = load_chain(A, (int32_t)i);
-  const int64_t LA = A.row_sizes[i];
-  int64_t pos = 0;
-  for (int64_t e = 0; e < LA; e++) {
-    const int64_t qa = ca.phys(e);
-    const int32_t k = A.cols[qa];
-    const V a = A.vals[qa];
-    const Chain cb = load_chain(B, k);
-    const int64_t LB = B.row_sizes[k];
-    for (int64_t j = tid; j < LB; j += nthr) {
-      const int64_t qb = cb.phys(j);
-      key[pos + j] = ((unsigned long long)(uint32_t)B.cols[qb] << 32) | (unsigned long long)(pos + j);
-      V pr;
-      if constexpr (sizeof(V) == 4) pr = __fmul_rn(a, B.vals[qb]);
-      else pr = __dmul_rn(a, B.vals[qb]);
-      prod[pos + j] = pr;
-    }
-    pos += LB;
+  __device__ __forceinline__ void total(const long long (&t)[2]) const {
+    ub[n] = t[0];
+    res[SG_R_PROD] = t[0];
+    res[SG_R_CAPS] = t[1];
   }
-  return pos;
-}
+};
 
-// Sort keys of the warp class: (column, product index p < 256) packed into
-// 32 bits when columns fit in 24 bits, else into 64.
-template <typename K>
+// The rows of the CTA class and of the global class, in row order.
+struct ListScan {
+  static constexpr int NS = 2, IT = SM_LIGHT;
+  using T = long long;
+  struct State {};
+  const long long *ub;
+  int warp_max;
+  unsigned *cta, *global;
+  __device__ __forceinline__ void load(int64_t i, bool ok, State &, T (&v)[2]) const {
+    const int c = ok ? sg_class(ub[i + 1] - ub[i], warp_max) : SG_EMPTY;
+    v[0] = c == SG_CTA;
+    v[1] = c == SG_GLOBAL;
+  }
+  __device__ __forceinline__ void emit(int64_t i, bool, const State &, const long long (&p)[2],
+                                       const T (&v)[2]) const {
+    if (v[0]) cta[p[0]] = (unsigned)i;
+    if (v[1]) global[p[1]] = (unsigned)i;
+  }
+  __device__ __forceinline__ void total(const long long (&)[2]) const {}
+};
+
+// Sort keys of the warp classes: (column, product index p < MAXP) packed into
+// 32 bits when the column bits and p's fit, else (256 products) into 64.
+template <typename K, int MAXP>
 struct SgKey {
-  static constexpr int S = sizeof(K) == 4 ? 8 : 32;
+  static constexpr int S = sizeof(K) == 8 ? 32 : MAXP == 256 ? 8 : 10;
+  static_assert((1 << (S < 31 ? S : 30)) >= MAXP, "p fits below the column");
   __device__ __forceinline__ static K make(int32_t col, int p) { return ((K)(uint32_t)col << S) | (K)p; }
   __device__ __forceinline__ static int32_t col(K k) { return (int32_t)(k >> S); }
   __device__ __forceinline__ static uint32_t idx(K k) { return (uint32_t)(k & ((K(1) << S) - 1)); }
 };
 
-// The warp class's expand (P_i <= 256): row i's A entries are taken 32 at
+// The warp classes' expand (P_i <= MAXP): row i's A entries are taken 32 at
 // a time, one per lane, each lane loading its entry's column k and value,
 // then B row k's length and segments, side by side (no load waits on another
 // entry's); the B-row lengths are scanned into product offsets, and lane l
-// produces products q = l, l + 32, ... of the group: the entry owning q is
-// found by a binary search over the lanes' offsets, and all B loads of the
-// group are issued before the first is used.  Same keys and products as
-// sg_expand (product p = the row's p-th product in A-entry-major order).
-template <typename V, typename K>
+// produces products q = l, l + 32, ... of the group.  The entry owning q: when
+// no B row of the group is empty, the starts within 32 products are a bit mask
+// (one warp OR) and the owner is the number of starts up to q, minus one (6
+// instructions against 20 of a search); else a binary search over the lanes'
+// offsets.  H x 32 products' B loads are issued before the first is used.
+// Product p = the row's p-th product in A-entry-major order.
+template <typename V, typename K, int MAXP>
 __device__ __forceinline__ int sg_expand_warp(const Mat<V> &A, const Mat<V> &B, int64_t i, int lane, K *key,
                                               V *prod) {
-  constexpr int H = 4;
+  constexpr int H = MAXP == SG_WARP_MAX ? 2 : 4;
   const int32_t LA = A.row_sizes[i];
   const Chain ca = load_chain_used(A, (int32_t)i, LA);
   int base = 0;
@@ -145,9 +172,11 @@ __device__ __forceinline__ int sg_expand_warp(const Mat<V> &A, const Mat<V> &B, 
     }
     const Chain cb = load_chain_used(B, kb, lb);
     const bool flat = __all_sync(FULL, cb.ns <= 1);  // every B row in its first segment (the common case)
+    const bool dense = __all_sync(FULL, lane >= nE || lb > 0);  // no empty B row among the entries
     const int incl = warp_incl_scan(lb);
     const int pos = incl - lb;
-    const int tot = __shfl_sync(FULL, incl, 31);  // base + tot <= P_i <= SG_WARP_MAX
+    const int tot = __shfl_sync(FULL, incl, 31);  // base + tot <= P_i <= MAXP
+    int started = 0;  // entries that start before the current 32 products (dense)
     // products in groups of H per lane: every B load of a group in flight at once
     for (int t0 = 0; t0 * 32 < tot; t0 += H) {
       int own[H];
@@ -161,11 +190,18 @@ __device__ __forceinline__ int sg_expand_warp(const Mat<V> &A, const Mat<V> &B, 
         bv[h] = V(0);
         if ((t0 + h) * 32 < tot) {  // warp-uniform
           int lo = 0;  // the last entry (< nE) whose offset is <= q: it owns q
+          if (dense) {
+            const unsigned sm =
+                __reduce_or_sync(FULL, lane < nE && (pos >> 5) == t0 + h ? 1u << (pos & 31) : 0u);
+            lo = started + __popc(sm & (0xffffffffu >> (31 - lane))) - 1;  // product 0 is a start: lo >= 0
+            started += __popc(sm);
+          } else {
 #pragma unroll
-          for (int st = 16; st > 0; st >>= 1) {
-            const int c = lo + st;  // <= 31
-            const int pc = __shfl_sync(FULL, pos, c);
-            if (c < nE && pc <= q) lo = c;
+            for (int st = 16; st > 0; st >>= 1) {
+              const int c = lo + st;  // <= 31
+              const int pc = __shfl_sync(FULL, pos, c);
+              if (c < nE && pc <= q) lo = c;
+            }
           }
           own[h] = lo;
           const int pj = __shfl_sync(FULL, pos, lo);
@@ -188,7 +224,7 @@ __device__ __forceinline__ int sg_expand_warp(const Mat<V> &A, const Mat<V> &B, 
         if ((t0 + h) * 32 < tot) {
           const V ao = __shfl_sync(FULL, a, own[h]);
           if (q < tot) {
-            key[base + q] = SgKey<K>::make(bc[h], base + q);
+            key[base + q] = SgKey<K, MAXP>::make(bc[h], base + q);
             V pr;
             if constexpr (sizeof(V) == 4) pr = __fmul_rn(ao, bv[h]);
             else pr = __dmul_rn(ao, bv[h]);
@@ -228,36 +264,52 @@ __device__ __forceinline__ void bitonic(K *key, int n2, int tid, int nthr, Sync 
 }
 
 // Bitonic sort of the 32*E keys held by a warp, E per lane: key i = lane*E + t
-// in v[t].  Steps with partner distance j < E swap within a lane's
-// registers, the others exchange with lane ^ (j / E) by shuffle; nothing
-// goes through shared memory.
+// in v[t].  The network whose comparators all ascend: a merge of two sorted
+// halves starts with the mirror image (i against i ^ (k - 1)), so no step
+// needs the direction of its block.  Steps with both keys in a lane are a min
+// and a max of registers; the others take the partner's key by shuffle and
+// one select (the lower lane keeps the smaller key).  Nothing goes through
+// shared memory.
 template <int E, typename K>
 __device__ __forceinline__ void warp_bitonic(K (&v)[E], int lane) {
   constexpr int N = 32 * E;
 #pragma unroll
   for (int k = 2; k <= N; k <<= 1) {
+    if (k <= E) {
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = 0; t < E; t++) {
+        const int q = t ^ (k - 1);
+        if (q > t) {
+          const K a = v[t], b = v[q];
+          v[t] = a < b ? a : b;
+          v[q] = a < b ? b : a;
+        }
+      }
+    } else {
+      const bool low = (lane & (k / E / 2)) == 0;
+      K o[E];
+#pragma unroll
+      for (int t = 0; t < E; t++) o[t] = __shfl_xor_sync(FULL, v[E - 1 - t], k / E - 1);
+#pragma unroll
+      for (int t = 0; t < E; t++) v[t] = (o[t] < v[t]) == low ? o[t] : v[t];
+    }
+#pragma unroll
+    for (int j = k >> 2; j > 0; j >>= 1) {
       if (j >= E) {
+        const bool low = (lane & (j / E)) == 0;
 #pragma unroll
         for (int t = 0; t < E; t++) {
-          const int i = lane * E + t;
           const K o = __shfl_xor_sync(FULL, v[t], j / E);
-          // the lower index of a pair keeps the smaller key in an ascending
-          // block (i & k == 0) and the larger in a descending one
-          const bool keep_min = ((i & k) == 0) == ((i & j) == 0);
-          v[t] = keep_min ? (o < v[t] ? o : v[t]) : (o > v[t] ? o : v[t]);
+          v[t] = (o < v[t]) == low ? o : v[t];
         }
       } else {
 #pragma unroll
         for (int t = 0; t < E; t++) {
           const int q = t ^ j;
           if (q > t) {
-            const bool up = ((lane * E + t) & k) == 0;
             const K a = v[t], b = v[q];
-            const bool sw = up ? (a > b) : (a < b);
-            v[t] = sw ? b : a;
-            v[q] = sw ? a : b;
+            v[t] = a < b ? a : b;
+            v[q] = a < b ? b : a;
           }
         }
       }
@@ -265,64 +317,114 @@ __device__ __forceinline__ void warp_bitonic(K (&v)[E], int lane) {
   }
 }
 
-// A warp-row's P keys (in key[0, P), P <= 32*E) sorted in place through
-// registers; slots past P take the largest key and end up past P.
+// Where sorted key i lies in shared memory: one word of padding per 32, so
+// that lanes writing their E consecutive keys hit different banks.
+__device__ __forceinline__ int sg_slot(int i) { return i + (i >> 5); }
+
+// A warp-row's P keys (in key[0, P), P <= 32*E) sorted through registers into
+// key[sg_slot(i)]; slots past P take the largest key and end up past P.
 template <int E, typename K>
 __device__ __forceinline__ void sort_row_keys(K *key, int P, int lane) {
   K v[E];
 #pragma unroll
-  for (int t = 0; t < E; t++) v[t] = lane * E + t < P ? key[lane * E + t] : ~K(0);
+  for (int t = 0; t < E; t++) v[t] = t * 32 + lane < P ? key[t * 32 + lane] : ~K(0);
   warp_bitonic<E>(v, lane);
+  __syncwarp();  // every key read before the first is overwritten
 #pragma unroll
-  for (int t = 0; t < E; t++) key[lane * E + t] = v[t];
+  for (int t = 0; t < E; t++) key[sg_slot(lane * E + t)] = v[t];
 }
 
-// Warp per row, P_i <= 256.
-template <typename V, typename K>
-__global__ void __launch_bounds__(SG_THREADS, 3) k_sg_warp(Mat<V> A, Mat<V> B, const unsigned *rows,
-                                                        const long long *starts, const long long *ub, int32_t *tcol,
-                                                        V *tval, long long *ucnt) {
-  using KO = SgKey<K>;
-  __shared__ K skey[SG_THREADS / 32][SG_WARP_MAX];
-  __shared__ V sprod[SG_THREADS / 32][SG_WARP_MAX];
+// A warp's keys and products in shared memory.
+template <typename V, typename K, int MAXP>
+struct SgWarp {
+  V prod[MAXP];
+  K key[MAXP + MAXP / 32];
+};
+
+// Warp per row: P_i <= 256 (CLS SG_WARP), 256 < P_i <= 1024 (CLS SG_WARP4).
+// Instruction issue bounds it (57% of the slots, DRAM 11%): expand, sort and
+// emit take about 1700 instructions of a 169-product row, 6900 of an
+// 841-product one, so what counts is few instructions and many warps --
+// 6 blocks of 256 threads per SM in the lower class (a few spilled registers
+// included; 3: 333 us, 4: 297 us of the kernel at 131072 rows of 169 FP64
+// products), 2 x 32 products' loads at a time (4: 6% slower, 8: 10%).  Rows of
+// 841 FP32 products in a CTA each, sorted as 64-bit keys in shared memory, took
+// 1022 us for 20011 rows; in a warp each, 32 keys a lane, 220 us.  Rows come
+// from a counter: a stride over the rows would give some warps only long rows
+// where lengths repeat with its period.
+template <typename V, typename K, int CLS>
+__global__ void __launch_bounds__(SG_THREADS, CLS == SG_WARP ? (sizeof(K) == 4 ? 6 : 4) : sizeof(V) == 4 ? 3 : 2)
+    k_sg_warp(Mat<V> A, Mat<V> B, const long long *ub, int warp_max, int G, unsigned long long *next, int32_t *tcol,
+              V *tval, long long *ucnt) {
+  constexpr int MAXP = CLS == SG_WARP ? SG_WARP_MAX : SG_WARP4_MAX;
+  using KO = SgKey<K, MAXP>;
+  extern __shared__ unsigned long long sg_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t b = starts[SG_WARP], e = starts[SG_WARP + 1];
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  SgWarp<V, K, MAXP> &sh = reinterpret_cast<SgWarp<V, K, MAXP> *>(sg_smem)[w];
   const unsigned lt = (1u << lane) - 1u;
-  K *key = skey[w];
-  V *prod = sprod[w];
-  for (int64_t it = b + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); it < e; it += nw) {
-    const int64_t i = rows[it];
-    const int P = sg_expand_warp(A, B, i, lane, key, prod);
-    __syncwarp();
-    if (P <= 32) sort_row_keys<1>(key, P, lane);
-    else if (P <= 64) sort_row_keys<2>(key, P, lane);
-    else if (P <= 128) sort_row_keys<4>(key, P, lane);
-    else sort_row_keys<8>(key, P, lane);
-    __syncwarp();
-    const int64_t base = ub[i];
-    int heads = 0;
-    for (int c0 = 0; c0 < P; c0 += 32) {
-      const int idx = c0 + lane;
-      const bool valid = idx < P;
-      const K k = valid ? key[idx] : K(0);
-      const bool head = valid && (idx == 0 || KO::col(key[idx - 1]) != KO::col(k));
-      const unsigned hm = __ballot_sync(FULL, head);
-      if (head) {
-        V v = prod[KO::idx(k)];
-        for (int j = idx + 1; j < P && KO::col(key[j]) == KO::col(k); j++) v = v + prod[KO::idx(key[j])];
-        const int64_t o = base + heads + __popc(hm & lt);
-        tcol[o] = KO::col(k);
-        tval[o] = v;
+  K *key = sh.key;
+  V *prod = sh.prod;
+  // rows in row order, G <= 32 at a time from one counter; the next G are asked
+  // for before these are worked on
+    unsigned long long r0 = 0;
+  if (lane == 0) r0 = atomicAdd(next, (unsigned long long)G);
+  r0 = __shfl_sync(FULL, r0, 0);
+  while (r0 < (unsigned long long)A.n_rows) {
+    const int64_t g0 = (int64_t)r0;
+    unsigned long long r1 = 0;
+    if (lane == 0) r1 = atomicAdd(next, (unsigned long long)G);
+    const bool mine = lane < G && g0 + lane < A.n_rows;
+    const long long u = mine ? ub[g0 + lane] : 0, u1 = mine ? ub[g0 + lane + 1] : 0;
+    unsigned todo = __ballot_sync(FULL, sg_class(u1 - u, warp_max) == CLS);
+    for (; todo; todo &= todo - 1) {
+      const int at = __ffs(todo) - 1;
+      const int64_t i = g0 + at;
+      const int64_t base = __shfl_sync(FULL, u, at);
+      const int P = sg_expand_warp<V, K, MAXP>(A, B, i, lane, key, prod);
+      __syncwarp();
+      if constexpr (CLS == SG_WARP) {
+        if (P <= 32) sort_row_keys<1>(key, P, lane);
+        else if (P <= 64) sort_row_keys<2>(key, P, lane);
+        else if (P <= 128) sort_row_keys<4>(key, P, lane);
+        else sort_row_keys<8>(key, P, lane);
+      } else {
+        if (P <= 512) sort_row_keys<16>(key, P, lane);
+        else sort_row_keys<32>(key, P, lane);
       }
-      heads += __popc(hm);
+      __syncwarp();
+      int heads = 0;
+      int32_t last = -1;  // the column before the current 32 keys
+      for (int c0 = 0; c0 < P; c0 += 32) {
+        const int idx = c0 + lane;
+        const bool valid = idx < P;
+        const K k = valid ? key[sg_slot(idx)] : ~K(0);
+        const int32_t c = KO::col(k);
+        int32_t before = __shfl_up_sync(FULL, c, 1);
+        if (lane == 0) before = last;
+        last = __shfl_sync(FULL, c, 31);
+        const bool head = valid && before != c;
+        const unsigned hm = __ballot_sync(FULL, head);
+        if (head) {
+          V v = prod[KO::idx(k)];
+          for (int j = idx + 1; j < P; j++) {
+            const K kj = key[sg_slot(j)];
+            if (KO::col(kj) != c) break;
+            v = v + prod[KO::idx(kj)];
+          }
+          const int64_t o = base + heads + __popc(hm & lt);
+          tcol[o] = c;
+          tval[o] = v;
+        }
+        heads += __popc(hm);
+      }
+      if (lane == 0) ucnt[i] = heads;
+      __syncwarp();
     }
-    if (lane == 0) ucnt[i] = heads;
-    __syncwarp();
+    r0 = __shfl_sync(FULL, r1, 0);
   }
 }
 
-// The CTA class's expand (256 < P_i <= 4096): row i's A entries are taken
+// The CTA class's expand (the class above): row i's A entries are taken
 // 256 at a time, one per thread (column, value, B row length and first
 // segment loaded side by side), the lengths scanned across the block into
 // product offsets, then each thread produces products q = tid, tid + 256,
@@ -407,11 +509,11 @@ __device__ __forceinline__ int sg_expand_cta(const Mat<V> &A, const Mat<V> &B, i
   return base;
 }
 
-// CTA per row, 256 < P_i <= 4096 (dynamic shared memory).
+// CTA per row, up to 4096 products (dynamic shared memory).
 template <typename V>
 __global__ void __launch_bounds__(SG_THREADS) k_sg_cta(Mat<V> A, Mat<V> B, const unsigned *rows,
-                                                       const long long *starts, const long long *ub, int32_t *tcol,
-                                                       V *tval, long long *ucnt) {
+                                                       int64_t n_rows, const long long *ub, int32_t *tcol, V *tval,
+                                                       long long *ucnt) {
   extern __shared__ unsigned long long sg_smem[];
   unsigned long long *key = sg_smem;
   V *prod = reinterpret_cast<V *>(sg_smem + SG_CTA_MAX);
@@ -420,8 +522,7 @@ __global__ void __launch_bounds__(SG_THREADS) k_sg_cta(Mat<V> A, Mat<V> B, const
   __shared__ int32_t sk[SG_THREADS], sst[SG_THREADS];
   __shared__ V sa[SG_THREADS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t b = starts[SG_CTA], e = starts[SG_CTA + 1];
-  for (int64_t it = b + blockIdx.x; it < e; it += gridDim.x) {
+  for (int64_t it = blockIdx.x; it < n_rows; it += gridDim.x) {
     const int64_t i = rows[it];
     const int P = sg_expand_cta(A, B, i, threadIdx.x, key, prod, soff, sk, sa, sst, wsum);
     const int n2 = next_pow2(P);
@@ -460,15 +561,13 @@ __global__ void __launch_bounds__(SG_THREADS) k_sg_cta(Mat<V> A, Mat<V> B, const
 
 // Global path: expand rows with P_i > 4096 into (key = slot<<cb | col, value = global product index).
 template <typename V>
-__global__ void k_sg_global_expand(Mat<V> A, Mat<V> B, const unsigned *rows, const long long *starts,
+__global__ void k_sg_global_expand(Mat<V> A, Mat<V> B, const unsigned *rows, int64_t n_rows,
                                    const long long *goff, int cb, unsigned long long *gkey, unsigned *gidx,
                                    V *gprod) {
   const int lane = threadIdx.x & 31;
-  const int64_t b = starts[SG_GLOBAL], e = starts[SG_GLOBAL + 1];
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t it = b + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); it < e; it += nw) {
-    const int64_t i = rows[it];
-    const int64_t slot = it - b;
+  for (int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; slot < n_rows; slot += nw) {
+    const int64_t i = rows[slot];
     const int64_t o = goff[slot];
     const Chain ca = load_chain(A, (int32_t)i);
     const int64_t LA = A.row_sizes[i];
@@ -502,17 +601,16 @@ __global__ void k_sg_global_flags(const unsigned long long *gkey, int64_t n, lon
 
 template <typename V>
 __global__ void k_sg_global_emit(const unsigned long long *gkey, const unsigned *gidx, const V *gprod, int64_t n,
-                                 const long long *hpos, const unsigned *rows, const long long *starts,
-                                 const long long *goff, const long long *ub, int cb, int32_t *tcol, V *tval,
+                                 const long long *hpos, const unsigned *rows, const long long *goff,
+                                 const long long *ub, int cb, int32_t *tcol, V *tval,
                                  long long *ucnt) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const unsigned long long cmask = (1ull << cb) - 1;
-  const int64_t b = starts[SG_GLOBAL];
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
     const unsigned long long k = gkey[q];
     if (q > 0 && gkey[q - 1] == k) continue;
     const int64_t slot = (int64_t)(k >> cb);
-    const int64_t i = rows[b + slot];
+    const int64_t i = rows[slot];
     V v = gprod[gidx[q]];
     for (int64_t j = q + 1; j < n && gkey[j] == k; j++) v = v + gprod[gidx[j]];
     const int64_t first = hpos[goff[slot]];  // head rank of the row's first product
@@ -525,12 +623,10 @@ __global__ void k_sg_global_emit(const unsigned long long *gkey, const unsigned 
 
 // slot products for the global class: goff[slot] = ub-like offsets of the
 // large rows in a dense staging array
-__global__ void k_sg_global_sizes(const unsigned *rows, const long long *starts, const long long *ub,
-                                  long long *gsz) {
-  const int64_t b = starts[SG_GLOBAL], e = starts[SG_GLOBAL + 1];
+__global__ void k_sg_global_sizes(const unsigned *rows, int64_t n_rows, const long long *ub, long long *gsz) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t it = b + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it <= e; it += stride)
-    gsz[it - b] = it < e ? ub[rows[it] + 1] - ub[rows[it]] : 0;
+  for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it <= n_rows; it += stride)
+    gsz[it] = it < n_rows ? ub[rows[it] + 1] - ub[rows[it]] : 0;
 }
 
 static int grid_for(int64_t n, int block) {
@@ -539,54 +635,63 @@ static int grid_for(int64_t n, int block) {
   return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
+// A warp class's launch: warps that stay and take rows from a counter.
+template <typename V, typename K, int CLS>
+static int sg_warp_rows(const Mat<V> &A, const Mat<V> &B, int64_t n_rows, const long long *ub, int warp_max,
+                        long long *next, int32_t *tcol, V *tval, long long *ucnt, cudaStream_t s) {
+  constexpr int W = SG_THREADS / 32;
+  constexpr size_t smem = sizeof(SgWarp<V, K, CLS == SG_WARP ? SG_WARP_MAX : SG_WARP4_MAX>) * W;
+  static const int g = [] {  // once, thread-safely: the kernel's shared-memory limit, then its grid
+    cudaFuncSetAttribute(k_sg_warp<V, K, CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return persistent_grid((const void *)k_sg_warp<V, K, CLS>, SG_THREADS, smem);
+  }();
+  // a warp asks for about GR rows of the class at a time
+  constexpr int64_t GR = CLS == SG_WARP ? 2 : 1;
+  const int64_t G = std::min<int64_t>(32, GR * A.n_rows / n_rows);
+  DCSR_LAUNCH((k_sg_warp<V, K, CLS>), (int)std::min<int64_t>(g, div_up(A.n_rows, G * W)), SG_THREADS, smem, s, A, B,
+              ub, warp_max, (int)G, (unsigned long long *)next, tcol, tval, ucnt);
+  return DCSR_OK;
+}
+
 template <typename V>
 static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStream_t s) {
   const int32_t n = hA->n_rows;
   Mat<V> A = hA->view<V>(), B = hB->view<V>();
   Arena ar;
-  ar.status = hC->stat + ST_STATUS;  // look-back timeouts reach C's status
-  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) * 4 + arena_bytes(n + 2, 4) * 2 + arena_bytes(8, 8) +
-                          radix_scratch_bytes(n) + scan_scratch_bytes(n + 2), s));
-  long long *cnt = ar.take<long long>(n + 2), *capub = ar.take<long long>(n + 2);
-  unsigned long long *k0 = ar.take<unsigned long long>(n + 2), *k1 = ar.take<unsigned long long>(n + 2);
-  unsigned *r0 = ar.take<unsigned>(n + 2), *r1 = ar.take<unsigned>(n + 2);
-  long long *starts = ar.take<long long>(8);  // [0..4] class starts, [5] products of the global class
+  DCSR_TRY(ar.reserve(arena_bytes(n + 2, 8) * 3 + arena_bytes(n + 2, 4) * 2 + arena_bytes(SG_R_WORDS, 8) +
+                          scan_scratch_bytes(n + 2),
+                      s));
+  long long *cnt = ar.take<long long>(n + 2), *ub = ar.take<long long>(n + 2), *ucnt = ar.take<long long>(n + 2);
+  unsigned *r_cta = ar.take<unsigned>(n + 2), *r_glob = ar.take<unsigned>(n + 2);
+  long long *res = ar.take<long long>(SG_R_WORDS);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  long long *ub = cnt;  // scanned in place
-  DCSR_CUDA(cudaMemsetAsync(starts, 0, sizeof(long long) * 8, s));
+  ar.status = res + SG_R_STATUS;  // look-back timeouts of the scans here
+  DCSR_CUDA(cudaMemsetAsync(res, 0, sizeof(long long) * SG_R_WORDS, s));
+  // rows of 257 to 1024 products: 32-bit keys (column, p) where the columns leave p its 10 bits
+  const int warp_max = hB->n_cols <= (1 << 22) ? SG_WARP4_MAX : SG_WARP_MAX;
   if (n > 0) {
-    DCSR_LAUNCH(k_sg_count<V>, grid_for((int64_t)n * 8, SG_THREADS), SG_THREADS, 0, s, A, B, hC->o, cnt, capub, k0,
-                r0, (unsigned long long *)(starts + 5));
-    if (n > 1) DCSR_TRY(radix_sort_pairs(&k0, &r0, &k1, &r1, n, 2, ar, s));
+    DCSR_LAUNCH(k_sg_count<V>, grid_for((int64_t)n * 8, SG_THREADS), SG_THREADS, 0, s, A, B, warp_max, cnt, res);
+    DCSR_TRY(scan_map(StageScan{cnt, hC->o, ub, ucnt, res, n}, n, ar, s));
   }
-  DCSR_LAUNCH(k_sg_classes, 1, 32, 0, s, k0, n, starts);
-  DCSR_TRY(scan2_i64(cnt, ub, hC->stat + ST_TOTAL, capub, capub, hC->stat + ST_AUX + 1, n + 1, ar, s));
   // the one read before the numeric pass: staging and C's pool are sized here
-  long long host[8];
-  DCSR_CUDA(cudaMemcpyAsync(host, starts, sizeof(long long) * 6, cudaMemcpyDeviceToHost, s));
-  DCSR_CUDA(cudaMemcpyAsync(host + 6, hC->stat + ST_TOTAL, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  DCSR_CUDA(cudaMemcpyAsync(host + 7, hC->stat + ST_AUX + 1, sizeof(long long), cudaMemcpyDeviceToHost, s));
-  long long st_word = 0;
-  DCSR_CUDA(cudaMemcpyAsync(&st_word, hC->stat + ST_STATUS, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  long long host[SG_R_WORDS];
+  DCSR_CUDA(cudaMemcpyAsync(host, res, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
-  if (st_word == DCSR_TIMEOUT) {
-    DCSR_CUDA(cudaMemsetAsync(hC->stat + ST_STATUS, 0, sizeof(long long), s));
+  if (host[SG_R_STATUS] == DCSR_TIMEOUT) {
     ar.release(s);
     return DCSR_TIMEOUT;
   }
-  const int64_t Pg = host[5], P = host[6], cap_bound = pool_capacity(hC->o, host[7]);
-  const int64_t n_global = host[SG_GLOBAL + 1] - host[SG_GLOBAL];
+  const int64_t Pg = host[SG_R_GPROD], P = host[SG_R_PROD], cap_bound = pool_capacity(hC->o, host[SG_R_CAPS]);
+  const int64_t n_cta = host[SG_CTA], n_global = host[SG_GLOBAL];
   if (Pg > 0xffffffffLL) return DCSR_NOT_SUPPORTED;
   // staging: row i's unique columns at ub[i]
   int32_t *tcol = nullptr;
   V *tval = nullptr;
-  long long *ucnt = nullptr;
   DCSR_CUDA(dcsr::dev_alloc((void **)&tcol, sizeof(int32_t) * (P + 1), s));
   DCSR_CUDA(dcsr::dev_alloc((void **)&tval, sizeof(V) * (P + 1), s));
-  DCSR_CUDA(dcsr::dev_alloc((void **)&ucnt, sizeof(long long) * (n + 2), s));
-  DCSR_CUDA(cudaMemsetAsync(ucnt, 0, sizeof(long long) * (n + 2), s));
+  ar.status = hC->stat + ST_STATUS;  // and from here on C's status, which load_from_rows reads
+  if (n_cta + n_global > 0) DCSR_TRY(scan_map(ListScan{ub, warp_max, r_cta, r_glob}, n, ar, s));
   const size_t cta_smem = SG_CTA_MAX * (sizeof(unsigned long long) + sizeof(V));
-  static const int g_warp = persistent_grid((const void *)k_sg_warp<double, unsigned long long>, SG_THREADS, 0);
   static const int g_cta = [] {  // once, thread-safely: the CTA kernels' shared-memory limit, then their grid
     cudaFuncSetAttribute(k_sg_cta<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(SG_CTA_MAX * (sizeof(unsigned long long) + sizeof(float))));
@@ -595,15 +700,16 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
     return persistent_grid((const void *)k_sg_cta<double>, SG_THREADS,
                            SG_CTA_MAX * (sizeof(unsigned long long) + sizeof(double)));
   }();
-  if (host[SG_WARP + 1] > host[SG_WARP]) {
-    if (hB->n_cols <= (1 << 24))  // (column, p) in 32-bit keys
-      DCSR_LAUNCH((k_sg_warp<V, unsigned>), g_warp, SG_THREADS, 0, s, A, B, r0, starts, ub, tcol, tval, ucnt);
-    else
-      DCSR_LAUNCH((k_sg_warp<V, unsigned long long>), g_warp, SG_THREADS, 0, s, A, B, r0, starts, ub, tcol, tval,
-                  ucnt);
+  if (host[SG_WARP] > 0) {
+    const bool narrow = hB->n_cols <= (1 << 24);  // (column, p) in 32-bit keys
+    DCSR_TRY((narrow ? sg_warp_rows<V, unsigned, SG_WARP> : sg_warp_rows<V, unsigned long long, SG_WARP>)(
+        A, B, host[SG_WARP], ub, warp_max, res + SG_R_NEXT, tcol, tval, ucnt, s));
   }
-  if (host[SG_CTA + 1] > host[SG_CTA])
-    DCSR_LAUNCH(k_sg_cta<V>, g_cta, SG_THREADS, cta_smem, s, A, B, r0, starts, ub, tcol, tval, ucnt);
+  if (host[SG_WARP4] > 0)
+    DCSR_TRY((sg_warp_rows<V, unsigned, SG_WARP4>(A, B, host[SG_WARP4], ub, warp_max, res + SG_R_NEXT4, tcol, tval,
+                                                  ucnt, s)));
+  if (n_cta > 0)
+    DCSR_LAUNCH(k_sg_cta<V>, g_cta, SG_THREADS, cta_smem, s, A, B, r_cta, n_cta, ub, tcol, tval, ucnt);
   Arena gg;
   if (n_global > 0) {
     // products of all large rows, laid out densely by slot, then one stable
@@ -618,16 +724,16 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
     V *gprod = (V *)gg.take<double>(Pg);
     long long *hpos = gg.take<long long>(Pg + 1);
     if (gg.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-    DCSR_LAUNCH(k_sg_global_sizes, grid_for(n_global + 1, 256), 256, 0, s, r0, starts, ub, goff);
+    DCSR_LAUNCH(k_sg_global_sizes, grid_for(n_global + 1, 256), 256, 0, s, r_glob, n_global, ub, goff);
     DCSR_TRY(scan_i64(goff, goff, n_global + 1, nullptr, gg, s));
     const int cb = bits_for(hB->n_cols);
-    DCSR_LAUNCH(k_sg_global_expand<V>, grid_for(n_global * 32, 256), 256, 0, s, A, B, r0, starts, goff, cb, gk0, gi0,
-                gprod);
+    DCSR_LAUNCH(k_sg_global_expand<V>, grid_for(n_global * 32, 256), 256, 0, s, A, B, r_glob, n_global, goff, cb,
+                gk0, gi0, gprod);
     DCSR_TRY(radix_sort_pairs(&gk0, &gi0, &gk1, &gi1, Pg, bits_for(n_global) + cb, gg, s));
     DCSR_LAUNCH(k_sg_global_flags, grid_for(Pg, 256), 256, 0, s, gk0, Pg, hpos);
     DCSR_TRY(scan_i64(hpos, hpos, Pg, nullptr, gg, s));
-    DCSR_LAUNCH(k_sg_global_emit<V>, grid_for(Pg, 256), 256, 0, s, gk0, gi0, gprod, Pg, hpos, r0, starts, goff, ub,
-                cb, tcol, tval, ucnt);
+    DCSR_LAUNCH(k_sg_global_emit<V>, grid_for(Pg, 256), 256, 0, s, gk0, gi0, gprod, Pg, hpos, r_glob, goff, ub, cb,
+                tcol, tval, ucnt);
   }
   // C's rows go straight from the staging area into C's pool (policy
   // capacities); the second and last synchronisation reads C's pool top
@@ -636,7 +742,6 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
   ar.release(s);
   dcsr::dev_free(tcol, s);
   dcsr::dev_free(tval, s);
-  dcsr::dev_free(ucnt, s);
   return st;
 }
 
