@@ -217,14 +217,14 @@ constexpr int64_t SM_ONE = SM_ONE_THREADS * SM_LIGHT;
 template <class F, class = void>
 struct ScanHasEmitAll : std::false_type {};
 template <class F>
-struct ScanHasEmitAll<F, std::void_t<decltype(F::EMIT_ALL)>> : std::true_type {};
+struct ScanHasEmitAll<F, std::void_t<decltype(F::EMIT_ALL)>> : std::bool_constant<F::EMIT_ALL> {};
 template <class F, class = void>
 struct ScanHasLoadAll : std::false_type {};
 template <class F>
 struct ScanHasLoadAll<F, std::void_t<decltype(F::LOAD_ALL)>> : std::true_type {};
 
 template <int TH, class F>
-__global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY ? 3 : 4) k_scan_map(F f, int64_t n, Lookback lb) {
+__global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY || ScanHasLoadAll<F>::value ? 3 : 4) k_scan_map(F f, int64_t n, Lookback lb) {
   constexpr int NS = F::NS, NW = TH / 32, SM_ITEMS = F::IT;
   __shared__ long long wsum[NS][NW];
   __shared__ long long sh_prefix[NS];

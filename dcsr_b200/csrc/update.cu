@@ -929,47 +929,150 @@ __global__ void k_coo_keys(const int32_t *rows, const int32_t *cols, int64_t n, 
   }
 }
 
-__global__ void k_group(const unsigned long long *keys, int64_t n, int merge, long long *flag) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    flag[i] = (!merge || i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
-}
-
-template <typename V>
-__global__ void k_group_emit(const unsigned long long *keys, const unsigned *perm, const int32_t *cols,
-                             const V *vals, int64_t n, int cb, int merge, int32_t n_cols, const long long *pos,
-                             int32_t *ocols, V *ovals, int32_t *rowcnt) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const unsigned long long cmask = (1ull << cb) - 1;
-  const int lane = threadIdx.x & 31;
-  // block-uniform trip count, so whole warps take part in the count below
-  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
-    const int64_t i = i0 + threadIdx.x;
-    int32_t r = -1;  // the row of the entry this thread emits
-    if (i < n) {
-      const unsigned long long k = keys[i];
-      if (!(merge && i > 0 && keys[i - 1] == k)) {
-        V v = vals[perm[i]];
-        if (merge)
-          for (int64_t j = i + 1; j < n && keys[j] == k; j++) v = v + vals[perm[j]];
-        int32_t c = merge ? (int32_t)(k & cmask) : cols[perm[i]];
-        if (c < 0 || c >= n_cols) c = 0;
-        ocols[pos[i]] = c;
-        ovals[pos[i]] = v;
-        r = merge ? (int32_t)(k >> cb) : (int32_t)k;
+// Sorted triples -> CSR columns and values and the rows' counts, in one pass:
+// a scan over group heads (MERGE: the first triple of each (row, column), the
+// group's values added up in input order; else every triple), whose position
+// is where the entry goes.  The pass is bound by the gather of the values
+// through the permutation (a random sector each: 540 MB of L2 traffic of 16.7M
+// triples), so a thread has its 8 triples' keys, then indices, then values in
+// flight together, before the look-back.  With a pass for flags, their scan
+// and a pass for the entries, 16 bytes of flags a triple written and read
+// twice, the three took 492 us of 16.7M triples; this one 272 us (3 blocks per
+// SM; 2 or 4, with more spilled registers: 20-40 us more).
+template <typename V, bool MERGE>
+struct CooScan {
+  static constexpr int NS = 1, IT = SM_LIGHT;
+  static constexpr bool LOAD_ALL = true, EMIT_ALL = MERGE;  // (no groups to add up in append mode)
+  using T = int32_t;
+  struct State {
+    unsigned long long key;
+    V val;
+    int32_t col;
+  };
+  const unsigned long long *keys;
+  const unsigned *perm;
+  const int32_t *cols;
+  const V *vals;
+  int64_t n;
+  int cb;
+  int32_t n_cols;
+  int32_t *ocols;
+  V *ovals;
+  int32_t *rowcnt;
+  __device__ __forceinline__ int32_t row(unsigned long long k) const { return (int32_t)(MERGE ? k >> cb : k); }
+  __device__ __forceinline__ void load_all(int64_t base, int64_t, State (&st)[IT], T (&v)[IT][1]) const {
+    const int lane = lane_id();
+    unsigned at[IT];
+#pragma unroll
+    for (int j = 0; j < IT; j++) {
+      const int64_t i = base + 32 * j;
+      st[j].key = i < n ? __ldcs(keys + i) : ~0ull;
+      at[j] = i < n ? __ldcs(perm + i) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < IT; j++) {
+      const int64_t i = base + 32 * j;
+      st[j].val = i < n ? vals[at[j]] : V(0);
+      st[j].col = 0;
+      if constexpr (!MERGE) st[j].col = i < n ? cols[at[j]] : 0;
+    }
+    // a triple is in the group of the one before it, or starts its own
+    const int64_t w0 = base - lane;  // the warp's first triple
+    unsigned long long carry = ~0ull;
+    if (MERGE && lane == 0 && w0 > 0 && w0 <= n) carry = keys[w0 - 1];
+#pragma unroll
+    for (int j = 0; j < IT; j++) {
+      const int64_t i = base + 32 * j;
+      unsigned long long prev = __shfl_up_sync(FULL, st[j].key, 1);
+      if (lane == 0) prev = carry;
+      carry = __shfl_sync(FULL, st[j].key, 31);
+      v[j][0] = i < n && !(MERGE && i > 0 && prev == st[j].key) ? 1 : 0;
+    }
+  }
+  // Groups of several triples: the head's value takes the others' in input
+  // order.  The triples of a warp are added by shuffle -- a step's groups side
+  // by side, a group that began in an earlier step by the whole warp -- and
+  // those past the warp's last 32 at a time, so a group's sum is a chain of
+  // additions, not of loads (a power-law graph's hottest edge comes up
+  // hundreds of times; a thread that walked its group through keys, indices
+  // and values held its warp for 0.6 us a triple).
+  __device__ __forceinline__ void emit_all(int64_t base, int64_t, State (&st)[IT], const T (&v)[IT][1]) const {
+    const int lane = lane_id();
+    const int64_t w1 = base - lane + 32 * IT;  // past the warp's triples
+    V cx = V(0);  // the sum of the last group so far, and where its head is
+    int jo = -1, lo = 0;
+#pragma unroll
+    for (int j = 0; j < IT; j++) {
+      const unsigned heads = __ballot_sync(FULL, v[j][0] != 0);
+      const unsigned same = __ballot_sync(FULL, base + 32 * j < n) & ~heads;
+      V x = st[j].val;
+      if (same) {
+        const unsigned rest = lane < 31 ? ~(same >> (lane + 1)) : FULL;
+        const int run = v[j][0] && rest ? __ffs(rest) - 1 : 0;  // triples of this head's group in this step
+        const int longest = (int)__reduce_max_sync(FULL, (unsigned)run);
+        for (int d = 1; d <= longest; d++) {
+          const V o = __shfl_down_sync(FULL, st[j].val, d);
+          if (d <= run) x = x + o;
+        }
+        if ((same & 1u) && jo >= 0) {  // the group open from an earlier step
+          const int lead = ~same ? __ffs(~same) - 1 : 32;
+          for (int q = 0; q < lead; q++) cx = cx + __shfl_sync(FULL, st[j].val, q);
+#pragma unroll
+          for (int i = 0; i < j; i++)
+            if (i == jo && lane == lo) st[i].val = cx;
+        }
+        st[j].val = x;
+      }
+      if (heads) {
+        jo = j;
+        lo = 31 - __clz(heads);
+        cx = __shfl_sync(FULL, x, lo);
       }
     }
-    // row counts, one atomic per row and warp: the keys are sorted, so a
-    // warp's entries are a few runs of one row each (a power-law graph's
-    // hottest rows otherwise took one atomic per entry on a single word)
-    const unsigned peers = __match_any_sync(FULL, r);
-    if (r >= 0 && __ffs(peers) - 1 == lane) atomicAdd(&rowcnt[r], __popc(peers));
+    if (jo < 0 || w1 >= n) return;
+    const unsigned long long k = __shfl_sync(FULL, st[IT - 1].key, 31);
+    bool more = keys[w1] == k;
+    if (!more) return;
+    for (int64_t at = w1; more; at += 32) {
+      const int64_t i = at + lane;
+      const unsigned in = __ballot_sync(FULL, i < n && keys[i < n ? i : w1] == k);
+      const int cnt = ~in ? __ffs(~in) - 1 : 32;
+      const V o = lane < cnt ? vals[perm[i]] : V(0);
+      for (int q = 0; q < cnt; q++) cx = cx + __shfl_sync(FULL, o, q);
+      more = cnt == 32;
+    }
+#pragma unroll
+    for (int i = 0; i < IT; i++)
+      if (i == jo && lane == lo) st[i].val = cx;
   }
-}
+  __device__ __forceinline__ void emit(int64_t i, bool ok, const State &st, const long long (&p)[1],
+                                       const T (&v)[1]) const {
+    const int lane = lane_id();
+    if (v[0]) {
+      int32_t c = MERGE ? (int32_t)(st.key & ((1ull << cb) - 1)) : st.col;
+      if (c < 0 || c >= n_cols) c = 0;
+      ocols[p[0]] = c;
+      ovals[p[0]] = st.val;
+    }
+    // row counts, one atomic per row and warp step: the keys are sorted, so 32
+    // triples are a few runs of one row each
+    const int32_t r = ok ? row(st.key) : -1;
+    const int32_t prev = __shfl_up_sync(FULL, r, 1);
+    const unsigned starts = __ballot_sync(FULL, lane == 0 || prev != r);
+    const unsigned heads = __ballot_sync(FULL, v[0] != 0);
+    if (r >= 0 && (starts >> lane & 1u)) {
+      const unsigned later = starts & ~((2u << lane) - 1u);  // lane 31: 2u << 31 is 0
+      const unsigned run = (later ? (later & -later) - 1u : FULL) & ~((1u << lane) - 1u);
+      const int c = __popc(heads & run);
+      if (c) atomicAdd(&rowcnt[r], c);
+    }
+  }
+  __device__ __forceinline__ void total(const long long (&)[1]) const {}
+};
 
 size_t coo_to_csr_scratch(dcsr_handle h, int64_t T) {
-  return 2 * arena_bytes(T, 8) + 2 * arena_bytes(T, 4) + arena_bytes(T + 1, 8) + arena_bytes(T, 4) +
-         arena_bytes(T, 8) + 3 * arena_bytes(h->n_rows + 2, 4) + radix_scratch_bytes(T) +
+  return 2 * arena_bytes(T, 8) + 2 * arena_bytes(T, 4) + arena_bytes(T, 4) + arena_bytes(T, 8) +
+         3 * arena_bytes(h->n_rows + 2, 4) + radix_scratch_bytes(T) +
          scan_scratch_bytes(std::max<int64_t>(T, h->n_rows + 1));
 }
 
@@ -979,7 +1082,6 @@ static int coo_impl(dcsr_handle h, const int32_t *rows, const int32_t *cols, con
   const int cb = bits_for(h->n_cols), rb = bits_for(h->n_rows);
   unsigned long long *k0 = ar.take<unsigned long long>(T), *k1 = ar.take<unsigned long long>(T);
   unsigned *p0 = ar.take<unsigned>(T), *p1 = ar.take<unsigned>(T);
-  long long *flag = ar.take<long long>(T + 1);
   int32_t *oc = ar.take<int32_t>(T);
   V *ov = (V *)ar.take<double>(T);
   int32_t *cnt = ar.take<int32_t>(h->n_rows + 2);
@@ -991,10 +1093,8 @@ static int coo_impl(dcsr_handle h, const int32_t *rows, const int32_t *cols, con
     DCSR_LAUNCH(k_coo_keys, grid_for(T, 256), 256, 0, s, rows, cols, T, h->n_rows, h->n_cols, cb, merge ? 1 : 0, k0,
                 p0, h->stat);
     DCSR_TRY(radix_sort_pairs(&k0, &p0, &k1, &p1, T, merge ? rb + cb : rb, ar, s));
-    DCSR_LAUNCH(k_group, grid_for(T, 256), 256, 0, s, k0, T, merge ? 1 : 0, flag);
-    DCSR_TRY(scan_i64(flag, flag, T, nullptr, ar, s));
-    DCSR_LAUNCH(k_group_emit<V>, grid_for(T, 256), 256, 0, s, k0, p0, cols, vals, T, cb, merge ? 1 : 0, h->n_cols,
-                flag, oc, ov, cnt);
+    if (merge) DCSR_TRY(scan_map(CooScan<V, true>{k0, p0, cols, vals, T, cb, h->n_cols, oc, ov, cnt}, T, ar, s));
+    else DCSR_TRY(scan_map(CooScan<V, false>{k0, p0, cols, vals, T, cb, h->n_cols, oc, ov, cnt}, T, ar, s));
   }
   DCSR_TRY(counts_scan(h, cnt, *rp, *caps, ar, s));
   *ocols = oc;
