@@ -26,7 +26,7 @@ __device__ __forceinline__ unsigned long long ld_vol(const unsigned long long *p
 // above a 32-bit value, so a word is published with one store and read with
 // one load -- no fences, no second load.  A sort's word per (tile, digit)
 // holds a count (kind 1: the tile's aggregate, 2: its inclusive prefix); a
-// scan has one 128-bit word per tile, tag and kind above up to two 48-bit
+// scan has one 128-bit word per tile, tag and kind above 96 bits of
 // sums, stored and loaded whole.  A word is current when its tag is the
 // kernel's; the tag repeats every 2^30 kernels on one area, so the kernel
 // whose last block advances the epoch to such a multiple clears the area
@@ -105,10 +105,14 @@ __device__ __forceinline__ void lb_store(unsigned long long *p, const LbWord &w)
 }
 template <int NS>
 __device__ __forceinline__ LbWord lb_word(unsigned long long e, int kind, const long long (&v)[NS]) {
-  static_assert(NS == 1 || NS == 2, "one or two sums");
+  static_assert(NS >= 1 && NS <= 3, "one to three sums");
   LbWord w;
   w.lo = (unsigned long long)v[0];
   w.hi = lb_pack(e, kind, 0);
+  if constexpr (NS == 3) {
+    w.lo = (w.lo & 0xffffffffull) | ((unsigned long long)v[1] << 32);
+    w.hi |= (unsigned long long)v[2] & 0xffffffffull;
+  }
   if constexpr (NS == 2) {
     const unsigned long long b = (unsigned long long)v[1];
     w.lo = (w.lo & 0xffffffffffffull) | (b << 48);
@@ -119,6 +123,7 @@ __device__ __forceinline__ LbWord lb_word(unsigned long long e, int kind, const 
 template <int NS>
 __device__ __forceinline__ long long lb_sum(const LbWord &w, int q) {
   if constexpr (NS == 1) return (long long)w.lo;
+  if constexpr (NS == 3) return (long long)(unsigned)(q == 0 ? w.lo : q == 1 ? w.lo >> 32 : w.hi);
   return q == 0 ? (long long)(w.lo & 0xffffffffffffull) : (long long)((w.lo >> 48) | ((w.hi & 0xffffffffull) << 16));
 }
 // Look-back words (8 bytes) that a scan of `tiles` tiles needs.

@@ -116,12 +116,10 @@ int debug_lookback(int spin_limit, int stall) {
   return DCSR_OK;
 }
 
-// Scan operands: one array, or two independent arrays of the same length
-// scanned by one launch (tiles [0, nt) scan the first, [nt, 2nt) the second).
 struct ScanArgs {
-  const long long *in[2];
-  long long *out[2];
-  long long *total[2];
+  const long long *in;
+  long long *out;
+  long long *total;
   int64_t n, nt;
 };
 
@@ -141,12 +139,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_1p(ScanArgs a, Lookback l
     if (lb_end(lb)) lb_advance(lb);
     return;
   }
-  const int arr = t >= a.nt ? 1 : 0;
-  const int64_t t0 = arr * a.nt;  // this array's first tile
-  const long long *__restrict__ in = a.in[arr];
-  long long *out = a.out[arr];
+  const long long *__restrict__ in = a.in;
+  long long *out = a.out;
   const int64_t n = a.n;
-  const int64_t base = (t - t0) * SCAN_TILE;
+  const int64_t base = t * SCAN_TILE;
 #pragma unroll
   for (int j = 0; j < SCAN_ITEMS; j++) {
     const int64_t i = base + j * SCAN_THREADS + threadIdx.x;
@@ -166,7 +162,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_1p(ScanArgs a, Lookback l
     const int lane = threadIdx.x;
     const long long agg[1] = {bt};
     long long before[1];
-    lb_lookback<1>(lb, e, t, t0, agg, before);
+    lb_lookback<1>(lb, e, t, 0, agg, before);
     const long long excl = before[0];
     if (lane == 0) sh_prefix = excl;
   }
@@ -183,7 +179,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_1p(ScanArgs a, Lookback l
     const int64_t i = base + j * SCAN_THREADS + threadIdx.x;
     if (i < n) out[i] = tile[j * SCAN_THREADS + threadIdx.x];
   }
-  if (threadIdx.x == 0 && a.total[arr] && base + SCAN_TILE >= n) *a.total[arr] = sh_prefix + bt;
+  if (threadIdx.x == 0 && a.total && base + SCAN_TILE >= n) *a.total = sh_prefix + bt;
   if (lb_end(lb)) lb_advance(lb);
 }
 
@@ -191,9 +187,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_1p(ScanArgs a, Lookback l
 // scans 4 consecutive values, one block scan, coalesced stores.
 constexpr int SCAN_SMALL = 1024 * 4;
 __global__ void __launch_bounds__(1024) k_scan_small(ScanArgs a) {
-  const long long *__restrict__ in = a.in[blockIdx.x];
-  long long *out = a.out[blockIdx.x];
-  long long *total = a.total[blockIdx.x];
+  const long long *__restrict__ in = a.in;
+  long long *out = a.out;
+  long long *total = a.total;
   const int64_t n = a.n;
   __shared__ long long tile[SCAN_SMALL];
   for (int i = threadIdx.x; i < SCAN_SMALL; i += 1024) tile[i] = i < n ? in[i] : 0;
@@ -223,7 +219,7 @@ int scan_i64(const long long *in, long long *out, int64_t n, long long *total, A
     if (total) DCSR_CUDA(cudaMemsetAsync(total, 0, sizeof(long long), s));
     return DCSR_OK;
   }
-  ScanArgs a{{in, nullptr}, {out, nullptr}, {total, nullptr}, n, div_up(n, SCAN_TILE)};
+  const ScanArgs a{in, out, total, n, div_up(n, SCAN_TILE)};
   if (n <= SCAN_SMALL) {
     DCSR_LAUNCH(k_scan_small, 1, 1024, 0, s, a);
     return DCSR_OK;
@@ -231,24 +227,6 @@ int scan_i64(const long long *in, long long *out, int64_t n, long long *total, A
   Lookback lb;
   DCSR_TRY(ar.lookback((size_t)(LB_SCAN_WORDS * a.nt), s, &lb));
   DCSR_LAUNCH(k_scan_1p, (unsigned)a.nt, SCAN_THREADS, 0, s, a, lb);
-  return DCSR_OK;
-}
-
-int scan2_i64(const long long *in0, long long *out0, long long *total0, const long long *in1, long long *out1,
-              long long *total1, int64_t n, Arena &ar, cudaStream_t s) {
-  if (n <= 0) {
-    if (total0) DCSR_CUDA(cudaMemsetAsync(total0, 0, sizeof(long long), s));
-    if (total1) DCSR_CUDA(cudaMemsetAsync(total1, 0, sizeof(long long), s));
-    return DCSR_OK;
-  }
-  ScanArgs a{{in0, in1}, {out0, out1}, {total0, total1}, n, div_up(n, SCAN_TILE)};
-  if (n <= SCAN_SMALL) {
-    DCSR_LAUNCH(k_scan_small, 2, 1024, 0, s, a);
-    return DCSR_OK;
-  }
-  Lookback lb;
-  DCSR_TRY(ar.lookback((size_t)(2 * LB_SCAN_WORDS * a.nt), s, &lb));
-  DCSR_LAUNCH(k_scan_1p, (unsigned)(2 * a.nt), SCAN_THREADS, 0, s, a, lb);
   return DCSR_OK;
 }
 
@@ -705,10 +683,10 @@ constexpr int OS_TILE = OS_T * OS_I;
 
 size_t lookback_slots(int64_t n) {
   // single-pass sorts: one slot per (tile, digit); larger ones: the scan of
-  // their histogram table; scans: a two-slot word per (smallest) tile, of two arrays
+  // their histogram table; scans: a two-slot word per (smallest) tile
   const int64_t sort = n <= RS_BIG ? div_up(n, OS_TILE) * RS_BINS
                                    : LB_SCAN_WORDS * div_up(div_up(n, RS_THREADS * 16) * RS_BINS, SCAN_TILE);
-  return (size_t)(std::max<int64_t>(sort, 2 * LB_SCAN_WORDS * div_up(n, SM_THREADS * SM_HEAVY)) + 1);
+  return (size_t)(std::max<int64_t>(sort, LB_SCAN_WORDS * div_up(n, SM_THREADS * SM_HEAVY)) + 1);
 }
 
 // Large inputs: three kernels per pass (tile histograms, table scan, scatter).

@@ -108,6 +108,10 @@ struct RowMany {
     }
     return lo;
   }
+  __device__ __forceinline__ int next_row(int i, int64_t g) const {  // the same, i holding an earlier row
+    while (i + 1 < count && its[i + 1].row0 <= g) i++;
+    return i;
+  }
   __device__ __forceinline__ int64_t units(int part) const { return pref[part * (count + 1) + count]; }
   __device__ __forceinline__ int locate(int part, int64_t u, int64_t &lu) const {
     const long long *p = pref + part * (count + 1);
@@ -123,68 +127,78 @@ struct RowMany {
 };
 
 // ---------------------------------------------------------------- schedule
-// Per row: lflag = (is_long << 32) | chunks, mflag = is_medium; two scans
-// give every long row its index and first chunk and every medium row its
-// slot, per matrix (differences of the scans at the matrix's first row).
-
-__device__ __forceinline__ void sched_flags_row(int32_t L, int32_t smax, int32_t lmin, long long &lf,
-                                                long long &mf) {
-  lf = L > lmin ? ((1ll << 32) | (long long)((L + CHUNK - 1) / CHUNK)) : 0;
-  mf = (L > smax && L <= lmin) ? 1 : 0;
-}
+// The long rows' indices and first chunks and the medium rows' slots, per
+// matrix: one scan over the rows of all matrices (sums modulo 2^32: only
+// differences within a matrix are used), which leaves the prefixes of the rows
+// that need one, and a pass that lists them.  A batch's first row of a matrix
+// may lie in any block, so the differences take the second pass.  (With flags
+// and their scan in memory, four kernels: 58 us in a batch of 48 matrices of 1000 to
+// 128000 rows, now 36.)
 
 template <typename V, typename Src>
-__global__ void k_sched_flags(Src src, int64_t R, long long *lflag, long long *mflag) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g <= R; g += stride) {
-    long long lf = 0, mf = 0;
-    if (g < R) {
+struct SchedScan {
+  static constexpr int NS = 3, IT = SM_LIGHT;
+  using T = int32_t;
+  struct State {
+    bool keep;  // long or medium, or the first or last row of its matrix
+  };
+  Src src;
+  uint4 *tmp;
+  // (a search per row: with one a thread and its rows following, as below, the
+  // kernel took 31 us instead of 24)
+  __device__ __forceinline__ void load(int64_t g, bool ok, State &st, T (&v)[3]) const {
+    v[0] = v[1] = v[2] = 0;
+    st.keep = false;
+    if (ok) {
       const RowItem<V> &it = src.item(src.find_row(g));
-      sched_flags_row(it.m.row_sizes[g - it.row0], it.short_max, it.long_min, lf, mf);
+      const int64_t r = g - it.row0;
+      const int32_t L = it.m.row_sizes[r];
+      if (L > it.long_min) {
+        v[0] = 1;
+        v[1] = (int32_t)(((int64_t)L + CHUNK - 1) / CHUNK);
+      } else if (L > it.short_max) {
+        v[2] = 1;
+      }
+      st.keep = L > it.short_max || r == 0 || r == it.m.n_rows - 1;
     }
-    lflag[g] = lf;
-    mflag[g] = mf;
   }
-}
+  __device__ __forceinline__ void emit(int64_t g, bool, const State &st, const long long (&p)[3],
+                                       const T (&)[3]) const {
+    if (st.keep) tmp[g] = make_uint4((unsigned)p[0], (unsigned)p[1], (unsigned)p[2], 0);
+  }
+  __device__ __forceinline__ void total(const long long (&)[3]) const {}
+};
 
+// Lists of the long and medium rows; per matrix the class counts and the
+// long-row offset sentinel (its last row's thread).
 template <typename V, typename Src>
-__global__ void k_sched_emit(Src src, int64_t R, const long long *lscan, const long long *mscan) {
+__global__ void k_sched_emit(Src src, int64_t R, const uint4 *tmp) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < R; g += stride) {
     const RowItem<V> &it = src.item(src.find_row(g));
     const int64_t r = g - it.row0;
     const int32_t L = it.m.row_sizes[r];
-    if (L > it.short_max) {
-      if (L > it.long_min) {
-        const long long s = lscan[g] - lscan[it.row0];
-        const int32_t li = (int32_t)(s >> 32);
-        const long long c0 = s & 0xffffffff, nc = (L + CHUNK - 1) / CHUNK;
-        const_cast<int32_t *>(it.long_rows)[li] = (int32_t)r;
-        const_cast<long long *>(it.long_off)[li] = c0;
-        it.long_cnt[li] = 0;
-        for (long long c = c0; c < c0 + nc; c++) const_cast<int2 *>(it.chunk_rl)[c] = make_int2((int32_t)r, li);
-      } else {
-        const_cast<int32_t *>(it.med_rows)[mscan[g] - mscan[it.row0]] = (int32_t)r;
-      }
+    const bool last = r == it.m.n_rows - 1;
+    if (L <= it.short_max && !last) continue;
+    const uint4 at = tmp[g], a0 = tmp[it.row0];
+    unsigned li = at.x - a0.x, c0 = at.y - a0.y, mi = at.z - a0.z;
+    if (L > it.long_min) {
+      const unsigned nc = (unsigned)(((int64_t)L + CHUNK - 1) / CHUNK);
+      const_cast<int32_t *>(it.long_rows)[li] = (int32_t)r;
+      const_cast<long long *>(it.long_off)[li] = c0;
+      it.long_cnt[li] = 0;
+      for (unsigned c = c0; c < c0 + nc; c++) const_cast<int2 *>(it.chunk_rl)[c] = make_int2((int32_t)r, (int32_t)li);
+      li++;
+      c0 += nc;
+    } else if (L > it.short_max) {
+      const_cast<int32_t *>(it.med_rows)[mi] = (int32_t)r;
+      mi++;
     }
-  }
-}
-
-// Per matrix (one warp each): class counts and the long-row offset sentinel.
-template <typename V, typename Src>
-__global__ void k_sched_info(Src src, const long long *lscan, const long long *mscan) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
-  for (int i = w; i < src.n_items(); i += nw) {
-    const RowItem<V> &it = src.item(i);
-    const int64_t a = it.row0, b = it.row0 + it.m.n_rows;
-    const long long ls = lscan[b] - lscan[a];
-    const int32_t n_long = (int32_t)(ls >> 32), n_chunks = (int32_t)(ls & 0xffffffff);
-    if (lane == 0) {
-      it.info[0] = n_long;
-      it.info[1] = n_chunks;
-      it.info[2] = (int32_t)(mscan[b] - mscan[a]);
-      const_cast<long long *>(it.long_off)[n_long] = n_chunks;
+    if (last) {
+      it.info[0] = (int32_t)li;
+      it.info[1] = (int32_t)c0;
+      it.info[2] = (int32_t)mi;
+      const_cast<long long *>(it.long_off)[li] = c0;
     }
   }
 }
@@ -247,26 +261,24 @@ static int grid_for(int64_t n, int block) {
   return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-size_t schedule_scratch_bytes(int64_t R) { return 2 * arena_bytes(R + 2, 8) + scan_scratch_bytes(R + 1); }
+size_t schedule_scratch_bytes(int64_t R) { return arena_bytes(R + 1, 16) + scan_scratch_bytes(R + 1); }
 
 // Needs schedule_scratch_bytes(R) free in the arena (reserved by the caller).
 template <typename V, typename Src>
-static int schedule_src(const Src &src, int count, int64_t R, Arena &ar, cudaStream_t s) {
-  long long *lf = ar.take<long long>(R + 2), *mf = ar.take<long long>(R + 2);
+static int schedule_src(const Src &src, int64_t R, Arena &ar, cudaStream_t s) {
+  if (R <= 0) return DCSR_OK;
+  uint4 *tmp = ar.take<uint4>(R + 1);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  const int g = grid_for(R + 1, 256);
-  DCSR_LAUNCH((k_sched_flags<V, Src>), g, 256, 0, s, src, R, lf, mf);
-  DCSR_TRY(scan2_i64(lf, lf, nullptr, mf, mf, nullptr, R + 1, ar, s));
-  DCSR_LAUNCH((k_sched_emit<V, Src>), g, 256, 0, s, src, R, lf, mf);
-  DCSR_LAUNCH((k_sched_info<V, Src>), grid_for((int64_t)count * 32, 256), 256, 0, s, src, lf, mf);
+  DCSR_TRY((scan_map(SchedScan<V, Src>{src, tmp}, R, ar, s)));
+  DCSR_LAUNCH((k_sched_emit<V, Src>), grid_for(R, 256), 256, 0, s, src, R, tmp);
   return DCSR_OK;
 }
 
 int schedule_many(const void *items_dev, int dtype, int count, int64_t R, Arena &ar, cudaStream_t s) {
   if (count == 0) return DCSR_OK;
   if (dtype == DCSR_F32)
-    return schedule_src<float>(RowMany<float>{(const RowItem<float> *)items_dev, count, nullptr}, count, R, ar, s);
-  return schedule_src<double>(RowMany<double>{(const RowItem<double> *)items_dev, count, nullptr}, count, R, ar, s);
+    return schedule_src<float>(RowMany<float>{(const RowItem<float> *)items_dev, count, nullptr}, R, ar, s);
+  return schedule_src<double>(RowMany<double>{(const RowItem<double> *)items_dev, count, nullptr}, R, ar, s);
 }
 
 template <typename V>
@@ -274,7 +286,7 @@ static int build_schedule_t(dcsr_handle h, cudaStream_t s, Arena &ar) {
   DCSR_TRY(ensure_part(h, 1, s));
   DCSR_TRY(ar.reserve(schedule_scratch_bytes(h->n_rows), s));
   RowOne<V> src{row_item<V>(h, nullptr, nullptr, 0, 0, 0.0, 0.0)};
-  DCSR_TRY(schedule_src<V>(src, 1, h->n_rows, ar, s));
+  DCSR_TRY(schedule_src<V>(src, h->n_rows, ar, s));
   h->bins_valid = true;
   return DCSR_OK;
 }
@@ -1040,11 +1052,18 @@ struct FlatManyScan {
   Src src;
   int64_t R;
   unsigned *tmp;
-  __device__ __forceinline__ void load(int64_t g, bool ok, State &, T (&v)[1]) const {
-    v[0] = 0;
-    if (ok) {
-      const RowItem<V> &it = src.item(src.find_row(g));
-      v[0] = it.m.row_sizes[g - it.row0];
+  static constexpr bool LOAD_ALL = true;
+  __device__ __forceinline__ void load_all(int64_t base, int64_t n, State (&)[IT], T (&v)[IT][1]) const {
+    int i = base < n ? src.find_row(base) : 0;  // one search a thread; its other rows follow
+#pragma unroll
+    for (int j = 0; j < IT; j++) {
+      const int64_t g = base + 32 * j;
+      v[j][0] = 0;
+      if (g < n) {
+        i = src.next_row(i, g);
+        const RowItem<V> &it = src.item(i);
+        v[j][0] = it.m.row_sizes[g - it.row0];
+      }
     }
   }
   __device__ __forceinline__ void emit(int64_t g, bool ok, const State &, const long long (&p)[1], const T (&)[1]) const {

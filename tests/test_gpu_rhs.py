@@ -50,3 +50,39 @@ def test_right_hand_sides(dcsr, k, dtype, layout):
             lim = tol * (abs(alpha) * bound.reshape(n, k) + abs(beta) * np.abs(y0[:, :k])) + 1e-300
             assert np.all(err <= lim), f"it {it} alpha {alpha}: {np.max(err / lim):.3g}"
             np.testing.assert_array_equal(got[:, k:], y0[:, k:])
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_classes_across_a_batch(dcsr, dtype):
+    """Long, medium and short rows first and last in their matrices, matrices
+    whose rows start anywhere in a block of the schedule's scan, thousands of
+    long rows: a batch's results are the single calls', bit for bit."""
+    rng = np.random.default_rng(5)
+    sizes = [1, 2, 255, 256, 257, 2047, 2048, 2049, 1, 5000]
+    work, want = [], []
+    for q, n in enumerate(sizes):
+        m, k = 3000, 2 + q % 7
+        lens = rng.choice([0, 1, 4, 31, 40, 70, 600], n, p=[0.2, 0.3, 0.2, 0.1, 0.1, 0.05, 0.05])
+        lens[0], lens[-1] = ([2500, 40], [64, 2049], [3, 700])[q % 3]
+        rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+        cols = np.concatenate([np.sort(rng.choice(m, L, replace=False)) for L in lens]).astype(np.int32)
+        vals = rng.uniform(-1, 1, cols.size)
+        vals = vals.astype(np.float32) if dtype == 0 else vals
+        pair = []
+        for _ in range(2):
+            A, _orc = make_pair(dcsr, n, m, dtype, 0)
+            A.set_row_classes(32, 256)
+            A.from_csr(rp, cols, vals)
+            pair.append(A)
+        x = torch.tensor(rng.uniform(-1, 1, (m, k)), dtype=pair[0].dtype).cuda()
+        work.append(dict(matrix=pair[0], x=x, y=torch.zeros(n, k, dtype=x.dtype, device="cuda")))
+        want.append(pair[1].spmv(x))
+    batch = dcsr.DcsrBatch(work)
+    for _ in range(2):
+        for w in work:
+            w["y"].fill_(7)
+        batch.run()
+        torch.cuda.synchronize()
+        for q, w in enumerate(work):
+            assert torch.equal(w["y"], want[q].view_as(w["y"])), f"matrix {q}"
+    batch.close()
