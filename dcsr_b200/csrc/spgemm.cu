@@ -344,12 +344,15 @@ struct SgWarp {
 // Warp per row: P_i <= 256 (CLS SG_WARP), 256 < P_i <= 1024 (CLS SG_WARP4).
 // Instruction issue bounds it (57% of the slots, DRAM 11%): expand, sort and
 // emit take about 1700 instructions of a 169-product row, 6900 of an
-// 841-product one, so what counts is few instructions and many warps --
-// 6 blocks of 256 threads per SM in the lower class (a few spilled registers
-// included; 3: 333 us, 4: 297 us of the kernel at 131072 rows of 169 FP64
-// products), 2 x 32 products' loads at a time (4: 6% slower, 8: 10%).  Rows of
-// 841 FP32 products in a CTA each, sorted as 64-bit keys in shared memory, took
-// 1022 us for 20011 rows; in a warp each, 32 keys a lane, 220 us.  Rows come
+// 841-product one, so what counts is few instructions and many warps.  The
+// lower class at 6 blocks of 256 threads per SM with 2 x 32 products' loads at
+// a time (a few spilled registers included): 286 us of 131072 rows of 169 FP64
+// products; 3 blocks and 4 x 32: 333 us; the whole call 647 us at 4 blocks and
+// 4 x 32, 623 at 4 and 2 x 32, 610 at 6.
+// The upper class ends at 1024 products: 32 keys a lane and 8 or 12 KB of
+// shared memory per warp still leave 3 or 2 blocks per SM; twice that would
+// leave one.  Rows of 841 FP32 products in a CTA each, sorted as 64-bit keys in
+// shared memory, took 1022 us for 20011 rows; in a warp each 215 us.  Rows come
 // from a counter: a stride over the rows would give some warps only long rows
 // where lengths repeat with its period.
 template <typename V, typename K, int CLS>

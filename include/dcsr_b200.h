@@ -206,14 +206,15 @@ int dcsr_get_status(dcsr_handle h, void *stream, int32_t *status);
 int dcsr_compact(dcsr_handle h, void *stream);
 /* Grow the pool to at least pool_cap entries (contents kept). */
 int dcsr_reserve(dcsr_handle h, int64_t pool_cap, void *stream);
-/* Recompute the SpMV row bins.  Replaces device::BinRows (include/load.h:583-610);
+/* Recompute the tables of the SpMV passes (entry offsets and tile rows; the
+ * row classes of k >= 2).  Replaces device::BinRows (include/load.h:583-610);
  * bins live in the handle (no process-global __constant__ table). */
 int dcsr_bin_rows(dcsr_handle h, void *stream);
-/* Row-class thresholds of the row passes (SpMV, reductions, export): rows of
- * at most short_max entries are streamed by 32-row blocks, rows above
- * long_min are split into CTA chunks, the others get a warp each.  Defaults
- * 64 / 512 (on a power-law graph rows of 512..4096 entries run about 1.3x
- * faster in CTA chunks than one warp each); 1 <= short_max <= 256,
+/* Row-class thresholds of the SpMV with two or more right-hand sides: rows of
+ * at most short_max entries are taken by 32-row blocks, rows above long_min
+ * are split into CTA chunks, the others get a warp each.  (One right-hand
+ * side, reductions and export run over tiles of entries and have no classes.)
+ * Defaults 64 / 512; 1 <= short_max <= 256,
  * max(short_max, 256) <= long_min <= 2^20.
  * The classes change only the order of floating-point additions: every path
  * (per call, batched, served) uses the handle's thresholds, so they agree
