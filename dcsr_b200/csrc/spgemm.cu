@@ -21,7 +21,8 @@
 // 4. layout  C's rows placed straight from the staging area into C's pool
 //            with C's slack policy; the pool is allocated at an upper bound
 //            (the policy capacity of P_i per row) so nothing waits for the
-//            unique counts.  Two synchronisations: the product counts (to size
+//            unique counts.  Two synchronisations (three with rows of the upper
+//            two classes, whose lists are checked): the product counts (to size
 //            the staging area) and C's pool top.
 // Sorting by (column, p) makes every sum run in product order, so values are
 // reproducible and match the CPU oracle bit for bit; explicit zeros are kept
@@ -342,8 +343,8 @@ struct SgWarp {
 };
 
 // Warp per row: P_i <= 256 (CLS SG_WARP), 256 < P_i <= 1024 (CLS SG_WARP4).
-// Instruction issue bounds it (57% of the slots, DRAM 11%): expand, sort and
-// emit take about 1700 instructions of a 169-product row, 6900 of an
+// Instruction issue bounds it (77% of the slots, DRAM 14%): expand, sort and
+// emit take about 1800 instructions of a 169-product row, 6700 of an
 // 841-product one, so what counts is few instructions and many warps.  The
 // lower class at 6 blocks of 256 threads per SM with 2 x 32 products' loads at
 // a time (a few spilled registers included): 286 us of 131072 rows of 169 FP64
@@ -687,13 +688,22 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
   const int64_t Pg = host[SG_R_GPROD], P = host[SG_R_PROD], cap_bound = pool_capacity(hC->o, host[SG_R_CAPS]);
   const int64_t n_cta = host[SG_CTA], n_global = host[SG_GLOBAL];
   if (Pg > 0xffffffffLL) return DCSR_NOT_SUPPORTED;
+  if (n_cta + n_global > 0) {
+    // (read back before the lists are used: a list that a timed-out look-back
+    // left unfinished must not reach a kernel)
+    DCSR_TRY(scan_map(ListScan{ub, warp_max, r_cta, r_glob}, n, ar, s));
+    DCSR_CUDA(cudaMemcpyAsync(host + SG_R_STATUS, res + SG_R_STATUS, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    DCSR_CUDA(cudaStreamSynchronize(s));
+    if (host[SG_R_STATUS] == DCSR_TIMEOUT) {
+      ar.release(s);
+      return DCSR_TIMEOUT;
+    }
+  }
   // staging: row i's unique columns at ub[i]
   int32_t *tcol = nullptr;
   V *tval = nullptr;
   DCSR_CUDA(dcsr::dev_alloc((void **)&tcol, sizeof(int32_t) * (P + 1), s));
   DCSR_CUDA(dcsr::dev_alloc((void **)&tval, sizeof(V) * (P + 1), s));
-  ar.status = hC->stat + ST_STATUS;  // and from here on C's status, which load_from_rows reads
-  if (n_cta + n_global > 0) DCSR_TRY(scan_map(ListScan{ub, warp_max, r_cta, r_glob}, n, ar, s));
   const size_t cta_smem = SG_CTA_MAX * (sizeof(unsigned long long) + sizeof(V));
   static const int g_cta = [] {  // once, thread-safely: the CTA kernels' shared-memory limit, then their grid
     cudaFuncSetAttribute(k_sg_cta<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -739,7 +749,7 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
                 tcol, tval, ucnt);
   }
   // C's rows go straight from the staging area into C's pool (policy
-  // capacities); the second and last synchronisation reads C's pool top
+  // capacities); the last synchronisation reads C's pool top
   const int st = load_from_rows(hC, ub, ucnt, tcol, tval, P, cap_bound, s);
   gg.release(s);
   ar.release(s);
