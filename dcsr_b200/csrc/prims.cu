@@ -242,7 +242,7 @@ int scan_i64(const long long *in, long long *out, int64_t n, long long *total, A
 //   up to RS_BIG          one histogram kernel for all digits (its last block
 //                         scans them), then per pass one scatter kernel: a
 //                         block takes the next tile, ranks its items per warp
-//                         with match_any (ties keep input order), publishes
+//                         through lane masks (ties keep input order), publishes
 //                         its digit counts, orders the tile in shared memory,
 //                         finds the items of each digit in the tiles before
 //                         it by decoupled look-back (one thread per digit,
