@@ -218,6 +218,14 @@ constexpr int SM_LIGHT = 8, SM_HEAVY = 4;
 constexpr int SM_THREADS = 256;
 constexpr int SM_ONE_THREADS = 1024;
 constexpr int64_t SM_ONE = SM_ONE_THREADS * SM_LIGHT;
+// Light functions of up to SM_FEW items take SM_THIN a thread: at 8 a thread a
+// scan of 131072 rows runs in 64 blocks, most SMs idle and each thread's eight
+// loads and stores one after the other (placing rows 20 -> 13 us at 131072 rows,
+// 18 -> 8 at 20011).  SM_FEW is 512 blocks of that size (148
+// SMs hold 592 at once; 1024 words of look-back area, which every area has);
+// above it the wide form fills the SMs as well.
+constexpr int SM_THIN = 2;
+constexpr int64_t SM_FEW = 512 * SM_THREADS * SM_THIN;
 
 template <class F, class = void>
 struct ScanHasEmitAll : std::false_type {};
@@ -228,9 +236,9 @@ struct ScanHasLoadAll : std::false_type {};
 template <class F>
 struct ScanHasLoadAll<F, std::void_t<decltype(F::LOAD_ALL)>> : std::true_type {};
 
-template <int TH, class F>
+template <int TH, class F, int SM_ITEMS = F::IT>
 __global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY || ScanHasLoadAll<F>::value ? 3 : 4) k_scan_map(F f, int64_t n, Lookback lb) {
-  constexpr int NS = F::NS, NW = TH / 32, SM_ITEMS = F::IT;
+  constexpr int NS = F::NS, NW = TH / 32;
   __shared__ long long wsum[NS][NW];
   __shared__ long long sh_prefix[NS];
   __shared__ unsigned sh_tile;
@@ -327,6 +335,14 @@ static int scan_map(const F &f, int64_t n, Arena &ar, cudaStream_t s) {
   if constexpr (F::IT == SM_LIGHT) {
     if (n <= SM_ONE) {
       DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
+      return DCSR_OK;
+    }
+  }
+  if constexpr (F::IT == SM_LIGHT && !ScanHasLoadAll<F>::value && !ScanHasEmitAll<F>::value) {
+    if (n <= SM_FEW) {
+      const int64_t few = div_up(n, SM_THREADS * SM_THIN);
+      DCSR_TRY(ar.lookback((size_t)(LB_SCAN_WORDS * few), s, &lb));
+      DCSR_LAUNCH((k_scan_map<SM_THREADS, F, SM_THIN>), (unsigned)few, SM_THREADS, 0, s, f, n, lb);
       return DCSR_OK;
     }
   }

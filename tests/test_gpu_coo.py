@@ -33,3 +33,27 @@ def test_load(dcsr, dtype, mode, keys):
         assert orc.load_coo(r, c, v) == 0
         assert_layout_equal(dev, orc, f"{T}")
         assert_content_equal(dev, orc, f"{T}")
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 8705, 262_143, 262_144, 262_145, 264_193])
+def test_row_scans(dcsr, n):
+    """Row counts where the scans over rows change form (one block, two and eight
+    rows a thread): load, compaction after an update, export."""
+    rng = np.random.default_rng(n)
+    m, T = 500, 40_000
+    at = rng.choice(n * m, T, replace=False)
+    at[:3] = [0, n * m - 1, (n - 1) * m]
+    at = np.unique(at)
+    r, c = (at // m).astype(np.int32), (at % m).astype(np.int32)
+    v = rng.standard_normal(at.size).astype(np.float32)
+    dev, orc = make_pair(dcsr, n, m, 0, 0)
+    dev.from_coo(r, c, v)
+    assert orc.load_coo(r, c, v) == 0
+    assert_layout_equal(dev, orc, "load")
+    u = rng.integers(0, n, 5000).astype(np.int32), rng.integers(0, m, 5000).astype(np.int32)
+    w = rng.standard_normal(5000).astype(np.float32)
+    assert dev.update(*u, w) == orc.update_auto(*u, w.astype(np.float64)) == 0
+    dev.compact()
+    orc.compact()
+    assert_layout_equal(dev, orc, "compacted")
+    assert_content_equal(dev, orc, "compacted")
