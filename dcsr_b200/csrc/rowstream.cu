@@ -17,8 +17,8 @@
 //          that finishes the last chunk sums them).
 // A row's result depends only on the row and its matrix (its length picks its
 // class, the block's lengths pick G, its position its tiles), never on which
-// launch or batch it runs in.  Sums are FP64, products too (k = 1: FP32 products
-// exact for matrices of up to FLAT_EXACT_ROWS rows, rounded to FP32 above);
+// launch or batch it runs in.  Sums are FP64, products too (k = 1, FP32
+// matrices of more than FLAT_EXACT_ROWS rows: products rounded to FP32);
 // every rounding step is an explicit round-to-nearest intrinsic.
 //
 // Reference: spmv_dcsr_bin* include/spmv.inl:364-622 (seven bin kernels on
@@ -736,36 +736,36 @@ __device__ __forceinline__ void write_row(const RowItem<V> &it, int32_t row, dou
   write_y<V, OP>(it.y + (int64_t)row * it.ldy, v, it.alpha, it.beta);
 }
 
-// FP32 matrices of at most this many rows sum exact products; larger ones
-// products rounded to FP32 (summed in FP64 either way), where the gathers and
-// instructions of many tiles count: 99 against 112 us on the R-MAT matrix, its
-// error against 64 bits 3.7e-8 (2.6e-8 with exact products, most of it the
-// result's own rounding).
+// FP32 matrices of at most this many rows multiply in FP64 (every product
+// exact, and within range whatever the factors), larger ones in FP32; both sum
+// in FP64.  FP64 products cost two conversions an entry: 132 against 99 us on
+// the R-MAT matrix of 2^20 rows, whose error against 64 bits is 3.7e-8 with
+// FP32 products (2.6e-8 with exact ones, most of it the result's own rounding).
+// The line is the one the library always had between its small and its large
+// matrices, so that results keep their precision and range on either side.
 constexpr int32_t FLAT_EXACT_ROWS = 32768;
 
 #ifndef DCSR_FLAT_MINB
 #define DCSR_FLAT_MINB 4
 #endif
-// EXACT (FP32 SpMV): products are kept with their rounding errors.
+// EXACT: an FP32 SpMV's products are kept in FP64 (FP64 products of a set's
+// matrices of up to FLAT_EXACT_ROWS rows, FP32 ones of the larger).
 template <typename V, int OP, typename Src, bool XU, bool EXACT>
 __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src src) {
   __shared__ __align__(16) unsigned s_run[FT_WARPS][FT_WIN], s_row[FT_WARPS][FT_WIN];
   // Products in tile order; before them, in an SpMV, the distances from an
   // entry's number to its slot, by run; and the rows by their first entries.
   // Shared memory is kept small: what it takes, the x gathers' L1 loses (33 KB
-  // a block ran 118 us on the R-MAT matrix where 25 KB ran 102, 17 KB 99).  EXACT
-  // adds each product's rounding error (one fused multiply-add), 112 us;
-  // FP64 products (two more conversions per entry) took 132 us.
-  constexpr bool OWN = OP != OP_SPMV, ERR = EXACT && OP == OP_SPMV && sizeof(V) == 4;
-  __shared__ __align__(16) V s_prod[FT_WARPS][FT_TILE];
-  __shared__ __align__(16) float s_err[ERR ? FT_WARPS : 1][ERR ? FT_TILE : 4];
+  // a block ran 118 us on the R-MAT matrix where 25 KB ran 102, 17 KB 99).
+  constexpr bool OWN = OP != OP_SPMV, WIDE = EXACT && OP == OP_SPMV && sizeof(V) == 4;
+  using P = typename std::conditional<WIDE, double, V>::type;
+  __shared__ __align__(16) P s_prod[FT_WARPS][FT_TILE];
   __shared__ int32_t s_sdel[OWN ? FT_WARPS : 1][OWN ? FT_TILE : 1];  // (the reductions': room of their own)
   __shared__ int32_t s_hrow[FT_WARPS][FT_TILE];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned *runs = s_run[w], *starts = s_row[w];
   int32_t *hrow = s_hrow[w], *sdel = OWN ? s_sdel[OWN ? w : 0] : reinterpret_cast<int32_t *>(s_prod[w]);
-  V *prod = s_prod[w];
-  float *err = s_err[ERR ? w : 0];
+  P *prod = s_prod[w];
   const int64_t total = src.units(P_TILES), nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
   FlatTile cur, nx;
@@ -781,9 +781,13 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
     const int32_t sx = __shfl_sync(FULL, cur.sg.x, 0), sy = __shfl_sync(FULL, cur.sg.y, 0);
     const bool inner = cnt > 0 && r0 == r1 && sx >= 0 && e0 + cnt - o0 <= sy - sx;
     const bool cont = o0 < e0;  // its first row began in an earlier tile
-    const bool exact = ERR && it.m.n_rows <= FLAT_EXACT_ROWS;  // (a set's larger matrices: as on their own)
+    const bool exact = WIDE && it.m.n_rows <= FLAT_EXACT_ROWS;  // (a set's larger matrices: as on their own)
+    auto product = [&](V a, V x) -> P {
+      if constexpr (WIDE)
+        if (exact) return mul_rn((double)a, (double)x);
+      return (P)mul_rn(a, x);
+    };
     double isum = op_init<double, OP>();
-    float ierr = 0.0f;
     if (inner) {
       const int32_t base = sx + (e0 - o0) + lane;
       V a[FT_WIN];
@@ -805,12 +809,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
           xv[i] = 32 * i + lane < cnt ? (XU ? __ldg(x + col[i]) : __ldg(x + (int64_t)col[i] * it.ldx)) : V(0);
 #pragma unroll
         for (int i = 0; i < FT_WIN; i++)
-          if (32 * i + lane < cnt) {
-            const V p = mul_rn(a[i], xv[i]);
-            isum = __dadd_rn((double)p, isum);
-            if constexpr (ERR) ierr = __fadd_rn(ierr, exact ? __fmaf_rn(a[i], xv[i], -p) : 0.0f);
-          }
-        if constexpr (ERR) isum = __dadd_rn(isum, (double)ierr);
+          if (32 * i + lane < cnt) isum = __dadd_rn((double)product(a[i], xv[i]), isum);
       } else {
 #pragma unroll
         for (int i = 0; i < FT_WIN; i++)
@@ -894,12 +893,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
         for (int i = 0; i < FT_WIN; i++)
           xv[i] = 32 * i + lane < cnt ? (XU ? __ldg(x + col[i]) : __ldg(x + (int64_t)col[i] * it.ldx)) : V(0);
 #pragma unroll
-        for (int i = 0; i < FT_WIN; i++) {
-          const bool in = 32 * i + lane < cnt;
-          const V p = mul_rn(a[i], xv[i]);
-          prod[32 * i + lane] = in ? p : V(0);
-          if constexpr (ERR) err[32 * i + lane] = in && exact ? __fmaf_rn(a[i], xv[i], -p) : 0.0f;
-        }
+        for (int i = 0; i < FT_WIN; i++) prod[32 * i + lane] = 32 * i + lane < cnt ? product(a[i], xv[i]) : P(0);
       } else {
 #pragma unroll
         for (int i = 0; i < FT_WIN; i++)
@@ -922,45 +916,32 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
     } else if (cnt > 0) {
       __syncwarp();
       // ---- sums: lane l holds entries 8l .. 8l+7
-      V pv[FT_WIN];
-      float ev[ERR ? FT_WIN : 1];
-      auto eight = [&](const auto *b, auto &v) {
-        using U = typename std::remove_cv<typename std::remove_reference<decltype(*b)>::type>::type;
+      P pv[FT_WIN];
 #pragma unroll
-        for (int q = 0; q < FT_WIN; q += 16 / (int)sizeof(U)) {
-          if constexpr (sizeof(U) == 4) {
-            const float4 f = *reinterpret_cast<const float4 *>(b + q);
-            v[q] = f.x; v[q + 1] = f.y; v[q + 2] = f.z; v[q + 3] = f.w;
-          } else {
-            const double2 f = *reinterpret_cast<const double2 *>(b + q);
-            v[q] = f.x; v[q + 1] = f.y;
-          }
+      for (int q = 0; q < FT_WIN; q += 16 / (int)sizeof(P)) {
+        if constexpr (sizeof(P) == 4) {
+          const float4 f = *reinterpret_cast<const float4 *>(prod + 8 * lane + q);
+          pv[q] = f.x; pv[q + 1] = f.y; pv[q + 2] = f.z; pv[q + 3] = f.w;
+        } else {
+          const double2 f = *reinterpret_cast<const double2 *>(prod + 8 * lane + q);
+          pv[q] = f.x; pv[q + 1] = f.y;
         }
-      };
-      eight(prod + 8 * lane, pv);
-      if constexpr (ERR) eight(err + 8 * lane, ev);
+      }
       const unsigned bits = (starts[lane >> 2] >> (8 * (lane & 3))) & 0xffu;
       double acc = op_init<double, OP>(), first = acc;
-      float ea = 0.0f;  // the errors of acc's products
-      auto piece = [&]() -> double {
-        if constexpr (ERR) return __dadd_rn(acc, (double)ea);
-        return acc;
-      };
       int at = -1;  // last row start in this lane
 #pragma unroll
       for (int q = 0; q < 8; q++) {
         if ((bits >> q) & 1) {
-          if (at < 0) first = piece();  // closes a row that began in an earlier lane (or the tile's first)
-          else write_row<V, OP>(it, hrow[at], piece());
+          if (at < 0) first = acc;  // closes a row that began in an earlier lane (or the tile's first)
+          else write_row<V, OP>(it, hrow[at], acc);
           at = 8 * lane + q;
           acc = op_init<double, OP>();
-          ea = 0.0f;
         }
         acc = op_comb<double, OP>((double)pv[q], acc);
-        if constexpr (ERR) ea = __fadd_rn(ea, ev[q]);
       }
       // open pieces carried over the lanes; the last start before each lane
-      double open = piece();
+      double open = acc;
       bool seen = at >= 0;
       int last = at < 0 ? 0 : at;
 #pragma unroll
