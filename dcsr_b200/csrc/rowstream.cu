@@ -440,6 +440,11 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
+// Maxima and minima take a where it beats b, so a NaN in b stays and one in a
+// is passed over.  A row's result is NaN when its first entry is, and else the
+// extreme of its entries that are numbers: a row starts from its first entry,
+// later ones are a, earlier results b.
+constexpr bool op_extreme(int op) { return op == OP_MAX || op == OP_MIN; }
 template <typename T, int OP>
 __device__ __forceinline__ T op_comb(T a, T b) {
   if (OP == OP_MAX) return a > b ? a : b;
@@ -787,7 +792,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
         if (exact) return mul_rn((double)a, (double)x);
       return (P)mul_rn(a, x);
     };
-    double isum = op_init<double, OP>();
+    double isum = op_init<double, OP>(), lead = 0.0;
     if (inner) {
       const int32_t base = sx + (e0 - o0) + lane;
       V a[FT_WIN];
@@ -811,6 +816,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
         for (int i = 0; i < FT_WIN; i++)
           if (32 * i + lane < cnt) isum = __dadd_rn((double)product(a[i], xv[i]), isum);
       } else {
+        lead = (double)a[0];
 #pragma unroll
         for (int i = 0; i < FT_WIN; i++)
           if (32 * i + lane < cnt) isum = op_comb<double, OP>(OP == OP_COUNT ? 1.0 : (double)a[i], isum);
@@ -909,6 +915,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
       for (int o = 16; o > 0; o >>= 1) isum = op_comb<double, OP>(isum, __shfl_xor_sync(FULL, isum, o));
       if (lane == 0) {
         double *part = it.fpart + 2 * (int64_t)cur.lt;
+        if (op_extreme(OP) && !cont) isum = op_comb<double, OP>(isum, lead);  // (the row's first entry)
         if (cont) part[0] = isum;
         else if (o01 > e0 + cnt) part[1] = isum;
         else write_row<V, OP>(it, r0, isum);
@@ -929,6 +936,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
       }
       const unsigned bits = (starts[lane >> 2] >> (8 * (lane & 3))) & 0xffu;
       double acc = op_init<double, OP>(), first = acc;
+      if (op_extreme(OP) && lane == 0 && !cont) acc = (double)pv[0];  // (position 0 has no start bit)
       int at = -1;  // last row start in this lane
 #pragma unroll
       for (int q = 0; q < 8; q++) {
@@ -936,7 +944,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
           if (at < 0) first = acc;  // closes a row that began in an earlier lane (or the tile's first)
           else write_row<V, OP>(it, hrow[at], acc);
           at = 8 * lane + q;
-          acc = op_init<double, OP>();
+          acc = op_extreme(OP) ? (double)pv[q] : op_init<double, OP>();
         }
         acc = op_comb<double, OP>((double)pv[q], acc);
       }
@@ -949,7 +957,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
         const double ov = __shfl_up_sync(FULL, open, d);
         const int os = __shfl_up_sync(FULL, (int)seen, d), ol = __shfl_up_sync(FULL, last, d);
         if (lane >= d) {
-          if (!seen) open = op_comb<double, OP>(open, ov);
+          if (!seen) open = op_comb<double, OP>(open, ov);  // ov: the earlier lanes'
           seen = seen || os;
           last = max(last, ol);
         }
@@ -957,7 +965,7 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
       double carry = __shfl_up_sync(FULL, open, 1);
       int before = __shfl_up_sync(FULL, last, 1);
       if (lane == 0) {
-        carry = op_init<double, OP>();
+        carry = op_extreme(OP) ? first : op_init<double, OP>();  // nothing came before
         before = 0;
       }
       double *part = it.fpart + 2 * (int64_t)cur.lt;

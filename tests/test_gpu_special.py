@@ -5,10 +5,13 @@ The right-hand sides and values are powers of two, infinities or NaN, so that
 every sum in 64 bits is exact (or a definite infinity or NaN) in whatever order
 it is taken, and results are compared for equality.  FP32 matrices of up to
 32768 rows multiply in 64 bits, larger ones in 32 (the reference below does the
-same)."""
+same).  Row maxima and minima follow the oracle: NaN when a row's first entry
+is, later NaNs passed over."""
 import numpy as np
 import pytest
 import torch
+
+from tests.helpers import make_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -82,3 +85,43 @@ def test_spmv_one_rhs(dcsr, n, dtype, alpha, beta):
     np.testing.assert_array_equal(y.cpu().numpy(), want)
     np.testing.assert_array_equal(y2.cpu().numpy(), expect(rows2, dtype, n2, alpha, 0.0, np.zeros(n2)))
     batch.close()
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_extremes_with_nan(dcsr, dtype):
+    """NaN first, inside, last and everywhere; infinities of both signs; rows
+    within a lane's eight entries, over lanes, over tiles and over more than
+    16 tiles, starting at every kind of place in a tile."""
+    rng = np.random.default_rng(5)
+    rows = []
+    for L in (1, 2, 3, 7, 8, 9, 31, 33, 255, 256, 257, 700, 5000):
+        for kind in ("first", "inside", "last", "all", "first_two", "minus_inf", "plus_inf", "none"):
+            v = rng.uniform(-1, 1, L)
+            if kind == "first":
+                v[0] = NAN
+            elif kind == "inside":
+                v[L // 2] = NAN
+            elif kind == "last":
+                v[-1] = NAN
+            elif kind == "all":
+                v[:] = NAN
+            elif kind == "first_two":
+                v[: min(2, L)] = NAN
+            elif kind == "minus_inf":
+                v[:] = -INF
+            elif kind == "plus_inf":
+                v[:] = INF
+            rows.append(v)
+            if kind == "inside":
+                rows.append(np.zeros(0))
+    rows = [rows[i] for i in rng.permutation(len(rows))] + rows  # (and in a regular order)
+    n, m = len(rows), 6000
+    rp = np.concatenate([[0], np.cumsum([len(v) for v in rows])]).astype(np.int32)
+    cols = np.concatenate([np.arange(len(v)) for v in rows]).astype(np.int32)
+    vals = np.concatenate(rows)
+    vals = vals.astype(np.float32) if dtype == 0 else vals
+    dev, orc = make_pair(dcsr, n, m, dtype, 0)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals.astype(np.float64)) == 0
+    for op in (dcsr.REDUCE_MAX, dcsr.REDUCE_MIN):
+        np.testing.assert_array_equal(dev.row_reduce(op).cpu().double().numpy(), orc.row_reduce(op))
