@@ -99,7 +99,7 @@ struct UpdMany {
 template <typename V, typename Src>
 __global__ void k_item_init(Src src, int count, long long *gstat) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid == 0) gstat[ST_LISTS] = 0;
+  if (tid == 0) gstat[ST_LISTS] = gstat[ST_RELOC] = 0;
   for (int i = tid; i < count; i += gridDim.x * blockDim.x) {
     long long *st = src.st(i);
     st[ST_AUX] = 0;
@@ -169,7 +169,7 @@ struct __align__(16) RowDesc {
   int32_t lo;         // MERGE: first insertion point
   int32_t info;       // bits 0..7: the new segment's layer (int8, -1 none); bit 8: relocated
   int32_t cap;        // capacity of a new segment (0: none)
-  int32_t tile0;      // relocated: its first tile
+  int32_t tile0;      // relocation tiles of the rows before it (relocated: its first tile)
   long long addr;     // the new segment's offset in the batch's allocation order
 };
 
@@ -187,7 +187,7 @@ struct UpdWork {
   V *nval;                      // [T] their values (batch-order sums)
   RowDesc *desc;                // [T] per touched row
   int32_t *small, *big;         // [T] touched rows to shift (or append to) in place
-  int32_t *reloc;               // [T] touched rows relocated, in order
+  int32_t *reloc;               // [T] touched rows relocated
 };
 
 // MERGE: scans (row heads, new columns) over the sorted batch.  A thread's
@@ -370,8 +370,7 @@ __global__ void k_check(Src src, int count) {
     check_item(src.mat(i), src.st(i));
 }
 
-// Scans (new-segment capacities; relocated rows and their tiles in one word)
-// over the touched rows.
+// Scans (new-segment capacities, relocation tiles) over the touched rows.
 // MERGE: new length, capacity, layer, relocation; APPEND: the reference's
 // segment walk and allocation size.  ONE: a single matrix (its check is done
 // here in MERGE mode).
@@ -419,7 +418,7 @@ struct PlanScan {
         if (reloc) {
           layer = 0;
           cap = policy_cap(m.o, nl);
-          v[1] = (1ll << 32) | ((nl + RT_TILE - 1) / RT_TILE);  // (relocated rows, tiles)
+          v[1] = (nl + RT_TILE - 1) / RT_TILE;
         } else {
           st.list = nl - ins0 > SMALL_AFF ? 2 : 1;
         }
@@ -458,27 +457,39 @@ struct PlanScan {
     v[0] = cap;
     st.info = (layer & 0xff) | (reloc << 8);
   }
-  // Lists of the rows to shift: a warp's rows of each take consecutive places,
-  // one atomic per warp for both (an atomic per list and step queued up on
-  // the two words).
+  // Lists of the rows to shift, and of the relocated ones: a warp's rows of
+  // each take consecutive places, one atomic per warp for the first two (an
+  // atomic per list and step queued up on the two words), one for the third.
   static constexpr bool EMIT_ALL = true;
   __device__ __forceinline__ void emit_all(int64_t base, int64_t, const State (&st)[IT], const T (&)[IT][2]) const {
     if (!MERGE) return;
-    unsigned ms[IT], mb[IT], ns = 0, nb = 0;
+    unsigned ms[IT], mb[IT], mr[IT], ns = 0, nb = 0, nr = 0;
 #pragma unroll
     for (int j = 0; j < IT; j++) {
       ms[j] = __ballot_sync(FULL, st[j].list == 1);
       mb[j] = __ballot_sync(FULL, st[j].list == 2);
+      mr[j] = __ballot_sync(FULL, st[j].row >= 0 && (st[j].info & 0x100));
       ns += __popc(ms[j]);
       nb += __popc(mb[j]);
+      nr += __popc(mr[j]);
     }
-    if (ns + nb == 0) return;  // the same in every lane
+    const unsigned lt = (1u << lane_id()) - 1u;
+    if (nr) {  // the same in every lane
+      unsigned long long at = 0;
+      if (lane_id() == 0) at = atomicAdd((unsigned long long *)&w.gstat[ST_RELOC], (unsigned long long)nr);
+      at = __shfl_sync(FULL, at, 0);
+#pragma unroll
+      for (int j = 0; j < IT; j++) {
+        if (mr[j] >> lane_id() & 1u) w.reloc[at + __popc(mr[j] & lt)] = (int32_t)(base + 32 * j);
+        at += __popc(mr[j]);
+      }
+    }
+    if (ns + nb == 0) return;
     unsigned long long at = 0;
     if (lane_id() == 0)
       at = atomicAdd((unsigned long long *)&w.gstat[ST_LISTS], ((unsigned long long)nb << 32) | ns);
     at = __shfl_sync(FULL, at, 0);
     unsigned as = (unsigned)at, ab = (unsigned)(at >> 32);
-    const unsigned lt = (1u << lane_id()) - 1u;
 #pragma unroll
     for (int j = 0; j < IT; j++) {
       const int32_t t = (int32_t)(base + 32 * j);
@@ -501,10 +512,9 @@ struct PlanScan {
     d.lo = st.lo;
     d.info = st.info;
     d.cap = (int32_t)v[0];
-    d.tile0 = (int32_t)(p[1] & 0xffffffff);
+    d.tile0 = (int32_t)p[1];
     d.addr = p[0];
     w.desc[t] = d;
-    if (MERGE && v[1] && (p[1] >> 32) < w.T) w.reloc[p[1] >> 32] = (int32_t)t;
     if (!ONE && (t == 0 || w.tmat[t - 1] != st.item)) {  // the first touched row of a matrix
       src.st(st.item)[ST_A0] = p[0];
       if (t > 0) src.st(w.tmat[t - 1])[ST_A1] = p[0];
@@ -512,8 +522,7 @@ struct PlanScan {
   }
   __device__ __forceinline__ void total(const long long (&t)[2]) const {
     w.gstat[ST_TOTAL] = t[0];
-    w.gstat[ST_TILES] = t[1] & 0xffffffff;
-    w.gstat[ST_RELOC] = t[1] >> 32;
+    w.gstat[ST_TILES] = t[1];
     if (ONE) {
       src.st(0)[ST_A1] = t[0];
       // MERGE: every input of the check is known (bad indices were flagged
@@ -695,11 +704,14 @@ __device__ __forceinline__ void apply_list(const Src &src, const UpdWork<V> &w, 
   }
 }
 
-// Relocation of rows into fresh segments, a warp per RT_TILE positions.
+// Relocation of rows into fresh segments, a warp per RT_TILE positions.  A
+// tile's row is the last touched row with no more tiles before it than the
+// tile's number (rows without tiles share theirs with the next row's): the
+// relocated rows need no order of their own, and no count in the plan's scan.
 template <typename V, typename Src>
 __device__ __forceinline__ void relocate_tiles(const Src &src, const UpdWork<V> &w, unsigned *mask) {
   const Sub<32> sub;
-  const int64_t ntiles = w.gstat[ST_TILES], nr = w.gstat[ST_RELOC];
+  const int64_t ntiles = w.gstat[ST_TILES], nt = w.gstat[ST_TOUCHED];
   const int lane = lane_id();
   const int64_t nw = (int64_t)gridDim.x * (blockDim.x / 32);
   // the number of leading i in [0, n) for which f(i) holds: 32 probes a step
@@ -717,8 +729,8 @@ __device__ __forceinline__ void relocate_tiles(const Src &src, const UpdWork<V> 
     return lo;
   };
   for (int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; q < ntiles; q += nw) {
-    const int64_t at = leading(nr, [&](int64_t i) { return w.desc[w.reloc[i]].tile0 <= q; }) - 1;
-    const RowDesc d = w.desc[w.reloc[at]];
+    const int64_t at = leading(nt, [&](int64_t i) { return w.desc[i].tile0 <= q; }) - 1;
+    const RowDesc d = w.desc[at];
     if (!src.st(d.item)[ST_GO]) continue;
     const Mat<V> &m = src.mat(d.item);
     const Chain ch = load_chain(m, d.row);

@@ -81,3 +81,59 @@ def test_batch_sizes_around_the_scan_tiles(dcsr, T):
             assert dev.update(r, c, v) == orc.update_auto(r, c, v) == 0
             assert_layout_equal(dev, orc, f"T={T}")
             assert_content_equal(dev, orc, f"T={T}")
+
+
+def grown_rows(rng, n, segs):
+    """n rows of 2 to 4 entries and triples that relocate most of them: a new
+    first column (reloc_min = 0), or one past each row's capacity (max_segs = 1)."""
+    lens = rng.integers(2, 5, n)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = np.concatenate([10 * np.arange(1, L + 1) for L in lens]).astype(np.int32)
+    each = 1 if segs else 7
+    hit = np.sort(rng.choice(n, n - n // 50, replace=False))  # some rows stay
+    r = np.repeat(hit, each).astype(np.int32)
+    c = (3 + np.tile(np.arange(each), hit.size) * 11 + (r % 5)).astype(np.int32)
+    order = rng.permutation(r.size)
+    return rp, cols, rng.uniform(-1, 1, cols.size), r[order], c[order], rng.uniform(-1, 1, r.size)
+
+
+@pytest.mark.parametrize("n", [66_000, 68_000, 140_000])
+@pytest.mark.parametrize("segs", [0, 1])
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_many_relocated_rows(dcsr, n, segs, dtype):
+    """More rows relocated by one update than 16 bits count (65536), and than
+    twice that."""
+    rng = np.random.default_rng(n + segs)
+    rp, cols, vals, r, c, v = grown_rows(rng, n, segs)
+    kw = dict(reloc_min=0) if segs else dict(max_segs=1)
+    dev, orc = make_pair(dcsr, n, M, dtype, 0, spare_x16=64, **kw)
+    ft = np.float32 if dtype == 0 else np.float64
+    vals, v = vals.astype(ft), v.astype(ft)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals.astype(np.float64)) == 0
+    for it in range(2):
+        assert dev.update(r, c + 60 * it, v) == orc.update_auto(r, c + 60 * it, v.astype(np.float64)) == 0
+        assert_layout_equal(dev, orc, f"update {it}")
+        assert_content_equal(dev, orc, f"update {it}")
+
+
+def test_many_relocated_rows_batched(dcsr):
+    """The same, counted over the matrices of a batch."""
+    import torch
+    work, orcs = [], []
+    for q, n in enumerate([40_000, 66_000, 3, 50_000]):
+        rng = np.random.default_rng(q)
+        rp, cols, vals, r, c, v = grown_rows(rng, n, 1)
+        dev, orc = make_pair(dcsr, n, M, 1, 0, spare_x16=64, reloc_min=0)
+        dev.from_csr(rp, cols, vals)
+        assert orc.load_csr(rp, cols, vals) == 0
+        assert orc.update_auto(r, c, v) == 0
+        work.append(dict(matrix=dev, rows=torch.tensor(r).cuda(), cols=torch.tensor(c).cuda(), vals=torch.tensor(v).cuda()))
+        orcs.append(orc)
+    batch = dcsr.DcsrBatch(work)
+    batch.run()
+    assert not batch.status().any()
+    for w, orc in zip(work, orcs):
+        assert_layout_equal(w["matrix"], orc, "batched")
+        assert_content_equal(w["matrix"], orc, "batched")
+    batch.close()
