@@ -118,9 +118,11 @@ struct Mat {
 // an epoch that the last block of every such kernel advances, the dynamic
 // tile counter and the finished-block counter that block resets, the radix
 // digit histograms (re-zeroed by the sort's last pass), and the look-back
-// words, each tagged with the epoch that wrote it (prims.cu).  Zeroed once at
-// allocation: a word left by an earlier kernel carries another epoch, so
-// nothing is cleared between kernels.
+// words, each tagged with the epoch that wrote it (lookback.cuh).  Zeroed once
+// at allocation: a word left by an earlier kernel carries another epoch, so
+// nothing is cleared between kernels.  The sort's words (8 bytes, all tagged)
+// and the scans' (16 bytes, one tag) lie in areas of their own: half of a
+// scan's word is bare sums, which a sort could take for a tag.
 // A wait that reaches its iteration limit gives up: it counts a fault,
 // marks the area's fault word with the kernel's epoch (the other waits of
 // that kernel then give up early instead of each spinning to the limit) and
@@ -138,13 +140,26 @@ struct Lookback {
   unsigned *tiles, *done;
   unsigned long long *fault;  // epoch tag + 1 of the last kernel whose wait gave up
   unsigned *hist;             // [8][256]
-  unsigned long long *flag;   // look-back words
-  unsigned long long slots;   // entries of flag
+  unsigned long long *flag;   // the sort's look-back words
+  unsigned long long *scan;   // the scans' (16-byte aligned)
+  unsigned long long slots;   // entries of each (even)
   long long *status;          // the operation's status word, or null
   LookbackGlobals *g;         // the device's wait limit, test switch and fault count
 };
 constexpr size_t LB_HEADER = 64 + 8 * 256 * 4;
 static_assert(LB_HEADER % 16 == 0, "look-back words of 16 bytes follow the header");
+// A look-back area of `slots` (even) words of each kind: its size, and its parts.
+constexpr size_t lb_bytes(size_t slots) { return LB_HEADER + 2 * 8 * slots; }
+inline void lb_parts(unsigned char *lb, size_t slots, Lookback *out) {
+  out->epoch = (unsigned long long *)lb;
+  out->tiles = (unsigned *)(lb + 8);
+  out->done = (unsigned *)(lb + 12);
+  out->fault = (unsigned long long *)(lb + 16);
+  out->hist = (unsigned *)(lb + 64);
+  out->flag = (unsigned long long *)(lb + LB_HEADER);
+  out->scan = out->flag + slots;
+  out->slots = slots;
+}
 
 // Stream-ordered scratch arena: one device buffer, bump-allocated per
 // operation, grown (stream-ordered free + malloc) when an operation needs more;
@@ -161,8 +176,8 @@ struct Arena {
   // Set when take() could not fit a request (a sizing bug): the caller
   // returns DCSR_OOM instead of launching with the null pointer.
   bool overflow = false;
-  // Look-back area with at least `slots` slots (grown, and zeroed, outside
-  // stream capture only: a captured graph must find it sized already).
+  // Look-back area with at least `slots` words of each kind (grown, and zeroed,
+  // outside stream capture only: a captured graph must find it sized already).
   int lookback(size_t slots, cudaStream_t s, Lookback *out) {
     if (slots > lb_slots || !lb) {
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -171,19 +186,13 @@ struct Arena {
       if (lb) DCSR_CUDA(dcsr::dev_free(lb, s));
       lb = nullptr;
       lb_slots = 0;
-      const size_t want = slots + slots / 4 + 1024;
-      const size_t bytes = LB_HEADER + 8 * want;
+      const size_t want = (slots + slots / 4 + 1024 + 1) & ~(size_t)1;
+      const size_t bytes = lb_bytes(want);
       DCSR_CUDA(dcsr::dev_alloc((void **)&lb, bytes, s));
       DCSR_CUDA(cudaMemsetAsync(lb, 0, bytes, s));
       lb_slots = want;
     }
-    out->epoch = (unsigned long long *)lb;
-    out->tiles = (unsigned *)(lb + 8);
-    out->done = (unsigned *)(lb + 12);
-    out->fault = (unsigned long long *)(lb + 16);
-    out->hist = (unsigned *)(lb + 64);
-    out->flag = (unsigned long long *)(lb + LB_HEADER);
-    out->slots = lb_slots;
+    lb_parts(lb, lb_slots, out);
     out->status = status;
     return lookback_globals(&out->g);
   }

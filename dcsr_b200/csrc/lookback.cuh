@@ -27,12 +27,14 @@ __device__ __forceinline__ unsigned long long ld_vol(const unsigned long long *p
 // one load -- no fences, no second load.  A sort's word per (tile, digit)
 // holds a count (kind 1: the tile's aggregate, 2: its inclusive prefix); a
 // scan has one 128-bit word per tile, tag and kind above 96 bits of
-// sums, stored and loaded whole.  A word is current when its tag is the
+// sums, stored and loaded whole.  The two kinds have areas of their own: the
+// lower half of a scan's word has no tag, and read as a sort's word its sums
+// could be taken for a current count.  A word is current when its tag is the
 // kernel's; the tag repeats every 2^30 kernels on one area, so the kernel
-// whose last block advances the epoch to such a multiple clears the area
+// whose last block advances the epoch to such a multiple clears both areas
 // (lb_advance) and a stale word never matches.
 constexpr unsigned long long LB_EMASK = (1ull << 30) - 1;
-__device__ __forceinline__ unsigned long long lb_pack(unsigned long long e, int kind, unsigned v) {
+__host__ __device__ __forceinline__ unsigned long long lb_pack(unsigned long long e, int kind, unsigned v) {
   return ((e & LB_EMASK) << 34) | ((unsigned long long)kind << 32) | v;
 }
 
@@ -68,13 +70,13 @@ __device__ __forceinline__ bool lb_end(const Lookback &lb) {
 }
 
 // The last block (all its threads): reset the counters and advance the
-// epoch; at a multiple of 2^30 clear the slots first (packed radix tags).
+// epoch; at a multiple of 2^30 clear the words first (their tags come round).
 __device__ __forceinline__ void lb_advance(const Lookback &lb) {
   __shared__ unsigned long long next;
   if (threadIdx.x == 0) next = ld_vol(lb.epoch) + 1;
   __syncthreads();
   if ((next & LB_EMASK) == 0)
-    for (unsigned long long i = threadIdx.x; i < lb.slots; i += blockDim.x) lb.flag[i] = 0;
+    for (unsigned long long i = threadIdx.x; i < lb.slots; i += blockDim.x) lb.flag[i] = lb.scan[i] = 0;
   __syncthreads();
   if (threadIdx.x == 0) {
     *(volatile unsigned *)lb.tiles = 0;
@@ -104,7 +106,7 @@ __device__ __forceinline__ void lb_store(unsigned long long *p, const LbWord &w)
                : "memory");
 }
 template <int NS>
-__device__ __forceinline__ LbWord lb_word(unsigned long long e, int kind, const long long (&v)[NS]) {
+__host__ __device__ __forceinline__ LbWord lb_word(unsigned long long e, int kind, const long long (&v)[NS]) {
   static_assert(NS >= 1 && NS <= 3, "one to three sums");
   LbWord w;
   w.lo = (unsigned long long)v[0];
@@ -121,7 +123,7 @@ __device__ __forceinline__ LbWord lb_word(unsigned long long e, int kind, const 
   return w;
 }
 template <int NS>
-__device__ __forceinline__ long long lb_sum(const LbWord &w, int q) {
+__host__ __device__ __forceinline__ long long lb_sum(const LbWord &w, int q) {
   if constexpr (NS == 1) return (long long)w.lo;
   if constexpr (NS == 3) return (long long)(unsigned)(q == 0 ? w.lo : q == 1 ? w.lo >> 32 : w.hi);
   return q == 0 ? (long long)(w.lo & 0xffffffffffffull) : (long long)((w.lo >> 48) | ((w.hi & 0xffffffffull) << 16));
@@ -142,7 +144,7 @@ __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long lo
                                             const long long (&agg)[NS], long long (&excl)[NS]) {
   const int lane = lane_id();
   const unsigned tag2 = (unsigned)(e & LB_EMASK) << 2;  // a current word's upper 32 bits, less its kind
-  unsigned long long *w = lb.flag;
+  unsigned long long *w = lb.scan;
 #pragma unroll
   for (int q = 0; q < NS; q++) excl[q] = 0;
   if (t == t0) {

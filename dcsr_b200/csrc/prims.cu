@@ -124,7 +124,7 @@ struct ScanArgs {
 };
 
 // Exclusive scan, one pass: tiles of SCAN_TILE values; warp 0 looks back over
-// 32 earlier tiles of its array at a time.  In place (in == out) is allowed.
+// the earlier tiles (lb_lookback).  In place (in == out) is allowed.
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_1p(ScanArgs a, Lookback lb) {
   __shared__ long long tile[SCAN_TILE];
   __shared__ unsigned sh_tile;
@@ -887,7 +887,8 @@ constexpr size_t NOALLOC_PART_BYTES = (size_t)(DCSR_NOALLOC_MAX_KEYS / RBK_PIECE
 constexpr size_t NOALLOC_LB_SLOTS = LB_SCAN_WORDS * ((DCSR_NOALLOC_MAX_KEYS + SCAN_TILE - 1) / SCAN_TILE) + 4;
 // (a multiple of 256: the look-back area behind it holds 16-byte words)
 constexpr size_t NOALLOC_ARENA_BYTES = (NOALLOC_POS_BYTES + 256 + NOALLOC_PART_BYTES + 256 + 255) / 256 * 256;
-constexpr size_t NOALLOC_BYTES = NOALLOC_ARENA_BYTES + LB_HEADER + 8 * NOALLOC_LB_SLOTS;
+static_assert(NOALLOC_LB_SLOTS % 2 == 0, "the scans' words start on 16 bytes");
+constexpr size_t NOALLOC_BYTES = NOALLOC_ARENA_BYTES + lb_bytes(NOALLOC_LB_SLOTS);
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
 
 static int noalloc_scratch(void **out) {

@@ -111,3 +111,29 @@ def test_reduce_by_key_long_runs(dcsr, runs):
         uk, start = np.unique(keys, return_index=True)
         np.testing.assert_array_equal(ko.cpu().numpy(), uk)
         np.testing.assert_array_equal(vo.cpu().double().numpy(), np.add.reduceat(vals, start))
+
+
+def test_schedule_scans_and_sorts_take_turns(dcsr):
+    """SpMVs with k >= 2 of a matrix with long rows (the schedule's scan carries
+    their chunk counts) alternate with updates large enough for the look-back
+    sort on one handle, over epochs that pass the chunk counts' values."""
+    rng = np.random.default_rng(21)
+    n, T = 20_000, 20_000
+    lens = rng.poisson(3.0, n)
+    lens[rng.choice(n, 90, replace=False)] = 2500
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(n, L, replace=False)) for L in lens if L]).astype(np.int32)
+    vals = rng.uniform(-1, 1, cols.size)
+    dev, orc = make_pair(dcsr, n, n, dcsr.F64, 0)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals) == 0
+    x = torch.tensor(rng.uniform(-1, 1, (n, 2))).cuda()
+    for it in range(60):
+        r = rng.integers(0, n, T).astype(np.int32)
+        c = rng.integers(0, 40, T).astype(np.int32)  # few columns: the structure settles
+        v = rng.uniform(-1, 1, T)
+        dev.spmv(x)
+        assert dev.update(r, c, v) == orc.update_auto(r, c, v) == 0
+        if it % 6 == 5:
+            assert_layout_equal(dev, orc, f"round {it}")
+            assert_content_equal(dev, orc, f"round {it}")
