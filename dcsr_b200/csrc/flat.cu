@@ -49,21 +49,21 @@ struct CompactScan {
   int64_t tiles;
   long long *top;
   __device__ __forceinline__ void load(int64_t i, bool ok, State &, T (&v)[2]) const {
-    v[0] = ok && i < n ? sizes[i] : 0;
-    v[1] = ok && i < n ? policy_cap(o, v[0]) : 0;
+    v[1] = ok && i < n ? sizes[i] : 0;
+    v[0] = ok && i < n ? policy_cap(o, v[1]) : 0;
   }
   __device__ __forceinline__ void emit(int64_t i, bool ok, const State &, const long long (&p)[2],
                                        const T (&v)[2]) const {
     if (ok && i < n) {
-      off[i] = (int32_t)p[0];
-      caps[i] = (int32_t)p[1];
+      off[i] = (int32_t)p[1];
+      caps[i] = (int32_t)p[0];
     }
-    flat_mark_tiles((int32_t)i, p[0], v[0], tile_row, tiles);
+    flat_mark_tiles((int32_t)i, p[1], v[1], tile_row, tiles);
   }
   __device__ __forceinline__ void total(const long long (&t)[2]) const {
-    off[n] = (int32_t)t[0];
-    caps[n] = (int32_t)t[1];
-    *top = t[1];
+    off[n] = (int32_t)t[1];
+    caps[n] = (int32_t)t[0];
+    *top = t[0];
   }
 };
 
@@ -102,20 +102,20 @@ struct CountScan {
   int32_t *rp, *caps;
   long long *top;
   __device__ __forceinline__ void load(int64_t i, bool ok, State &, T (&v)[2]) const {
-    v[0] = ok && i < n ? cnt[i] : 0;
-    v[1] = ok && i < n ? policy_cap(o, v[0]) : 0;
+    v[1] = ok && i < n ? cnt[i] : 0;
+    v[0] = ok && i < n ? policy_cap(o, v[1]) : 0;
   }
   __device__ __forceinline__ void emit(int64_t i, bool ok, const State &, const long long (&p)[2],
                                        const T (&)[2]) const {
     if (ok && i < n) {
-      rp[i] = (int32_t)p[0];
-      caps[i] = (int32_t)p[1];
+      rp[i] = (int32_t)p[1];
+      caps[i] = (int32_t)p[0];
     }
   }
   __device__ __forceinline__ void total(const long long (&t)[2]) const {
-    rp[n] = (int32_t)t[0];
-    caps[n] = (int32_t)t[1];
-    *top = t[1];
+    rp[n] = (int32_t)t[1];
+    caps[n] = (int32_t)t[0];
+    *top = t[0];
   }
 };
 
@@ -133,25 +133,25 @@ struct PlaceScan {
   int64_t tiles;
   long long *top;
   __device__ __forceinline__ void load(int64_t i, bool ok, State &, T (&v)[2]) const {
-    v[0] = ok && i < n ? lens[i] : 0;
-    v[1] = ok && i < n ? policy_cap(o, v[0]) : 0;
+    v[1] = ok && i < n ? lens[i] : 0;
+    v[0] = ok && i < n ? policy_cap(o, v[1]) : 0;
   }
   __device__ __forceinline__ void emit(int64_t i, bool ok, const State &, const long long (&p)[2],
                                        const T (&v)[2]) const {
     if (ok && i < n) {
-      off[i] = (int32_t)p[0];
-      caps[i] = (int32_t)p[1];
-      row_sizes[i] = (int32_t)v[0];
-      *reinterpret_cast<int2 *>(seg + 2 * i) = make_int2((int32_t)p[1], (int32_t)(p[1] + v[1]));
+      off[i] = (int32_t)p[1];
+      caps[i] = (int32_t)p[0];
+      row_sizes[i] = (int32_t)v[1];
+      *reinterpret_cast<int2 *>(seg + 2 * i) = make_int2((int32_t)p[0], (int32_t)(p[0] + v[0]));
       for (int l = 1; l < max_segs; l++)
         *reinterpret_cast<int2 *>(seg + (int64_t)l * pitch + 2 * i) = make_int2(-1, -1);
     }
-    flat_mark_tiles((int32_t)i, p[0], v[0], tile_row, tiles);
+    flat_mark_tiles((int32_t)i, p[1], v[1], tile_row, tiles);
   }
   __device__ __forceinline__ void total(const long long (&t)[2]) const {
-    off[n] = (int32_t)t[0];
-    caps[n] = row_sizes[n] = (int32_t)t[1];
-    *top = t[1];
+    off[n] = (int32_t)t[1];
+    caps[n] = row_sizes[n] = (int32_t)t[0];
+    *top = t[0];
   }
 };
 

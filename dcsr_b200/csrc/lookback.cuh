@@ -88,7 +88,9 @@ __device__ __forceinline__ void lb_advance(const Lookback &lb) {
 
 // A scan's 128-bit look-back word (16-byte aligned), written and read as one
 // relaxed access: hi = tag | kind | 32 bits, lo = 64 bits; the 96 bits hold
-// one 64-bit sum or two of 48 bits.
+// one sum of 64 bits, one of 64 and one of 32, or three of 32 (the 32-bit ones
+// modulo 2^32).  Of two sums the first is the one that may be large: layout
+// capacities, whose options allow 2^31 entries a row.
 struct LbWord {
   unsigned long long lo, hi;
 };
@@ -115,18 +117,14 @@ __host__ __device__ __forceinline__ LbWord lb_word(unsigned long long e, int kin
     w.lo = (w.lo & 0xffffffffull) | ((unsigned long long)v[1] << 32);
     w.hi |= (unsigned long long)v[2] & 0xffffffffull;
   }
-  if constexpr (NS == 2) {
-    const unsigned long long b = (unsigned long long)v[1];
-    w.lo = (w.lo & 0xffffffffffffull) | (b << 48);
-    w.hi |= (b >> 16) & 0xffffffffull;
-  }
+  if constexpr (NS == 2) w.hi |= (unsigned long long)v[1] & 0xffffffffull;
   return w;
 }
 template <int NS>
 __host__ __device__ __forceinline__ long long lb_sum(const LbWord &w, int q) {
   if constexpr (NS == 1) return (long long)w.lo;
   if constexpr (NS == 3) return (long long)(unsigned)(q == 0 ? w.lo : q == 1 ? w.lo >> 32 : w.hi);
-  return q == 0 ? (long long)(w.lo & 0xffffffffffffull) : (long long)((w.lo >> 48) | ((w.hi & 0xffffffffull) << 16));
+  return q == 0 ? (long long)w.lo : (long long)(unsigned)w.hi;
 }
 // Look-back words (8 bytes) that a scan of `tiles` tiles needs.
 constexpr int LB_SCAN_WORDS = 2;

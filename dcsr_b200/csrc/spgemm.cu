@@ -83,9 +83,11 @@ __global__ void __launch_bounds__(SG_THREADS) k_sg_count(Mat<V> A, Mat<V> B, int
   if (threadIdx.x == 0 && gprod) atomicAdd((unsigned long long *)&res[SG_R_GPROD], gprod);
 }
 
-// Staging offsets ub (n + 1) from the product counts, and the capacities that
-// C's layout policy gives rows of P_i entries added up (an upper bound of the
-// pool, whatever the rows' unique columns); no unique columns yet.
+// The capacities that C's layout policy gives rows of P_i entries added up (an
+// upper bound of the pool, whatever the rows' unique columns), and the staging
+// offsets ub (n + 1) from the product counts; no unique columns yet.  The
+// products may pass the 32 bits of a second sum only where the capacities, at
+// least as many, pass the pool's range: the call then ends before they are used.
 struct StageScan {
   static constexpr int NS = 2, IT = SM_LIGHT;
   using T = long long;
@@ -95,20 +97,20 @@ struct StageScan {
   long long *ub, *ucnt, *res;
   int32_t n;
   __device__ __forceinline__ void load(int64_t i, bool ok, State &, T (&v)[2]) const {
-    v[0] = ok ? cnt[i] : 0;
-    v[1] = ok ? policy_cap(o, v[0]) : 0;
+    v[1] = ok ? cnt[i] : 0;
+    v[0] = ok ? policy_cap(o, v[1]) : 0;
   }
   __device__ __forceinline__ void emit(int64_t i, bool ok, const State &, const long long (&p)[2],
                                        const T (&)[2]) const {
     if (ok) {
-      ub[i] = p[0];
+      ub[i] = p[1];
       ucnt[i] = 0;
     }
   }
   __device__ __forceinline__ void total(const long long (&t)[2]) const {
-    ub[n] = t[0];
-    res[SG_R_PROD] = t[0];
-    res[SG_R_CAPS] = t[1];
+    ub[n] = t[1];
+    res[SG_R_PROD] = t[1];
+    res[SG_R_CAPS] = t[0];
   }
 };
 
@@ -687,7 +689,14 @@ static int spgemm_impl(dcsr_handle hA, dcsr_handle hB, dcsr_handle hC, cudaStrea
   }
   const int64_t Pg = host[SG_R_GPROD], P = host[SG_R_PROD], cap_bound = pool_capacity(hC->o, host[SG_R_CAPS]);
   const int64_t n_cta = host[SG_CTA], n_global = host[SG_GLOBAL];
-  if (Pg > 0xffffffffLL) return DCSR_NOT_SUPPORTED;
+  // C's pool is allocated for cap_bound entries: out of its index range, no
+  // staging either
+  const int refused = Pg > 0xffffffffLL ? DCSR_NOT_SUPPORTED
+                      : host[SG_R_CAPS] > 0x7fffffffLL || cap_bound > 0x7fffffffLL ? DCSR_OOM : DCSR_OK;
+  if (refused != DCSR_OK) {
+    ar.release(s);
+    return refused;
+  }
   if (n_cta + n_global > 0) {
     // (read back before the lists are used: a list that a timed-out look-back
     // left unfinished must not reach a kernel)

@@ -1,7 +1,7 @@
 // The look-back words of the single-pass scans and sorts on the CPU: where
-// the two kinds lie in an area, and that no word a scan leaves can be read as
-// a current one by a sort on the same area, in whatever order operations
-// with whatever sums alternate.
+// the two kinds lie in an area, that no word a scan leaves can be read as a
+// current one by a sort on the same area, in whatever order operations with
+// whatever sums alternate, and the range of the sums that a scan's word carries.
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -45,6 +45,26 @@ int main() {
       }
       for (size_t i = 0; i < slots; i++) CHECK(!sort_takes(lb.flag[i], e + 1));
     }
+  }
+  // what a word carries: a sum of 64 bits; sums of 64 and of 32; three of 32
+  const long long big[] = {0, 1, 65535ll << 32, 1ll << 48, (1ll << 48) + 12345, 1ll << 61, INT64_MAX};
+  const long long small[] = {0, 1, 65536, 0x7fffffffll, 0xffffffffll};
+  for (unsigned long long e : {1ull, 77ull, LB_EMASK}) {
+    for (long long a : big) {
+      const long long v1[1] = {a};
+      CHECK(lb_sum<1>(lb_word<1>(e, 1, v1), 0) == a);
+      for (long long b : small) {
+        const long long v2[2] = {a, b};
+        const LbWord w = lb_word<2>(e, 2, v2);
+        CHECK(lb_sum<2>(w, 0) == a && lb_sum<2>(w, 1) == b && w.hi >> 32 == ((e << 2) | 2));
+      }
+    }
+    for (long long a : small)
+      for (long long b : small) {
+        const long long v3[3] = {a, b, a};
+        const LbWord w = lb_word<3>(e, 1, v3);
+        CHECK(lb_sum<3>(w, 0) == a && lb_sum<3>(w, 1) == b && lb_sum<3>(w, 2) == a && w.hi >> 32 == ((e << 2) | 1));
+      }
   }
   printf("ok\n");
   return 0;
