@@ -34,6 +34,7 @@ struct OffsetsScan {
     flat_mark_tiles((int32_t)i, p[0], v[0], tile_row, tiles);
   }
   __device__ __forceinline__ void total(const long long (&t)[1]) const { off[n] = (int32_t)t[0]; }
+  __device__ __forceinline__ void fault() const { off[n] = FLAT_BAD; }
 };
 
 // Row lengths -> CSR row pointer, tile rows and the offsets of the policy's
@@ -153,6 +154,7 @@ struct PlaceScan {
     caps[n] = row_sizes[n] = (int32_t)t[0];
     *top = t[0];
   }
+  __device__ __forceinline__ void fault() const { off[n] = FLAT_BAD; }
 };
 
 // Where the entries come from / go to: CSR order, a row's start given by an

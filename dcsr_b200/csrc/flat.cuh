@@ -27,6 +27,9 @@ constexpr int32_t FT_ROWS = 512;
 constexpr int FT_THREADS = 256;
 constexpr int FT_WARPS = FT_THREADS / 32;
 
+// The entry count (off[n]) of tables whose scan gave up a look-back wait: no
+// tile, so no pass reads a row's offsets or a tile's row from them.
+constexpr int32_t FLAT_BAD = -1;
 inline int64_t flat_tiles(int64_t entries) { return div_up(entries, FT_TILE); }
 
 // The tiles that start within row r's entries [off, off+len) (called by whole

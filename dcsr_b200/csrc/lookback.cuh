@@ -44,6 +44,7 @@ __host__ __device__ __forceinline__ unsigned long long lb_pack(unsigned long lon
 __device__ __forceinline__ void lb_give_up(const Lookback &lb, unsigned long long e) {
   atomicAdd(&lb.g->faults, 1ull);
   *(volatile unsigned long long *)lb.fault = (e & LB_EMASK) + 1;
+  __threadfence();  // before the block counts as finished
   if (lb.status) atomicCAS(reinterpret_cast<unsigned long long *>(lb.status), 0ull, (unsigned long long)DCSR_TIMEOUT);
 }
 // True when another wait of this kernel (epoch e) gave up already.
@@ -209,6 +210,8 @@ __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long lo
 //   emit(i, ok, st, excl[NS], v[NS]) item i's prefix; called by whole warps (with a member
 //                                    EMIT_ALL after emit_all(base, n, st[], v[][NS]))
 //   total(tot[NS])                   one thread, the totals
+//   fault()                          (if there) one thread, last of all, when a look-back wait gave up:
+//                                    marks the result so that kernels behind it do not use it
 // A warp takes 32*IT consecutive items, item j*32 + lane in lane's j-th step
 // (coalesced, and every step's prefix by a warp scan in registers -- no
 // staging through shared memory), a block SM_THREADS*IT.  Light functions
@@ -235,6 +238,11 @@ template <class F, class = void>
 struct ScanHasLoadAll : std::false_type {};
 template <class F>
 struct ScanHasLoadAll<F, std::void_t<decltype(F::LOAD_ALL)>> : std::true_type {};
+
+template <class F, class = void>
+struct ScanHasFault : std::false_type {};
+template <class F>
+struct ScanHasFault<F, std::void_t<decltype(&F::fault)>> : std::true_type {};
 
 template <int TH, class F, int SM_ITEMS = F::IT>
 __global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY || ScanHasLoadAll<F>::value ? 3 : 4) k_scan_map(F f, int64_t n, Lookback lb) {
@@ -318,8 +326,13 @@ __global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY ||
 #pragma unroll
     for (int q = 0; q < NS; q++) tot[q] = (single ? 0 : sh_prefix[q]) + agg[q];
     f.total(tot);
+    if constexpr (ScanHasFault<F>::value) __threadfence();  // (fault() may write over it from another block)
   }
-  if (!single && lb_end(lb)) lb_advance(lb);
+  if (!single && lb_end(lb)) {
+    if constexpr (ScanHasFault<F>::value)
+      if (threadIdx.x == 0 && lb_faulted(lb, e)) f.fault();
+    lb_advance(lb);
+  }
 }
 
 // n >= 1 items.  Needs LB_SCAN_WORDS look-back slots per SM_THREADS*IT items.

@@ -604,8 +604,11 @@ int dcsr_nnz(dcsr_handle h, int64_t *nnz, void *stream) {
     int32_t t = 0;
     DCSR_CUDA(cudaMemcpyAsync(&t, h->flat_off + h->n_rows, sizeof(t), cudaMemcpyDeviceToHost, s));
     DCSR_CUDA(cudaStreamSynchronize(s));
-    *nnz = t;
-    return DCSR_OK;
+    if (t >= 0) {
+      *nnz = t;
+      return DCSR_OK;
+    }
+    h->flat_valid = false;  // the tables' scan gave up
   }
   DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX + 1, 0, sizeof(long long), s));
   if (h->n_rows > 0)

@@ -143,7 +143,8 @@ struct SchedScan {
     bool keep;  // long or medium, or the first or last row of its matrix
   };
   Src src;
-  uint4 *tmp;
+  int64_t R;
+  uint4 *tmp;  // [R + 1]: the last one nonzero when the scan gave up
   // (a search per row: with one a thread and its rows following, as below, the
   // kernel took 31 us instead of 24)
   __device__ __forceinline__ void load(int64_t g, bool ok, State &st, T (&v)[3]) const {
@@ -166,21 +167,24 @@ struct SchedScan {
                                        const T (&)[3]) const {
     if (st.keep) tmp[g] = make_uint4((unsigned)p[0], (unsigned)p[1], (unsigned)p[2], 0);
   }
-  __device__ __forceinline__ void total(const long long (&)[3]) const {}
+  __device__ __forceinline__ void total(const long long (&)[3]) const { tmp[R].x = 0; }
+  __device__ __forceinline__ void fault() const { tmp[R].x = 1; }
 };
 
 // Lists of the long and medium rows; per matrix the class counts and the
-// long-row offset sentinel (its last row's thread).
+// long-row offset sentinel (its last row's thread).  None of either when the
+// scan gave up.
 template <typename V, typename Src>
 __global__ void k_sched_emit(Src src, int64_t R, const uint4 *tmp) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const bool bad = tmp[R].x != 0;
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < R; g += stride) {
     const RowItem<V> &it = src.item(src.find_row(g));
     const int64_t r = g - it.row0;
-    const int32_t L = it.m.row_sizes[r];
+    const int32_t L = bad ? 0 : it.m.row_sizes[r];
     const bool last = r == it.m.n_rows - 1;
     if (L <= it.short_max && !last) continue;
-    const uint4 at = tmp[g], a0 = tmp[it.row0];
+    const uint4 at = bad ? make_uint4(0, 0, 0, 0) : tmp[g], a0 = bad ? at : tmp[it.row0];
     unsigned li = at.x - a0.x, c0 = at.y - a0.y, mi = at.z - a0.z;
     if (L > it.long_min) {
       const unsigned nc = (unsigned)(((int64_t)L + CHUNK - 1) / CHUNK);
@@ -269,7 +273,7 @@ static int schedule_src(const Src &src, int64_t R, Arena &ar, cudaStream_t s) {
   if (R <= 0) return DCSR_OK;
   uint4 *tmp = ar.take<uint4>(R + 1);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
-  DCSR_TRY((scan_map(SchedScan<V, Src>{src, tmp}, R, ar, s)));
+  DCSR_TRY((scan_map(SchedScan<V, Src>{src, R, tmp}, R, ar, s)));
   DCSR_LAUNCH((k_sched_emit<V, Src>), grid_for(R, 256), 256, 0, s, src, R, tmp);
   return DCSR_OK;
 }
@@ -1058,12 +1062,18 @@ struct FlatManyScan {
   __device__ __forceinline__ void emit(int64_t g, bool ok, const State &, const long long (&p)[1], const T (&)[1]) const {
     if (ok) tmp[g] = (unsigned)p[0];
   }
-  __device__ __forceinline__ void total(const long long (&t)[1]) const { tmp[R] = (unsigned)t[0]; }
+  __device__ __forceinline__ void total(const long long (&t)[1]) const {
+    tmp[R] = (unsigned)t[0];
+    tmp[R + 1] = 0;
+  }
+  __device__ __forceinline__ void fault() const { tmp[R + 1] = 1; }
 };
 
+// (tmp[R + 1]: the scan gave up, every matrix's tables are bad)
 template <typename V, typename Src>
 __global__ void __launch_bounds__(256) k_flat_tables(Src src, int64_t R, const unsigned *tmp) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const bool bad = tmp[R + 1] != 0;
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x; b < R; b += stride) {
     const int64_t g = b + threadIdx.x;
     int32_t r = 0, o = 0, len = 0;
@@ -1072,10 +1082,12 @@ __global__ void __launch_bounds__(256) k_flat_tables(Src src, int64_t R, const u
       i = src.find_row(g);
       const RowItem<V> &it = src.item(i);
       r = (int32_t)(g - it.row0);
-      o = (int32_t)(tmp[g] - tmp[it.row0]);
-      len = (int32_t)(tmp[g + 1] - tmp[g]);
+      if (!bad) {
+        o = (int32_t)(tmp[g] - tmp[it.row0]);
+        len = (int32_t)(tmp[g + 1] - tmp[g]);
+      }
       const_cast<int32_t *>(it.off)[r] = o;
-      if (r == it.m.n_rows - 1) const_cast<int32_t *>(it.off)[r + 1] = o + len;
+      if (r == it.m.n_rows - 1) const_cast<int32_t *>(it.off)[r + 1] = bad ? FLAT_BAD : o + len;
     }
     // (a warp may hold rows of several matrices: tiles are marked per row)
     const RowItem<V> &it = src.item(i);

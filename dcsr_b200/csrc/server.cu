@@ -489,6 +489,11 @@ int retire(dcsr_server s, Slot &sl) {
   for (auto &q : sl.reqs) {
     if (q.r.kind != DCSR_REQ_EXPORT) continue;
     q.nnz = sl.nnz_host[q.item];
+    if (q.nnz < 0) {  // the offsets' scan gave up
+      q.status = DCSR_TIMEOUT;
+      q.nnz = 0;
+      s->mats[q.r.matrix]->flat_valid = false;
+    }
     if (q.nnz > q.r.cap) q.status = DCSR_BAD_ARG;
     const int64_t n_copy = q.nnz < q.r.cap ? q.nnz : q.r.cap;
     if (!q.direct && n_copy > 0) {
