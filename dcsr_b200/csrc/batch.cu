@@ -358,6 +358,13 @@ void BatchCore::mark_scheduled() {
     for (int i : g.idx) (g.k == 1 ? items[i].matrix->flat_valid : items[i].matrix->bins_valid) = true;
 }
 
+void BatchCore::note_statuses(const long long *host) {
+  bool timeout = false;  // (a wait of the batch's own: its tables are all built by the same scans)
+  for (size_t j = 0; j < upd.size(); j++) timeout |= host[2 * j] == DCSR_TIMEOUT;
+  if (timeout)
+    for (auto &it : items) note_status(it.matrix, DCSR_TIMEOUT);
+}
+
 void BatchCore::release() {
   // Device buffers: stream-ordered frees on the legacy default stream (after
   // the work queued on blocking streams; the host does not wait).  The pinned
@@ -492,6 +499,7 @@ int dcsr_batch_status(dcsr_batch b, int32_t *statuses, void *stream) {
     const int j = b->core.upd_of[i];
     statuses[i] = j >= 0 ? (int32_t)b->status_host[2 * j] : DCSR_OK;
   }
+  b->core.note_statuses(b->status_host);
   b->status_read = true;
   return DCSR_OK;
 }

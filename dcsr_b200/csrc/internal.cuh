@@ -136,6 +136,11 @@ int unit_prefix_many(const void *const *items, const int *counts, long long *con
                      int dtype, cudaStream_t s);
 template <typename V>
 RowItem<V> row_item(dcsr_handle h, const void *x, void *y, int64_t ldx, int64_t ldy, double alpha, double beta);
+// An operation of the handle reported `status`: after a timeout its tables may
+// be those of the scan that gave up, and are built anew.
+inline void note_status(dcsr_handle h, int status) {
+  if (status == DCSR_TIMEOUT) h->flat_valid = h->bins_valid = false;
+}
 // Size the handle's chunk table and chunk partials (K results per chunk).
 int ensure_part(dcsr_handle h, int K, cudaStream_t s);
 // DCSR -> CSR writing at most `limit` entries (the row pointer is complete).
@@ -214,6 +219,8 @@ struct BatchCore {
   // 2j, 2j+1) into host memory (async); clears the device statuses.
   int status_async(long long *host, cudaStream_t s);
   void mark_scheduled();
+  // The words status_async fetched have arrived: a timeout's tables are stale.
+  void note_statuses(const long long *host);
   void release();
 };
 

@@ -510,6 +510,7 @@ int dcsr_from_csr(dcsr_handle h, const int32_t *row_ptr, const int32_t *cols, co
   if (aux & AUX_BAD_ROWPTR) return DCSR_BAD_ARG;
   if (aux & AUX_BAD_INDEX) return DCSR_BAD_INDEX;
   if (host[ST_STATUS] == DCSR_TIMEOUT) {  // the scan's look-back gave up
+    note_status(h, DCSR_TIMEOUT);
     DCSR_TRY(clear_status(h, s));
     return DCSR_TIMEOUT;
   }
@@ -539,6 +540,7 @@ int dcsr_from_coo(dcsr_handle h, const int32_t *rows, const int32_t *cols, const
   long long host[ST_WORDS];
   DCSR_TRY(read_stat(h, s, host));
   if (host[ST_STATUS] == DCSR_TIMEOUT) {  // a look-back wait of the sort or scan gave up
+    note_status(h, DCSR_TIMEOUT);
     DCSR_TRY(clear_status(h, s));
     return DCSR_TIMEOUT;
   }
@@ -651,6 +653,7 @@ int dcsr_update_sync(dcsr_handle h, const int32_t *rows, const int32_t *cols, co
   if (!h || nnz < 0 || (nnz > 0 && (!rows || !cols || !vals))) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   long long host[ST_WORDS];
+  h->bins_valid = h->flat_valid = false;  // (their own timeout's report, if any, is cleared unread)
   DCSR_TRY(clear_status(h, s));
   DCSR_TRY(update_async(h, rows, cols, vals, nnz, s));
   DCSR_TRY(read_stat(h, s, host));
@@ -679,6 +682,7 @@ int dcsr_get_status(dcsr_handle h, void *stream, int32_t *status) {
   long long host[ST_WORDS];
   DCSR_TRY(read_stat(h, s, host));
   *status = (int32_t)host[ST_STATUS];
+  note_status(h, *status);
   return clear_status(h, s);
 }
 

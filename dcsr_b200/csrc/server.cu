@@ -454,6 +454,7 @@ int retire(dcsr_server s, Slot &sl) {
   sl.h_retire = Clock::now();
   sl.repairs = sl.grows = 0;
   if (sl.statuses) {
+    if (!sl.single) sl.core.note_statuses(sl.status_host);
     for (size_t i = 0; i < sl.items.size(); i++) {
       const int ui = sl.item_upd[i];
       if (ui < 0) continue;
@@ -463,6 +464,7 @@ int retire(dcsr_server s, Slot &sl) {
       const int j = sl.single ? 0 : sl.core.upd_of[i];
       int status = (int)sl.status_host[2 * j];
       const long long need = sl.status_host[2 * j + 1];
+      note_status(h, status);
       if (status != DCSR_OK) {
         sl.repairs++;
         if (status == DCSR_POOL_EXHAUSTED || status == DCSR_LAYER_OVERFLOW)

@@ -84,3 +84,25 @@ def test_bad_tables_are_not_used(dcsr, pair, op):
     assert_content_equal(dev, orc, op)
     x = torch.ones(N, dtype=torch.float64).cuda()
     np.testing.assert_allclose(dev.spmv(x).cpu().numpy(), orc.spmv(np.ones(N)), rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize("op", ["csr", "spmv", "spmv2", "sum", "bins"])
+def test_tables_are_rebuilt_after_a_timeout(dcsr, pair, op):
+    """Once the timeout has been read, export, entry count, SpMV and reductions
+    build their tables anew: no update is needed in between."""
+    dev, orc = pair
+    small_update(dev, orc, 1)
+    ops, _, _ = operations(dcsr, dev)
+    small_update(dev, orc, 2)
+    stalled(dcsr, dev, lambda: ops[op]())
+    assert dev.get_status() == dcsr.TIMEOUT
+    assert dev.nnz() == orc.export_csr()[1].size
+    assert_content_equal(dev, orc, op)
+    rng = np.random.default_rng(9)
+    for k in (1, 2):
+        x = rng.uniform(-1, 1, (N, k))
+        got = dev.spmv(torch.tensor(x if k > 1 else x[:, 0].copy()).cuda()).cpu().numpy().reshape(N, k)
+        for j in range(k):
+            np.testing.assert_allclose(got[:, j], orc.spmv(x[:, j].copy()), rtol=0, atol=1e-10)
+    np.testing.assert_allclose(dev.row_reduce(dcsr.REDUCE_SUM).cpu().numpy(), orc.row_reduce(0), rtol=0, atol=1e-10)
+    assert dev.get_status() == dcsr.OK
