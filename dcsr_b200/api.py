@@ -127,6 +127,7 @@ _SIGS = {
     "dcsr_launch_count": (C.c_uint64, []),
     "dcsr_spin_faults": (C.c_int, [C.POINTER(C.c_int64)]),
     "dcsr_debug_lookback": (_i32, [_i32, _i32]),
+    "dcsr_debug_fail_alloc": (_i32, [_i32]),
     "dcsr_snapshot_bytes": (_i32, [_vp, C.POINTER(_i64), _vp]),
     "dcsr_snapshot": (_i32, [_vp, _vp, _i64, _vp]),
     "dcsr_snapshot_header": (_i32, [_vp, _i64, C.POINTER(_i32), C.POINTER(_i32), C.POINTER(_i32), C.POINTER(Opts)]),
@@ -177,6 +178,11 @@ def spin_faults() -> int:
 def debug_lookback(spin_limit: int = 0, stall_first_tile: bool = False):
     """Test hook: look-back wait limit (0: default) and the first-tile stall switch."""
     _check(lib().dcsr_debug_lookback(spin_limit, 1 if stall_first_tile else 0), "dcsr_debug_lookback")
+
+
+def debug_fail_alloc(nth: int = 0):
+    """The nth device allocation of the library from now on fails (0: none; for tests)."""
+    _check(lib().dcsr_debug_fail_alloc(nth), "dcsr_debug_fail_alloc")
 
 
 def pool_reserve(nbytes: int, stream=None):

@@ -33,6 +33,8 @@ void debug_check(cudaStream_t s, const char *kernel, const char *file, int line)
 // buffer the library allocates goes through these two calls.
 cudaError_t dev_alloc_raw(void **p, size_t bytes, cudaStream_t s);
 cudaError_t dev_free(void *p, cudaStream_t s);
+// Test hook: the nth allocation from now fails (once); 0: none does.
+void fail_alloc(int nth);
 template <typename T>
 inline cudaError_t dev_alloc(T **p, size_t bytes, cudaStream_t s) {
   return dev_alloc_raw(reinterpret_cast<void **>(p), bytes, s);

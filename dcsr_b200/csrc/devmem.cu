@@ -68,9 +68,14 @@ bool capturing(cudaStream_t s) {
   return cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
 }
 
+std::atomic<int> g_fail_alloc{0};
+
 }  // namespace
 
+void fail_alloc(int nth) { g_fail_alloc = nth; }
+
 cudaError_t dev_alloc_raw(void **p, size_t bytes, cudaStream_t s) {
+  if (g_fail_alloc.load(std::memory_order_relaxed) > 0 && --g_fail_alloc == 0) return cudaErrorMemoryAllocation;
   int dev = 0;
   if (g_region_devices > 0 && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < MAX_DEVICES &&
       !capturing(s)) {

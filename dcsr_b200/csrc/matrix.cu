@@ -153,7 +153,9 @@ static int alloc_pool(dcsr_handle h, int64_t cap, int32_t **cols, void **vals, i
     return DCSR_OK;
   }
   DCSR_CUDA(dcsr::dev_alloc((void **)cols, cap * sizeof(int32_t), s));
-  DCSR_CUDA(dcsr::dev_alloc(vals, cap * h->vsize(), s));
+  const cudaError_t e = dcsr::dev_alloc(vals, cap * h->vsize(), s);
+  if (e != cudaSuccess) dcsr::dev_free(*cols, s);
+  DCSR_CUDA(e);
   *got = cap;
   return DCSR_OK;
 }
@@ -197,6 +199,8 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   if (top > 0x7fffffffLL) return DCSR_OOM;
   int64_t cap = pool_capacity(h->o, top);
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
+  // every allocation before the first change: one that fails leaves the matrix as it was
+  DCSR_TRY(ensure_flat(h, s, cap));
   int32_t *nc;
   void *nv;
   int64_t got;
@@ -207,7 +211,6 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   h->buf_cap = got;
   h->pool_cap = cap;
   h->bins_valid = h->flat_valid = false;
-  DCSR_TRY(ensure_flat(h, s));
   DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, s));
   h->flat_valid = true;  // the load knows the offsets: the export and the row passes find them
   // A load is a one-off: a resident matrix keeps no load-sized scratch (the
@@ -231,6 +234,8 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   int32_t *caps = ar.take<int32_t>(n + 2);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   if (cap_bound > 0x7fffffffLL) return DCSR_OOM;
+  // every allocation before the first change: one that fails leaves the matrix as it was
+  DCSR_TRY(ensure_flat(h, s, bound));
   int32_t *nc;
   void *nv;
   int64_t got;
@@ -239,15 +244,17 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   h->cols = nc;
   h->vals = nv;
   h->buf_cap = got;
+  h->pool_cap = cap_bound;
   h->bins_valid = h->flat_valid = false;
-  DCSR_TRY(ensure_flat(h, s, bound));
   DCSR_TRY(place_rows_scan(h, lens, caps, ar, s));
   DCSR_TRY(place_rows_copy(h, caps, src_off, scols, svals, bound, s));
   long long host[ST_WORDS];
   DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
   h->scratch.release(s);
-  if (host[ST_STATUS] == DCSR_TIMEOUT) {
+  if (host[ST_STATUS] == DCSR_TIMEOUT) {  // the placement's scan gave up: an empty matrix, not its offsets
+    DCSR_CUDA(cudaMemsetAsync(h->row_sizes, 0, sizeof(int32_t) * ((size_t)n + 1), s));
+    DCSR_CUDA(cudaMemsetAsync(h->seg, 0xff, sizeof(int32_t) * (size_t)h->pitch * h->o.max_segs, s));
     DCSR_TRY(clear_status(h, s));
     return DCSR_TIMEOUT;
   }
@@ -870,6 +877,11 @@ int dcsr_pool_usage(int64_t *reserved, int64_t *free_bytes, int64_t *fallback_al
 
 int dcsr_debug_lookback(int32_t spin_limit, int32_t stall_first_tile) {
   return dcsr::debug_lookback(spin_limit, stall_first_tile ? 1 : 0);
+}
+
+int dcsr_debug_fail_alloc(int32_t nth) {
+  dcsr::fail_alloc(nth);
+  return DCSR_OK;
 }
 
 int dcsr_spin_faults(int64_t *count) {

@@ -213,6 +213,7 @@ int ensure_part(dcsr_handle h, int K, cudaStream_t s) {
   if (max_chunks(h) > h->chunk_cap) {
     if (h->chunk_rl) DCSR_CUDA(dcsr::dev_free(h->chunk_rl, s));
     h->chunk_rl = nullptr;
+    h->chunk_cap = 0;  // (should the allocation fail)
     DCSR_CUDA(dcsr::dev_alloc((void **)&h->chunk_rl, sizeof(int2) * max_chunks(h), s));
     h->chunk_cap = max_chunks(h);
     h->bins_valid = false;  // the chunk table is gone
@@ -221,6 +222,7 @@ int ensure_part(dcsr_handle h, int K, cudaStream_t s) {
   if (need <= h->part_cap) return DCSR_OK;
   if (h->part) DCSR_CUDA(dcsr::dev_free(h->part, s));
   h->part = nullptr;
+  h->part_cap = 0;
   DCSR_CUDA(dcsr::dev_alloc((void **)&h->part, sizeof(double) * need, s));
   h->part_cap = need;
   return DCSR_OK;

@@ -454,6 +454,10 @@ int dcsr_spin_faults(int64_t *count);
  * For tests only; synchronises the device; not thread-safe with running
  * operations. */
 int dcsr_debug_lookback(int32_t spin_limit, int32_t stall_first_tile);
+/* Failure-handling test hook (no counterpart in the reference): the nth device
+ * allocation of the library from now on fails as if memory had run out, once
+ * (nth = 1: the next one; 0: none does).  For tests only. */
+int dcsr_debug_fail_alloc(int32_t nth);
 /* Make sure at least `bytes` of device memory reserved for this library are
  * free on the current device: when the reserved regions have less free, a
  * new region of the difference is mapped (on `stream`, then synchronised)
