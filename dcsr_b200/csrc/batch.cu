@@ -171,7 +171,7 @@ int BatchCore::plan(const dcsr_batch_item *its, int n, cudaStream_t s, bool all_
   for (int i = 0; i < n; i++) {
     if (!its[i].x || its[i].matrix->n_rows == 0) continue;
     const bool flat = its[i].k == 1;
-    if (!all_schedules && its[i].nnz == 0 && (flat ? its[i].matrix->flat_valid : its[i].matrix->bins_valid)) continue;
+    if (!all_schedules && its[i].nnz == 0 && (flat ? its[i].matrix->flat : its[i].matrix->bins).ready(0)) continue;
     in_sched[i] = 1;
     if (flat) {
       R1 += its[i].matrix->n_rows;
@@ -353,9 +353,9 @@ int BatchCore::status_async(long long *host, cudaStream_t s) {
 
 void BatchCore::mark_scheduled() {
   for (auto &it : items)
-    if (it.nnz > 0) it.matrix->bins_valid = it.matrix->flat_valid = false;
+    if (it.nnz > 0) it.matrix->bins.valid = it.matrix->flat.valid = false;
   for (auto &g : groups)
-    for (int i : g.idx) (g.k == 1 ? items[i].matrix->flat_valid : items[i].matrix->bins_valid) = true;
+    for (int i : g.idx) (g.k == 1 ? items[i].matrix->flat : items[i].matrix->bins).valid = true;
 }
 
 void BatchCore::note_statuses(const long long *host) {

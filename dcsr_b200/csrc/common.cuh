@@ -224,12 +224,67 @@ struct Arena {
     used = off + n * sizeof(T);
     return (T *)(base + off);
   }
+  // After a one-off operation: everything but a look-back area of at most
+  // keep_slots words of each kind.
+  void trim(size_t keep_slots, cudaStream_t s) {
+    if (base) dcsr::dev_free(base, s);
+    base = nullptr;
+    cap = used = 0;
+    if (lb && lb_slots > keep_slots) {
+      dcsr::dev_free(lb, s);
+      lb = nullptr;
+      lb_slots = 0;
+    }
+  }
   void release(cudaStream_t s) {
     if (base) dcsr::dev_free(base, s);
     if (lb) dcsr::dev_free(lb, s);
     base = nullptr;
     lb = nullptr;
     cap = used = lb_slots = 0;
+  }
+};
+
+// The id of the capture stream s is in (0: none).
+unsigned long long capture_id(cudaStream_t s);
+
+// Whether tables made from a matrix's row lengths are those of its present
+// rows, as far as the host can tell.  An operation in a stream capture changes
+// nothing when it is called but each time the graph runs, unseen: tables that
+// a capture's last update left behind stay good over its runs only if the same
+// capture builds them after it, and are built in every later call otherwise.
+struct RowTables {
+  bool valid = false;                // built since the rows last changed (outside captures)
+  unsigned long long cap_rows = 0;   // the last capture that changes the rows
+  unsigned long long cap_built = 0;  // the last capture that builds the tables after its changes
+  unsigned long long pending = 0;    // a capture that changes the rows and does not build the tables
+  bool loose = false;                // there are several of those
+  // cap: the capture of the calling stream (0: none)
+  bool ready(unsigned long long cap) const {
+    if (cap && (cap == cap_rows || cap == cap_built)) return cap == cap_built;
+    return valid && !pending && !loose;
+  }
+  bool seen_capture() const { return cap_rows || cap_built; }
+  void changed(unsigned long long cap) {
+    if (!cap) {
+      valid = false;
+      return;
+    }
+    loose |= pending && pending != cap;
+    pending = cap_rows = cap;
+    if (cap_built == cap) cap_built = 0;
+  }
+  void built(unsigned long long cap) {
+    if (!cap) {
+      valid = true;
+      return;
+    }
+    cap_built = cap;
+    if (pending == cap) pending = 0;
+  }
+  void drop() {
+    valid = false;
+    cap_built = 0;
   }
 };
 
@@ -261,7 +316,7 @@ struct dcsr_matrix_s {
   // Row-class thresholds of the row passes (rows of at most short_max
   // entries are streamed by row blocks, rows above long_min are chunked).
   int32_t short_max = 64, long_min = 512;
-  bool bins_valid = false;
+  dcsr::RowTables bins;
   // Flat tables (one value per entry: k = 1 SpMV, row reductions; export):
   // the rows' CSR offsets, the row of every tile of 256 entries, two partial
   // sums per tile.  They depend on the row lengths alone.
@@ -269,7 +324,7 @@ struct dcsr_matrix_s {
   int32_t *flat_tile = nullptr;  // [flat_tiles]
   double *flat_part = nullptr;   // [2 * flat_tiles]
   int64_t flat_tiles = 0;
-  bool flat_valid = false;
+  dcsr::RowTables flat;
   dcsr::Arena scratch;
   // Pool buffers: buf_cap >= pool_cap entries are allocated.  The buffers a
   // compaction or growth replaced stay as this matrix's spare (within a

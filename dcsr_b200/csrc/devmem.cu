@@ -72,6 +72,16 @@ std::atomic<int> g_fail_alloc{0};
 
 }  // namespace
 
+unsigned long long capture_id(cudaStream_t s) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &cs, &id) != cudaSuccess) {
+    (void)cudaGetLastError();  // (the legacy stream beside another stream's capture)
+    return 0;
+  }
+  return cs == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 void fail_alloc(int nth) { g_fail_alloc = nth; }
 
 cudaError_t dev_alloc_raw(void **p, size_t bytes, cudaStream_t s) {

@@ -123,6 +123,10 @@ int short_split(int64_t blocks, int k);
 // valid.
 int ensure_flat(dcsr_handle h, cudaStream_t s, int64_t entries = 0);
 int build_flat(dcsr_handle h, cudaStream_t s, Arena *ar = nullptr);
+// Those tables ready for a call on s: built unless they are valid.
+int ready_flat(dcsr_handle h, cudaStream_t s, Arena *ar = nullptr);
+// Look-back words that a build of either kind of tables needs.
+size_t table_slots(dcsr_handle h);
 // Of `count` matrices at once (items: device RowItem<V>[count], row0 = their
 // first rows in a common row space of R rows).  Needs flat_scratch_bytes(R)
 // free in the arena.
@@ -139,7 +143,9 @@ RowItem<V> row_item(dcsr_handle h, const void *x, void *y, int64_t ldx, int64_t 
 // An operation of the handle reported `status`: after a timeout its tables may
 // be those of the scan that gave up, and are built anew.
 inline void note_status(dcsr_handle h, int status) {
-  if (status == DCSR_TIMEOUT) h->flat_valid = h->bins_valid = false;
+  if (status != DCSR_TIMEOUT) return;
+  h->flat.drop();
+  h->bins.drop();
 }
 // Size the handle's chunk table and chunk partials (K results per chunk).
 int ensure_part(dcsr_handle h, int K, cudaStream_t s);

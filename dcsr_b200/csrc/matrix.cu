@@ -190,6 +190,14 @@ static size_t load_scratch_bytes(dcsr_handle h) {
   return arena_bytes(h->n_rows + 2, 4) + scan_scratch_bytes(h->n_rows + 1);
 }
 
+// A load is a one-off: a resident matrix keeps no load-sized scratch (the
+// stream-ordered pool keeps the memory for the next allocation), only a
+// look-back area of about the size that builds of its tables need.
+static void trim_scratch(dcsr_handle h, cudaStream_t s) {
+  const size_t need = table_slots(h);
+  h->scratch.trim(need ? 2 * need + 2048 : 0, s);
+}
+
 // The end of a CSR or COO load, after the host has read the status words
 // (host): a fresh pool for the policy capacities (caps), the layout and the
 // entries.  nnz bounds the row pointer's entries.
@@ -210,12 +218,10 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   h->vals = nv;
   h->buf_cap = got;
   h->pool_cap = cap;
-  h->bins_valid = h->flat_valid = false;
+  h->bins.valid = h->flat.valid = false;
   DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, s));
-  h->flat_valid = true;  // the load knows the offsets: the export and the row passes find them
-  // A load is a one-off: a resident matrix keeps no load-sized scratch (the
-  // stream-ordered pool keeps the memory for the next allocation).
-  h->scratch.release(s);
+  h->flat.valid = true;  // the load knows the offsets: the export and the row passes find them
+  trim_scratch(h, s);
   return DCSR_OK;
 }
 
@@ -245,13 +251,13 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   h->vals = nv;
   h->buf_cap = got;
   h->pool_cap = cap_bound;
-  h->bins_valid = h->flat_valid = false;
+  h->bins.valid = h->flat.valid = false;
   DCSR_TRY(place_rows_scan(h, lens, caps, ar, s));
   DCSR_TRY(place_rows_copy(h, caps, src_off, scols, svals, bound, s));
   long long host[ST_WORDS];
   DCSR_CUDA(cudaMemcpyAsync(host, h->stat, sizeof(host), cudaMemcpyDeviceToHost, s));
   DCSR_CUDA(cudaStreamSynchronize(s));
-  h->scratch.release(s);
+  trim_scratch(h, s);
   if (host[ST_STATUS] == DCSR_TIMEOUT) {  // the placement's scan gave up: an empty matrix, not its offsets
     DCSR_CUDA(cudaMemsetAsync(h->row_sizes, 0, sizeof(int32_t) * ((size_t)n + 1), s));
     DCSR_CUDA(cudaMemsetAsync(h->seg, 0xff, sizeof(int32_t) * (size_t)h->pitch * h->o.max_segs, s));
@@ -262,7 +268,7 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
   if (cap > got) return DCSR_OOM;  // the caller's bound was not one (a bug)
   h->pool_cap = cap;
-  h->flat_valid = true;
+  h->flat.valid = true;
   return DCSR_OK;
 }
 
@@ -354,7 +360,7 @@ int compact(dcsr_handle h, cudaStream_t s) {
   h->pool_cap = cap;
   // the schedule's row descriptors hold segment starts, which moved (the
   // flat tables follow the row lengths, which did not change)
-  h->bins_valid = false;
+  h->bins.valid = false;
   // the scratch (sized by this matrix's earlier updates) stays for the
   // update a repair runs next: re-allocating it there stalled repairs
   return DCSR_OK;
@@ -609,7 +615,7 @@ int dcsr_from_hyb(dcsr_handle h, const int32_t *ell_cols, const void *ell_vals, 
 int dcsr_nnz(dcsr_handle h, int64_t *nnz, void *stream) {
   if (!h || !nnz) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  if (h->flat_valid) {  // the offsets' last word
+  if (h->flat.ready(0)) {  // the offsets' last word
     int32_t t = 0;
     DCSR_CUDA(cudaMemcpyAsync(&t, h->flat_off + h->n_rows, sizeof(t), cudaMemcpyDeviceToHost, s));
     DCSR_CUDA(cudaStreamSynchronize(s));
@@ -617,7 +623,7 @@ int dcsr_nnz(dcsr_handle h, int64_t *nnz, void *stream) {
       *nnz = t;
       return DCSR_OK;
     }
-    h->flat_valid = false;  // the tables' scan gave up
+    h->flat.drop();  // the tables' scan gave up
   }
   DCSR_CUDA(cudaMemsetAsync(h->stat + ST_AUX + 1, 0, sizeof(long long), s));
   if (h->n_rows > 0)
@@ -634,7 +640,7 @@ static int export_impl(dcsr_handle h, int32_t *row_ptr, int32_t *rows, int32_t *
   const int32_t n = h->n_rows;
   // the flat tables are the export's offsets too; built here when stale (a
   // later SpMV or reduction finds them)
-  if (!h->flat_valid) DCSR_TRY(build_flat(h, s, arp));
+  DCSR_TRY(ready_flat(h, s, arp));
   if (row_ptr)
     DCSR_CUDA(cudaMemcpyAsync(row_ptr, h->flat_off, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyDeviceToDevice, s));
   return export_rows(h, h->flat_off, h->flat_tile, cols, vals, rows, limit, s);
@@ -660,7 +666,7 @@ int dcsr_update_sync(dcsr_handle h, const int32_t *rows, const int32_t *cols, co
   if (!h || nnz < 0 || (nnz > 0 && (!rows || !cols || !vals))) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   long long host[ST_WORDS];
-  h->bins_valid = h->flat_valid = false;  // (their own timeout's report, if any, is cleared unread)
+  h->bins.valid = h->flat.valid = false;  // (their own timeout's report, if any, is cleared unread)
   DCSR_TRY(clear_status(h, s));
   DCSR_TRY(update_async(h, rows, cols, vals, nnz, s));
   DCSR_TRY(read_stat(h, s, host));
@@ -818,7 +824,7 @@ int dcsr_restore(dcsr_handle h, const void *host_buf, int64_t buf_bytes, void *s
     p += 4 * (size_t)hd.top;
     DCSR_CUDA(cudaMemcpyAsync(h->vals, p, h->vsize() * (size_t)hd.top, cudaMemcpyHostToDevice, s));
   }
-  h->bins_valid = h->flat_valid = false;
+  h->bins.valid = h->flat.valid = false;
   DCSR_CUDA(cudaStreamSynchronize(s));  // the host buffer may be released on return
   return DCSR_OK;
 }
@@ -835,7 +841,7 @@ int dcsr_set_row_classes(dcsr_handle h, int32_t short_max, int32_t long_min) {
   if (h->short_max != short_max || h->long_min != long_min) {
     h->short_max = short_max;
     h->long_min = long_min;
-    h->bins_valid = false;  // rows change class: rebuild the schedule before the next pass
+    h->bins.valid = false;  // rows change class: rebuild the schedule before the next pass
   }
   return DCSR_OK;
 }

@@ -216,7 +216,7 @@ int ensure_part(dcsr_handle h, int K, cudaStream_t s) {
     h->chunk_cap = 0;  // (should the allocation fail)
     DCSR_CUDA(dcsr::dev_alloc((void **)&h->chunk_rl, sizeof(int2) * max_chunks(h), s));
     h->chunk_cap = max_chunks(h);
-    h->bins_valid = false;  // the chunk table is gone
+    h->bins.drop();  // the chunk table is gone
   }
   const int64_t need = max_chunks(h) * K;
   if (need <= h->part_cap) return DCSR_OK;
@@ -289,11 +289,13 @@ int schedule_many(const void *items_dev, int dtype, int count, int64_t R, Arena 
 
 template <typename V>
 static int build_schedule_t(dcsr_handle h, cudaStream_t s, Arena &ar) {
+  const unsigned long long cap = capture_id(s);
+  if (!cap) DCSR_TRY(ensure_flat(h, s));  // (so that a capture may build those tables too)
   DCSR_TRY(ensure_part(h, 1, s));
   DCSR_TRY(ar.reserve(schedule_scratch_bytes(h->n_rows), s));
   RowOne<V> src{row_item<V>(h, nullptr, nullptr, 0, 0, 0.0, 0.0)};
   DCSR_TRY(schedule_src<V>(src, h->n_rows, ar, s));
-  h->bins_valid = true;
+  h->bins.built(cap);
   return DCSR_OK;
 }
 
@@ -309,13 +311,14 @@ int build_schedule(dcsr_handle h, cudaStream_t s, Arena *ar) {
 int ensure_flat(dcsr_handle h, cudaStream_t s, int64_t entries) {
   const int64_t need = flat_tiles(std::max(h->pool_cap, entries)) + 1;
   if (h->flat_off && need <= h->flat_tiles) return DCSR_OK;
+  if (capture_id(s)) return DCSR_NOT_SUPPORTED;  // (memory allocated in a capture is the graph's)
   if (!h->flat_off) DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_off, sizeof(int32_t) * ((size_t)h->n_rows + 2), s));
   if (h->flat_tile) DCSR_CUDA(dcsr::dev_free(h->flat_tile, s));
   if (h->flat_part) DCSR_CUDA(dcsr::dev_free(h->flat_part, s));
   h->flat_tile = nullptr;
   h->flat_part = nullptr;
   h->flat_tiles = 0;
-  h->flat_valid = false;
+  h->flat.drop();
   const int64_t want = need + need / 4;
   DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_tile, sizeof(int32_t) * want, s));
   DCSR_CUDA(dcsr::dev_alloc((void **)&h->flat_part, sizeof(double) * 2 * want, s));
@@ -328,7 +331,24 @@ int build_flat(dcsr_handle h, cudaStream_t s, Arena *ar) {
   a.status = h->stat + ST_STATUS;
   DCSR_TRY(ensure_flat(h, s));
   DCSR_TRY(flat_offsets(h, h->flat_off, h->flat_tile, h->flat_tiles, a, s));
-  h->flat_valid = true;
+  h->flat.built(capture_id(s));
+  return DCSR_OK;
+}
+
+size_t table_slots(dcsr_handle h) {
+  if (h->n_rows <= SM_ONE) return 0;
+  return (size_t)(LB_SCAN_WORDS * div_up(h->n_rows, SM_THREADS * (h->n_rows <= SM_FEW ? SM_THIN : SM_LIGHT)));
+}
+
+int ready_flat(dcsr_handle h, cudaStream_t s, Arena *ar) {
+  const bool seen = h->flat.seen_capture();
+  if (!h->flat.ready(seen ? capture_id(s) : 0)) return build_flat(h, s, ar);
+  // A load leaves the tables built: the area that a build in a capture needs is
+  // sized by the first call that finds them so.
+  if (!ar && table_slots(h) > h->scratch.lb_slots && !capture_id(s)) {
+    Lookback lb;
+    DCSR_TRY(h->scratch.lookback(table_slots(h), s, &lb));
+  }
   return DCSR_OK;
 }
 
@@ -1262,10 +1282,10 @@ int spmv_call(dcsr_handle h, const void *x, int32_t k, int64_t ldx, void *y, int
               cudaStream_t s, Arena *ar) {
   if (h->n_rows == 0) return DCSR_OK;
   if (k == 1) {
-    if (!h->flat_valid) DCSR_TRY(build_flat(h, s, ar));
+    DCSR_TRY(ready_flat(h, s, ar));
   } else {
     DCSR_TRY(ensure_part(h, rhs_family(k), s));
-    if (!h->bins_valid) DCSR_TRY(build_schedule(h, s, ar));
+    if (!h->bins.ready(h->bins.seen_capture() ? capture_id(s) : 0)) DCSR_TRY(build_schedule(h, s, ar));
   }
   if (h->dtype == DCSR_F32)
     return spmv_dispatch<float>(h, (const float *)x, k, ldx, (float *)y, ldy, alpha, beta, s);
@@ -1284,7 +1304,7 @@ extern "C" int dcsr_row_reduce(dcsr_handle h, int32_t op, void *y, void *stream)
   if (!h || (h->n_rows > 0 && !y) || op < 0 || op > 3) return DCSR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   if (h->n_rows == 0) return DCSR_OK;
-  if (!h->flat_valid) DCSR_TRY(build_flat(h, s));
+  DCSR_TRY(ready_flat(h, s));
   if (h->dtype == DCSR_F32) return reduce_dispatch<float>(h, op, (float *)y, s);
   return reduce_dispatch<double>(h, op, (double *)y, s);
 }

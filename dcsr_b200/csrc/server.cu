@@ -494,7 +494,7 @@ int retire(dcsr_server s, Slot &sl) {
     if (q.nnz < 0) {  // the offsets' scan gave up
       q.status = DCSR_TIMEOUT;
       q.nnz = 0;
-      s->mats[q.r.matrix]->flat_valid = false;
+      s->mats[q.r.matrix]->flat.drop();
     }
     if (q.nnz > q.r.cap) q.status = DCSR_BAD_ARG;
     const int64_t n_copy = q.nnz < q.r.cap ? q.nnz : q.r.cap;

@@ -894,7 +894,9 @@ static int update_one(dcsr_handle h, const int32_t *rows, const int32_t *cols, c
   UpdOne<V> src{h->view<V>(), rows, cols, vals};
   DCSR_TRY((update_pipeline<V, true>(src, 1, T, h->o.mode == DCSR_MERGE, bits_for(h->n_rows), bits_for(h->n_cols), h->stat,
                                      ar, s)));
-  h->bins_valid = h->flat_valid = false;
+  const unsigned long long cap = capture_id(s);
+  h->bins.changed(cap);
+  h->flat.changed(cap);
   return DCSR_OK;
 }
 
