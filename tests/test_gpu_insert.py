@@ -137,3 +137,68 @@ def test_many_relocated_rows_batched(dcsr):
         assert_layout_equal(w["matrix"], orc, "batched")
         assert_content_equal(w["matrix"], orc, "batched")
     batch.close()
+
+
+COUNTS = [1, 2, 3, 4, 5, 6, 7, 31, 32, 33, 35, 36, 37, 63, 64, 65, 127, 128, 129, 131, 132, 133, 134, 259, 260, 261, 1000, 20_000]
+
+
+def repeated(rng, per_count, n, cols_of):
+    """Triples whose (row, column) pairs come COUNTS times each."""
+    r, c = [], []
+    for q in range(per_count):
+        for i, k in enumerate(COUNTS):
+            r.append(np.full(k, (q * len(COUNTS) + 7 * i) % n))
+            c.append(np.full(k, cols_of(q, i)))
+    r, c = np.concatenate(r), np.concatenate(c)
+    order = rng.permutation(r.size)
+    return r[order].astype(np.int32), c[order].astype(np.int32), rng.uniform(-1, 1, r.size)
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("per_count", [1, 9])
+def test_repeated_pairs(dcsr, dtype, per_count):
+    """Pairs that come once to 20,000 times in an update, new and existing
+    columns, added up in batch order, alone and in a batch."""
+    import torch
+    rng = np.random.default_rng(per_count)
+    lens = rng.integers(0, 40, 500)
+    rp, cols, vals = build(rng, lens)
+    ft = np.float32 if dtype == 0 else np.float64
+    dev, orc = make_pair(dcsr, 500, M, dtype, 0)
+    bat, _ = make_pair(dcsr, 500, M, dtype, 0)
+    for m in (dev, bat):
+        m.from_csr(rp, cols, vals.astype(ft))
+    assert orc.load_csr(rp, cols, vals.astype(ft).astype(np.float64)) == 0
+    for it in range(3):  # the second round's pairs are all there
+        r, c, v = repeated(rng, per_count, 500, lambda q, i: 10 * (1 + i % 5) if (q + i + it // 2) % 2 else 1003 + 11 * i + q)
+        v = v.astype(ft)
+        assert dev.update(r, c, v) == orc.update_auto(r, c, v.astype(np.float64)) == 0
+        assert_layout_equal(dev, orc, f"update {it}")
+        assert_content_equal(dev, orc, f"update {it}")
+        batch = dcsr.DcsrBatch([dict(matrix=bat, rows=torch.tensor(r).cuda(), cols=torch.tensor(c).cuda(),
+                                     vals=torch.tensor(v).cuda())])
+        batch.run()
+        batch.repair(batch.status())
+        assert_content_equal(bat, orc, f"batched update {it}")
+        batch.close()
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_append_many_to_a_row(dcsr, dtype):
+    """Append mode: rows that take one to 20,000 triples in an update, on rows of
+    no, one and several segments."""
+    rng = np.random.default_rng(2)
+    n = 3 * len(COUNTS)
+    lens = rng.integers(0, 30, n)
+    rp, cols, vals = build(rng, lens)
+    ft = np.float32 if dtype == 0 else np.float64
+    dev, orc = make_pair(dcsr, n, M, dtype, 1)
+    dev.from_csr(rp, cols, vals.astype(ft))
+    assert orc.load_csr(rp, cols, vals.astype(ft).astype(np.float64)) == 0
+    for it in range(3):
+        r = np.concatenate([np.full(k, (3 * i + it * 5) % n) for i, k in enumerate(COUNTS)])
+        r = r[rng.permutation(r.size)].astype(np.int32)
+        c, v = rng.integers(0, M, r.size).astype(np.int32), rng.uniform(-1, 1, r.size).astype(ft)
+        assert dev.update(r, c, v) == orc.update_auto(r, c, v.astype(np.float64)) == 0
+        assert_layout_equal(dev, orc, f"append {it}")
+        assert_content_equal(dev, orc, f"append {it}")
