@@ -113,7 +113,8 @@ size_t schedule_scratch_bytes(int64_t R);
 int spmv_many(const void *items_dev, int dtype, int count, int k, long long *pref, cudaStream_t s,
               bool prefixed = false, int split = 1);
 // The kernel family of a k: 1 (flat pass), 2, 4 or 8; and whether x's rows can
-// be read 16 bytes a lane (packed, aligned, k the family's width).
+// be read in vectors of 16 bytes (8 where a row is no multiple of 16): packed,
+// aligned, k even.
 inline int rhs_family(int32_t k) { return k == 1 ? 1 : k == 2 ? 2 : k <= 4 ? 4 : 8; }
 bool rhs_vec(const void *x, int32_t k, int64_t ldx, size_t vsize);
 // Warps per 32-row short-row block for an SpMV pass over `blocks` blocks with k RHS.

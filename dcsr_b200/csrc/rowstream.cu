@@ -500,7 +500,7 @@ __device__ __forceinline__ void write_y(V *y, double v, double alpha, double bet
 // half the speed.
 template <typename V, int K, bool VEC>
 __device__ __forceinline__ void load_x(const V *__restrict__ p, V (&v)[K]) {
-  if constexpr (VEC && K * sizeof(V) >= 16) {
+  if constexpr (VEC && K * sizeof(V) % 16 == 0) {
 #pragma unroll
     for (int q = 0; q < K; q += 16 / (int)sizeof(V)) {
       if constexpr (sizeof(V) == 4) {
@@ -511,9 +511,12 @@ __device__ __forceinline__ void load_x(const V *__restrict__ p, V (&v)[K]) {
         v[q] = t.x; v[q + 1] = t.y;
       }
     }
-  } else if constexpr (VEC) {  // FP32, K = 2
-    const float2 t = __ldg(reinterpret_cast<const float2 *>(p));
-    v[0] = t.x; v[1] = t.y;
+  } else if constexpr (VEC) {  // FP32, K = 2 or 6
+#pragma unroll
+    for (int q = 0; q < K; q += 2) {
+      const float2 t = __ldg(reinterpret_cast<const float2 *>(p + q));
+      v[q] = t.x; v[q + 1] = t.y;
+    }
   } else {
 #pragma unroll
     for (int q = 0; q < K; q++) v[q] = __ldg(p + q);
@@ -659,7 +662,9 @@ template <typename V, int FAM, int PART>
 __device__ __forceinline__ void rows_unit_k(const RowItem<V> &it, int64_t lu, int split, double (*red)[8],
                                             int *last_flag) {
   if (it.skip && *it.skip) return;  // a batch matrix whose update was rejected: y untouched
-  if (it.vec) {  // k = 2, 4 or 8
+  if (FAM == 8 && it.vec && it.k == 6) {
+    rows_unit<V, FAM == 8 ? 6 : FAM, true, PART>(it, lu, split, red, last_flag);
+  } else if (it.vec) {  // k = 2, 4 or 8
     rows_unit<V, FAM, true, PART>(it, lu, split, red, last_flag);
   } else if constexpr (FAM == 2) {
     rows_unit<V, 2, false, PART>(it, lu, split, red, last_flag);
@@ -1194,8 +1199,8 @@ int short_split(int64_t blocks, int k) {
 }
 
 bool rhs_vec(const void *x, int32_t k, int64_t ldx, size_t vsize) {
-  const size_t rb = (size_t)k * vsize, al = rb >= 16 ? 16 : rb;  // a lane's load
-  return (k == 2 || k == 4 || k == 8) && ldx == k && (uintptr_t)x % al == 0;
+  const size_t al = (size_t)k * vsize % 16 == 0 ? 16 : 8;  // a lane's load
+  return k % 2 == 0 && ldx == k && (uintptr_t)x % al == 0;
 }
 
 template <typename V>

@@ -86,3 +86,27 @@ def test_classes_across_a_batch(dcsr, dtype):
         for q, w in enumerate(work):
             assert torch.equal(w["y"], want[q].view_as(w["y"])), f"matrix {q}"
     batch.close()
+
+
+@pytest.mark.parametrize("k", [2, 4, 6, 8])
+@pytest.mark.parametrize("off", [0, 1, 2, 4])
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_packed_rows_of_every_alignment(dcsr, k, off, dtype):
+    """Packed x at each multiple of a value: rows read in vectors of 16 or 8
+    bytes, or value by value, give the same sums in the same order."""
+    rng = np.random.default_rng(k)
+    n, m = len(LENS), 9100
+    rp = np.concatenate([[0], np.cumsum(LENS)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(m, L, replace=False)) for L in LENS if L]).astype(np.int32)
+    dev, _ = make_pair(dcsr, n, m, dtype, 0)
+    dev.from_csr(rp, cols, torch.tensor(rng.uniform(-1, 1, cols.size), dtype=dev.dtype).cuda())
+    x = torch.tensor(rng.uniform(-1, 1, (m, k)), dtype=dev.dtype).cuda()
+    s = torch.cuda.current_stream().cuda_stream
+    wide = torch.zeros(m, k + 1, dtype=dev.dtype).cuda()
+    wide[:, :k] = x
+    want, y = torch.empty(n, k, dtype=dev.dtype).cuda(), torch.empty(n, k, dtype=dev.dtype).cuda()
+    assert dcsr.lib().dcsr_spmv(dev.h, wide.data_ptr(), k, k + 1, want.data_ptr(), k, 1.0, 0.0, s) == 0
+    xb = torch.zeros(m * k + 4, dtype=dev.dtype).cuda()
+    xb[off : off + m * k] = x.reshape(-1)
+    assert dcsr.lib().dcsr_spmv(dev.h, xb[off:].data_ptr(), k, k, y.data_ptr(), k, 1.0, 0.0, s) == 0
+    assert torch.equal(y, want)
