@@ -314,7 +314,9 @@ int BatchCore::enqueue(cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEv
   }
   const int nu = (int)upd.size();
   if (T > 0 && nu > 0) {
-    DCSR_TRY(update_many(img_dev, dtype, nu, T, merge, rb, cb, gstat, ar, s));
+    int64_t pool = 0;
+    for (int i : upd) pool += items[i].matrix->pool_cap;
+    DCSR_TRY(update_many(img_dev, dtype, nu, T, pool, merge, rb, cb, gstat, ar, s));
     const int g = (nu + 255) / 256;
     if (dtype == DCSR_F32)
       DCSR_LAUNCH(k_batch_gate<float>, g, 256, 0, s, (const BatchItem<float> *)img_dev, nu, skip);

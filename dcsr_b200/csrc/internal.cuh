@@ -66,9 +66,10 @@ struct BatchItem {
   long long T;     // its triple count
 };
 // Update `count` matrices at once (items_dev: device BatchItem<V>[count],
-// toff prefix over T); gstat: batch-global status words.
-int update_many(const void *items_dev, int dtype, int count, int64_t T, bool merge, int rb, int cb, long long *gstat,
-                Arena &ar, cudaStream_t s);
+// toff prefix over T); pool: their pools' entries together; gstat: batch-global
+// status words.
+int update_many(const void *items_dev, int dtype, int count, int64_t T, int64_t pool, bool merge, int rb, int cb,
+                long long *gstat, Arena &ar, cudaStream_t s);
 size_t update_scratch_bytes(int64_t T, size_t vsize);
 int compact(dcsr_handle h, cudaStream_t s);
 int build_schedule(dcsr_handle h, cudaStream_t s, Arena *ar = nullptr);

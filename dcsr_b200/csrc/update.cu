@@ -924,9 +924,10 @@ static int update_plan(const Src &src, const UpdWork<V> &w, Arena &ar, cudaStrea
 
 // The update of `count` matrices (one Src) with T triples in total.
 // gstat: batch-global status words (ST_TOUCHED, ST_TILES, ST_RELOC, ST_TOTAL, ST_LISTS).
+// pool: pool entries of all matrices, an upper bound of what relocations move.
 template <typename V, bool ONE, typename Src>
-static int update_pipeline(const Src &src, int count, int64_t T, bool merge, int rb, int cb, long long *gstat,
-                           Arena &ar, cudaStream_t s) {
+static int update_pipeline(const Src &src, int count, int64_t T, int64_t pool, bool merge, int rb, int cb,
+                           long long *gstat, Arena &ar, cudaStream_t s) {
   const int ib = count > 1 ? bits_for(count) : 0;
   const KeyFmt f{cb, rb, merge ? 1 : 0};
   const int bits = ib + rb + (merge ? cb : 0);
@@ -971,8 +972,12 @@ static int update_pipeline(const Src &src, int count, int64_t T, bool merge, int
   if (merge) {
     static const int g_apply = persistent_grid((const void *)k_apply_rows<V, Src>, UPD_THREADS, 0);
     DCSR_LAUNCH((k_apply_existing<V, Src>), gT, 256, 0, s, src, w);
-    DCSR_LAUNCH((k_apply_rows<V, Src>), (int)std::min<int64_t>(g_apply, div_up(T, UPD_THREADS / 32)), UPD_THREADS, 0, s,
-                src, w);
+    // warps for the triples' rows, and for the tiles of the rows they may
+    // relocate: one triple can move a row of millions (20 triples into rows of 1M
+    // and 2M entries: 205 us, 1170 with warps for the triples alone)
+    const int64_t warps = std::max(T, div_up(pool, RT_TILE));
+    DCSR_LAUNCH((k_apply_rows<V, Src>), (int)std::min<int64_t>(g_apply, div_up(warps, UPD_THREADS / 32)), UPD_THREADS, 0,
+                s, src, w);
   } else {
     static const int g_apply = persistent_grid((const void *)k_apply_append<V, Src>, UPD_THREADS, 0);
     DCSR_LAUNCH((k_apply_append<V, Src>), (int)std::min<int64_t>(g_apply, div_up(T, UPD_THREADS / 8)), UPD_THREADS, 0,
@@ -986,7 +991,7 @@ template <typename V>
 static int update_one(dcsr_handle h, const int32_t *rows, const int32_t *cols, const V *vals, int64_t T,
                       cudaStream_t s, Arena &ar) {
   UpdOne<V> src{h->view<V>(), rows, cols, vals};
-  DCSR_TRY((update_pipeline<V, true>(src, 1, T, h->o.mode == DCSR_MERGE, bits_for(h->n_rows), bits_for(h->n_cols), h->stat,
+  DCSR_TRY((update_pipeline<V, true>(src, 1, T, h->pool_cap, h->o.mode == DCSR_MERGE, bits_for(h->n_rows), bits_for(h->n_cols), h->stat,
                                      ar, s)));
   const unsigned long long cap = capture_id(s);
   h->bins.changed(cap);
@@ -1005,19 +1010,19 @@ int update_async(dcsr_handle h, const int32_t *rows, const int32_t *cols, const 
 }
 
 template <typename V>
-static int update_many_t(const BatchItem<V> *items_dev, int count, int64_t T, bool merge, int rb, int cb,
+static int update_many_t(const BatchItem<V> *items_dev, int count, int64_t T, int64_t pool, bool merge, int rb, int cb,
                          long long *gstat, Arena &ar, cudaStream_t s) {
   UpdMany<V> src{items_dev, count};
-  return update_pipeline<V, false>(src, count, T, merge, rb, cb, gstat, ar, s);
+  return update_pipeline<V, false>(src, count, T, pool, merge, rb, cb, gstat, ar, s);
 }
 
-int update_many(const void *items_dev, int dtype, int count, int64_t T, bool merge, int rb, int cb, long long *gstat,
-                Arena &ar, cudaStream_t s) {
+int update_many(const void *items_dev, int dtype, int count, int64_t T, int64_t pool, bool merge, int rb, int cb,
+                long long *gstat, Arena &ar, cudaStream_t s) {
   if (T == 0 || count == 0) return DCSR_OK;
   ar.status = gstat + ST_STATUS;  // a look-back wait that gives up reports DCSR_TIMEOUT for the batch
   if (dtype == DCSR_F32)
-    return update_many_t<float>((const BatchItem<float> *)items_dev, count, T, merge, rb, cb, gstat, ar, s);
-  return update_many_t<double>((const BatchItem<double> *)items_dev, count, T, merge, rb, cb, gstat, ar, s);
+    return update_many_t<float>((const BatchItem<float> *)items_dev, count, T, pool, merge, rb, cb, gstat, ar, s);
+  return update_many_t<double>((const BatchItem<double> *)items_dev, count, T, pool, merge, rb, cb, gstat, ar, s);
 }
 
 // ------------------------------------------------------------- COO -> CSR

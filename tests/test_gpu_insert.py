@@ -202,3 +202,24 @@ def test_append_many_to_a_row(dcsr, dtype):
         assert dev.update(r, c, v) == orc.update_auto(r, c, v.astype(np.float64)) == 0
         assert_layout_equal(dev, orc, f"append {it}")
         assert_content_equal(dev, orc, f"append {it}")
+
+
+@pytest.mark.parametrize("T", [1, 20])
+def test_few_triples_move_long_rows(dcsr, T):
+    """One and twenty triples whose rows, of 400,000 and 1,000,000 entries,
+    are relocated whole."""
+    rng = np.random.default_rng(T)
+    m = 3_000_000
+    lens = [3, 1_000_000, 0, 400_000, 5]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(m, L, replace=False)) for L in lens if L]).astype(np.int32)
+    vals = rng.uniform(-1, 1, cols.size)
+    dev, orc = make_pair(dcsr, 5, m, 1, 0)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals) == 0
+    for it in range(3):
+        r = (1 + 2 * (np.arange(T) % 2)).astype(np.int32)
+        c, v = rng.integers(0, m, T).astype(np.int32), rng.uniform(-1, 1, T)
+        assert dev.update(r, c, v) == orc.update_auto(r, c, v) == 0
+        assert_layout_equal(dev, orc, f"update {it}")
+        assert_content_equal(dev, orc, f"update {it}")
