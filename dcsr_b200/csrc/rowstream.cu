@@ -1018,9 +1018,16 @@ __global__ void __launch_bounds__(FT_THREADS, DCSR_FLAT_MINB) k_flat_rows(Src sr
 }
 
 // Rows over several tiles (a thread per tile in which one begins, a warp for
-// more than 16 tiles) and empty rows (a thread per row).
+// more than 16 tiles, the block for more than 512: a row of 2M entries has 7800,
+// 60 us a load at a time by one warp, 7 to 10 by the block) and empty rows (a thread
+// per row).  The row's length alone gives the order of the additions.
+constexpr int FIX_WARP = 16, FIX_BLOCK = 512;
 template <typename V, int OP, typename Src>
 __global__ void __launch_bounds__(FT_THREADS) k_flat_fix(Src src) {
+  __shared__ double s_sum[FT_WARPS];
+  __shared__ int64_t s_tile;
+  __shared__ int s_n;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t nt = src.units(P_TBLOCKS), total = nt + src.units(P_RBLOCKS);
   for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
     int64_t lu;
@@ -1043,20 +1050,41 @@ __global__ void __launch_bounds__(FT_THREADS) k_flat_fix(Src src) {
     double v = 0.0;
     if (r >= 0) {
       v = it.fpart[2 * i + 1];
-      if (nh <= 16)
+      if (nh <= FIX_WARP)
         for (int32_t q = 1; q <= nh; q++) v = op_comb<double, OP>(it.fpart[2 * (i + q)], v);
     }
-    unsigned big = __ballot_sync(FULL, nh > 16);
-    while (big) {  // lanes take heads lane, lane+32, ... in order, then a fixed tree
-      const int s = __ffs(big) - 1;
-      big &= big - 1;
-      const int64_t ti = __shfl_sync(FULL, i, s);
-      const int32_t n = __shfl_sync(FULL, nh, s);
+    // the heads a .. b of the row that begins in tile t: lanes take every 32nd
+    // in order, then a fixed tree
+    auto heads = [&](int64_t t, int32_t a, int32_t b) {
       double p = op_init<double, OP>();
-      for (int32_t q = 1 + lane_id(); q <= n; q += 32) p = op_comb<double, OP>(it.fpart[2 * (ti + q)], p);
+#pragma unroll 4
+      for (int32_t q = a + lane; q <= b; q += 32) p = op_comb<double, OP>(it.fpart[2 * (t + q)], p);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) p = op_comb<double, OP>(p, __shfl_xor_sync(FULL, p, o));
-      if (lane_id() == s) v = op_comb<double, OP>(p, v);
+      return p;
+    };
+    unsigned big = __ballot_sync(FULL, nh > FIX_WARP && nh <= FIX_BLOCK);
+    while (big) {
+      const int s = __ffs(big) - 1;
+      big &= big - 1;
+      const double p = heads(__shfl_sync(FULL, i, s), 1, __shfl_sync(FULL, nh, s));
+      if (lane == s) v = op_comb<double, OP>(p, v);
+    }
+    // (of FT_THREADS tiles, one at most begins such a row)
+    static_assert(FIX_BLOCK >= FT_THREADS, "one row per unit");
+    if (__syncthreads_or(nh > FIX_BLOCK)) {
+      if (nh > FIX_BLOCK) {
+        s_tile = i;
+        s_n = nh;
+      }
+      __syncthreads();
+      const int32_t per = (s_n + FT_WARPS - 1) / FT_WARPS, to = (w + 1) * per;
+      const double p = heads(s_tile, 1 + w * per, to < s_n ? to : s_n);
+      if (lane == 0) s_sum[w] = p;
+      __syncthreads();
+      if (nh > FIX_BLOCK)
+        for (int q = 0; q < FT_WARPS; q++) v = op_comb<double, OP>(s_sum[q], v);
+      __syncthreads();  // (the shared words are free)
     }
     if (r >= 0) write_row<V, OP>(it, r, v);
   }

@@ -171,3 +171,22 @@ def test_csr_check_finds_one_fault(dcsr, nnz, at):
     with pytest.raises(dcsr.DcsrError) as e:
         dev.from_csr(short, cols, vals)
     assert e.value.status == dcsr.BAD_ARG
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("lead", [0, 1, 255])
+def test_rows_over_many_tiles(dcsr, lead, dtype):
+    """Rows over about 16 tiles (where a thread stops adding their parts) and
+    about 512 (where a warp does), side by side, starting anywhere in a tile."""
+    rng = np.random.default_rng(lead)
+    m = 300_000
+    lens = [lead] + [t * 256 + d for t in (15, 16, 17, 18, 511, 512, 513, 514, 1000) for d in (0, 1, 255)] + [0, 3, 700 * 256]
+    n = len(lens)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    cols = np.concatenate([np.sort(rng.choice(m, L, replace=False)) for L in lens if L]).astype(np.int32)
+    vals = rng.uniform(-1, 1, cols.size)
+    vals = vals.astype(np.float32) if dtype == 0 else vals
+    dev, orc = make_pair(dcsr, n, m, dtype, 0)
+    dev.from_csr(rp, cols, vals)
+    assert orc.load_csr(rp, cols, vals.astype(np.float64)) == 0
+    check_rows(dcsr, dev, orc, rng, "loaded")
