@@ -215,8 +215,11 @@ __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long lo
 // A warp takes 32*IT consecutive items, item j*32 + lane in lane's j-th step
 // (coalesced, and every step's prefix by a warp scan in registers -- no
 // staging through shared memory), a block SM_THREADS*IT.  Light functions
-// (IT = 8) of up to SM_ONE items run in one block without look-back; heavy
-// ones (IT = 4: searches, plans) spread over blocks from 1024 items on.
+// (IT = 8) of up to SM_ONE items run in one block without look-back, with as
+// few items a thread as its 1024 threads allow (a few rows of many tiles each
+// are then marked by as many warps as can be: 500 rows of 78 tiles %B% us,
+// 43 with eight rows a lane in two warps); heavy ones (IT = 4: searches, plans)
+// spread over blocks from 1024 items on.
 constexpr int SM_LIGHT = 8, SM_HEAVY = 4;
 constexpr int SM_THREADS = 256;
 constexpr int SM_ONE_THREADS = 1024;
@@ -326,7 +329,8 @@ __global__ void __launch_bounds__(TH, TH > SM_THREADS ? 1 : F::IT == SM_HEAVY ||
 #pragma unroll
     for (int q = 0; q < NS; q++) tot[q] = (single ? 0 : sh_prefix[q]) + agg[q];
     f.total(tot);
-    if constexpr (ScanHasFault<F>::value) __threadfence();  // (fault() may write over it from another block)
+    if constexpr (ScanHasFault<F>::value)
+      if (!single) __threadfence();  // (fault() may write over it from another block)
   }
   if (!single && lb_end(lb)) {
     if constexpr (ScanHasFault<F>::value)
@@ -341,6 +345,21 @@ static int scan_map(const F &f, int64_t n, Arena &ar, cudaStream_t s) {
   Lookback lb;
   std::memset(&lb, 0, sizeof(lb));
   const int64_t nt = div_up(n, SM_THREADS * F::IT);
+  constexpr bool ANY = F::IT == SM_LIGHT && !ScanHasLoadAll<F>::value && !ScanHasEmitAll<F>::value;  // items a thread
+  if constexpr (ANY) {
+    if (n <= SM_ONE_THREADS) {
+      DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F, 1>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
+      return DCSR_OK;
+    }
+    if (n <= 2 * SM_ONE_THREADS) {
+      DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F, 2>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
+      return DCSR_OK;
+    }
+    if (n <= 4 * SM_ONE_THREADS) {
+      DCSR_LAUNCH((k_scan_map<SM_ONE_THREADS, F, 4>), 1, SM_ONE_THREADS, 0, s, f, n, lb);
+      return DCSR_OK;
+    }
+  }
   if (nt == 1) {
     DCSR_LAUNCH((k_scan_map<SM_THREADS, F>), 1, SM_THREADS, 0, s, f, n, lb);
     return DCSR_OK;
@@ -351,7 +370,7 @@ static int scan_map(const F &f, int64_t n, Arena &ar, cudaStream_t s) {
       return DCSR_OK;
     }
   }
-  if constexpr (F::IT == SM_LIGHT && !ScanHasLoadAll<F>::value && !ScanHasEmitAll<F>::value) {
+  if constexpr (ANY) {
     if (n <= SM_FEW) {
       const int64_t few = div_up(n, SM_THREADS * SM_THIN);
       DCSR_TRY(ar.lookback((size_t)(LB_SCAN_WORDS * few), s, &lb));
