@@ -525,10 +525,9 @@ __device__ __forceinline__ void load_x(const V *__restrict__ p, V (&v)[K]) {
 
 // acc += a*x over logical entries [c0, c1) of a row, lane j of G: entries j,
 // j+G, ... of each segment, UN of them in flight.
-template <typename V, int K, bool VEC>
+template <typename V, int K, bool VEC, int UN = (K <= 2 ? 8 : 4)>
 __device__ __forceinline__ void accum_row(const Mat<V> &m, const V *__restrict__ x, int64_t ldx, const Chain &ch,
                                           int32_t c0, int32_t c1, int j, int G, double (&acc)[K]) {
-  constexpr int UN = K <= 2 ? 8 : 4;
   int32_t before = 0;
 #pragma unroll
   for (int l = 0; l < MAX_SEGS; l++) {
@@ -590,7 +589,9 @@ __device__ __forceinline__ void rows_unit(const RowItem<V> &it, int64_t lu, int 
     const int32_t nch = (len + CHUNK - 1) / CHUNK, chunk = nch == 1 ? 0 : (int32_t)(lu - it.long_off[li]);
     const Chain ch = load_chain(m, row);
     const int32_t c0 = chunk * CHUNK, c1 = len - c0 > CHUNK ? c0 + CHUNK : len;
-    accum_row<V, K, VEC>(m, x, it.ldx, ch, c0, c1, threadIdx.x, RS_THREADS_, acc);
+    // FP64: four entries in flight as well for K = 2 (rows of 600 entries: 74 us of
+    // 6M, 90 with eight, of which a thread has two or three; of 5000: 79 and 85)
+    accum_row<V, K, VEC, K <= 2 && sizeof(V) == 4 ? 8 : 4>(m, x, it.ldx, ch, c0, c1, threadIdx.x, RS_THREADS_, acc);
     reduce(32);
     if (lane == 0)
 #pragma unroll
