@@ -594,6 +594,10 @@ int dcsr_batch_autotune(dcsr_batch b, void *stream, int32_t *short_max, int32_t 
   int32_t best_s = c.items[0].matrix->short_max, best_l = c.items[0].matrix->long_min;
   int best_split = 0;
   float best = -1.0f;
+  // only passes of two or more right-hand sides have classes and splits: a set
+  // without them is timed as it is
+  bool has_k2 = false;
+  for (const auto &it : items) has_k2 |= it.k >= 2;
   int st = DCSR_OK;
   if (!items.empty()) {
     BatchCore tmp;
@@ -602,7 +606,8 @@ int dcsr_batch_autotune(dcsr_batch b, void *stream, int32_t *short_max, int32_t 
     cudaEventCreate(&e1);
     // three timed runs (after one warm-up) of the SpMV pass under one setting
     auto measure = [&](int32_t sm, int32_t lm, int split, float &sum) -> int {
-      for (auto &it : items) dcsr_set_row_classes(it.matrix, sm, lm);
+      if (has_k2)
+        for (auto &it : items) dcsr_set_row_classes(it.matrix, sm, lm);
       tmp.split_force = split;
       DCSR_TRY(tmp.plan(items.data(), (int)items.size(), s, true));
       DCSR_TRY(tmp.upload(s, true));
@@ -625,7 +630,9 @@ int dcsr_batch_autotune(dcsr_batch b, void *stream, int32_t *short_max, int32_t 
     // changes which warp takes a row's lane group, never a row's result)
     const int32_t shorts[] = {32, 64, 128};
     const int32_t longs[] = {512, 1024, 4096, 16384};
+    if (!has_k2) st = measure(0, 0, 0, best);
     for (int32_t sm : shorts) {
+      if (!has_k2) break;
       for (int32_t lm : longs) {
         float sum = 0.0f;
         if ((st = measure(sm, lm, 0, sum)) != DCSR_OK) break;
@@ -637,8 +644,6 @@ int dcsr_batch_autotune(dcsr_batch b, void *stream, int32_t *short_max, int32_t 
       }
       if (st != DCSR_OK) break;
     }
-    bool has_k2 = false;
-    for (const auto &g : tmp.groups) has_k2 |= g.k >= 2;
     for (int split = 1; st == DCSR_OK && has_k2 && split <= 8; split *= 2) {
       float sum = 0.0f;
       if ((st = measure(best_s, best_l, split, sum)) != DCSR_OK) break;
@@ -659,7 +664,8 @@ int dcsr_batch_autotune(dcsr_batch b, void *stream, int32_t *short_max, int32_t 
     for (int i : g.idx) blocks += div_up(c.items[i].matrix->n_rows, 32);
     g.split = best_split > 0 ? best_split : short_split(blocks, g.k);
   }
-  for (auto &it : c.items) dcsr_set_row_classes(it.matrix, best_s, best_l);
+  if (has_k2)
+    for (auto &it : c.items) dcsr_set_row_classes(it.matrix, best_s, best_l);
   if (yscratch) dcsr::dev_free(yscratch, s);
   DCSR_CUDA(cudaStreamSynchronize(s));
   if (st != DCSR_OK) return st;

@@ -324,7 +324,8 @@ int dcsr_batch_destroy(dcsr_batch b);
  * the k >= 2 passes (1, 2, 4, 8 against the automatic rule).  Sets the
  * fastest thresholds on every matrix and the split on the batch (a captured
  * graph must be captured again to use them), returns the thresholds
- * (best_us: the best time per run).  The split never changes a result; the
+ * (best_us: the best time per run).  A set whose SpMVs all have one right-hand
+ * side has no classes: it is timed, and its matrices' thresholds are kept.  The split never changes a result; the
  * thresholds move rows between classes, which sum in different orders.
  * Synchronises. */
 int dcsr_batch_autotune(dcsr_batch b, void *stream, int32_t *short_max, int32_t *long_min, float *best_us);

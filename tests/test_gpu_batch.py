@@ -299,3 +299,21 @@ def test_grow_nearly_full_pools(dcsr):
             ref[0].reserve(la.pool_cap)  # the reference follows the growth
     assert grown_total >= 1
     batch.close()
+
+
+def test_autotune_without_classes(dcsr):
+    """A set of one right-hand side each has no row classes to tune: every
+    matrix keeps its own thresholds, and the set is timed."""
+    rng = np.random.default_rng(31)
+    _, _, work = build_set(dcsr, rng, torch.float32, dcsr.MERGE, [(3000, 3000, 6, (), 200, 1), (500, 500, 90, (), 50, 1)])
+    own = [(40, 700), (90, 1500)]
+    for w, (s, l) in zip(work, own):
+        w["matrix"].set_row_classes(s, l)
+    y = [w["y"].clone() for w in work]
+    batch = dcsr.DcsrBatch(work)
+    sm, lm, us = batch.autotune()
+    assert (sm, lm) == own[0] and us > 0
+    for w, o, y0 in zip(work, own, y):
+        assert w["matrix"].row_classes() == o
+        assert torch.equal(w["y"], y0)
+    batch.close()
