@@ -309,7 +309,7 @@ int BatchCore::enqueue(cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEv
     DCSR_CUDA(cudaStreamWaitEvent(s2, fork, 0));
     for (auto &g : groups)
       if (g.side)
-        DCSR_TRY(spmv_many(img_dev + g.off, dtype, (int)g.idx.size(), g.k, pref + g.pref_off, s2, true, g.split));
+        DCSR_TRY(spmv_many(img_dev + g.off, dtype, (int)g.idx.size(), g.k, pref + g.pref_off, g.split, s2));
     DCSR_CUDA(cudaEventRecord(join, s2));
   }
   const int nu = (int)upd.size();
@@ -335,7 +335,7 @@ int BatchCore::enqueue(cudaStream_t s, cudaStream_t s2, cudaEvent_t fork, cudaEv
   DCSR_TRY(prefixes(false));
   for (auto &g : groups)
     if (!g.side || !beside)
-      DCSR_TRY(spmv_many(img_dev + g.off, dtype, (int)g.idx.size(), g.k, pref + g.pref_off, s, true, g.split));
+      DCSR_TRY(spmv_many(img_dev + g.off, dtype, (int)g.idx.size(), g.k, pref + g.pref_off, g.split, s));
   if (beside) DCSR_CUDA(cudaStreamWaitEvent(s, join, 0));
   return DCSR_OK;
 }

@@ -508,7 +508,7 @@ int persistent_grid(const void *kernel, int block, size_t smem);
 int sm_count();
 
 // -------------------------------------------------------------- primitives
-// (scan.cu / radix.cu)
+// (prims.cu)
 
 // Exclusive scan of int64 values; out may alias in; *total (device) = sum.
 int scan_i64(const long long *in, long long *out, int64_t n, long long *total, Arena &ar, cudaStream_t s);

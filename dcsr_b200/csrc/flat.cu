@@ -264,16 +264,15 @@ __global__ void __launch_bounds__(FT_THREADS) k_flat_copy(FlatCopy<V> a) {
               __shfl_sync(FULL, cur.sg.x, 0) >= 0;
     if (inner) {
       const int32_t o = __shfl_sync(FULL, cur.o, 0), dd = __shfl_sync(FULL, cur.dd, 0) - o;
-      const SD sd = SRC == AT_POOL ? (SD)(__shfl_sync(FULL, cur.sg.x, 0) - o) : (SD)(__shfl_sync(FULL, cur.so, 0) - o);
+      const int32_t sd = __shfl_sync(FULL, cur.sg.x, 0) - o;
 #pragma unroll
       for (int i = 0; i < FT_WIN; i++) {
         const int p = 32 * i + lane;
         dst[i] = 0xffffffffu;
         if (p < cnt) {
-          if constexpr (SRC != AT_FLAT) {
-            const SD src = (SD)(e0 + p) + sd;
-            c[i] = __ldcs(a.scols + src);
-            v[i] = __ldcs(a.svals + src);
+          if constexpr (SRC == AT_POOL) {  // (only there)
+            c[i] = __ldcs(a.scols + (e0 + p + sd));
+            v[i] = __ldcs(a.svals + (e0 + p + sd));
           }
           dst[i] = (unsigned)(DST == AT_FLAT ? e0 + p : e0 + p + dd);
           if constexpr (ROWS) row[i] = r0;

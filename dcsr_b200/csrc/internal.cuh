@@ -107,12 +107,10 @@ int schedule_many(const void *items_dev, int dtype, int count, int64_t R, Arena 
 size_t schedule_scratch_bytes(int64_t R);
 // y = A x for `count` matrices (items: device RowItem<V>[count]) of one k
 // family: kf = 1 (flat pass), 2, 4 or 8, every item's k <= kf (each item's own
-// k / vec are read by the kernel); pref: device scratch of 3*(count+1) long
-// longs (the unit prefixes).
-// prefixed: the group's unit prefixes were computed already (unit_prefix_many,
-// with the same split); split: warps per 32-row block of short rows (short_split)
-int spmv_many(const void *items_dev, int dtype, int count, int k, long long *pref, cudaStream_t s,
-              bool prefixed = false, int split = 1);
+// k / vec are read by the kernel); pref: the group's unit prefixes, 3*(count+1)
+// long longs on the device, computed by unit_prefix_many with the same split:
+// warps per 32-row block of short rows (short_split; 0 for the flat pass).
+int spmv_many(const void *items_dev, int dtype, int count, int k, const long long *pref, int split, cudaStream_t s);
 // The kernel family of a k: 1 (flat pass), 2, 4 or 8; and whether x's rows can
 // be read in vectors of 16 bytes (8 where a row is no multiple of 16): packed,
 // aligned, k even.

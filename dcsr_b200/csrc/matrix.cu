@@ -358,9 +358,7 @@ int compact(dcsr_handle h, cudaStream_t s) {
   h->vals = nv;
   h->buf_cap = got;
   h->pool_cap = cap;
-  // the schedule's row descriptors hold segment starts, which moved (the
-  // flat tables follow the row lengths, which did not change)
-  h->bins.valid = false;
+  // (the row tables follow the row lengths, which did not change)
   // the scratch (sized by this matrix's earlier updates) stays for the
   // update a repair runs next: re-allocating it there stalled repairs
   return DCSR_OK;

@@ -417,8 +417,7 @@ __device__ __forceinline__ void warp_digit_ranks(D &&dg, O &&ok, unsigned (&rank
 #ifndef DCSR_OS_MINB
 #define DCSR_OS_MINB 3
 #endif
-// One pass of the mid tier (the first RS_BINS threads own a digit each in the
-// middle).  PACK: keys_in holds key << ib | index words, or (FIRST) the bare
+// One pass of the mid tier (a thread owns a digit in the middle).  PACK: keys_in holds key << ib | index words, or (FIRST) the bare
 // keys, packed here with their input positions; LAST unpacks to keys_out and
 // vals_out.  Not PACK: keys and indices side by side.
 template <int TH, int IT, bool PACK, bool FIRST, bool LAST>
@@ -428,7 +427,8 @@ __global__ void __launch_bounds__(TH, DCSR_OS_MINB) k_radix_onesweep(const unsig
                                                            unsigned *__restrict__ vals_out, int64_t n, int pass,
                                                            int ib, int last_pass, Lookback lb) {
   constexpr int TILE = TH * IT, WARPS = TH / 32;
-  static_assert(TH >= RS_BINS && TILE >= 2 * WARPS * RS_BINS * 4 / 8, "rank tables fit the tile's room");
+  static_assert(TH == RS_BINS, "a thread per digit");
+  static_assert(TILE >= 2 * WARPS * RS_BINS * 4 / 8, "rank tables fit the tile's room");
   extern __shared__ __align__(16) unsigned char os_sm[];
   unsigned long long *sw = reinterpret_cast<unsigned long long *>(os_sm);  // the tile in digit order
   unsigned *sv = reinterpret_cast<unsigned *>(sw + TILE);                   // (not PACK) its indices
@@ -439,13 +439,12 @@ __global__ void __launch_bounds__(TH, DCSR_OS_MINB) k_radix_onesweep(const unsig
   __shared__ unsigned sh_tile;
   __shared__ unsigned long long sh_ep;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
-  const bool owner = TH == RS_BINS || d < RS_BINS;
   lb_begin(lb, &sh_tile, &sh_ep);
   for (int i = lane; i < RS_BINS; i += 32) {
     wcnt[warp][i] = 0;
     mask[warp][i] = 0;
   }
-  const unsigned gbase = owner ? __ldcg(lb.hist + pass * RS_BINS + d) : 0u;
+  const unsigned gbase = __ldcg(lb.hist + pass * RS_BINS + d);
   __syncthreads();
   const int64_t t = sh_tile;
   const unsigned long long e = sh_ep;
@@ -482,20 +481,18 @@ __global__ void __launch_bounds__(TH, DCSR_OS_MINB) k_radix_onesweep(const unsig
   auto publish = [&](unsigned kind, unsigned v) {
     *(volatile unsigned long long *)(lb.flag + slot) = ((unsigned long long)(tag2 | kind) << 32) | v;
   };
-  if (owner) {
 #pragma unroll
-    for (int w = 0; w < WARPS; w++) {
-      const unsigned c = wcnt[w][d];
-      wcnt[w][d] = run;
-      run += c;
-    }
-    // published before the tile is put in order: later tiles can look back
-    if (t > 0) publish(1, run);
-    else if (!lb.g->stall) publish(2, run);
+  for (int w = 0; w < WARPS; w++) {
+    const unsigned c = wcnt[w][d];
+    wcnt[w][d] = run;
+    run += c;
   }
+  // published before the tile is put in order: later tiles can look back
+  if (t > 0) publish(1, run);
+  else if (!lb.g->stall) publish(2, run);
   unsigned all;
   const unsigned ds = block_excl_scan(run, &all);
-  if (owner) dstart[d] = ds;
+  dstart[d] = ds;
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < IT; j++) {
@@ -509,7 +506,7 @@ __global__ void __launch_bounds__(TH, DCSR_OS_MINB) k_radix_onesweep(const unsig
   // items of digit d in the tiles before this one: look back over windows of
   // LB_W earlier tiles (their flags loaded together), consuming published
   // aggregates up to the nearest published inclusive prefix
-  if (owner) {
+  {
     unsigned excl = 0;
     if (t > 0) {
       const int limit = lb.g->spin_limit;
@@ -675,10 +672,7 @@ size_t radix_scratch_bytes(int64_t n) {
 #ifndef DCSR_OS_I
 #define DCSR_OS_I 16
 #endif
-#ifndef DCSR_OS_T
-#define DCSR_OS_T 256
-#endif
-constexpr int OS_I = DCSR_OS_I, OS_T = DCSR_OS_T;
+constexpr int OS_I = DCSR_OS_I, OS_T = RS_BINS;
 constexpr int OS_TILE = OS_T * OS_I;
 
 size_t lookback_slots(int64_t n) {

@@ -60,7 +60,6 @@ template <typename V>
 struct RowOne {
   RowItem<V> it;
   int split = 1;
-  __device__ __forceinline__ int n_items() const { return 1; }
   __device__ __forceinline__ const RowItem<V> &item(int) const { return it; }
   __device__ __forceinline__ int find_row(int64_t) const { return 0; }
   __device__ __forceinline__ int64_t units(int part) const {
@@ -97,7 +96,6 @@ struct RowMany {
   int count;
   const long long *pref;  // [3][count+1] unit prefixes per class (short blocks counted split times)
   int split = 1;
-  __device__ __forceinline__ int n_items() const { return count; }
   __device__ __forceinline__ const RowItem<V> &item(int i) const { return its[i]; }
   __device__ __forceinline__ int find_row(int64_t g) const {  // matrix holding global row g
     int lo = 0, hi = count;
@@ -406,12 +404,7 @@ __device__ __forceinline__ void unit_prefix_block(const RowItem<V> *its, int cou
   if (threadIdx.x < 3) pref[threadIdx.x * (count + 1) + count] = carry[threadIdx.x];
 }
 
-template <typename V>
-__global__ void __launch_bounds__(1024) k_unit_prefix(const RowItem<V> *its, int count, long long *pref, int split) {
-  unit_prefix_block(its, count, pref, split);
-}
-
-// Several SpMV groups' prefixes in one launch, one block per group.
+// The SpMV groups' prefixes in one launch, one block per group.
 template <typename V>
 struct PrefixJobs {
   const RowItem<V> *its[MAX_PREFIX_JOBS];
@@ -1259,13 +1252,10 @@ static int reduce_dispatch(dcsr_handle h, int32_t op, V *y, cudaStream_t s) {
   return DCSR_BAD_ARG;
 }
 
-// Batched SpMV over a set of matrices of one k family: kf = 1 (k = 1,
-// streamed short rows), 2, 4 or 8 (each item's k <= kf, read by the kernel).
+// Batched SpMV over a set of matrices of one k family: kf = 1 (flat pass), 2,
+// 4 or 8 (each item's k <= kf, read by the kernel).
 template <typename V>
-static int spmv_many_t(const RowItem<V> *its, int count, int kf, long long *pref, bool prefixed, int split,
-                       cudaStream_t s) {
-  if (kf == 1) split = 0;  // flat units
-  if (!prefixed) DCSR_LAUNCH(k_unit_prefix<V>, 1, 1024, 0, s, its, count, pref, split);
+static int spmv_many_t(const RowItem<V> *its, int count, int kf, const long long *pref, int split, cudaStream_t s) {
   RowMany<V> src{its, count, pref, split};
   switch (kf) {
     case 1: return launch_flat_src<V, OP_SPMV, false, sizeof(V) == 4>(src, -1, -1, s);
@@ -1276,12 +1266,11 @@ static int spmv_many_t(const RowItem<V> *its, int count, int kf, long long *pref
   return DCSR_BAD_ARG;
 }
 
-int spmv_many(const void *items_dev, int dtype, int count, int k, long long *pref, cudaStream_t s, bool prefixed,
-              int split) {
+int spmv_many(const void *items_dev, int dtype, int count, int k, const long long *pref, int split, cudaStream_t s) {
   if (count == 0) return DCSR_OK;
   if (dtype == DCSR_F32)
-    return spmv_many_t<float>((const RowItem<float> *)items_dev, count, k, pref, prefixed, split, s);
-  return spmv_many_t<double>((const RowItem<double> *)items_dev, count, k, pref, prefixed, split, s);
+    return spmv_many_t<float>((const RowItem<float> *)items_dev, count, k, pref, split, s);
+  return spmv_many_t<double>((const RowItem<double> *)items_dev, count, k, pref, split, s);
 }
 
 template <typename V>

@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(SG_THREADS, CLS == SG_WARP ? (sizeof(K) == 4 ?
   V *prod = sh.prod;
   // rows in row order, G <= 32 at a time from one counter; the next G are asked
   // for before these are worked on
-    unsigned long long r0 = 0;
+  unsigned long long r0 = 0;
   if (lane == 0) r0 = atomicAdd(next, (unsigned long long)G);
   r0 = __shfl_sync(FULL, r0, 0);
   while (r0 < (unsigned long long)A.n_rows) {
