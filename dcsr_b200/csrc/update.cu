@@ -848,29 +848,30 @@ __global__ void k_finish(Src src, UpdWork<V> w, int count, int merge) {
 // triples of one row: 0.76 ms, 6.1 with one at a time in each of the 8 lanes).
 template <typename V, typename Src>
 __global__ void __launch_bounds__(UPD_THREADS) k_apply_append(Src src, UpdWork<V> w) {
-  constexpr int S = 8, U = 4, FIRST = 64;
+  constexpr int S = 8, FIRST = 64;
   const Sub<S> sub;
   const int lane = lane_id();
   const int64_t nt = w.gstat[ST_TOUCHED];
   const int64_t step = (int64_t)gridDim.x * blockDim.x / S;
-  // triples j0, j0 + lanes, ... below j1 of row d
-  auto put = [&](const RowDesc &d, const Chain &ch, int32_t j0, int32_t j1, int lanes) {
-    const Mat<V> &m = src.mat(d.item);
+  // triples j0, j0 + lanes, ... below j1 of a row of len entries before, U in flight
+  auto put = [&](auto u_, int item, int32_t n0, int32_t len, const Chain &ch, int32_t j0, int32_t j1, int lanes) {
+    constexpr int U = decltype(u_)::value;
+    const Mat<V> &m = src.mat(item);
     for (; j0 < j1; j0 += U * lanes) {
       int64_t p[U];
       int32_t c[U];
       V v[U];
 #pragma unroll
-      for (int u = 0; u < U; u++) p[u] = j0 + u * lanes < j1 ? src.local(d.item, w.perm[d.n0 + j0 + u * lanes]) : -1;
+      for (int u = 0; u < U; u++) p[u] = j0 + u * lanes < j1 ? src.local(item, w.perm[n0 + j0 + u * lanes]) : -1;
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        c[u] = p[u] >= 0 ? src.ucols(d.item)[p[u]] : 0;
-        v[u] = p[u] >= 0 ? src.uvals(d.item)[p[u]] : V(0);
+        c[u] = p[u] >= 0 ? src.ucols(item)[p[u]] : 0;
+        v[u] = p[u] >= 0 ? src.uvals(item)[p[u]] : V(0);
       }
 #pragma unroll
       for (int u = 0; u < U; u++)
         if (p[u] >= 0) {
-          const int64_t q = ch.phys(d.len + j0 + u * lanes);
+          const int64_t q = ch.phys(len + j0 + u * lanes);
           m.cols[q] = c[u];
           m.vals[q] = v[u];
         }
@@ -888,18 +889,15 @@ __global__ void __launch_bounds__(UPD_THREADS) k_apply_append(Src src, UpdWork<V
     if (on) {
       const Mat<V> &m = src.mat(d.item);
       ch = row_chain(src, d, m, sub.sl == 0);
-      put(d, ch, sub.sl, d.mnew < FIRST ? d.mnew : FIRST, S);
+      put(std::integral_constant<int, 1>(), d.item, d.n0, d.len, ch, sub.sl, d.mnew < FIRST ? d.mnew : FIRST, S);
       if (sub.sl == 0) m.row_sizes[d.row] = d.len + d.mnew;
     }
     unsigned longs = __ballot_sync(FULL, on && sub.sl == 0 && d.mnew > FIRST);
     while (longs) {
       const int s = __ffs(longs) - 1;
       longs &= longs - 1;
-      RowDesc e;
-      e.item = __shfl_sync(FULL, d.item, s);
-      e.n0 = __shfl_sync(FULL, d.n0, s);
-      e.len = __shfl_sync(FULL, d.len, s);
-      put(e, shfl_chain(ch, s), FIRST + lane, __shfl_sync(FULL, d.mnew, s), 32);
+      put(std::integral_constant<int, 4>(), __shfl_sync(FULL, d.item, s), __shfl_sync(FULL, d.n0, s),
+          __shfl_sync(FULL, d.len, s), shfl_chain(ch, s), FIRST + lane, __shfl_sync(FULL, d.mnew, s), 32);
     }
   }
 }
