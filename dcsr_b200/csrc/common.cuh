@@ -188,7 +188,8 @@ struct Arena {
       if (lb) DCSR_CUDA(dcsr::dev_free(lb, s));
       lb = nullptr;
       lb_slots = 0;
-      const size_t want = (slots + slots / 4 + 1024 + 1) & ~(size_t)1;
+      // (a multiple of 16, and 8: the scans' words start on a line of 128 bytes)
+      const size_t want = (slots + slots / 4 + 1024 + 15) / 16 * 16 + 8;
       const size_t bytes = lb_bytes(want);
       DCSR_CUDA(dcsr::dev_alloc((void **)&lb, bytes, s));
       DCSR_CUDA(cudaMemsetAsync(lb, 0, bytes, s));
