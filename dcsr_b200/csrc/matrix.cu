@@ -190,6 +190,28 @@ static size_t load_scratch_bytes(dcsr_handle h) {
   return arena_bytes(h->n_rows + 2, 4) + scan_scratch_bytes(h->n_rows + 1);
 }
 
+// A fresh pool of cap entries for a load, and flat tables for that many
+// entries.  Both allocations come before the first change: one that fails
+// leaves the matrix as it was.
+static int replace_pool(dcsr_handle h, int64_t cap, int64_t entries, cudaStream_t s) {
+  int32_t *nc;
+  void *nv;
+  int64_t got;
+  DCSR_TRY(alloc_pool(h, cap, &nc, &nv, &got, s));
+  const int st = ensure_flat(h, s, entries);
+  if (st != DCSR_OK) {
+    dcsr::dev_free(nc, s);
+    dcsr::dev_free(nv, s);
+    return st;
+  }
+  free_pool(h, s);
+  h->cols = nc;
+  h->vals = nv;
+  h->buf_cap = got;
+  h->pool_cap = cap;
+  return DCSR_OK;
+}
+
 // A load is a one-off: a resident matrix keeps no load-sized scratch (the
 // stream-ordered pool keeps the memory for the next allocation), only a
 // look-back area of about the size that builds of its tables need.
@@ -207,17 +229,7 @@ static int load_csr(dcsr_handle h, const int32_t *rp, const int32_t *caps, const
   if (top > 0x7fffffffLL) return DCSR_OOM;
   int64_t cap = pool_capacity(h->o, top);
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
-  // every allocation before the first change: one that fails leaves the matrix as it was
-  DCSR_TRY(ensure_flat(h, s, cap));
-  int32_t *nc;
-  void *nv;
-  int64_t got;
-  DCSR_TRY(alloc_pool(h, cap, &nc, &nv, &got, s));
-  free_pool(h, s);
-  h->cols = nc;
-  h->vals = nv;
-  h->buf_cap = got;
-  h->pool_cap = cap;
+  DCSR_TRY(replace_pool(h, cap, cap, s));
   h->bins.valid = h->flat.valid = false;
   DCSR_TRY(place_csr(h, rp, caps, cols, vals, nnz, s));
   h->flat.valid = true;  // the load knows the offsets: the export and the row passes find them
@@ -240,17 +252,11 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   int32_t *caps = ar.take<int32_t>(n + 2);
   if (ar.overflow) return DCSR_OOM;  // scratch sizing bug: no kernel sees a null pointer
   if (cap_bound > 0x7fffffffLL) return DCSR_OOM;
-  // every allocation before the first change: one that fails leaves the matrix as it was
-  DCSR_TRY(ensure_flat(h, s, bound));
-  int32_t *nc;
-  void *nv;
-  int64_t got;
-  DCSR_TRY(alloc_pool(h, cap_bound, &nc, &nv, &got, s));
-  free_pool(h, s);
-  h->cols = nc;
-  h->vals = nv;
-  h->buf_cap = got;
-  h->pool_cap = cap_bound;
+  if (table_slots(h)) {  // (the placement's scan, before the pool is replaced)
+    Lookback lb;
+    DCSR_TRY(ar.lookback(table_slots(h), s, &lb));
+  }
+  DCSR_TRY(replace_pool(h, cap_bound, bound, s));
   h->bins.valid = h->flat.valid = false;
   DCSR_TRY(place_rows_scan(h, lens, caps, ar, s));
   DCSR_TRY(place_rows_copy(h, caps, src_off, scols, svals, bound, s));
@@ -266,7 +272,7 @@ int load_from_rows(dcsr_handle h, const long long *src_off, const long long *len
   }
   int64_t cap = pool_capacity(h->o, host[ST_TOTAL]);
   if (cap > 0x7fffffffLL) cap = 0x7fffffffLL;
-  if (cap > got) return DCSR_OOM;  // the caller's bound was not one (a bug)
+  if (cap > h->buf_cap) return DCSR_OOM;  // the caller's bound was not one (a bug)
   h->pool_cap = cap;
   h->flat.valid = true;
   return DCSR_OK;
