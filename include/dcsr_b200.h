@@ -230,8 +230,9 @@ int dcsr_get_row_classes(dcsr_handle h, int32_t *short_max, int32_t *long_min);
  * device::spmv(dcsr, x, y, streams) (include/spmv.h:121-248). */
 int dcsr_spmv(dcsr_handle h, const void *x, int32_t k, int64_t ldx, void *y, int64_t ldy, double alpha,
               double beta, void *stream);
-/* y[r] = op over row r's entries (sum / max / min / count).  The reference
- * computes row sums as SpMV with x = 1. */
+/* y[r] = op over row r's entries (sum / max / min / count; 0 for an empty
+ * row).  Max and min are NaN where the row's first entry is, and pass over
+ * later NaNs.  The reference computes row sums as SpMV with x = 1. */
 int dcsr_row_reduce(dcsr_handle h, int32_t op, void *y, void *stream);
 /* C = A*B.  C must be a handle created with n_rows = A.n_rows, n_cols =
  * B.n_cols and A's dtype; its content is replaced.  Rows sorted, explicit
