@@ -217,8 +217,8 @@ __device__ __forceinline__ void lb_lookback(const Lookback &lb, unsigned long lo
 // staging through shared memory), a block SM_THREADS*IT.  Light functions
 // (IT = 8) of up to SM_ONE items run in one block without look-back, with as
 // few items a thread as its 1024 threads allow (a few rows of many tiles each
-// are then marked by as many warps as can be: 500 rows of 78 tiles %B% us,
-// 43 with eight rows a lane in two warps); heavy ones (IT = 4: searches, plans)
+// are then marked by as many warps as can be: 500 rows of 78 tiles 8.8 us,
+// 46 with eight rows a lane in two warps); heavy ones (IT = 4: searches, plans)
 // spread over blocks from 1024 items on.
 constexpr int SM_LIGHT = 8, SM_HEAVY = 4;
 constexpr int SM_THREADS = 256;
